@@ -285,11 +285,18 @@ DEV void pair_mul(const LanePair &lp, const fp &a0, const fp &b0, const fp &a1, 
   r0 = pair_sel(lp, r, o);
   r1 = pair_sel(lp, o, r);
 }
+// r0 = a0^2, r1 = a1^2 the same way.
+DEV void pair_sqr(const LanePair &lp, const fp &a0, const fp &a1, fp &r0, fp &r1) {
+  const fp r = fp_sqr(pair_sel(lp, a0, a1));
+  const fp o = pair_swap(lp, r);
+  r0 = pair_sel(lp, r, o);
+  r1 = pair_sel(lp, o, r);
+}
 DEV g1 g1_dbl_pair(const LanePair &lp, const g1 &p) {
   if (g1_is_inf(p)) return p;
   const fp U = fp_dbl(p.Y);
   fp V, X2, W, S, ZZ3, M2, WY, ZZZ3;
-  pair_mul(lp, U, U, p.X, p.X, V, X2);
+  pair_sqr(lp, U, p.X, V, X2);
   const fp M = fp_add(fp_dbl(X2), X2);
   pair_mul(lp, U, V, p.X, V, W, S);
   pair_mul(lp, V, p.ZZ, M, M, ZZ3, M2);
@@ -312,7 +319,7 @@ DEV g1 g1_add_aff_pair(const LanePair &lp, const g1 &p, const g1a &q) {
     return g1_inf();
   }
   fp PP, RR, PPP, Q, ZZ3, YP, ZZZ3, T;
-  pair_mul(lp, P, P, R, R, PP, RR);
+  pair_sqr(lp, P, R, PP, RR);
   pair_mul(lp, P, PP, p.X, PP, PPP, Q);
   g1 r;
   r.X = fp_sub(fp_sub(RR, PPP), fp_dbl(Q));
@@ -335,7 +342,7 @@ DEV g1 g1_add_pair(const LanePair &lp, const g1 &p, const g1 &q) {
     return g1_inf();
   }
   fp PP, RR, PPP, Q, Z1, Z2, ZZ3, ZZZ3, SP, T;
-  pair_mul(lp, P, P, R, R, PP, RR);
+  pair_sqr(lp, P, R, PP, RR);
   pair_mul(lp, P, PP, U1, PP, PPP, Q);
   g1 r;
   r.X = fp_sub(fp_sub(RR, PPP), fp_dbl(Q));
@@ -412,11 +419,17 @@ DEV void quad_mul(const LaneQuad &q, const fp &a0, const fp &b0, const fp &a1, c
   if (N > 2) r2 = quad_from(q, mine, 2);
   if (N > 3) r3 = quad_from(q, mine, 3);
 }
+// r0 = a0^2, r1 = a1^2 (roles 0 and 1; the others repeat role 0's).
+DEV void quad_sqr2(const LaneQuad &q, const fp &a0, const fp &a1, fp &r0, fp &r1) {
+  const fp mine = fp_sqr(quad_pick(q, a0, a1, a0, a0));
+  r0 = quad_from(q, mine, 0);
+  r1 = quad_from(q, mine, 1);
+}
 DEV g1 g1_dbl_quad(const LaneQuad &q, const g1 &p) {
   if (g1_is_inf(p)) return p;
   const fp U = fp_dbl(p.Y);
   fp V, X2, W, S, ZZ3, M2, T, WY, ZZZ3, unused;
-  quad_mul<2>(q, U, U, p.X, p.X, U, U, U, U, V, X2, unused, unused);
+  quad_sqr2(q, U, p.X, V, X2);
   const fp M = fp_add(fp_dbl(X2), X2);
   quad_mul<4>(q, U, V, p.X, V, V, p.ZZ, M, M, W, S, ZZ3, M2);
   g1 r;
@@ -437,7 +450,7 @@ DEV g1 g1_add_aff_quad(const LaneQuad &lq, const g1 &p, const g1a &q) {
     if (fp_is_zero(R)) return g1_dbl_quad(lq, g1_from_aff(q));
     return g1_inf();
   }
-  quad_mul<2>(lq, P, P, R, R, P, P, P, P, PP, RR, unused, unused);
+  quad_sqr2(lq, P, R, PP, RR);
   quad_mul<3>(lq, P, PP, p.X, PP, p.ZZ, PP, P, P, PPP, Q, ZZ3, unused);
   g1 r;
   r.X = fp_sub(fp_sub(RR, PPP), fp_dbl(Q));

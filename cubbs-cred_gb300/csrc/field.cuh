@@ -4,8 +4,8 @@
 //
 // The tower and encodings follow the curve arithmetic the reference protocol
 // delegates to (bls12_381_plus 0.8.18; reference device types are SPPARK
-// fp_t/fr_t/fp2_t, prepare_b_msm.cu:40-49, pairing.cuh:3-321).  Multiplication
-// is CIOS over inline-PTX carry chains generated by gen_field_ptx.py.
+// fp_t/fr_t/fp2_t, prepare_b_msm.cu:40-49, pairing.cuh:3-321).  Products are
+// Montgomery rows on inline-PTX carry chains generated by gen_field_ptx.py.
 #pragma once
 #include <stdint.h>
 
@@ -42,7 +42,7 @@ DEV fp fp_sub(const fp &a, const fp &b) { fp r; fp_sub_raw(r.w, a.w, b.w); retur
 DEV fp fp_dbl(const fp &a) { return fp_add(a, a); }
 DEV fp fp_neg(const fp &a) { return fp_sub(fp_zero(), a); }
 // CIOS Montgomery product over the carry chains of field_ptx.cuh (one row per
-// limb of b; every row is a dependent carry chain).
+// limb of b; every row is a dependent carry chain), for the tests.
 DEV fp fp_mul_cios_inl(const fp &a, const fp &b) {
   uint32_t t[25];
   _Pragma("unroll") for (int i = 0; i < 13; i++) t[i] = 0;
@@ -55,70 +55,29 @@ DEV fp fp_mul_cios_inl(const fp &a, const fp &b) {
   return r;
 }
 
-// The Montgomery product a b / 2^384 mod p (fully reduced) used everywhere:
-// carry-save accumulation instead of carry chains.  T_j = (hi_j : lo_j) are
-// 64-bit partial sums of limb position j; each row adds a_j b_i to every T_j
-// (a mad.lo.cc / madc.hi pair), splits every sum into its low word and the
-// high word of its right neighbour (N_j = lo(T_j) + hi(T_{j-1}) <= 2^33 - 2,
-// an add.cc / addc pair, so the next 32 x 32-bit product cannot overflow 64
-// bits), adds m p_j, and splits again while shifting one limb down.  No step
-// depends on a carry from another limb, so the twelve products of a row
-// issue back to back.  One carry pass at the end and one conditional
-// subtraction of p finish it.
-// Bounds: a, b < p; every partial sum stays below 2^64 (the worst case is
-// (2^33 - 2) + (2^32 - 1)^2 = 2^64 - 1) and the final value is below 2p.
-// Written in PTX: from the same arithmetic in C++ 64-bit integers the
-// compiler put many of the splits' carry additions on the FMA pipe, beside
-// the multiplies (522 FMA-pipe and 511 ALU instructions a product); here 324
-// and 587.  Measured on GB300, one warp, chains of dependent products: 1965
-// cycles a product against 2316 for the C++ form (and 2802 for CIOS); about
-// the same with two warps per SM sub-partition (1830 vs 1860 cycles of the
-// sub-partition a product) and 3 % slower with four (1813 vs 1753).  Every
-// carry flag lives inside one asm statement.
+// The Montgomery product a b / 2^384 mod p (fully reduced) used everywhere, and
+// its square: interleaved Montgomery rows on an even and an odd carry chain
+// (fp_mont_mul / fp_mont_sqr of field_ptx.cuh), which the compiler turns into
+// one 64-bit multiply-add with carry in and out per limb product.
+// What bounds it: the multiplier.  On GB300 an SM sub-partition takes a 64-bit
+// multiply-add every 4 cycles from two or more warps and every 6 from a lone
+// warp, whatever their dependencies; other integer instructions cost one issue
+// slot each, hidden behind the multiplies of a lone warp.  The product has 288
+// multiply-adds, 12 multiplies and 77 other instructions (counted by ncu), the
+// square 222, 12 and 155.  The carry-save form this replaces (every row split
+// into low and high words) had the same multiplies and 587 others.  Cycles of
+// the sub-partition per dependent product at 1 / 2 / 4 warps: 1816 / 1234 /
+// 1195 against 1983 / 1849 / 1828; the square 1507 / 1083 / 1005.
 DEV fp fp_mul_inl(const fp &a, const fp &b) {
-  const fp pm = FP_MOD_INIT;
-  uint32_t lo[12], hi[12];  // T_j = hi_j : lo_j
-#pragma unroll
-  for (int j = 0; j < 12; j++) lo[j] = hi[j] = 0;
-#pragma unroll
-  for (int i = 0; i < 12; i++) {
-    const uint32_t bi = b.w[i];
-#pragma unroll
-    for (int j = 0; j < 12; j++)
-      asm("mad.lo.cc.u32 %0, %2, %3, %0;\n\tmadc.hi.u32 %1, %2, %3, %1;"
-          : "+r"(lo[j]), "+r"(hi[j])
-          : "r"(a.w[j]), "r"(bi));
-    uint32_t nl[12], nh[12];  // N_j = nh_j : nl_j
-    nl[0] = lo[0];
-    nh[0] = 0;
-#pragma unroll
-    for (int j = 1; j < 12; j++)
-      asm("add.cc.u32 %0, %2, %3;\n\taddc.u32 %1, 0, 0;" : "=r"(nl[j]), "=r"(nh[j]) : "r"(lo[j]), "r"(hi[j - 1]));
-    const uint32_t n12 = hi[11];
-    const uint32_t m = nl[0] * FP_PINV;
-#pragma unroll
-    for (int j = 0; j < 12; j++)
-      asm("mad.lo.cc.u32 %0, %2, %3, %0;\n\tmadc.hi.u32 %1, %2, %3, %1;"
-          : "+r"(nl[j]), "+r"(nh[j])
-          : "r"(m), "r"(pm.w[j]));
-#pragma unroll
-    for (int j = 0; j < 11; j++)
-      asm("add.cc.u32 %0, %2, %3;\n\taddc.u32 %1, 0, 0;" : "=r"(lo[j]), "=r"(hi[j]) : "r"(nl[j + 1]), "r"(nh[j]));
-    asm("add.cc.u32 %0, %2, %3;\n\taddc.u32 %1, 0, 0;" : "=r"(lo[11]), "=r"(hi[11]) : "r"(n12), "r"(nh[11]));
-  }
-  // t = sum_j T_j 2^(32 j): t_j = lo_j + hi_(j-1) + carry (the value is below 2p < 2^384)
-  uint32_t t[12];
-  asm("add.cc.u32 %0, %12, 0;\n\taddc.cc.u32 %1, %13, %24;\n\taddc.cc.u32 %2, %14, %25;\n\t"
-      "addc.cc.u32 %3, %15, %26;\n\taddc.cc.u32 %4, %16, %27;\n\taddc.cc.u32 %5, %17, %28;\n\t"
-      "addc.cc.u32 %6, %18, %29;\n\taddc.cc.u32 %7, %19, %30;\n\taddc.cc.u32 %8, %20, %31;\n\t"
-      "addc.cc.u32 %9, %21, %32;\n\taddc.cc.u32 %10, %22, %33;\n\taddc.u32 %11, %23, %34;"
-      : "=r"(t[0]), "=r"(t[1]), "=r"(t[2]), "=r"(t[3]), "=r"(t[4]), "=r"(t[5]), "=r"(t[6]), "=r"(t[7]), "=r"(t[8]),
-        "=r"(t[9]), "=r"(t[10]), "=r"(t[11])
-      : "r"(lo[0]), "r"(lo[1]), "r"(lo[2]), "r"(lo[3]), "r"(lo[4]), "r"(lo[5]), "r"(lo[6]), "r"(lo[7]), "r"(lo[8]),
-        "r"(lo[9]), "r"(lo[10]), "r"(lo[11]), "r"(hi[0]), "r"(hi[1]), "r"(hi[2]), "r"(hi[3]), "r"(hi[4]), "r"(hi[5]),
-        "r"(hi[6]), "r"(hi[7]), "r"(hi[8]), "r"(hi[9]), "r"(hi[10]));
-  fp r;
-  fp_reduce_once(r.w, t);
+  fp t, r;
+  fp_mont_mul(t.w, a.w, b.w);
+  fp_reduce_once(r.w, t.w);
+  return r;
+}
+DEV fp fp_sqr_inl(const fp &a) {
+  fp t, r;
+  fp_mont_sqr(t.w, a.w);
+  fp_reduce_once(r.w, t.w);
   return r;
 }
 // One out-of-line copy of the product per translation unit: with the body
@@ -127,7 +86,7 @@ DEV fp fp_mul_inl(const fp &a, const fp &b) {
 // sub-partition cannot hide (measured 2.6x slower G1 doubling).
 DEVNI fp fp_mul(fp a, fp b) { return fp_mul_inl(a, b); }
 DEVNI fp fp_mul_cios(fp a, fp b) { return fp_mul_cios_inl(a, b); }
-DEV fp fp_sqr(const fp &a) { return fp_mul(a, a); }
+DEVNI fp fp_sqr(fp a) { return fp_sqr_inl(a); }
 
 // raw canonical limbs (little-endian words) -> Montgomery
 DEV fp fp_to_mont(const fp &a) { const fp r2 = FP_R2_INIT; return fp_mul(a, r2); }
@@ -423,51 +382,15 @@ DEV bool fr_eq(const fr &a, const fr &b) {
 }
 DEV fr fr_add(const fr &a, const fr &b) { fr r; fr_add_raw(r.w, a.w, b.w); return r; }
 DEV fr fr_sub(const fr &a, const fr &b) { fr r; fr_sub_raw(r.w, a.w, b.w); return r; }
-// Montgomery product mod r (R = 2^256, fully reduced): the carry-save rows of
-// fp_mul_inl over 8 limbs, in PTX for the same reason (the carry additions stay
-// on the ALU pipe).  Bounds: a, b < r; partial sums below 2^64; result below 2r.
+// Montgomery product mod r (R = 2^256, fully reduced): the rows of fp_mul_inl
+// over 8 limbs.
 DEV fr fr_mul_inl(const fr &a, const fr &b) {
-  const fr rm = FR_MOD_INIT;
-  uint32_t lo[8], hi[8];
-#pragma unroll
-  for (int j = 0; j < 8; j++) lo[j] = hi[j] = 0;
-#pragma unroll
-  for (int i = 0; i < 8; i++) {
-    const uint32_t bi = b.w[i];
-#pragma unroll
-    for (int j = 0; j < 8; j++)
-      asm("mad.lo.cc.u32 %0, %2, %3, %0;\n\tmadc.hi.u32 %1, %2, %3, %1;"
-          : "+r"(lo[j]), "+r"(hi[j])
-          : "r"(a.w[j]), "r"(bi));
-    uint32_t nl[8], nh[8];
-    nl[0] = lo[0];
-    nh[0] = 0;
-#pragma unroll
-    for (int j = 1; j < 8; j++)
-      asm("add.cc.u32 %0, %2, %3;\n\taddc.u32 %1, 0, 0;" : "=r"(nl[j]), "=r"(nh[j]) : "r"(lo[j]), "r"(hi[j - 1]));
-    const uint32_t n8 = hi[7];
-    const uint32_t m = nl[0] * FR_PINV;
-#pragma unroll
-    for (int j = 0; j < 8; j++)
-      asm("mad.lo.cc.u32 %0, %2, %3, %0;\n\tmadc.hi.u32 %1, %2, %3, %1;"
-          : "+r"(nl[j]), "+r"(nh[j])
-          : "r"(m), "r"(rm.w[j]));
-#pragma unroll
-    for (int j = 0; j < 7; j++)
-      asm("add.cc.u32 %0, %2, %3;\n\taddc.u32 %1, 0, 0;" : "=r"(lo[j]), "=r"(hi[j]) : "r"(nl[j + 1]), "r"(nh[j]));
-    asm("add.cc.u32 %0, %2, %3;\n\taddc.u32 %1, 0, 0;" : "=r"(lo[7]), "=r"(hi[7]) : "r"(n8), "r"(nh[7]));
-  }
-  uint32_t t[8];
-  asm("add.cc.u32 %0, %8, 0;\n\taddc.cc.u32 %1, %9, %16;\n\taddc.cc.u32 %2, %10, %17;\n\taddc.cc.u32 %3, %11, %18;\n\t"
-      "addc.cc.u32 %4, %12, %19;\n\taddc.cc.u32 %5, %13, %20;\n\taddc.cc.u32 %6, %14, %21;\n\taddc.u32 %7, %15, %22;"
-      : "=r"(t[0]), "=r"(t[1]), "=r"(t[2]), "=r"(t[3]), "=r"(t[4]), "=r"(t[5]), "=r"(t[6]), "=r"(t[7])
-      : "r"(lo[0]), "r"(lo[1]), "r"(lo[2]), "r"(lo[3]), "r"(lo[4]), "r"(lo[5]), "r"(lo[6]), "r"(lo[7]),
-        "r"(hi[0]), "r"(hi[1]), "r"(hi[2]), "r"(hi[3]), "r"(hi[4]), "r"(hi[5]), "r"(hi[6]));
-  fr r;
-  fr_reduce_once(r.w, t);
+  fr t, r;
+  fr_mont_mul(t.w, a.w, b.w);
+  fr_reduce_once(r.w, t.w);
   return r;
 }
-// The CIOS form it replaced (carry chains of field_ptx.cuh), kept for the tests.
+// The CIOS form (carry chains of field_ptx.cuh), kept for the tests.
 DEV fr fr_mul_cios_inl(const fr &a, const fr &b) {
   uint32_t t[17];
   _Pragma("unroll") for (int i = 0; i < 9; i++) t[i] = 0;

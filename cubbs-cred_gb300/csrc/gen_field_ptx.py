@@ -4,12 +4,13 @@ limbs) as inline-PTX carry chains (mad.lo.cc / madc.hi.cc / addc / subc).
 
 Run:  python gen_field_ptx.py   (rewrites field_ptx.cuh beside this file)
 
-The multiplication is operand-scanning CIOS: for each limb b_i of the second
-operand, one asm block adds lo(a*b_i) and hi(a*b_i), computes the Montgomery
-quotient m = t0 * (-p^-1 mod 2^32), and adds lo(m*p) and hi(m*p).  Each block
-keeps its carry flag local, so no condition code crosses asm statements.  The
-modulus words are embedded as immediates.  Intermediate values stay below
-2^(32n+32), which the bounds in the comments of field_ptx.cuh document.
+The product in use is gen_mont's: rows of 64-bit multiply-adds on an even and
+an odd carry chain (gen_mont_sqr: the square).  The rows of operand-scanning
+CIOS are kept for the tests: for each limb b_i of the second operand, one asm
+block adds lo(a*b_i) and hi(a*b_i), computes the Montgomery quotient
+m = t0 * (-p^-1 mod 2^32), and adds lo(m*p) and hi(m*p).  Each block keeps its
+carry flag local, so no condition code crosses asm statements.  The modulus
+words are embedded as immediates.  Intermediate values stay below 2^(32n+32).
 """
 import pathlib
 
@@ -181,6 +182,153 @@ def gen_lazy(name, mod, n):
     return "\n".join(out)
 
 
+def asm_fn(name, n, body, operands):
+    """An inline function `name`(r, operand arrays...) around one asm block; %0..%{n-1} are r."""
+    outs = ", ".join(f'"=&r"(r[{i}])' for i in range(n))
+    ins = ", ".join(f'"r"({v}[{i}])' for v in operands for i in range(n))
+    args = ", ".join(f"const uint32_t *{v}" for v in operands)
+    text = "\\n\\t".join(body)
+    return (f"__device__ __forceinline__ void {name}(uint32_t *r, {args}) {{\n"
+            f'  asm("{text}" : {outs} : {ins});\n}}\n')
+
+
+def wide_chain(lines, acc, xs, y, first_carry=False, carry_out=True, fresh=False, fresh_top=False):
+    """acc (2 len(xs) words) += sum_k xs[k] y 2^(64 k), one carry chain of 64-bit multiply-adds.
+    first_carry: the chain starts from the carry flag; carry_out: it ends in it; fresh: acc is written, not added to
+    (no carries at all); fresh_top: the top pair of acc counts as zero."""
+    for k, x in enumerate(xs):
+        lo, hi = acc[2 * k], acc[2 * k + 1]
+        if fresh:
+            lines.append(f"mul.lo.u32 {lo}, {x}, {y};")
+            lines.append(f"mul.hi.u32 {hi}, {x}, {y};")
+            continue
+        c = "c" if k or first_carry else ""
+        cc = ".cc" if carry_out or k < len(xs) - 1 else ""
+        zero = fresh_top and k == len(xs) - 1
+        lines.append(f"mad{c}.lo.cc.u32 {lo}, {x}, {y}, {'0' if zero else lo};")
+        lines.append(f"madc.hi{cc}.u32 {hi}, {x}, {y}, {'0' if zero else hi};")
+
+
+def gen_mont(name, mod, n):
+    """{name}_mont_mul(r, a, b) = a b / 2^(32n) mod mod up to one mod too large, and {name}_mont_mul2(r, a, b, c, d)
+    = (a b + c d) / 2^(32n) the same way.
+
+    The running sum is kept in two arrays of n words: E at limbs 0..n-1 holds the products of even limb distance, O
+    at limbs 1..n those of odd distance, so a row b_i adds its n products as two carry chains of n/2 64-bit
+    multiply-adds whose words line up in pairs.  Then m = E_0 (-mod^-1), a row m mod in the same way, and E_0 is
+    zero.  Dropping that limb turns O into the next E and E's words 2.. into the next O; the word E_1 left over is
+    added to the next E_0 and its carry enters the next row's O chain.
+    Bounds: the sum before a shift is below 2^32 (a + mod + the sum before), so operands with
+    a (+ c) < 2^(32n) - 3 mod never carry out of limb n, and the result is below mod + (a b (+ c d)) / 2^(32n)."""
+    assert n % 2 == 0
+    ml = limbs(mod, n)
+    pinv = (-pow(mod, -1, 1 << 32)) % (1 << 32)
+    odd = [f"0x{ml[j]:08x}" for j in range(1, n, 2)]
+    even = [f"0x{ml[j]:08x}" for j in range(0, n, 2)]
+
+    def build(pairs):
+        body = [f"{{ .reg .u32 x<{n}>; .reg .u32 y<{n}>; .reg .u32 m;"]
+        op = [[f"%{n * (k + 1) + j}" for j in range(n)] for k in range(2 * pairs)]
+        E, O = [f"x{j}" for j in range(n)], [f"y{j}" for j in range(n)]
+        for i in range(n):
+            for k in range(pairs):
+                a, b = op[2 * k], op[2 * k + 1][i]
+                if i == 0 and k == 0:
+                    wide_chain(body, O, a[1::2], b, fresh=True)
+                    wide_chain(body, E, a[0::2], b, fresh=True)
+                    continue
+                if k == 0:
+                    body.append(f"add.cc.u32 {E[0]}, {E[0]}, {left};")
+                wide_chain(body, O, a[1::2], b, first_carry=k == 0, carry_out=False, fresh_top=k == 0 and i > 0)
+                wide_chain(body, E, a[0::2], b)
+                body.append(f"addc.u32 {O[n - 1]}, {O[n - 1]}, 0;")
+            body.append(f"mul.lo.u32 m, {E[0]}, 0x{pinv:08x};")
+            wide_chain(body, O, odd, "m", carry_out=False)
+            wide_chain(body, E, even, "m")
+            body.append(f"addc.u32 {O[n - 1]}, {O[n - 1]}, 0;")
+            left = E[1]
+            E, O = O, E[2:] + E[:2]  # the two top words of the new O count as zero (fresh_top)
+        body.append(f"add.cc.u32 %0, {E[0]}, {left};")
+        for j in range(1, n):
+            body.append(f"addc{'.cc' if j < n - 1 else ''}.u32 %{j}, {E[j]}, {O[j - 1] if j < n - 1 else '0'};")
+        body.append("}")
+        return body
+
+    return (f"// r = a b / 2^{32 * n} mod p, up to one p too large (interleaved Montgomery rows on even / odd carry "
+            f"chains).\n" + asm_fn(f"{name}_mont_mul", n, build(1), "ab")
+            + f"// r = (a b + c d) / 2^{32 * n} mod p, up to one p too large: one reduction for both products.\n"
+            + asm_fn(f"{name}_mont_mul2", n, build(2), "abcd"))
+
+
+def gen_mont_sqr(name, mod, n):
+    """{name}_mont_sqr(r, a) = a^2 / 2^(32n) mod mod up to one mod too large: the n(n-1)/2 cross products in an even
+    (t) and an odd (u) array of carry chains, doubled by shifts, the n squares added in one chain, then n reduction
+    rows on the low words as in {name}_mont_mul and the high words added at the end (222 multiply-adds for n = 12
+    instead of 288)."""
+    ml = limbs(mod, n)
+    pinv = (-pow(mod, -1, 1 << 32)) % (1 << 32)
+    odd = [f"0x{ml[j]:08x}" for j in range(1, n, 2)]
+    even = [f"0x{ml[j]:08x}" for j in range(0, n, 2)]
+    a = [f"%{n + j}" for j in range(n)]
+    L = [f"{{ .reg .u32 t<{2 * n}>; .reg .u32 u<{2 * n}>; .reg .u32 m;"]
+    live = {"t": set(), "u": set()}
+    for i in range(n - 1):
+        for par, R in ((0, "t"), (1, "u")):
+            chain = False
+            js = [j for j in range(i + 1, n) if (i + j) % 2 == par]
+            for j in js:
+                k = i + j
+                if k in live[R]:
+                    L.append(f"mad{'c' if chain else ''}.lo.cc.u32 {R}{k}, {a[i]}, {a[j]}, {R}{k};")
+                    L.append(f"madc.hi.cc.u32 {R}{k + 1}, {a[i]}, {a[j]}, {R}{k + 1};")
+                    chain = True
+                elif chain:  # a fresh pair takes the chain's carry and cannot overflow
+                    L.append(f"madc.lo.cc.u32 {R}{k}, {a[i]}, {a[j]}, 0;")
+                    L.append(f"madc.hi.u32 {R}{k + 1}, {a[i]}, {a[j]}, 0;")
+                    chain = False
+                else:
+                    L.append(f"mul.lo.u32 {R}{k}, {a[i]}, {a[j]};")
+                    L.append(f"mul.hi.u32 {R}{k + 1}, {a[i]}, {a[j]};")
+                live[R] |= {k, k + 1}
+            if chain:  # the carry past the last pair: a word that holds nothing but such carries
+                k = i + js[-1] + 2
+                if k in live[R]:
+                    L.append(f"addc.u32 {R}{k}, {R}{k}, 0;")
+                else:
+                    L.append(f"addc.u32 {R}{k}, 0, 0;")
+                    live[R].add(k)
+                    if k + 1 < 2 * n:
+                        L.append(f"mov.u32 {R}{k + 1}, 0;")
+                        live[R].add(k + 1)
+    for k in range(1, 2 * n):  # t = t + u
+        x, y = (f"{R}{k}" if k in live[R] else "0" for R in "tu")
+        L.append(f"add{'c' if k > 1 else ''}{'.cc' if k < 2 * n - 1 else ''}.u32 t{k}, {x}, {y};")
+    L.append("shf.l.clamp.b32 u1, 0, t1, 1;")  # u = 2 t
+    for k in range(2, 2 * n):
+        L.append(f"shf.l.clamp.b32 u{k}, t{k - 1}, t{k}, 1;")
+    L.append(f"mul.lo.u32 t0, {a[0]}, {a[0]};")  # t = u + the squares
+    L.append(f"mad.hi.cc.u32 t1, {a[0]}, {a[0]}, u1;")
+    for j in range(1, n):
+        L.append(f"madc.lo.cc.u32 t{2 * j}, {a[j]}, {a[j]}, u{2 * j};")
+        L.append(f"madc.hi{'.cc' if j < n - 1 else ''}.u32 t{2 * j + 1}, {a[j]}, {a[j]}, u{2 * j + 1};")
+    E, O = [f"t{j}" for j in range(n)], [f"u{j}" for j in range(n)]
+    for i in range(n):
+        L.append(f"mul.lo.u32 m, {E[0]}, 0x{pinv:08x};")
+        wide_chain(L, O, odd, "m", first_carry=i > 0, carry_out=False, fresh=i == 0, fresh_top=True)
+        wide_chain(L, E, even, "m")
+        L.append(f"addc.u32 {O[n - 1]}, {O[n - 1]}, 0;")
+        left = E[1]
+        E, O = O, E[2:] + E[:2]
+        L.append(f"add.cc.u32 {E[0]}, {E[0]}, {left};")  # its carry enters the next O chain
+    for j in range(1, n):
+        L.append(f"addc{'.cc' if j < n - 1 else ''}.u32 {E[j]}, {E[j]}, {O[j - 1] if j < n - 1 else '0'};")
+    L.append(f"add.cc.u32 %0, {E[0]}, t{n};")
+    for j in range(1, n):
+        L.append(f"addc{'.cc' if j < n - 1 else ''}.u32 %{j}, {E[j]}, t{n + j};")
+    L.append("}")
+    return (f"// r = a^2 / 2^{32 * n} mod p, up to one p too large.\n" + asm_fn(f"{name}_mont_sqr", n, L, "a"))
+
+
 def main():
     text = [
         "// GENERATED by gen_field_ptx.py -- do not edit by hand.",
@@ -190,7 +338,10 @@ def main():
         "",
         gen_field("fp", P, 12),
         gen_lazy("fp", P, 12),
+        gen_mont("fp", P, 12),
+        gen_mont_sqr("fp", P, 12),
         gen_field("fr", R, 8),
+        gen_mont("fr", R, 8),
     ]
     dst = pathlib.Path(__file__).with_name("field_ptx.cuh")
     dst.write_text("\n".join(text) + "\n")

@@ -54,7 +54,7 @@ DEV g1 zabs_unrolled_bits(g1 p) {
 }
 
 // op 0: Fp product of canonical BE inputs; op 1: Fp inverse; op 2: Fp sqrt (0 if none);
-// op 3: variable-time Fp inverse; op 4: Fp product by CIOS carry chains
+// op 3: variable-time Fp inverse; op 4: Fp product by CIOS carry chains; op 5: Fp square
 __global__ void k_fp_test(const uint8_t *a, const uint8_t *b, uint32_t n, int op, uint8_t *out, int32_t *st) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -63,6 +63,7 @@ __global__ void k_fp_test(const uint8_t *a, const uint8_t *b, uint32_t n, int op
   if (ok) {
     if (op == 0) r = fp_mul(x, y);
     else if (op == 4) r = fp_mul_cios(x, y);
+    else if (op == 5) r = fp_sqr(x);
     else if (op == 1) r = fp_inv(x);
     else if (op == 3) r = fp_inv_vartime(x);
     else ok = fp_sqrt(x, r);
@@ -373,9 +374,9 @@ extern "C" int32_t cubbs_bbs_gpu_latency_probe_for_test_v2(double *cycles, int32
   }
 }
 
-// Fp products per second (1e9) of the carry-save product (fp_mul) and the
+// Fp products per second (1e9) of the product in use (fp_mul) and of the
 // CIOS product with `wps[k]` warps per SM (blocks of 32 threads,
-// sm_count * wps[k] blocks): rates[2k] carry-save, rates[2k + 1] CIOS.
+// sm_count * wps[k] blocks): rates[2k] fp_mul, rates[2k + 1] CIOS.
 extern "C" int32_t cubbs_bbs_gpu_fpmul_rates_for_test_v2(const int32_t *wps, int32_t n, double *rates) {
   if (!wps || !rates || n <= 0 || n > 8) return CUBBS_BBS_GPU_ERR_INVALID_INPUT;
   for (int k = 0; k < n; k++)

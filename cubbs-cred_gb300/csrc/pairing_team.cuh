@@ -186,10 +186,7 @@ template <int W = 32> DEVNI void run(fp *sl, int lane, int prog, int bar = 0) {
       if (type == PP_MUL) {
         const fp x = (tw & PP_F_PLAIN_A) ? ld(sl, e0.y & PP_SLOT_MASK) : wsum(sl, terms_lo(e0, e1), na);
         const fp y = (tw & PP_F_PLAIN_B) ? ld(sl, (e1.x >> 16) & PP_SLOT_MASK) : wsum(sl, terms_hi(e1), nb);
-        // one dependent product per lane, inlined: the PTX carry-save form
-        // (1965 cycles a product on one warp against 2802 for the CIOS form
-        // this replaced; the aggregated check 1.88 -> 1.73 ms, C1 Verify
-        // 17.2k -> 18.1k ops/s on GB300)
+        // one dependent product per lane, inlined
         r = fp_mul_inl(x, y);
       } else if (type == PP_LIN) {
         r = (tw & PP_F_UNIT) ? lin(sl, e0, na) : wsum(sl, terms_lo(e0, e1), na);

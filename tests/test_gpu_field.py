@@ -28,6 +28,17 @@ def test_fp_mul_carry_save(gpu, oracle):
     assert [g[1] for g in cs] == [oracle.fp_mul(x, y) for x, y in zip(a, b)]
 
 
+@pytest.mark.parametrize("values", ["edges", "random"])
+def test_fp_sqr(gpu, oracle, values):
+    """The square (its own carry chains) against the oracle's product: limbs of all ones, single bits at every limb
+    boundary, the largest residues, and random values."""
+    p = oracle.P_MOD
+    xs = [p - 1, p - 2, 0, 1, 2, (p - 1) // 2, (p + 1) // 2, (1 << 380) - 1]
+    xs += [1 << (32 * k + b) for k in range(12) for b in (0, 15, 28)] + [(1 << (32 * k)) - 1 for k in range(1, 12)]
+    a = [x.to_bytes(48, "big") for x in xs] if values == "edges" else rand_fp(oracle, b"sqr", 1024)
+    assert [g[1] for g in gpu.fp_op_for_test(5, a, a)] == [oracle.fp_mul(x, x) for x in a]
+
+
 def test_fp_inv_sqrt(gpu, oracle):
     a = rand_fp(oracle, b"inv", 16)
     inv = gpu.fp_op_for_test(1, a, a)
