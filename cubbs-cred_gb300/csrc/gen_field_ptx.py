@@ -143,7 +143,8 @@ def gen_field(name, mod, n):
 def gen_lazy(name, mod, n):
     """Unreduced sums for short signed sums of reduced values (at most 6 terms
     of [0, mod], so every partial sum stays below 6 mod < 2^(32n)):
-    {name}_acc_add (plain add), {name}_from_mod (mod - a) and {name}_csub{k}
+    {name}_acc_add / _acc_sub (plain add and subtract; _x: of n + 1 words),
+    {name}_acc_add_3mod (a + 3 mod), {name}_from_mod (mod - a) and {name}_csub{k}
     (subtract k*mod when the value is at least k*mod, k = 4, 2, 1), which bring
     a value below 8 mod back to [0, mod)."""
     assert 6 * mod < 1 << (32 * n)
@@ -159,6 +160,30 @@ def gen_lazy(name, mod, n):
     w(f'  asm("' + "\\n\\t".join(body) + f'" : {outs} : {ins2});')
     w("}")
     ml = limbs(mod, n)
+    body = [f"sub.cc.u32 %0, %{n}, %{2 * n};"]
+    for j in range(1, n):
+        body.append(f"sub{'c.cc' if j < n - 1 else 'c'}.u32 %{j}, %{n + j}, %{2 * n + j};")
+    w(f"__device__ __forceinline__ void {name}_acc_sub(uint32_t *r, const uint32_t *a, const uint32_t *b) {{")
+    w(f'  asm("' + "\\n\\t".join(body) + f'" : {outs} : {ins2});')
+    w("}")
+    m3 = limbs(3 * mod, n)
+    body = [f"add.cc.u32 %0, %{n}, 0x{m3[0]:08x};"]
+    for j in range(1, n):
+        body.append(f"add{'c.cc' if j < n - 1 else 'c'}.u32 %{j}, %{n + j}, 0x{m3[j]:08x};")
+    w(f"__device__ __forceinline__ void {name}_acc_add_3mod(uint32_t *r, const uint32_t *a) {{")
+    w(f'  asm("' + "\\n\\t".join(body) + f'" : {outs} : {ins1});')
+    w("}")
+    # sums of n + 1 words
+    k = n + 1
+    for nm, op in (("acc_add_x", "add"), ("acc_sub_x", "sub")):
+        body = [f"{op}.cc.u32 %0, %{k}, %{2 * k};"]
+        for j in range(1, k):
+            body.append(f"{op}{'c.cc' if j < k - 1 else 'c'}.u32 %{j}, %{k + j}, %{2 * k + j};")
+        outx = ", ".join(f'"=&r"(r[{i}])' for i in range(k))
+        insx = ", ".join(f'"r"({v}[{i}])' for v in "ab" for i in range(k))
+        w(f"__device__ __forceinline__ void {name}_{nm}(uint32_t *r, const uint32_t *a, const uint32_t *b) {{")
+        w(f'  asm("' + "\\n\\t".join(body) + f'" : {outx} : {insx});')
+        w("}")
     body = [f"sub.cc.u32 %0, 0x{ml[0]:08x}, %{n};"]
     for j in range(1, n):
         body.append(f"sub{'c.cc' if j < n - 1 else 'c'}.u32 %{j}, 0x{ml[j]:08x}, %{n + j};")

@@ -1579,8 +1579,7 @@ void run_pgen(Runtime &rt, OpBatch &b, uint8_t *dmapdst) {
 // Verify on three streams, as ProofVerify: the signature decode (stream2, no
 // subgroup check) and its GLV term run beside the message hash, the domain and
 // the B-MSM (stream); the subgroup check runs on stream4; the pairing checks
-// follow the finish kernel.  Small batches take the two-warp pairing kernel
-// (lower latency per check).
+// follow the finish kernel.
 void run_verify(Runtime &rt, OpBatch &b, uint8_t *dmapdst) {
   cudaStream_t s = rt.stream, s2 = rt.stream2, s4 = rt.stream4;
   size_t n = b.n, nm = b.ml.count(), npts = b.pts48.size() / 48;

@@ -8,8 +8,9 @@
 // (native/cuda/src/kernels/pairing.cuh:376-478, host :579-737).
 #include <cstdlib>
 
-#include "pairing_team.cuh"
 #include "runtime.cuh"
+
+#include "pairing_quad.cuh"
 
 namespace cubbs {
 
@@ -90,15 +91,14 @@ __global__ void __launch_bounds__(64) k_pairing_check_split(const PairJob *jobs,
   if (lane == 0) ok[item] = one ? 1 : 0;
 }
 
-// The same with a two-warp team per pair (four warps per check): team t runs
-// the Miller loop of pair t on named barrier 1 + t, then team 0 multiplies
-// the two values and runs the final exponentiation.  Phases of up to 64
-// products take one round (pairing_team.cuh).
-__global__ void __launch_bounds__(128) k_pairing_check_split_wide(const PairJob *jobs, uint32_t n,
-                                                                  const line2 *lines, uint8_t *ok) {
-  extern __shared__ __align__(16) uint8_t pp_smem[];
-  const int team = threadIdx.x >> 6, lane = threadIdx.x & 63, bar = 1 + team;
-  fp *sl = reinterpret_cast<fp *>(pp_smem) + team * PP_SLOTS;
+// One check per block of four warps (pairing_quad.cuh).  Calls of n checks
+// through the pairing-equality entry point (decode included), one warp per
+// check -> this: 1: 3.86 -> 2.44 ms, 152: 3.95 -> 2.53, 608: 4.09 -> 3.04, 1216: 4.94 -> 4.33,
+// 4864: 12.4 -> 12.0; no size prefers the one-warp form, which is left for CUBBS_BBS_PAIR_TEAM=32
+// and for the units of the uneven-MSM engine.
+__global__ void __launch_bounds__(128) k_pairing_check_team(const PairJob *jobs, uint32_t n, const line2 *lines,
+                                                            uint8_t *ok) {
+  __shared__ __align__(16) pq::Mem mem;
   const uint32_t item = blockIdx.x;
   if (item >= n) return;
   const PairJob &j = jobs[item];
@@ -106,20 +106,11 @@ __global__ void __launch_bounds__(128) k_pairing_check_split_wide(const PairJob 
     if (threadIdx.x == 0 && j.active == 0) ok[item] = 0;
     return;
   }
-  const bool skip = (j.flags >> team) & 1;
-  const line2 *L = lines + (size_t)(team ? j.slot_b : j.slot_a) * MILLER_LINES;
-  pp::miller_one<64>(sl, lane, team ? j.pb : j.pa, L, skip, bar);
-  __syncthreads();
-  if (team != 0) return;
-  if (lane < 12) pp::st(sl, PP_REG(PP_REG_X) + lane, pp::ld(sl + PP_SLOTS, PP_REG(PP_REG_F) + lane));
-  pp::team_sync<64>(bar);
-  pp::run<64>(sl, lane, PP_MUL_F_F_X, bar);
-  pp::run<64>(sl, lane, PP_CONJ_F, bar);  // z < 0
-  const bool one = pp::final_exp_is_one<64>(sl, lane, bar);
-  if (lane == 0) ok[item] = one ? 1 : 0;
+  const bool one = pq::pairing_check(&mem, j, lines);
+  if (threadIdx.x == 0) ok[item] = one ? 1 : 0;
 }
 
-// Two-warp teams unless CUBBS_BBS_PAIR_TEAM=32 (one warp per pair).
+// Four warps per check unless CUBBS_BBS_PAIR_TEAM=32 (one warp per pair).
 static bool wide_pair_teams() {
   static const bool v = [] {
     const char *e = std::getenv("CUBBS_BBS_PAIR_TEAM");
@@ -132,13 +123,11 @@ void launch_pairing_check_split(cudaStream_t s, const PairJob *jobs, uint32_t n,
   const size_t smem = 2 * (size_t)PP_SLOTS * sizeof(fp);
   static const bool attr = [smem] {
     CUBBS_CHECK(cudaFuncSetAttribute(k_pairing_check_split, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    CUBBS_CHECK(
-        cudaFuncSetAttribute(k_pairing_check_split_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     return true;
   }();
   (void)attr;
   if (!n) return;
-  if (wide_pair_teams()) k_pairing_check_split_wide<<<n, 128, smem, s>>>(jobs, n, lines, ok);
+  if (wide_pair_teams()) k_pairing_check_team<<<n, 128, 0, s>>>(jobs, n, lines, ok);
   else k_pairing_check_split<<<n, 64, smem, s>>>(jobs, n, lines, ok);
 }
 
@@ -218,7 +207,9 @@ void launch_pairing_check(cudaStream_t s, const PairJob *jobs, uint32_t n, const
     return true;
   }();
   (void)attr;
-  if (n) k_pairing_check_warp<<<n, 32, smem, s>>>(jobs, n, lines, ok);
+  if (!n) return;
+  if (wide_pair_teams()) k_pairing_check_team<<<n, 128, 0, s>>>(jobs, n, lines, ok);
+  else k_pairing_check_warp<<<n, 32, smem, s>>>(jobs, n, lines, ok);
 }
 
 }  // namespace cubbs

@@ -1,0 +1,299 @@
+// Four-warp pairing check: one block of 128 lanes evaluates
+//     e(P_a, Q_a) * e(P_b, Q_b) == 1
+// for the launches whose latency is one check's: both lines share one Miller
+// loop, and an Fp12 operation is one round of products and one round of signed
+// sums (tables of gen_pairing_quad.py, checked there on exact integers).
+//
+// What bounds it: a lone warp's product, 1730 cycles of multiply-adds at six
+// cycles each (field.cuh), in a chain of 315 cyclotomic squarings, 136 Miller
+// rounds and about 40 others.  So every operation is cut to one product deep
+// (two in a Miller step): schoolbook Fp2 products on up to 128 lanes, one warp
+// per SM sub-partition, all outputs as sums of products.  The sums take
+// 2^g lanes an output, four slots a lane, carry chains instead of
+// weighted multiply-adds, and one reduction by a multiple of p from a table.
+// The cyclotomic squaring is 30 products: it stays in one warp, without block
+// barriers.  Against the two-warp teams per pair that this replaces (LIN
+// phases of at most 14 weighted terms, four to six a product): see
+// k_pairing_check_team.
+#pragma once
+#include "pairing_team.cuh"
+
+#include "pairing_quad_program.cuh"
+
+namespace pq {
+
+static_assert(PQ_SLOTS >= PP_SLOTS, "the inverse runs on the same slots");
+struct Mem {
+  fp slot[PQ_SLOTS];
+  fp mul_p[PQ_QMAX];  // k p
+};
+
+DEV fp ld(const fp *sl, uint32_t off) {
+  const uint4 *p = reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(sl) + off);
+  const uint4 a = p[0], b = p[1], c = p[2];
+  return {{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w}};
+}
+DEV void st(fp *sl, uint32_t off, const uint32_t *w) {
+  uint4 *p = reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(sl) + off);
+  p[0] = make_uint4(w[0], w[1], w[2], w[3]);
+  p[1] = make_uint4(w[4], w[5], w[6], w[7]);
+  p[2] = make_uint4(w[8], w[9], w[10], w[11]);
+}
+
+// slot[out] = (slot[a] [+ slot[a2]]) (slot[b] [+ slot[b2]]) << dbl, not fully
+// reduced: operands below 2.1 p give a product below 1.42 p.
+DEV void product(fp *sl, const uint4 &e) {
+  fp a = ld(sl, e.x & 0xffffu), b = ld(sl, e.x >> 16);
+  if (e.w & 0x10u) {  // the same on every lane of a phase
+    const fp a2 = ld(sl, e.y & 0xffffu), b2 = ld(sl, e.y >> 16);
+    fp_acc_add(a.w, a.w, a2.w);
+    fp_acc_add(b.w, b.w, b2.w);
+  }
+  const uint32_t sh = (e.w >> 5) & 1u;
+#pragma unroll
+  for (int j = 11; j > 0; j--) b.w[j] = __funnelshift_l(b.w[j - 1], b.w[j], sh);
+  b.w[0] <<= sh;
+  fp r;
+  fp_mont_mul(r.w, a.w, b.w);
+  if ((e.z & 0xffffu) != PQ_NONE) st(sl, e.z & 0xffffu, r.w);
+}
+
+// 3p + slot[p0] + slot[p1] - slot[m0] - slot[m1], in (0, 6p)
+DEV fp lane_sum(const fp *sl, uint32_t plus, uint32_t minus) {
+  const fp p0 = ld(sl, plus & 0xffffu), p1 = ld(sl, plus >> 16), m0 = ld(sl, minus & 0xffffu),
+           m1 = ld(sl, minus >> 16);
+  fp t;
+  fp_acc_add_3mod(t.w, p0.w);
+  fp_acc_add(t.w, t.w, p1.w);
+  fp_acc_sub(t.w, t.w, m0.w);
+  fp_acc_sub(t.w, t.w, m1.w);
+  return t;
+}
+
+// The 13-word value v < PQ_QMAX p brought below 1.001 p: the quotient from its
+// top 32 bits (bits 360..391) in single precision, a little low so that it
+// never exceeds v / p, and that multiple of p taken off.
+DEV void reduce13(const fp *mul_p, const uint32_t *v, uint32_t *r) {
+  constexpr float K = (float)(256.0 / 436277739.0 * (1.0 - 1.0 / 1048576.0));  // 436277739 = floor(p / 2^352) + 1
+  const uint32_t q = (uint32_t)(__uint2float_rz(__funnelshift_l(v[11], v[12], 24)) * K);
+  const fp m = ld(mul_p, q * (uint32_t)sizeof(fp));
+  fp_acc_sub(r, v, m.w);
+}
+
+DEV void add_lane(uint32_t *v, int d) {
+  uint32_t o[13];
+#pragma unroll
+  for (int j = 0; j < 13; j++) o[j] = __shfl_xor_sync(0xffffffffu, v[j], d);
+  fp_acc_add_x(v, v, o);
+}
+
+// One output per 2^g lanes; every lane of the warp calls it.
+DEV void sums(Mem *m, const uint4 &e) {
+  const int g = (int)(e.w >> 4) & 7;
+  if (g == 7) return;
+  uint32_t v[13];
+  const fp t = lane_sum(m->slot, e.x, e.y);
+#pragma unroll
+  for (int j = 0; j < 12; j++) v[j] = t.w[j];
+  v[12] = 0;
+#pragma unroll 1
+  for (int d = 1; d < (1 << g); d <<= 1) add_lane(v, d);
+  if ((e.z & 0xffffu) != PQ_NONE) {
+    uint32_t r[12];
+    reduce13(m->mul_p, v, r);
+    st(m->slot, e.z & 0xffffu, r);
+  }
+}
+
+// Runs program `prog`; every lane of the block calls it, and the block is in
+// step before and after.
+static __device__ __noinline__ void run(Mem *m, int prog) {
+  const int lane = threadIdx.x;
+  const int ph0 = PQ_FIRST[prog], ph1 = PQ_FIRST[prog + 1];
+  uint4 e = __ldg(&PQ_ENTRY[ph0 * PQ_LANES + lane]);
+#pragma unroll 1
+  for (int ph = ph0; ph < ph1; ph++) {
+    const uint4 nx = __ldg(&PQ_ENTRY[min(ph + 1, ph1 - 1) * PQ_LANES + lane]);
+    if (e.w & 1u) sums(m, e);
+    else if ((e.z & 0xffffu) != PQ_NONE) product(m->slot, e);
+    __syncthreads();
+    e = nx;
+  }
+}
+
+// Register R squared n times in the cyclotomic subgroup, on one warp.  An
+// output is 3 A + post with A on a lane pair (two lane sums) and post one
+// slot added or subtracted on the odd lane.
+static __device__ __noinline__ void cyclo(Mem *m, int n) {
+  const int lane = threadIdx.x & 31;
+  const uint4 em = __ldg(&PQ_CYCLO_M[lane]), es = __ldg(&PQ_CYCLO_S[lane]);
+#pragma unroll 1
+  for (; n > 0; n--) {
+    product(m->slot, em);
+    __syncwarp();
+    const fp t = lane_sum(m->slot, es.x, es.y);
+    const fp pp = ld(m->slot, es.z >> 16), pm = ld(m->slot, es.w);
+    uint32_t a[13], v[13];
+    v[0] = t.w[0] << 1;
+#pragma unroll
+    for (int j = 1; j < 12; j++) v[j] = __funnelshift_l(t.w[j - 1], t.w[j], 1);
+    v[12] = t.w[11] >> 31;
+#pragma unroll
+    for (int j = 0; j < 12; j++) a[j] = t.w[j];
+    a[12] = 0;
+    fp_acc_add_x(v, v, a);  // 3 t
+#pragma unroll
+    for (int j = 0; j < 12; j++) a[j] = pp.w[j];
+    fp_acc_add_x(v, v, a);
+#pragma unroll
+    for (int j = 0; j < 12; j++) a[j] = pm.w[j];
+    fp_acc_sub_x(v, v, a);
+    add_lane(v, 1);
+    __syncwarp();  // every lane has read its slots
+    if ((es.z & 0xffffu) != PQ_NONE) {
+      uint32_t r[12];
+      reduce13(m->mul_p, v, r);
+      st(m->slot, es.z & 0xffffu, r);
+    }
+    __syncwarp();
+  }
+}
+
+// Register `dst` = register `src`.
+DEV void copy_reg(Mem *m, int dst, int src) {
+  const int t = threadIdx.x;
+  if (t < 36) {
+    const uint4 *s = reinterpret_cast<const uint4 *>(&m->slot[PP_REG(src)]);
+    reinterpret_cast<uint4 *>(&m->slot[PP_REG(dst)])[t] = s[t];
+  }
+  __syncthreads();
+}
+// R = R^|z| with R = the base held in the register that mul_prog multiplies by.
+DEV void exp_by_zabs(Mem *m, int mul_prog) {
+#pragma unroll 1
+  for (int k = 0; k < 6; k++) {
+    // |z| = 2^63 + 2^62 + 2^60 + 2^57 + 2^48 + 2^16
+    const int n = k < 3 ? k + 1 : k == 3 ? 9 : k == 4 ? 32 : 16;
+    if (threadIdx.x < 32) cyclo(m, n);
+    __syncthreads();
+    if (k < 5) run(m, mul_prog);
+  }
+}
+
+// Registers r's slots fully reduced (S outputs are below 1.001 p).
+DEV void canonical(Mem *m, int r) {
+  const int t = threadIdx.x;
+  if (t < 12) {
+    fp &v = m->slot[PP_REG(r) + t];
+    fp_csub1(v.w, v.w);
+  }
+  __syncthreads();
+}
+
+// Component c (A.c0, A.c1, B.c0, B.c1) of a line; a skipped pair has the line 1.
+DEV fp line_part(const line2 *L, bool skip, int idx, int c) {
+  if (skip) return c == 0 ? fp_one() : fp_zero();
+  const line2 &l = L[idx];
+  return c == 0 ? l.a.c0 : c == 1 ? l.a.c1 : c == 2 ? l.b.c0 : l.b.c1;
+}
+
+// The whole check; true on every lane when the product of the pairings is 1.
+// All 128 lanes of the block call it.
+template <class Job> DEV bool pairing_check(Mem *m, const Job &j, const line2 *lines) {
+  const int t = threadIdx.x;
+  const bool skip[2] = {(j.flags & 1) != 0, (j.flags & 2) != 0};
+  const line2 *const L[2] = {lines + (size_t)j.slot_a * MILLER_LINES, lines + (size_t)j.slot_b * MILLER_LINES};
+  fp *sl = m->slot;
+  // constants, points, F = 1
+  if (t < PQ_QMAX) {
+    const fp pm = FP_MOD_INIT;
+    uint64_t c = 0;
+    for (int k = 0; k < 12; k++) {
+      c += (uint64_t)pm.w[k] * (uint32_t)t;
+      m->mul_p[t].w[k] = (uint32_t)c;
+      c >>= 32;
+    }
+  } else if (t < PQ_QMAX + 10) {
+    const fp2 g[6] = C_FROB_GAMMA;
+    const int k = t - PQ_QMAX;
+    const fp2 &ge = g[1 + (k >> 1)];
+    sl[PP_GAMMA_BASE + k] = (k & 1) ? ge.c1 : ge.c0;
+  } else if (t < PQ_QMAX + 14) {
+    const int k = t - PQ_QMAX - 10, p = k >> 1;
+    const g1a &pt = p ? j.pb : j.pa;
+    sl[PP_PT_BASE + k] = skip[p] ? fp_zero() : ((k & 1) ? pt.y : pt.x);
+  } else if (t == PQ_QMAX + 14) {
+    sl[PP_ZERO_SLOT] = fp_zero();
+  } else if (t >= 96 && t < 108) {
+    sl[PP_REG(PP_REG_F) + t - 96] = t == 96 ? fp_one() : fp_zero();
+  } else if (t >= 112 && t < 120) {
+    sl[PP_LINE_BASE + t - 112] = line_part(L[(t - 112) >> 2], skip[(t - 112) >> 2], 0, t & 3);
+  }
+  __syncthreads();
+  run(m, PQ_LINE);
+  // Miller loop: the lanes that no product of a step's first round uses fetch
+  // the next step's lines, whose B xP the second round multiplies
+  const int lp = (t >> 2) & 1;
+  const bool fetch = t >= 120;
+  int idx = 1;
+#pragma unroll 1
+  for (int i = 62; i >= 0; i--) {
+#pragma unroll 1
+    for (int add = 0; add <= (int)zabs_bit(i); add++) {
+      const int ph = PQ_FIRST[add ? PQ_ADD : PQ_DBL];
+      const uint4 *tab = &PQ_ENTRY[ph * PQ_LANES + t];
+      uint4 e = __ldg(tab);
+      fp next = fp_zero();
+      if (fetch && idx < MILLER_LINES) next = line_part(L[lp], skip[lp], idx, t & 3);
+      idx++;
+      const uint4 e1 = __ldg(tab + PQ_LANES), e2 = __ldg(tab + 2 * PQ_LANES), e3 = __ldg(tab + 3 * PQ_LANES);
+#pragma unroll 1
+      for (int k = 0; k < 2; k++) {
+        if ((e.z & 0xffffu) != PQ_NONE) product(sl, e);
+        __syncthreads();
+        if (k == 0 && fetch) sl[PP_LINE_BASE + t - 120] = next;
+        sums(m, k ? e3 : e1);
+        __syncthreads();
+        e = e2;
+      }
+    }
+  }
+  // F holds the conjugate of the Miller value f (z < 0), so f^(p^6 - 1) =
+  // F conj(F)^-1 = F conj(F^-1); then the powers as in final_exponentiation of
+  // pairing.cuh (b^(z^2) needs no conjugation: both signs cancel)
+  canonical(m, PP_REG_F);
+  if (t < 64) pp::run<64>(sl, t, PP_INV_U_F, 1);
+  __syncthreads();
+  if (t < 5) sl[PQ_NORM2_BASE + t] = PQ_NORM2[t];  // the inverse's temporaries lie over these slots
+  __syncthreads();
+  run(m, PQ_T_F_CU);
+  run(m, PQ_T_T2_T);
+  copy_reg(m, PP_REG_R, PP_REG_T);
+  exp_by_zabs(m, PQ_R_R_T);
+  run(m, PQ_A_CRT);  // a = t^z conj(t)
+  copy_reg(m, PP_REG_R, PP_REG_A);
+  exp_by_zabs(m, PQ_R_R_A);
+  run(m, PQ_A_CRA);  // a = a^z conj(a)
+  copy_reg(m, PP_REG_R, PP_REG_A);
+  exp_by_zabs(m, PQ_R_R_A);
+  run(m, PQ_X_FROB_A);
+  run(m, PQ_A_X_CR);  // b = a^z a^p
+  copy_reg(m, PP_REG_R, PP_REG_A);
+  exp_by_zabs(m, PQ_R_R_A);
+  copy_reg(m, PP_REG_X, PP_REG_R);
+  exp_by_zabs(m, PQ_R_R_X);  // b^(z^2)
+  run(m, PQ_R_A2_R);         // b^(z^2) b^(p^2)
+  run(m, PQ_R_R_CA);
+  run(m, PQ_R_R_T);
+  run(m, PQ_R_R_T);
+  run(m, PQ_R_R_T);
+  canonical(m, PP_REG_R);
+  bool one = true;
+  if (t < 12) {
+    const fp v = sl[PP_REG(PP_REG_R) + t];
+    one = t == 0 ? fp_eq(v, fp_one()) : fp_is_zero(v);
+  }
+  return __syncthreads_and(one);
+}
+
+}  // namespace pq
