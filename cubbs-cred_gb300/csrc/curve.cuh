@@ -727,53 +727,6 @@ DEV g1 g1_mul_glv_quad(const LaneQuad &lq, g1a p, fr k) {
   return acc;
 }
 
-// k * P on eight lanes: the quad of lanes 8j .. 8j+3 computes s P and the quad
-// of lanes 8j+4 .. 8j+7 computes q [lambda]P = q phi(P) (k = q lambda + s),
-// each with its own doubling chain (half the additions of the shared chain
-// each); the first quad adds the second quad's sum.  Lanes of the first quad
-// return k * P.  All eight lanes must call it.
-DEV g1 g1_mul_glv_octet(const LaneQuad &lq, g1a p, fr k) {
-  uint32_t s[4], q[4];
-  glv_split(k, s, q);
-  const int half = (threadIdx.x >> 2) & 1;
-  int8_t d[33];
-  recode_w4(half ? q : s, d);
-  if (half) {
-    const fp beta = C_GLV_BETA;
-    p.x = fp_mul(p.x, beta);  // phi(P) = (beta x, -y) = [lambda]P
-    p.y = fp_neg(p.y);
-  }
-  g1 tab[8];
-  tab[0] = g1_from_aff(p);
-  tab[1] = g1_dbl_quad(lq, g1_from_aff(p));
-  #pragma unroll 1
-  for (int i = 2; i < 8; i++) tab[i] = g1_add_aff_quad(lq, tab[i - 1], p);
-  g1 acc = g1_inf();
-  #pragma unroll 1
-  for (int i = 32; i >= 0; i--) {
-    if (i != 32) {
-      acc = g1_dbl_quad(lq, acc); acc = g1_dbl_quad(lq, acc); acc = g1_dbl_quad(lq, acc); acc = g1_dbl_quad(lq, acc);
-    }
-    const int a = d[i];
-    if (a) {
-      g1 t = tab[(a > 0 ? a : -a) - 1];
-      acc = g1_add_quad(lq, acc, a > 0 ? t : g1_neg(t));
-    }
-  }
-  // both quads meet here: the first takes the second's sum
-  const unsigned oct = 0xFFu << (threadIdx.x & 24);
-  g1 other;
-#pragma unroll
-  for (int i = 0; i < 12; i++) {
-    other.X.w[i] = __shfl_xor_sync(oct, acc.X.w[i], 4);
-    other.Y.w[i] = __shfl_xor_sync(oct, acc.Y.w[i], 4);
-    other.ZZ.w[i] = __shfl_xor_sync(oct, acc.ZZ.w[i], 4);
-    other.ZZZ.w[i] = __shfl_xor_sync(oct, acc.ZZZ.w[i], 4);
-  }
-  if (half) return acc;
-  return g1_add_quad(lq, acc, other);
-}
-
 // ------------------------------------------------------------------ G2 (Jacobian over Fp2)
 struct g2a { fp2 x, y; };
 struct g2j { fp2 X, Y, Z; };

@@ -320,6 +320,17 @@ def main():
     betas = [(-1 + s) * inv(2) % P, (-1 - s) * inv(2) % P]
     zz = ec_mul(lam, (G1X, G1Y))
     beta = [b for b in betas if (b * G1X % P, (-G1Y) % P) == zz][0]
+    # E': y^2 = x^3 + 2/3 through (x, y) -> (s^2 x, s^3 y), s^6 = (2/3) / 4: 3 b' = 2 keeps the multiples in the
+    # complete addition law small
+    s6 = inv(6)
+    s3 = sqrt(s6)
+    m, w = (P - 1) // 9, next(g for g in range(2, 50) if pow(g, (P - 1) // 3, P) != 1)
+
+    def cube_root(a):  # 9 divides p - 1, 27 does not
+        x = pow(a, pow(3, -1, m), P)
+        return next(x * pow(w, m * k, P) % P for k in range(9) if pow(x * pow(w, m * k, P) % P, 3, P) == a % P)
+    s1 = next(cube_root(t) for t in (s3, P - s3) if pow(t, (P - 1) // 3, P) == 1)
+    assert pow(s1, 6, P) == s6
     # Frobenius gammas for Fp12 = Fp2[w]/(w^6 - xi)
     def f2mul(a, b):
         return ((a[0] * b[0] - a[1] * b[1]) % P, (a[0] * b[1] + a[1] * b[0]) % P)
@@ -356,6 +367,10 @@ def main():
         f"#define C_G2_GEN_Y1 {fp_init(G2Y1)}",
         f"// beta: [z^2](x, y) = (beta x, -y) on G1, z^2 = 0x{lam:x}",
         f"#define C_GLV_BETA {fp_init(beta)}",
+        "// E': y^2 = x^3 + 2/3, (x, y) -> (s^2 x, s^3 y): s^2, s^3, beta s^2",
+        f"#define C_B3_S2 {fp_init(s1 * s1)}",
+        f"#define C_B3_S3 {fp_init(pow(s1, 3, P))}",
+        f"#define C_B3_BETA_S2 {fp_init(beta * s1 * s1)}",
         f"#define C_GLV_LAMBDA_LO 0x{lam & ((1 << 64) - 1):016x}ull",
         f"#define C_GLV_LAMBDA_HI 0x{lam >> 64:016x}ull",
         f"#define C_SSWU_A {fp_init(SSWU_A)}",

@@ -10,6 +10,7 @@
 // decode and compress run on the device.
 #include <cstdlib>
 
+#include "g1_ladder.cuh"
 #include "runtime.cuh"
 
 namespace cubbs {
@@ -195,20 +196,47 @@ __global__ void __launch_bounds__(128) k_var_mul_quad(const g1a *points, const V
   const g1 r = g1_mul_glv_quad(lq, points[j.point], scalars[i]);
   if (lq.role == 0) out[i] = r;
 }
-// Eight lanes per job (g1_mul_glv_octet): one quad per GLV half.
-__global__ void __launch_bounds__(128) k_var_mul_octet(const g1a *points, const VarJob *jobs, const fr *scalars,
+// Two ladders of eight lanes per job (g1_ladder.cuh), one per GLV half; two
+// jobs a warp, one warp a block.
+__global__ void __launch_bounds__(32) k_var_mul_ladder(const g1a *points, const VarJob *jobs, const fr *scalars,
                                                        uint32_t n, g1 *out) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  const uint32_t i = t >> 3;
-  if (i >= n) return;  // the eight lanes of a job leave together
-  const LaneQuad lq = LaneQuad::here();
-  const VarJob j = jobs[i];
-  if (j.flags & 1) {
-    if ((t & 7) == 0) out[i] = g1_inf();
-    return;
+  __shared__ __align__(16) gl::Mem mem;
+  if (n == 0) return;
+  const int lane = threadIdx.x & 31, role = lane & 7, half = (lane >> 3) & 1;
+  const uint32_t i = 2 * blockIdx.x + (lane >> 4);
+  const uint32_t j = min(i, n - 1);  // a warp's spare ladders repeat the last job
+  const VarJob job = jobs[j];
+  const bool inf = job.flags & 1;
+  g1a p;
+  p.x = p.y = fp_one();
+  if (!inf) p = points[job.point];
+  gl::start(&mem, p, half != 0);
+  uint32_t s[4], q[4];
+  glv_split(scalars[j], s, q);
+  gl::ladder128(&mem, half ? q : s);
+  // the first ladder takes the second's sum (its entry 0), and leaves E'
+  fp *sl = mem.slot[lane >> 3];
+  if (!half && role < 3) sl[gl::TAB + (role == 2 ? 3 : role)] = mem.slot[(lane >> 3) + 1][gl::AX + role];
+  __syncwarp();
+  gl::add_digit(&mem, 1);
+  if (!half && role < 2) {
+    const fp s2 = C_B3_S2, s3 = C_B3_S3;
+    fp v[2];  // (X Z, s^2 Z^2) or (Y Z^2, s^3 Z^3)
+    const fp z = sl[gl::AZ];
+    fp zz = z;
+    if (role == 1) zz = fp_mul(z, z);
+    v[0] = fp_mul(sl[gl::AX + role], zz);
+    v[1] = fp_mul(fp_mul(zz, z), role ? s3 : s2);
+    if (i < n) {
+      if (inf) {
+        const g1 o = g1_inf();
+        v[0] = role ? o.Y : o.X;
+        v[1] = fp_zero();
+      }
+      (role ? out[i].Y : out[i].X) = v[0];
+      (role ? out[i].ZZZ : out[i].ZZ) = v[1];
+    }
   }
-  const g1 r = g1_mul_glv_octet(lq, points[j.point], scalars[i]);
-  if ((t & 7) == 0) out[i] = r;
 }
 __global__ void __launch_bounds__(128) k_var_mul(const g1a *points, const VarJob *jobs, const fr *scalars,
                                                  uint32_t n, g1 *out) {
@@ -256,6 +284,41 @@ __global__ void __launch_bounds__(64) k_g1_subgroup_quad(const g1a *pts, const i
   if (lq.role == 0) bad[i] = outside ? 1 : 0;
 }
 
+// One ladder of eight lanes per point (g1_ladder.cuh), four points a warp, one
+// warp a block: phi(P) == -[z^2]P, that is [z^2]P == (beta x, -y).
+__global__ void __launch_bounds__(32) k_g1_subgroup_ladder(const g1a *pts, const int32_t *status, uint32_t n,
+                                                           int32_t *bad) {
+  __shared__ __align__(16) gl::Mem mem;
+  const int lane = threadIdx.x & 31, role = lane & 7;
+  const uint32_t i = 4 * blockIdx.x + (lane >> 3), j = min(i, n - 1);
+  const bool ok = status[j] == DEC_OK;
+  g1a p;
+  p.x = p.y = fp_one();
+  if (ok) p = pts[j];
+  gl::start(&mem, p, false);
+  fp *sl = mem.slot[lane >> 3];
+  gl::mul_zabs(&mem);
+  gl::store_entry(sl, role, 1);  // keep the first entry (P) for the comparison
+  if (role < 4) {  // swap entries 0 and 1: the second half multiplies [|z|]P
+    const fp t = sl[gl::TAB + role];
+    sl[gl::TAB + role] = sl[gl::TAB + 4 + role];
+    sl[gl::TAB + 4 + role] = t;
+  }
+  __syncwarp();
+  gl::mul_zabs(&mem);
+  if (role == 0 && i < n) {
+    const fp beta = C_GLV_BETA;
+    fp X = sl[gl::AX], Y = sl[gl::AY], Z = sl[gl::AZ], x = sl[gl::TAB + 4], y = sl[gl::TAB + 5];
+    fp_csub1(X.w, X.w);
+    fp_csub1(Y.w, Y.w);
+    fp_csub1(Z.w, Z.w);
+    fp_csub1(x.w, x.w);
+    fp_csub1(y.w, y.w);
+    const bool in = !fp_is_zero(Z) && fp_eq(X, fp_mul(fp_mul(x, beta), Z)) && fp_eq(Y, fp_mul(fp_neg(y), Z));
+    bad[i] = ok && !in ? 1 : 0;
+  }
+}
+
 // CUBBS_BBS_VAR_LANES (1, 2, 4 or 8; else 0: chosen by launch size).
 int var_lanes_setting() {
   static const int v = [] {
@@ -266,22 +329,24 @@ int var_lanes_setting() {
   return v;
 }
 // Lanes per job for a launch of n jobs: the CUBBS_BBS_VAR_LANES setting, else
-// by size.  A few jobs leave the GPU idle, so each job's chain of products is
-// spread over more lanes (8: the two GLV halves on a quad each); thousands of
-// jobs fill the GPU, where lane pairs spend the fewest instructions per job.
-// Measured on GB300: in the 1024-proof ProofVerify step (4096 jobs) 2 lanes
-// 4.47 ms, 4 lanes 5.08, 8 lanes 5.40; Verify of 64 signatures (64 jobs) 8
-// lanes 12 % faster than 2.
-static int lanes_for(uint32_t n, int max_lanes) {
-  int l = var_lanes_setting();
-  if (l == 0) l = n <= 1024 ? 8 : n <= 2048 ? 4 : 2;
-  return l > max_lanes ? max_lanes : l;
+// by size.  Few jobs leave the GPU idle, so each takes ladders of eight lanes
+// (g1_ladder.cuh); thousands fill it, where lane pairs spend fewer
+// instructions a job.  Measured on GB300, 8 lanes against 2: Verify of 64
+// (64 terms) 1.72 ms against 2.45 on the lane octets before the ladders,
+// Verify of 1000 (1000 terms) 2.79 against 3.43; ProofVerify of 1024 over 64
+// keys (4096 terms, 3072 points) 3.36 against 3.37; ProofGen of 1024 (7168
+// terms) 6.21 against 5.91.  Lane quads were slower than one or the other at
+// every size (3.78, 3.66 and 6.29 ms) and are left for the setting.
+static int lanes_for(uint32_t n) {
+  const int l = var_lanes_setting();
+  return l ? l : n <= 2048 ? 8 : 2;
 }
 
 void launch_g1_subgroup(cudaStream_t s, const g1a *pts, const int32_t *status, uint32_t n, int32_t *bad, int lanes) {
   if (!n) return;
-  if (lanes == 0) lanes = lanes_for(n, 4);
-  if (lanes >= 4) k_g1_subgroup_quad<<<blocks_for(4 * (size_t)n, 64), 64, 0, s>>>(pts, status, n, bad);
+  if (lanes == 0) lanes = lanes_for(n);
+  if (lanes == 8) k_g1_subgroup_ladder<<<blocks_for(n, 4), 32, 0, s>>>(pts, status, n, bad);
+  else if (lanes == 4) k_g1_subgroup_quad<<<blocks_for(4 * (size_t)n, 64), 64, 0, s>>>(pts, status, n, bad);
   else if (lanes == 2) k_g1_subgroup<<<blocks_for(2 * (size_t)n, 32), 32, 0, s>>>(pts, status, n, bad);
   else k_g1_subgroup_lane<<<blocks_for(n, 32), 32, 0, s>>>(pts, status, n, bad);
 }
@@ -329,8 +394,8 @@ void launch_fixed_msm(cudaStream_t s, const FixedTable &t, const fr *scalars, ui
 void launch_var_mul(cudaStream_t s, const g1a *points, const VarJob *jobs, const fr *scalars, uint32_t n, g1 *out,
                     int lanes) {
   if (!n) return;
-  if (lanes == 0) lanes = lanes_for(n, 8);
-  if (lanes == 8) k_var_mul_octet<<<blocks_for(8 * (size_t)n, 128), 128, 0, s>>>(points, jobs, scalars, n, out);
+  if (lanes == 0) lanes = lanes_for(n);
+  if (lanes == 8) k_var_mul_ladder<<<blocks_for(n, 2), 32, 0, s>>>(points, jobs, scalars, n, out);
   else if (lanes == 4) k_var_mul_quad<<<blocks_for(4 * (size_t)n, 128), 128, 0, s>>>(points, jobs, scalars, n, out);
   else if (lanes == 2) k_var_mul_pair<<<blocks_for(2 * (size_t)n, 128), 128, 0, s>>>(points, jobs, scalars, n, out);
   else k_var_mul<<<blocks_for(n, 128), 128, 0, s>>>(points, jobs, scalars, n, out);
@@ -341,7 +406,7 @@ cudaError_t warm_decode_and_var_mul_kernels(uint8_t *any_device_buffer) {
   k_var_mul<<<1, 128>>>(nullptr, nullptr, nullptr, 0, nullptr);
   k_var_mul_pair<<<1, 128>>>(nullptr, nullptr, nullptr, 0, nullptr);
   k_var_mul_quad<<<1, 128>>>(nullptr, nullptr, nullptr, 0, nullptr);
-  k_var_mul_octet<<<1, 128>>>(nullptr, nullptr, nullptr, 0, nullptr);
+  k_var_mul_ladder<<<1, 32>>>(nullptr, nullptr, nullptr, 0, nullptr);
   return cudaGetLastError();
 }
 void launch_g1_compress(cudaStream_t s, const g1 *pts, uint32_t n, uint8_t *out48) {

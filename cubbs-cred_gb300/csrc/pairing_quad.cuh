@@ -17,28 +17,20 @@
 // k_pairing_check_team.
 #pragma once
 #include "pairing_team.cuh"
+#include "slots.cuh"
 
 #include "pairing_quad_program.cuh"
 
 namespace pq {
 
 static_assert(PQ_SLOTS >= PP_SLOTS, "the inverse runs on the same slots");
+static_assert(PQ_QMAX == slots::QMAX, "the bounds checked by the generator");
 struct Mem {
   fp slot[PQ_SLOTS];
   fp mul_p[PQ_QMAX];  // k p
 };
 
-DEV fp ld(const fp *sl, uint32_t off) {
-  const uint4 *p = reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(sl) + off);
-  const uint4 a = p[0], b = p[1], c = p[2];
-  return {{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w}};
-}
-DEV void st(fp *sl, uint32_t off, const uint32_t *w) {
-  uint4 *p = reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(sl) + off);
-  p[0] = make_uint4(w[0], w[1], w[2], w[3]);
-  p[1] = make_uint4(w[4], w[5], w[6], w[7]);
-  p[2] = make_uint4(w[8], w[9], w[10], w[11]);
-}
+using namespace slots;
 
 // slot[out] = (slot[a] [+ slot[a2]]) (slot[b] [+ slot[b2]]) << dbl, not fully
 // reduced: operands below 2.1 p give a product below 1.42 p.
@@ -58,41 +50,12 @@ DEV void product(fp *sl, const uint4 &e) {
   if ((e.z & 0xffffu) != PQ_NONE) st(sl, e.z & 0xffffu, r.w);
 }
 
-// 3p + slot[p0] + slot[p1] - slot[m0] - slot[m1], in (0, 6p)
-DEV fp lane_sum(const fp *sl, uint32_t plus, uint32_t minus) {
-  const fp p0 = ld(sl, plus & 0xffffu), p1 = ld(sl, plus >> 16), m0 = ld(sl, minus & 0xffffu),
-           m1 = ld(sl, minus >> 16);
-  fp t;
-  fp_acc_add_3mod(t.w, p0.w);
-  fp_acc_add(t.w, t.w, p1.w);
-  fp_acc_sub(t.w, t.w, m0.w);
-  fp_acc_sub(t.w, t.w, m1.w);
-  return t;
-}
-
-// The 13-word value v < PQ_QMAX p brought below 1.001 p: the quotient from its
-// top 32 bits (bits 360..391) in single precision, a little low so that it
-// never exceeds v / p, and that multiple of p taken off.
-DEV void reduce13(const fp *mul_p, const uint32_t *v, uint32_t *r) {
-  constexpr float K = (float)(256.0 / 436277739.0 * (1.0 - 1.0 / 1048576.0));  // 436277739 = floor(p / 2^352) + 1
-  const uint32_t q = (uint32_t)(__uint2float_rz(__funnelshift_l(v[11], v[12], 24)) * K);
-  const fp m = ld(mul_p, q * (uint32_t)sizeof(fp));
-  fp_acc_sub(r, v, m.w);
-}
-
-DEV void add_lane(uint32_t *v, int d) {
-  uint32_t o[13];
-#pragma unroll
-  for (int j = 0; j < 13; j++) o[j] = __shfl_xor_sync(0xffffffffu, v[j], d);
-  fp_acc_add_x(v, v, o);
-}
-
 // One output per 2^g lanes; every lane of the warp calls it.
 DEV void sums(Mem *m, const uint4 &e) {
   const int g = (int)(e.w >> 4) & 7;
   if (g == 7) return;
   uint32_t v[13];
-  const fp t = lane_sum(m->slot, e.x, e.y);
+  const fp t = lane_sum(m->slot, e.x & 0xffffu, e.x >> 16, e.y & 0xffffu, e.y >> 16);
 #pragma unroll
   for (int j = 0; j < 12; j++) v[j] = t.w[j];
   v[12] = 0;
@@ -131,7 +94,7 @@ static __device__ __noinline__ void cyclo(Mem *m, int n) {
   for (; n > 0; n--) {
     product(m->slot, em);
     __syncwarp();
-    const fp t = lane_sum(m->slot, es.x, es.y);
+    const fp t = lane_sum(m->slot, es.x & 0xffffu, es.x >> 16, es.y & 0xffffu, es.y >> 16);
     const fp pp = ld(m->slot, es.z >> 16), pm = ld(m->slot, es.w);
     uint32_t a[13], v[13];
     v[0] = t.w[0] << 1;
@@ -206,13 +169,7 @@ template <class Job> DEV bool pairing_check(Mem *m, const Job &j, const line2 *l
   fp *sl = m->slot;
   // constants, points, F = 1
   if (t < PQ_QMAX) {
-    const fp pm = FP_MOD_INIT;
-    uint64_t c = 0;
-    for (int k = 0; k < 12; k++) {
-      c += (uint64_t)pm.w[k] * (uint32_t)t;
-      m->mul_p[t].w[k] = (uint32_t)c;
-      c >>= 32;
-    }
+    m->mul_p[t] = multiple_of_p((uint32_t)t);
   } else if (t < PQ_QMAX + 10) {
     const fp2 g[6] = C_FROB_GAMMA;
     const int k = t - PQ_QMAX;

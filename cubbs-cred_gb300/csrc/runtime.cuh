@@ -293,7 +293,7 @@ void launch_decode_p1(cudaStream_t s, g1a *gens, uint8_t *gens_c, int suite);
 void launch_build_table(cudaStream_t s, const g1a *gens, int g0, int g1n, FixedTable t, g1a *bases,
                         g1 *scratch_xyzz, fp *scratch_prod);
 // decode N compressed G1 points: status DEC_*; affine out
-// lanes per point: 1, 2 or 4 (0: chosen by the point count or CUBBS_BBS_VAR_LANES)
+// lanes per point: 1, 2, 4 or 8 (0: chosen by the point count or CUBBS_BBS_VAR_LANES)
 void launch_g1_subgroup(cudaStream_t s, const g1a *pts, const int32_t *status, uint32_t n, int32_t *bad,
                         int lanes = 0);
 int var_lanes_setting();
@@ -307,7 +307,7 @@ struct VarJob {
   uint32_t point;  // index into the point array
   uint32_t flags;  // bit0: point is infinity (result infinity)
 };
-// lanes per job: 1, 2, 4 or 8 (0: chosen by the job count or CUBBS_BBS_VAR_LANES)
+// lanes per job: 1, 2, 4, or 8 for each half (0: chosen by the job count or CUBBS_BBS_VAR_LANES)
 void launch_var_mul(cudaStream_t s, const g1a *points, const VarJob *jobs, const fr *scalars, uint32_t n,
                     g1 *out, int lanes = 0);
 void launch_g1_compress(cudaStream_t s, const g1 *pts, uint32_t n, uint8_t *out48);

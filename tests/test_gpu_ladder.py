@@ -1,0 +1,35 @@
+"""The eight-lane G1 ladders: launches that leave lanes of a warp over, scalars at the edges of the signed 4-bit digits
+and of the GLV split, the identity, and the membership test on points in and out of G1, of small order too."""
+import pytest
+
+from helpers import scalar
+from tests.test_gpu_parity import _on_curve_outside_g1
+
+pytestmark = pytest.mark.gpu
+LAMBDA = 0xAC45A4010001A4020000000100000000
+INF = bytes([0xC0]) + bytes(47)
+
+
+@pytest.mark.parametrize("n", [1, 2, 3, 8])
+def test_terms(gpu, oracle, n):
+    p1, gens = oracle.generators(4)
+    r = oracle.R_MOD
+    ks = [0, 1, 2, 7, 8, 9, 15, 16, 17, 128, LAMBDA - 1, LAMBDA, LAMBDA + 1, 8 * LAMBDA + 8, (1 << 128) - 1, 1 << 128,
+          int("88" * 16, 16), int("77" * 16, 16) * LAMBDA % r, r - 1, r - LAMBDA]
+    ks += [int.from_bytes(scalar(b"ladder", b"k", i), "big") for i in range(4)]
+    pts = [p1] + gens[:3]
+    for at in range(0, len(ks), n):  # n one-term MSMs a call: fewer than the bucket engine takes
+        msms = [([pts[(at + j) % 4]], [k.to_bytes(32, "big")]) for j, k in enumerate(ks[at:at + n])]
+        assert gpu.g1_msm_batch(msms) == [(0, oracle.g1_mul(p[0], s[0])) for p, s in msms], at
+    assert gpu.g1_msm_batch([([INF], [ks[3].to_bytes(32, "big")])] * n) == [(0, INF)] * n
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 6])
+def test_membership(gpu, oracle, n):
+    p1, gens = oracle.generators(4)
+    order3 = [bytes([0x80 | sign]) + bytes(47) for sign in (0, 0x20)]  # (0, 2) and (0, -2)
+    pts = [(p1, 0), (_on_curve_outside_g1(oracle, b"ladder"), 1), (order3[0], 1), (gens[0], 0), (order3[1], 1),
+           (gens[1], 0)]
+    got = gpu.g1_subgroup_for_test([p for p, _ in pts[:n]])
+    assert got == [(0, bad) for _, bad in pts[:n]]
+    assert gpu.g1_subgroup_for_test([INF] * n) == [(1, 0)] * n
