@@ -72,92 +72,154 @@ __device__ const Op ADD = {
     {{E0, ZERO, E4, ZERO, AX, 1}, {E1, ZERO, E3, ZERO, NONE, 2}, {E5, ZERO, E4, ZERO, AY, 1}, {P0, ZERO, E3, ZERO, NONE, 6},
      {E2, ZERO, E5, ZERO, AZ, 1}, {P0, ZERO, E0, ZERO, NONE, 3}, GL_IDLE_M, GL_IDLE_M}};
 
+// The addition on y^2 = x^3 + 4 itself (3b = 12), for sums of points given as
+// projective triples (add_points).
+__device__ const Op ADD4 = {
+    {{AX, ZERO, BY_TAB | 0, ZERO, P0, 1}, {AY, ZERO, BY_TAB | 1, ZERO, P1, 1}, {AZ, ZERO, BY_TAB | 3, ZERO, P2, 1},
+     {AZ, ZERO, BY_TAB | 3, ZERO, P3, 12}, {AX, AY, BY_TAB | 0, BY_TAB | 1, P4, 1},
+     {AY, AZ, BY_TAB | 1, BY_TAB | 3, P5, 1}, {AX, AZ, BY_TAB | 0, BY_TAB | 3, P6, 1}, GL_IDLE_M},
+    {{P4, ZERO, P0, P1, E0}, {P1, P2, P5, ZERO, E1}, {P5, ZERO, P1, P2, E2}, {P6, ZERO, P0, P2, E3},
+     {P1, ZERO, P3, ZERO, E4}, {P1, P3, ZERO, ZERO, E5}, GL_IDLE_S, GL_IDLE_S},
+    {{E0, ZERO, E4, ZERO, AX, 1}, {E1, ZERO, E3, ZERO, NONE, 12}, {E5, ZERO, E4, ZERO, AY, 1},
+     {P0, ZERO, E3, ZERO, NONE, 36}, {E2, ZERO, E5, ZERO, AZ, 1}, {P0, ZERO, E0, ZERO, NONE, 3}, GL_IDLE_M, GL_IDLE_M}};
+
 DEV uint32_t at(uint32_t slot) { return slot * (uint32_t)sizeof(fp); }
 
-// One product per lane; PAIR: an output is the sum of two neighbouring lanes'.
-template <bool PAIR> DEV void mul_round(Mem *m, fp *sl, const Mul &e, uint32_t b, uint32_t b2) {
-  fp x = ld(sl, at(e.a)), y = ld(sl, at(b));
-  if (!PAIR) {
-    const fp x2 = ld(sl, at(e.a2)), y2 = ld(sl, at(b2));
+// One lane's part of an operation, as slot addresses (k: the constants; a
+// negative out: nothing stored).
+struct Role {
+  uint32_t a, a2, b, b2, k1, p0, p1, m0, m1, c, d, k2;
+  int32_t out1, sum, out2;
+};
+// acc, x, y, z: addresses of the accumulator's X and of the operand's
+// coordinates; tmp: that of ZERO .. E5.
+DEV Role role_of(const Op &op, uint32_t acc, uint32_t x, uint32_t y, uint32_t z, uint32_t tmp) {
+  auto where = [&](uint32_t s) {
+    return s & BY_TAB ? (s == (BY_TAB | 0) ? x : s == (BY_TAB | 1) ? y : z)
+                      : s - AX < 3u ? acc + at(s - AX) : tmp + at(s);
+  };
+  auto to = [&](uint32_t s) { return s == NONE ? -1 : (int32_t)where(s); };
+  const int r = threadIdx.x & 7;
+  const Mul f = op.first[r], g = op.second[r];
+  const Sum u = op.sum[r];
+  return {where(f.a), where(f.a2), where(f.b), where(f.b2), f.k, where(u.p0), where(u.p1), where(u.m0), where(u.m1),
+          where(g.a), where(g.b), g.k, to(f.out), to(u.out), to(g.out)};
+}
+// Where a lane's first-round operands b, b2 come from in an addition: 0 a fixed
+// slot, 1, 2, 3 the operand's X, Y, Z.
+struct Operand {
+  uint32_t b, b2;
+  DEV static uint32_t code(uint32_t s) { return !(s & BY_TAB) ? 0 : s == (BY_TAB | 0) ? 1 : s == (BY_TAB | 1) ? 2 : 3; }
+  DEV static Operand of(const Op &op) {
+    const Mul f = op.first[threadIdx.x & 7];
+    return {code(f.b), code(f.b2)};
+  }
+  DEV void set(Role &r, uint32_t x, uint32_t y, uint32_t z) const {
+    if (b) r.b = b == 1 ? x : b == 2 ? y : z;
+    if (b2) r.b2 = b2 == 1 ? x : b2 == 2 ? y : z;
+  }
+};
+
+// The operation on the slots of `r`; octets with `live` false compute and store
+// nothing.  All lanes of the warp call it.
+DEV void apply(const Role &r, uint32_t mul_p, bool live) {
+  uint32_t v[13], w[12];
+  {
+    fp x = ld(r.a), y = ld(r.b);
+    const fp x2 = ld(r.a2), y2 = ld(r.b2);
     fp_acc_add(x.w, x.w, x2.w);
     fp_acc_add(y.w, y.w, y2.w);
+    fp t;
+    fp_mont_mul(t.w, x.w, y.w);
+    scale(v, t.w, r.k1);
+    reduce13(mul_p, v, w);
+    __syncwarp();  // every lane has read its operands
+    if (live && r.out1 >= 0) st((uint32_t)r.out1, w);
+    __syncwarp();
   }
-  fp t;
-  fp_mont_mul(t.w, x.w, y.w);
-  uint32_t v[13], r[12];
-  scale(v, t.w, e.k);
-  if (PAIR) add_lane(v, 1);
-  reduce13(m->mul_p, v, r);
-  __syncwarp();  // every lane has read its operands
-  if (e.out != NONE) st(sl, at(e.out), r);
-  __syncwarp();
+  {
+    const fp t = lane_sum(r.p0, r.p1, r.m0, r.m1);
+    if (live && r.sum >= 0) st((uint32_t)r.sum, t.w);
+    __syncwarp();
+  }
+  {
+    const fp x = ld(r.c), y = ld(r.d);
+    fp t;
+    fp_mont_mul(t.w, x.w, y.w);
+    scale(v, t.w, r.k2);
+    add_lane(v, 1);
+    reduce13(mul_p, v, w);
+    __syncwarp();
+    if (live && r.out2 >= 0) st((uint32_t)r.out2, w);
+    __syncwarp();
+  }
 }
 
-// acc = op(acc, table entry): x, y, z are the slots of the entry's coordinates
-// (ignored by a doubling).  All lanes of the warp call it.
-static __device__ __noinline__ void apply(Mem *m, const Op *op, uint32_t x, uint32_t y, uint32_t z) {
-  const int role = threadIdx.x & 7;
-  fp *sl = m->slot[(threadIdx.x & 31) >> 3];
-  auto pick = [&](uint32_t s) { return !(s & BY_TAB) ? s : s == (BY_TAB | 0) ? x : s == (BY_TAB | 1) ? y : z; };
-  const Mul f = op->first[role], s = op->second[role];
-  const Sum u = op->sum[role];
-  mul_round<false>(m, sl, f, pick(f.b), pick(f.b2));
-  const fp t = lane_sum(sl, at(u.p0), at(u.p1), at(u.m0), at(u.m1));
-  if (u.out != NONE) st(sl, at(u.out), t.w);
-  __syncwarp();
-  mul_round<true>(m, sl, s, s.b, ZERO);
-}
-DEV void dbl(Mem *m) { apply(m, &DBL, ZERO, ZERO, ZERO); }
-// acc += digit * P for digit in -8 .. 8 (entry |digit| - 1; 0 adds the identity)
-DEV void add_digit(Mem *m, int digit) {
-  const uint32_t e = TAB + 4 * (uint32_t)(abs(digit) - 1);
-  apply(m, &ADD, digit ? e : ZERO, digit ? e + (digit < 0 ? 2 : 1) : ONE, digit ? e + 3 : ZERO);
-}
 // table entry k = acc
 DEV void store_entry(fp *sl, int role, int k) {
   if (role < 4) {
-    fp v = ld(sl, at(role == 0 ? AX : role == 3 ? AZ : AY));
+    fp v = sl[role == 0 ? AX : role == 3 ? AZ : AY];
     if (role == 2) {
       fp_csub1(v.w, v.w);
       fp_from_mod(v.w, v.w);
     }
-    st(sl, at(TAB + 4 * k + role), v.w);
+    sl[TAB + 4 * k + role] = v;
   }
   __syncwarp();
 }
+
+// A warp's four ladders: the lanes' parts of a doubling and of an addition.
+struct Ladders {
+  Role dbl, add;
+  Operand operand;
+  uint32_t tab, mul_p;  // addresses of table entry 0 and of the multiples of p
+  fp *sl;
+  int role;
+  // acc *= 2, or acc += digit * P for digit in -8 .. 8 (entry |digit| - 1; 0
+  // adds the identity).  One copy in the code: the loops select the operation.
+  DEV void step(bool doubling, int digit) const {
+    Role r = add;
+    const uint32_t e = tab + at(4 * (uint32_t)(abs(digit) - 1)), zero = tab - at(TAB);
+    operand.set(r, digit ? e : zero, digit ? e + at(digit < 0 ? 2 : 1) : tab + at(ONE - TAB), digit ? e + at(3) : zero);
+    if (doubling) r = dbl;
+    apply(r, mul_p, true);
+  }
+};
 
 // The constants, ladder state and base point: acc = entry 0 = the image on E'
 // of (x, y), or of phi(x, y) = (beta x, -y).  All lanes of the warp call it.
-DEV void start(Mem *m, const g1a &p, bool phi) {
+DEV Ladders start(Mem *m, const g1a &p, bool phi) {
   const int lane = threadIdx.x & 31, role = lane & 7;
   fp *sl = m->slot[lane >> 3];
   for (int k = lane; k < QMAX; k += 32) m->mul_p[k] = multiple_of_p((uint32_t)k);
-  const fp s2 = C_B3_S2, bs2 = C_B3_BETA_S2, s3 = C_B3_S3;
-  if (role == 0) sl[ZERO] = fp_zero();
-  if (role == 1) sl[ONE] = fp_one();
-  if (role == 2) sl[AX] = p.x;
-  if (role == 3) sl[AY] = phi ? fp_neg(p.y) : p.y;
-  if (role == 4) sl[AZ] = fp_one();
-  if (role == 5) sl[E0] = phi ? bs2 : s2;
-  if (role == 6) sl[E1] = s3;
+  if (role == 0) {
+    const fp s2 = C_B3_S2, bs2 = C_B3_BETA_S2;
+    sl[AX] = fp_mul(p.x, phi ? bs2 : s2);
+    sl[ZERO] = fp_zero();
+  } else if (role == 1) {
+    const fp s3 = C_B3_S3;
+    sl[AY] = fp_mul(phi ? fp_neg(p.y) : p.y, s3);
+    sl[ONE] = fp_one();
+  } else if (role == 2) {
+    sl[AZ] = fp_one();
+  }
   __syncwarp();
-  const Mul e = {(uint8_t)(role ? AY : AX), ZERO, (uint8_t)(role ? E1 : E0), ZERO,
-                 (uint8_t)(role == 0 ? AX : role == 1 ? AY : NONE), 1};
-  mul_round<false>(m, sl, e, e.b, ZERO);
   store_entry(sl, role, 0);
+  Ladders l;
+  const uint32_t a = addr(sl);
+  l.dbl = role_of(DBL, a + at(AX), a, a, a, a);
+  l.add = role_of(ADD, a + at(AX), a, a, a, a);
+  l.operand = Operand::of(ADD);
+  l.tab = a + at(TAB);
+  l.mul_p = addr(m->mul_p);
+  l.sl = sl;
+  l.role = role;
+  return l;
 }
 
-// k P for four ladders: half 0 or 1 of a GLV term on each (sh: the half's 128-bit
-// scalar).  Returns with the multiple in the accumulator.
-DEV void ladder128(Mem *m, const uint32_t sh[4]) {
-  const int lane = threadIdx.x & 31, role = lane & 7;
-  fp *sl = m->slot[lane >> 3];
-#pragma unroll 1
-  for (int k = 1; k < 8; k++) {  // entries 2P .. 8P
-    if (k == 1) dbl(m);
-    else add_digit(m, 1);
-    store_entry(sl, role, k);
-  }
+// acc = k P on each of the four ladders (sh: k's 128-bit half of a GLV term),
+// then acc += the point that `join` has stored as entry 0.
+template <class Join> DEV void ladder128(const Ladders &l, const uint32_t sh[4], const Join &join) {
   // signed digits: nibbles of sh + 0x888...8, less 8
   uint32_t d[5];
   uint64_t c = 0;
@@ -168,29 +230,120 @@ DEV void ladder128(Mem *m, const uint32_t sh[4]) {
     c >>= 32;
   }
   d[4] = (uint32_t)c;
-  if (role == 0) sl[AX] = fp_zero();
-  if (role == 1) sl[AY] = fp_one();
-  if (role == 2) sl[AZ] = fp_zero();
-  __syncwarp();
-  add_digit(m, (int)d[4]);
+  // steps 0..6: entries 2P .. 8P; 7: the top digit into the identity; then 32
+  // times four doublings and a digit; last: the join
+  constexpr int BUILD = 7, MAIN = BUILD + 1, END = MAIN + 5 * 32;
+  int quint = 0;
 #pragma unroll 1
-  for (int i = 31; i >= 0; i--) {
-#pragma unroll 1
-    for (int k = 0; k < 4; k++) dbl(m);
-    add_digit(m, (int)(d[3] >> 28) - 8);
-    d[3] = __funnelshift_l(d[2], d[3], 4);
-    d[2] = __funnelshift_l(d[1], d[2], 4);
-    d[1] = __funnelshift_l(d[0], d[1], 4);
-    d[0] <<= 4;
+  for (int i = 0; i <= END; i++) {
+    bool doubling = i == 0;
+    int digit = 1;
+    if (i == BUILD) {
+      digit = (int)d[4];
+      if (l.role == 0) l.sl[AX] = fp_zero();
+      if (l.role == 1) l.sl[AY] = fp_one();
+      if (l.role == 2) l.sl[AZ] = fp_zero();
+      __syncwarp();
+    } else if (i == END) {
+      join();
+      __syncwarp();
+    } else if (i >= MAIN) {
+      doubling = quint < 4;
+      digit = (int)(d[3] >> 28) - 8;
+      quint = doubling ? quint + 1 : 0;
+      if (!doubling) {
+        d[3] = __funnelshift_l(d[2], d[3], 4);
+        d[2] = __funnelshift_l(d[1], d[2], 4);
+        d[1] = __funnelshift_l(d[0], d[1], 4);
+        d[0] <<= 4;
+      }
+    }
+    l.step(doubling, digit);
+    if (i < BUILD) store_entry(l.sl, l.role, i + 1);
   }
 }
 
-// acc = [|z|] acc, entry 0 being acc at the start
-DEV void mul_zabs(Mem *m) {
+// acc = [z^2] acc for acc = entry 0 = P; entry 1 is P afterwards.
+DEV void mul_z2(const Ladders &l) {
 #pragma unroll 1
-  for (int i = 62; i >= 0; i--) {
-    dbl(m);
-    if (zabs_bit(i)) add_digit(m, 1);
+  for (int half = 0; half < 2; half++) {
+    bool add = false;
+#pragma unroll 1
+    for (int i = 62; i >= 0;) {
+      l.step(!add, 1);
+      add = !add && zabs_bit(i);
+      if (!add) i--;
+    }
+    if (half) break;
+    store_entry(l.sl, l.role, 1);
+    if (l.role < 4) {  // swap entries 0 and 1: the second half multiplies [|z|]P
+      const fp t = l.sl[TAB + l.role];
+      l.sl[TAB + l.role] = l.sl[TAB + 4 + l.role];
+      l.sl[TAB + 4 + l.role] = t;
+    }
+    __syncwarp();
+  }
+}
+
+// ---- sums of many points
+// Projective triples (X, Y, Z) in shared memory, added in place by the lane
+// octets of a warp: a level of a tree sum is one complete addition of two
+// products' depth for up to four pairs, where every lane adding its neighbour's
+// XYZZ point (g1_add and shuffles) is fourteen products deep for half of the
+// lanes.
+constexpr uint32_t TRIPLE = 3 * (uint32_t)sizeof(fp);       // an odd number of 16-byte units
+constexpr uint32_t TMP_SLOTS = 19;                          // ZERO .. E5, one more to keep it odd
+constexpr uint32_t TMP_BYTES = TMP_SLOTS * (uint32_t)sizeof(fp);
+
+DEV void put_triple(fp *t, const g1 &p) {
+  const bool inf = g1_is_inf(p);
+  t[0] = fp_mul(p.X, p.ZZZ);
+  t[1] = inf ? fp_one() : fp_mul(p.Y, p.ZZ);
+  t[2] = fp_mul(p.ZZ, p.ZZZ);
+}
+// Per warp: the octets' scratch (TMP_BYTES each from `tmp`, zero slots set) and
+// their parts of an addition.
+struct Adder {
+  Role add;
+  Operand operand;
+  uint32_t mul_p;
+  bool acc_a, acc_a2, acc_out;  // which of the lane's slots lie in the accumulator
+  DEV static Adder on(uint32_t tmp, uint32_t mul_p) {
+    const uint32_t oct = (threadIdx.x & 31) >> 3, t = tmp + oct * TMP_BYTES;
+    const Mul f = ADD4.first[threadIdx.x & 7], g = ADD4.second[threadIdx.x & 7];
+    return {role_of(ADD4, 0, 0, 0, 0, t), Operand::of(ADD4), mul_p, f.a - AX < 3u, f.a2 - AX < 3u, g.out != NONE};
+  }
+  // For e < count: the triple (e / d) stride + e % d (in steps of `step` bytes
+  // from base) takes the one d further on.  One warp, all lanes.
+  DEV void level(uint32_t base, uint32_t count, uint32_t d, uint32_t stride, uint32_t step) const {
+    const uint32_t oct = (threadIdx.x & 31) >> 3;
+#pragma unroll 1
+    for (uint32_t e0 = 0; e0 < count; e0 += 4) {
+      const uint32_t e = min(e0 + oct, count - 1), acc = base + ((e / d) * stride + e % d) * step, op = acc + d * step;
+      Role r = add;
+      if (acc_a) r.a += acc;
+      if (acc_a2) r.a2 += acc;
+      if (acc_out) r.out2 += acc;
+      operand.set(r, op, op + at(1), op + at(2));
+      apply(r, mul_p, e0 + oct < count);
+    }
+  }
+};
+// The triple at t as an XYZZ point, written by the octet's lanes 0..2.
+DEV void get_triple(const fp *t, int role, g1 *out) {
+  if (role > 2) return;
+  const fp z = t[2];
+  const fp zz = fp_mul(z, role == 0 ? t[0] : z);  // X Z, or Z^2
+  if (role == 0) {
+    out->X = zz;
+  } else {
+    const fp c = fp_mul(zz, role == 1 ? t[1] : z);  // Y Z^2, or Z^3
+    if (role == 1) {
+      out->Y = c;
+    } else {
+      out->ZZ = zz;
+      out->ZZZ = c;
+    }
   }
 }
 

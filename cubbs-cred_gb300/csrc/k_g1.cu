@@ -8,6 +8,8 @@
 // GLV variable base (kernels/variable_base_universal.cuh:25-331), BLST decode
 // and compress on the host (native/cuda/src/g1_msm_blst.cpp:614-732).  Here
 // decode and compress run on the device.
+#include <algorithm>
+#include <cmath>
 #include <cstdlib>
 
 #include "g1_ladder.cuh"
@@ -87,81 +89,109 @@ __global__ void __launch_bounds__(64) k_table_build(const g1a *bases, int g0, in
   }
 }
 
-// w-bit field of a raw 256-bit scalar starting at bit pos
-DEV uint32_t scalar_bits(const fr &s, int pos, int w) {
-  if (pos >= 256) return 0;
-  int wi = pos >> 5, sh = pos & 31;
-  uint64_t lo = s.w[wi];
-  uint64_t hi = wi + 1 < 8 ? s.w[wi + 1] : 0;
-  uint64_t v = (lo | (hi << 32)) >> sh;
-  return (uint32_t)(v & ((1u << w) - 1));
+// w-bit field of a raw 256-bit scalar in memory, starting at bit pos < 256
+DEV uint32_t scalar_bits(const uint32_t *s, int pos, int w) {
+  const int wi = pos >> 5;
+  const uint32_t lo = s[wi], hi = wi + 1 < 8 ? s[wi + 1] : 0;
+  return __funnelshift_r(lo, hi, pos & 31) & ((1u << w) - 1);
 }
 
-// Signed w-bit digit of window k of scalar s (digits in (-half, half], a
-// digit above half becomes d - 2^w with a carry into the next window).  The
-// carry into window k is recomputed from the windows below it, so any window
-// can be taken alone; the work is a few integer operations per window, next
-// to the mixed addition the digit costs.
-DEV uint32_t fixed_digit(const fr &s, int k, int w, uint32_t half, bool &neg) {
+// Signed w-bit digit of window k of scalar s: digits in (-half, half], a digit
+// above half becomes d - 2^w with a carry into the next window.  The carry
+// into window k is 1 when the window below it is above half, 0 when it is
+// less, and that window's own carry when it is half: one more window is read
+// almost always.
+DEV uint32_t fixed_digit(const uint32_t *s, int k, int w, uint32_t half, bool &neg) {
   uint32_t carry = 0;
   #pragma unroll 1
-  for (int i = 0; i < k; i++) carry = scalar_bits(s, i * w, w) + carry > half ? 1u : 0u;
-  uint32_t d = scalar_bits(s, k * w, w) + carry;
+  for (int i = k - 1; i >= 0; i--) {
+    const uint32_t v = scalar_bits(s, i * w, w);
+    if (v != half) {
+      carry = v > half ? 1u : 0u;
+      break;
+    }
+  }
+  const uint32_t d = scalar_bits(s, k * w, w) + carry;
   neg = d > half;
   return neg ? (1u << w) - d : d;  // 2^w - d is 0 for d = 2^w (the carry alone)
 }
-// Sum of the points of the L-lane groups of a warp (valid on each group's first lane).
-template <int L> DEV g1 group_sum_g1(g1 acc) {
-  #pragma unroll 1
-  for (int d = L / 2; d > 0; d >>= 1) {
-    g1 o;
-#pragma unroll
-    for (int i = 0; i < 12; i++) {
-      o.X.w[i] = __shfl_down_sync(0xffffffffu, acc.X.w[i], d, L);
-      o.Y.w[i] = __shfl_down_sync(0xffffffffu, acc.Y.w[i], d, L);
-      o.ZZ.w[i] = __shfl_down_sync(0xffffffffu, acc.ZZ.w[i], d, L);
-      o.ZZZ.w[i] = __shfl_down_sync(0xffffffffu, acc.ZZZ.w[i], d, L);
-    }
-    acc = g1_add(acc, o);
-  }
-  return acc;
-}
 
 // Fixed-base MSM: row r = sum_g scalars[r*stride + g] * G_g, g < nterms[r].
-// A row runs on a group of L lanes (L = 4 .. 32): its (generator, window)
-// units g * nwin + k are dealt round robin to the group's lanes, so every lane
+// A row runs on a group of L lanes, L a power of two: 4 .. 32 (a block of
+// one warp, 32 / L rows) or L / 32 warps (a block, one row).  Its (generator,
+// window) units g * nwin + k are dealt round robin to the lanes, so every lane
 // does the same number of mixed additions whatever the row's length (give or
 // take one); each nonzero digit costs one table lookup and one mixed addition,
-// and the lanes' sums are added by shuffles within the group.  The warps take
-// rows in a grid-stride loop, a warp 32 / L rows at a time (every lane of a
-// warp runs the same iterations, as the shuffles need).
-template <int L>
-__global__ void __launch_bounds__(128) k_fixed_msm(FixedTable t, const fr *scalars, uint32_t stride,
-                                                   const uint32_t *nterms, uint32_t rows, g1 *out) {
-  constexpr uint32_t PER_WARP = 32 / L;
-  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t lane = threadIdx.x & 31, sub = lane % L, grp = lane / L;
+// and the next unit's table entry (a random 96-byte read from HBM) is fetched
+// while the current one is added.  The lanes' sums are added as projective
+// triples by the lane octets (g1_ladder.cuh, tree_level): 9 levels of a 32-lane
+// row take 41 thousand cycles where five rounds of shuffled full additions
+// took 140 thousand, so that short rows can spread over many lanes.
+// Dynamic shared memory: fixed_smem of the block's warps.
+constexpr uint32_t fixed_smem(uint32_t warps) { return warps * (32 * gl::TRIPLE + 4 * gl::TMP_BYTES); }
+template <int THREADS>  // the largest block: few rows spread over 256 or 512 lanes take the form with fewer registers
+__global__ void __launch_bounds__(THREADS) k_fixed_msm(FixedTable t, const fr *scalars, uint32_t stride,
+                                                   const uint32_t *nterms, uint32_t rows, uint32_t L, g1 *out) {
+  extern __shared__ __align__(16) uint8_t fixed_mem[];
+  __shared__ __align__(16) fp mul_p[slots::QMAX];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  const uint32_t per_block = L < 32 ? 32 / L : 1, sub = threadIdx.x & (L - 1);
+  const uint32_t row = blockIdx.x * per_block + threadIdx.x / L;
   const uint32_t half = (uint32_t)t.half, nwin = (uint32_t)t.nwin;
+  fp *base = reinterpret_cast<fp *>(fixed_mem);
+  for (uint32_t k = threadIdx.x; k < slots::QMAX; k += blockDim.x) mul_p[k] = slots::multiple_of_p(k);
+  const uint32_t tmp = warps * 32 * gl::TRIPLE + warp * 4 * gl::TMP_BYTES;
+  if ((lane & 7) == 0)
+    *reinterpret_cast<fp *>(fixed_mem + tmp + (lane >> 3) * gl::TMP_BYTES + gl::at(gl::ZERO)) = fp_zero();
+
+  const uint32_t units = row < rows ? nterms[row] * nwin : 0;
+  g1 acc = g1_inf();
+  g1a next;
+  bool have = false, neg = false;
+  auto fetch = [&](uint32_t u) {
+    have = false;
+    if (u >= units) return;
+    const uint32_t g = u / nwin, k = u - g * nwin;
+    const uint32_t d = fixed_digit(scalars[(size_t)row * stride + g].w, (int)k, t.w, half, neg);
+    have = d != 0;
+    if (have) next = t.entries[((size_t)g * nwin + k) * half + d - 1];
+  };
+  fetch(sub);
   #pragma unroll 1
-  for (uint32_t base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * PER_WARP; base < rows;
-       base += warps * PER_WARP) {
-    const uint32_t row = base + grp;
-    const uint32_t units = row < rows ? nterms[row] * nwin : 0;
-    g1 acc = g1_inf();
-    #pragma unroll 1
-    for (uint32_t u = sub; u < units; u += L) {
-      const uint32_t g = u / nwin, k = u - g * nwin;
-      const fr sc = scalars[(size_t)row * stride + g];
-      bool neg;
-      const uint32_t d = fixed_digit(sc, (int)k, t.w, half, neg);
-      if (d) {
-        g1a e = t.entries[((size_t)g * nwin + k) * half + d - 1];
-        if (neg) e.y = fp_neg(e.y);
-        acc = g1_add_aff_inl(acc, e);  // inlined: no struct arguments through the stack
-      }
+  for (uint32_t u = sub; u < units; u += L) {
+    g1a e = next;
+    const bool use = have;
+    if (neg) e.y = fp_neg(e.y);
+    fetch(u + L);
+    if (use) acc = g1_add_aff_inl(acc, e);  // inlined: no struct arguments through the stack
+  }
+  gl::put_triple(base + 3 * threadIdx.x, acc);
+  __syncthreads();  // the triples, the multiples of p and the zero slots
+  // each warp adds its own 32 triples (32 / L rows of L, or one part of a row),
+  // then the first warp the warps' sums; one loop, one copy of the addition
+  const uint32_t in_warp = L < 32 ? L : 32;
+  const gl::Adder adder = gl::Adder::on(slots::addr(fixed_mem) + tmp, slots::addr(mul_p));
+  const uint32_t groups = 32 / in_warp;
+  uint32_t first = slots::addr(base + 3 * 32 * warp), span = in_warp, step = gl::TRIPLE, d = in_warp / 2;
+  #pragma unroll 1
+  for (bool across = false;; d >>= 1) {
+    if (d == 0) {
+      if (across || L <= 32) break;
+      across = true;
+      __syncthreads();
+      if (warp != 0) return;
+      first = slots::addr(base);
+      step = 32 * gl::TRIPLE;
+      d = warps / 2;
+      span = warps;
     }
-    acc = group_sum_g1<L>(acc);
-    if (sub == 0 && row < rows) out[row] = acc;
+    adder.level(first, groups * d, d, span, step);
+  }
+  // one octet per row (up to four at a time) writes it
+  #pragma unroll 1
+  for (uint32_t k = lane >> 3; k < per_block; k += 4) {
+    const uint32_t r = blockIdx.x * per_block + k;
+    if (r < rows) gl::get_triple(base + 3 * k * in_warp, (int)(lane & 7), &out[r]);
   }
 }
 
@@ -210,15 +240,14 @@ __global__ void __launch_bounds__(32) k_var_mul_ladder(const g1a *points, const 
   g1a p;
   p.x = p.y = fp_one();
   if (!inf) p = points[job.point];
-  gl::start(&mem, p, half != 0);
+  const gl::Ladders l = gl::start(&mem, p, half != 0);
   uint32_t s[4], q[4];
   glv_split(scalars[j], s, q);
-  gl::ladder128(&mem, half ? q : s);
-  // the first ladder takes the second's sum (its entry 0), and leaves E'
-  fp *sl = mem.slot[lane >> 3];
-  if (!half && role < 3) sl[gl::TAB + (role == 2 ? 3 : role)] = mem.slot[(lane >> 3) + 1][gl::AX + role];
-  __syncwarp();
-  gl::add_digit(&mem, 1);
+  fp *sl = l.sl;
+  // the first ladder takes the second's sum as its entry 0, and leaves E'
+  gl::ladder128(l, half ? q : s, [&] {
+    if (!half && role < 3) sl[gl::TAB + (role == 2 ? 3 : role)] = mem.slot[(lane >> 3) + 1][gl::AX + role];
+  });
   if (!half && role < 2) {
     const fp s2 = C_B3_S2, s3 = C_B3_S3;
     fp v[2];  // (X Z, s^2 Z^2) or (Y Z^2, s^3 Z^3)
@@ -295,17 +324,9 @@ __global__ void __launch_bounds__(32) k_g1_subgroup_ladder(const g1a *pts, const
   g1a p;
   p.x = p.y = fp_one();
   if (ok) p = pts[j];
-  gl::start(&mem, p, false);
-  fp *sl = mem.slot[lane >> 3];
-  gl::mul_zabs(&mem);
-  gl::store_entry(sl, role, 1);  // keep the first entry (P) for the comparison
-  if (role < 4) {  // swap entries 0 and 1: the second half multiplies [|z|]P
-    const fp t = sl[gl::TAB + role];
-    sl[gl::TAB + role] = sl[gl::TAB + 4 + role];
-    sl[gl::TAB + 4 + role] = t;
-  }
-  __syncwarp();
-  gl::mul_zabs(&mem);
+  const gl::Ladders l = gl::start(&mem, p, false);
+  const fp *sl = l.sl;
+  gl::mul_z2(l);
   if (role == 0 && i < n) {
     const fp beta = C_GLV_BETA;
     fp X = sl[gl::AX], Y = sl[gl::AY], Z = sl[gl::AZ], x = sl[gl::TAB + 4], y = sl[gl::TAB + 5];
@@ -362,34 +383,51 @@ void launch_build_table(cudaStream_t s, const g1a *gens, int g0, int g1n, FixedT
   const int run = std::min(t.half, 256);
   k_table_build<<<blocks_for((size_t)nb * (t.half / run), 64), 64, 0, s>>>(bases, g0, g1n, t, run, scratch, prod);
 }
-// Lanes per row (CUBBS_BBS_FIXED_LANES forces 4, 8, 16 or 32): a launch whose
-// rows give at most two warps per SM sub-partition at 32 lanes a row is bound
-// by one row's latency, so a row gets the whole warp; a larger launch is bound
-// by issue, where the shuffle reduction (log2 L full additions on every lane)
-// outweighs a shorter chain, so short rows share a warp: 16 lanes for rows of
-// 256 units or more, else 8.
-static int fixed_lanes_for(uint32_t rows, uint32_t stride, int nwin) {
-  static const int forced = [] {
+// Lanes per row (CUBBS_BBS_FIXED_LANES forces 4, 8, 16 or 32): the power of two
+// that a model of the launch finds fastest.  A lane does units / L mixed
+// additions of ten products; the tree sum is `passes` additions of two
+// products' depth; a product costs a lone warp of an SM sub-partition 1816
+// cycles and each of several warps 1215.
+static uint32_t fixed_lanes_for(uint32_t rows, uint32_t stride, int nwin) {
+  static const uint32_t forced = [] {
     const char *e = std::getenv("CUBBS_BBS_FIXED_LANES");
     const int x = e && *e ? std::atoi(e) : 0;
-    return (x == 4 || x == 8 || x == 16 || x == 32) ? x : 0;
+    return (uint32_t)((x == 4 || x == 8 || x == 16 || x == 32) ? x : 0);
   }();
   if (forced) return forced;
   int dev = 0, sms = 152;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if ((size_t)rows <= (size_t)sms * 8) return 32;
-  return (size_t)stride * nwin >= 256 ? 16 : 8;
+  const double units = (double)stride * nwin;
+  uint32_t best = 4;
+  double best_cost = 0;
+  for (uint32_t L = 4; L <= 512; L *= 2) {
+    const uint32_t in_warp = L < 32 ? L : 32, warps = L < 32 ? 1 : L / 32;
+    double passes = 0;
+    for (uint32_t d = in_warp / 2; d > 0; d >>= 1) passes += (32 / in_warp * d + 3) / 4;
+    for (uint32_t d = warps / 2; d > 0; d >>= 1) passes += (d + 3) / 4;
+    const double products = std::ceil(units / L) * 10 + 3 + 2.4 * passes;
+    const double total = (double)rows * L / 32, per = std::ceil(total / (4.0 * sms));
+    const double cost = products * (per <= 1 ? 1816 : per * 1215);
+    if (L == 4 || cost < best_cost) {
+      best = L;
+      best_cost = cost;
+    }
+  }
+  return best;
 }
 void launch_fixed_msm(cudaStream_t s, const FixedTable &t, const fr *scalars, uint32_t stride,
                       const uint32_t *nterms, uint32_t rows, g1 *out) {
   if (!rows) return;
-  const int L = fixed_lanes_for(rows, stride, t.nwin);
-  const size_t threads = (size_t)(rows + 32 / L - 1) / (32 / L) * 32;
-  const unsigned blocks = blocks_for(threads, 128);
-  if (L == 32) k_fixed_msm<32><<<blocks, 128, 0, s>>>(t, scalars, stride, nterms, rows, out);
-  else if (L == 16) k_fixed_msm<16><<<blocks, 128, 0, s>>>(t, scalars, stride, nterms, rows, out);
-  else if (L == 8) k_fixed_msm<8><<<blocks, 128, 0, s>>>(t, scalars, stride, nterms, rows, out);
-  else k_fixed_msm<4><<<blocks, 128, 0, s>>>(t, scalars, stride, nterms, rows, out);
+  const uint32_t L = fixed_lanes_for(rows, stride, t.nwin), threads = L < 32 ? 32 : L, per_block = L < 32 ? 32 / L : 1;
+  static const bool attr = [] {
+    CUBBS_CHECK(cudaFuncSetAttribute(k_fixed_msm<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fixed_smem(16)));
+    return true;
+  }();
+  (void)attr;
+  const unsigned blocks = (rows + per_block - 1) / per_block;
+  const size_t smem = fixed_smem(threads / 32);
+  if (threads <= 128) k_fixed_msm<128><<<blocks, threads, smem, s>>>(t, scalars, stride, nterms, rows, L, out);
+  else k_fixed_msm<512><<<blocks, threads, smem, s>>>(t, scalars, stride, nterms, rows, L, out);
 }
 void launch_var_mul(cudaStream_t s, const g1a *points, const VarJob *jobs, const fr *scalars, uint32_t n, g1 *out,
                     int lanes) {

@@ -29,15 +29,16 @@ struct Mem {
   fp slot[PQ_SLOTS];
   fp mul_p[PQ_QMAX];  // k p
 };
+constexpr uint32_t MUL_P = PQ_SLOTS * (uint32_t)sizeof(fp);  // from the slots
 
 using namespace slots;
-
 // slot[out] = (slot[a] [+ slot[a2]]) (slot[b] [+ slot[b2]]) << dbl, not fully
-// reduced: operands below 2.1 p give a product below 1.42 p.
-DEV void product(fp *sl, const uint4 &e) {
-  fp a = ld(sl, e.x & 0xffffu), b = ld(sl, e.x >> 16);
+// reduced: operands below 2.1 p give a product below 1.42 p.  sl: address of
+// the slots.
+DEV void product(uint32_t sl, const uint4 &e) {
+  fp a = ld(sl + (e.x & 0xffffu)), b = ld(sl + (e.x >> 16));
   if (e.w & 0x10u) {  // the same on every lane of a phase
-    const fp a2 = ld(sl, e.y & 0xffffu), b2 = ld(sl, e.y >> 16);
+    const fp a2 = ld(sl + (e.y & 0xffffu)), b2 = ld(sl + (e.y >> 16));
     fp_acc_add(a.w, a.w, a2.w);
     fp_acc_add(b.w, b.w, b2.w);
   }
@@ -47,15 +48,15 @@ DEV void product(fp *sl, const uint4 &e) {
   b.w[0] <<= sh;
   fp r;
   fp_mont_mul(r.w, a.w, b.w);
-  if ((e.z & 0xffffu) != PQ_NONE) st(sl, e.z & 0xffffu, r.w);
+  if ((e.z & 0xffffu) != PQ_NONE) st(sl + (e.z & 0xffffu), r.w);
 }
 
 // One output per 2^g lanes; every lane of the warp calls it.
-DEV void sums(Mem *m, const uint4 &e) {
+DEV void sums(uint32_t sl, const uint4 &e) {
   const int g = (int)(e.w >> 4) & 7;
   if (g == 7) return;
   uint32_t v[13];
-  const fp t = lane_sum(m->slot, e.x & 0xffffu, e.x >> 16, e.y & 0xffffu, e.y >> 16);
+  const fp t = lane_sum(sl + (e.x & 0xffffu), sl + (e.x >> 16), sl + (e.y & 0xffffu), sl + (e.y >> 16));
 #pragma unroll
   for (int j = 0; j < 12; j++) v[j] = t.w[j];
   v[12] = 0;
@@ -63,22 +64,22 @@ DEV void sums(Mem *m, const uint4 &e) {
   for (int d = 1; d < (1 << g); d <<= 1) add_lane(v, d);
   if ((e.z & 0xffffu) != PQ_NONE) {
     uint32_t r[12];
-    reduce13(m->mul_p, v, r);
-    st(m->slot, e.z & 0xffffu, r);
+    reduce13(sl + MUL_P, v, r);
+    st(sl + (e.z & 0xffffu), r);
   }
 }
 
 // Runs program `prog`; every lane of the block calls it, and the block is in
 // step before and after.
-static __device__ __noinline__ void run(Mem *m, int prog) {
+static __device__ __noinline__ void run(uint32_t sl, int prog) {
   const int lane = threadIdx.x;
   const int ph0 = PQ_FIRST[prog], ph1 = PQ_FIRST[prog + 1];
   uint4 e = __ldg(&PQ_ENTRY[ph0 * PQ_LANES + lane]);
 #pragma unroll 1
   for (int ph = ph0; ph < ph1; ph++) {
     const uint4 nx = __ldg(&PQ_ENTRY[min(ph + 1, ph1 - 1) * PQ_LANES + lane]);
-    if (e.w & 1u) sums(m, e);
-    else if ((e.z & 0xffffu) != PQ_NONE) product(m->slot, e);
+    if (e.w & 1u) sums(sl, e);
+    else if ((e.z & 0xffffu) != PQ_NONE) product(sl, e);
     __syncthreads();
     e = nx;
   }
@@ -87,15 +88,15 @@ static __device__ __noinline__ void run(Mem *m, int prog) {
 // Register R squared n times in the cyclotomic subgroup, on one warp.  An
 // output is 3 A + post with A on a lane pair (two lane sums) and post one
 // slot added or subtracted on the odd lane.
-static __device__ __noinline__ void cyclo(Mem *m, int n) {
+static __device__ __noinline__ void cyclo(uint32_t sl, int n) {
   const int lane = threadIdx.x & 31;
   const uint4 em = __ldg(&PQ_CYCLO_M[lane]), es = __ldg(&PQ_CYCLO_S[lane]);
 #pragma unroll 1
   for (; n > 0; n--) {
-    product(m->slot, em);
+    product(sl, em);
     __syncwarp();
-    const fp t = lane_sum(m->slot, es.x & 0xffffu, es.x >> 16, es.y & 0xffffu, es.y >> 16);
-    const fp pp = ld(m->slot, es.z >> 16), pm = ld(m->slot, es.w);
+    const fp t = lane_sum(sl + (es.x & 0xffffu), sl + (es.x >> 16), sl + (es.y & 0xffffu), sl + (es.y >> 16));
+    const fp pp = ld(sl + (es.z >> 16)), pm = ld(sl + es.w);
     uint32_t a[13], v[13];
     v[0] = t.w[0] << 1;
 #pragma unroll
@@ -115,8 +116,8 @@ static __device__ __noinline__ void cyclo(Mem *m, int n) {
     __syncwarp();  // every lane has read its slots
     if ((es.z & 0xffffu) != PQ_NONE) {
       uint32_t r[12];
-      reduce13(m->mul_p, v, r);
-      st(m->slot, es.z & 0xffffu, r);
+      reduce13(sl + MUL_P, v, r);
+      st(sl + (es.z & 0xffffu), r);
     }
     __syncwarp();
   }
@@ -132,14 +133,14 @@ DEV void copy_reg(Mem *m, int dst, int src) {
   __syncthreads();
 }
 // R = R^|z| with R = the base held in the register that mul_prog multiplies by.
-DEV void exp_by_zabs(Mem *m, int mul_prog) {
+DEV void exp_by_zabs(uint32_t sl, int mul_prog) {
 #pragma unroll 1
   for (int k = 0; k < 6; k++) {
     // |z| = 2^63 + 2^62 + 2^60 + 2^57 + 2^48 + 2^16
     const int n = k < 3 ? k + 1 : k == 3 ? 9 : k == 4 ? 32 : 16;
-    if (threadIdx.x < 32) cyclo(m, n);
+    if (threadIdx.x < 32) cyclo(sl, n);
     __syncthreads();
-    if (k < 5) run(m, mul_prog);
+    if (k < 5) run(sl, mul_prog);
   }
 }
 
@@ -167,6 +168,7 @@ template <class Job> DEV bool pairing_check(Mem *m, const Job &j, const line2 *l
   const bool skip[2] = {(j.flags & 1) != 0, (j.flags & 2) != 0};
   const line2 *const L[2] = {lines + (size_t)j.slot_a * MILLER_LINES, lines + (size_t)j.slot_b * MILLER_LINES};
   fp *sl = m->slot;
+  const uint32_t at = addr(sl);
   // constants, points, F = 1
   if (t < PQ_QMAX) {
     m->mul_p[t] = multiple_of_p((uint32_t)t);
@@ -187,7 +189,7 @@ template <class Job> DEV bool pairing_check(Mem *m, const Job &j, const line2 *l
     sl[PP_LINE_BASE + t - 112] = line_part(L[(t - 112) >> 2], skip[(t - 112) >> 2], 0, t & 3);
   }
   __syncthreads();
-  run(m, PQ_LINE);
+  run(at, PQ_LINE);
   // Miller loop: the lanes that no product of a step's first round uses fetch
   // the next step's lines, whose B xP the second round multiplies
   const int lp = (t >> 2) & 1;
@@ -206,10 +208,10 @@ template <class Job> DEV bool pairing_check(Mem *m, const Job &j, const line2 *l
       const uint4 e1 = __ldg(tab + PQ_LANES), e2 = __ldg(tab + 2 * PQ_LANES), e3 = __ldg(tab + 3 * PQ_LANES);
 #pragma unroll 1
       for (int k = 0; k < 2; k++) {
-        if ((e.z & 0xffffu) != PQ_NONE) product(sl, e);
+        if ((e.z & 0xffffu) != PQ_NONE) product(at, e);
         __syncthreads();
         if (k == 0 && fetch) sl[PP_LINE_BASE + t - 120] = next;
-        sums(m, k ? e3 : e1);
+        sums(at, k ? e3 : e1);
         __syncthreads();
         e = e2;
       }
@@ -223,27 +225,27 @@ template <class Job> DEV bool pairing_check(Mem *m, const Job &j, const line2 *l
   __syncthreads();
   if (t < 5) sl[PQ_NORM2_BASE + t] = PQ_NORM2[t];  // the inverse's temporaries lie over these slots
   __syncthreads();
-  run(m, PQ_T_F_CU);
-  run(m, PQ_T_T2_T);
+  run(at, PQ_T_F_CU);
+  run(at, PQ_T_T2_T);
   copy_reg(m, PP_REG_R, PP_REG_T);
-  exp_by_zabs(m, PQ_R_R_T);
-  run(m, PQ_A_CRT);  // a = t^z conj(t)
+  exp_by_zabs(at, PQ_R_R_T);
+  run(at, PQ_A_CRT);  // a = t^z conj(t)
   copy_reg(m, PP_REG_R, PP_REG_A);
-  exp_by_zabs(m, PQ_R_R_A);
-  run(m, PQ_A_CRA);  // a = a^z conj(a)
+  exp_by_zabs(at, PQ_R_R_A);
+  run(at, PQ_A_CRA);  // a = a^z conj(a)
   copy_reg(m, PP_REG_R, PP_REG_A);
-  exp_by_zabs(m, PQ_R_R_A);
-  run(m, PQ_X_FROB_A);
-  run(m, PQ_A_X_CR);  // b = a^z a^p
+  exp_by_zabs(at, PQ_R_R_A);
+  run(at, PQ_X_FROB_A);
+  run(at, PQ_A_X_CR);  // b = a^z a^p
   copy_reg(m, PP_REG_R, PP_REG_A);
-  exp_by_zabs(m, PQ_R_R_A);
+  exp_by_zabs(at, PQ_R_R_A);
   copy_reg(m, PP_REG_X, PP_REG_R);
-  exp_by_zabs(m, PQ_R_R_X);  // b^(z^2)
-  run(m, PQ_R_A2_R);         // b^(z^2) b^(p^2)
-  run(m, PQ_R_R_CA);
-  run(m, PQ_R_R_T);
-  run(m, PQ_R_R_T);
-  run(m, PQ_R_R_T);
+  exp_by_zabs(at, PQ_R_R_X);  // b^(z^2)
+  run(at, PQ_R_A2_R);         // b^(z^2) b^(p^2)
+  run(at, PQ_R_R_CA);
+  run(at, PQ_R_R_T);
+  run(at, PQ_R_R_T);
+  run(at, PQ_R_R_T);
   canonical(m, PP_REG_R);
   bool one = true;
   if (t < 12) {

@@ -9,16 +9,25 @@ namespace slots {
 
 constexpr int QMAX = 72;  // multiples of p in the table of reduce13
 
-DEV fp ld(const fp *sl, uint32_t off) {  // off in bytes
-  const uint4 *p = reinterpret_cast<const uint4 *>(reinterpret_cast<const uint8_t *>(sl) + off);
-  const uint4 a = p[0], b = p[1], c = p[2];
-  return {{a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w, c.x, c.y, c.z, c.w}};
+// Slots are addressed by their 32-bit shared-memory addresses: a pointer that
+// crosses an out-of-line call would be a generic one.
+DEV uint32_t addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
+DEV fp ld(uint32_t a) {
+  fp r;
+#pragma unroll
+  for (int k = 0; k < 3; k++)
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(r.w[4 * k]), "=r"(r.w[4 * k + 1]), "=r"(r.w[4 * k + 2]), "=r"(r.w[4 * k + 3])
+                 : "r"(a + 16 * k)
+                 : "memory");
+  return r;
 }
-DEV void st(fp *sl, uint32_t off, const uint32_t *w) {
-  uint4 *p = reinterpret_cast<uint4 *>(reinterpret_cast<uint8_t *>(sl) + off);
-  p[0] = make_uint4(w[0], w[1], w[2], w[3]);
-  p[1] = make_uint4(w[4], w[5], w[6], w[7]);
-  p[2] = make_uint4(w[8], w[9], w[10], w[11]);
+DEV void st(uint32_t a, const uint32_t *w) {
+#pragma unroll
+  for (int k = 0; k < 3; k++)
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(a + 16 * k), "r"(w[4 * k]), "r"(w[4 * k + 1]),
+                 "r"(w[4 * k + 2]), "r"(w[4 * k + 3])
+                 : "memory");
 }
 
 // k p for the table of reduce13
@@ -35,9 +44,9 @@ DEV fp multiple_of_p(uint32_t k) {
   return r;
 }
 
-// 3p + slot[p0] + slot[p1] - slot[m0] - slot[m1], in (0, 6p)
-DEV fp lane_sum(const fp *sl, uint32_t p0, uint32_t p1, uint32_t m0, uint32_t m1) {
-  const fp a = ld(sl, p0), b = ld(sl, p1), c = ld(sl, m0), d = ld(sl, m1);
+// 3p + [p0] + [p1] - [m0] - [m1], in (0, 6p)
+DEV fp lane_sum(uint32_t p0, uint32_t p1, uint32_t m0, uint32_t m1) {
+  const fp a = ld(p0), b = ld(p1), c = ld(m0), d = ld(m1);
   fp t;
   fp_acc_add_3mod(t.w, a.w);
   fp_acc_add(t.w, t.w, b.w);
@@ -49,10 +58,10 @@ DEV fp lane_sum(const fp *sl, uint32_t p0, uint32_t p1, uint32_t m0, uint32_t m1
 // The 13-word value v < QMAX p brought below 1.001 p: the quotient from its top
 // 32 bits (bits 360..391) in single precision, a little low so that it never
 // exceeds v / p, and that multiple of p taken off.
-DEV void reduce13(const fp *mul_p, const uint32_t *v, uint32_t *r) {
+DEV void reduce13(uint32_t mul_p, const uint32_t *v, uint32_t *r) {
   constexpr float K = (float)(256.0 / 436277739.0 * (1.0 - 1.0 / 1048576.0));  // 436277739 = floor(p / 2^352) + 1
   const uint32_t q = (uint32_t)(__uint2float_rz(__funnelshift_l(v[11], v[12], 24)) * K);
-  const fp m = ld(mul_p, q * (uint32_t)sizeof(fp));
+  const fp m = ld(mul_p + q * (uint32_t)sizeof(fp));
   fp_acc_sub(r, v, m.w);
 }
 

@@ -33,3 +33,26 @@ def test_membership(gpu, oracle, n):
     got = gpu.g1_subgroup_for_test([p for p, _ in pts[:n]])
     assert got == [(0, bad) for _, bad in pts[:n]]
     assert gpu.g1_subgroup_for_test([INF] * n) == [(1, 0)] * n
+
+
+@pytest.mark.parametrize("rows", [1, 3, 45, 700, 1400])
+def test_fixed_rows(gpu, oracle, rows):
+    """Fixed-base rows from one (a block of warps) to many (several rows a warp), with scalars whose windows sit on
+    either side of half at every table width, zero and r - 1 rows among them."""
+    p1, gens = oracle.generators(11)
+    pts, r = [p1] + gens, oracle.R_MOD
+
+    def edge(w, d):  # every window half + d
+        return sum(((1 << (w - 1)) + d) << (w * k) for k in range(255 // w)) % r
+    kinds = [0, r - 1, 1] + [edge(w, d) for w in (8, 14, 16, 19, 20) for d in (-1, 0, 1)]
+
+    def row(i):
+        if i % 97 == 1:
+            return [bytes(32)] * 12
+        return [(kinds[(i + k) % len(kinds)]).to_bytes(32, "big") if (i + k) % 3 == 0 else scalar(b"rows", b"%d" % i, k)
+                for k in range(12)]
+    scalars = [row(i) for i in range(rows)]
+    got = gpu.g1_msm_common_points(pts, scalars)
+    assert all(c == 0 for c, _, _ in got)
+    for i in sorted({0, 1, 2, 7, 8, 15, 16, 31, 32, 98, rows // 2, rows - 2, rows - 1} & set(range(rows))):
+        assert got[i][2] == oracle.g1_msm(pts, scalars[i]), i
