@@ -32,15 +32,8 @@ namespace cubbs {
 
 // ----------------------------------------------------------------------------- raw Fr helpers
 DEVNI fr frr_mul(fr a, fr b) { return fr_mul(a, fr_to_mont(b)); }
-DEV fr frr_inv(fr a) { return fr_from_mont(fr_inv(fr_to_mont(a))); }
 DEV fr frr_neg(const fr &a) { return fr_sub(fr_zero(), a); }
 DEV fr frr_one() { fr r = fr_zero(); r.w[0] = 1; return r; }
-
-DEV void sha_fr_be(sha_ctx &c, const fr &raw) {
-  uint8_t b[32];
-  fr_raw_to_be32(raw, b);
-  sha_bytes(c, b, 32);
-}
 
 // Debug record of item 0 of the last ProofGen / ProofVerify finish kernel:
 // [0,48) T1, [48,96) T2, [96,128) domain BE, [128,160) challenge BE,
@@ -71,45 +64,66 @@ struct PvItem {
   int32_t status;  // host-side status
 };
 
+// Entries of the increasing list idx[0 .. n) below v.
+DEV uint32_t count_below(const uint32_t *idx, uint32_t n, uint32_t v) {
+  uint32_t lo = 0, hi = n;
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi) / 2;
+    if (idx[mid] < v) lo = mid + 1;
+    else hi = mid;
+  }
+  return lo;
+}
+
+// The kernels that build an item's scalar row (or its responses) run one block
+// per item, a thread per term: one thread per item walked the terms one after
+// another (1024 items of 100: 0.30 ms for k_pv_rows, 0.11 ms for the copies).
+constexpr unsigned ROW_THREADS = 64;
+
 // Parse the scalars of the proof and build its T2 fixed-base row.  Needs no
 // decoded point, so the fixed-base MSM can run while the points decode.
-__global__ void __launch_bounds__(128) k_pv_rows(PvItem *items, uint32_t n, const uint8_t *blob, const fr *msc,
-                                                 const fr *domain, fr *rows, uint32_t stride, uint32_t *nterms) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  PvItem it = items[i];
-  bool ok = it.status == ST_OK && it.pk_status != DEC_BAD;
+__global__ void __launch_bounds__(ROW_THREADS) k_pv_rows(PvItem *items, const uint8_t *blob, const fr *msc,
+                                                         const fr *domain, fr *rows, uint32_t stride,
+                                                         uint32_t *nterms) {
+  const uint32_t i = blockIdx.x, t = threadIdx.x;
+  const PvItem it = items[i];
   const uint8_t *pr = blob + it.proof_off;
-  fr ecap, r1cap, r3cap, c;
-  if (ok) ok = fr_raw_from_be32(pr + 144, ecap) && fr_raw_from_be32(pr + 176, r1cap) &&
-               fr_raw_from_be32(pr + 208, r3cap) && fr_raw_from_be32(pr + 240 + 32 * it.U, c);
-  #pragma unroll 1
-  for (uint32_t j = 0; j < it.U && ok; j++) {
-    fr t;
-    ok = fr_raw_from_be32(pr + 240 + 32 * j, t);
+  // the item's scalars, e^, r1^, r3^, m^_j .. and c: proof_off + 144 + 32 k, k < U + 4
+  bool ok = it.status == ST_OK && it.pk_status != DEC_BAD;
+  if (ok) {
+    #pragma unroll 1
+    for (uint32_t k = t; k < it.U + 4; k += ROW_THREADS) {
+      fr s;
+      ok = fr_raw_from_be32(pr + 144 + 32 * k, s) && ok;
+    }
   }
-  fr *row = rows + (size_t)i * stride;
-  if (!ok) {
-    items[i].status = ST_INVALID;
-    nterms[i] = 0;
+  if (!__syncthreads_and(ok)) {
+    if (t == 0) {
+      items[i].status = ST_INVALID;
+      nterms[i] = 0;
+    }
     return;
   }
-  nterms[i] = it.L + 2;
-  row[0] = c;
-  row[1] = frr_mul(domain[i], c);
+  fr c;
+  fr_raw_from_be32(pr + 240 + 32 * it.U, c);
+  fr *row = rows + (size_t)i * stride;
+  if (t == 0) {
+    nterms[i] = it.L + 2;
+    row[0] = c;
+  }
+  const fr cm = fr_to_mont(c);
   const uint32_t *idx = reinterpret_cast<const uint32_t *>(blob + it.idx_off);
-  uint32_t k = 0, u = 0;
   #pragma unroll 1
-  for (uint32_t m = 0; m < it.L; m++) {
-    if (k < it.R && idx[k] == m) {
-      row[2 + m] = frr_mul(msc[it.msg_base + k], c);
-      k++;
+  for (uint32_t m = t; m < it.L + 1; m += ROW_THREADS) {  // the domain, then the messages
+    fr s;
+    if (m == 0) {
+      s = fr_mul(domain[i], cm);
     } else {
-      fr t;
-      fr_raw_from_be32(pr + 240 + 32 * u, t);
-      row[2 + m] = t;
-      u++;
+      const uint32_t k = count_below(idx, it.R, m - 1);
+      if (k < it.R && idx[k] == m - 1) s = fr_mul(msc[it.msg_base + k], cm);
+      else fr_raw_from_be32(pr + 240 + 32 * (m - 1 - k), s);
     }
+    row[1 + m] = s;
   }
 }
 
@@ -623,14 +637,21 @@ __global__ void __launch_bounds__(64) k_sign_prep(SignItem *items, uint32_t n, c
     nterms[i] = 0;
     return;
   }
-  // A = B / (sk + e) = sum_g (s_g / (sk + e)) G_g: scale the B row (execution.rs:3400-3447)
-  fr inv = frr_inv(ske);
-  fr *row = rows + (size_t)i * stride;
+  // A = B / (sk + e) = sum_g (s_g / (sk + e)) G_g: the B row scaled (execution.rs:3400-3447), by k_sign_rows
+  rows[(size_t)i * stride] = fr_inv_raw(ske);
   nterms[i] = it.L + 2;
-  row[0] = inv;
-  row[1] = frr_mul(domain[i], inv);
+}
+// The rest of each row, from its factor in the first place.
+__global__ void __launch_bounds__(ROW_THREADS) k_sign_rows(const SignItem *items, const fr *msc, const fr *domain,
+                                                           fr *rows, uint32_t stride, const uint32_t *nterms) {
+  const uint32_t i = blockIdx.x, terms = nterms[i];
+  if (terms == 0) return;
+  const uint32_t base = items[i].msg_base;
+  fr *row = rows + (size_t)i * stride;
+  const fr f = fr_to_mont(row[0]);
   #pragma unroll 1
-  for (uint32_t k = 0; k < it.L; k++) row[2 + k] = frr_mul(msc[it.msg_base + k], inv);
+  for (uint32_t g = 1 + threadIdx.x; g < terms; g += ROW_THREADS)
+    row[g] = fr_mul(g == 1 ? domain[i] : msc[base + g - 2], f);
 }
 
 __global__ void __launch_bounds__(64) k_sign_finish(SignItem *items, uint32_t n, const g1 *A, const fr *e,
@@ -660,25 +681,23 @@ struct VerifyItem {
 
 // B-MSM row of each signature (needs no decoded point, so the fixed-base MSM
 // runs while the signature's A decodes).
-__global__ void __launch_bounds__(128) k_verify_rows(VerifyItem *items, uint32_t n, const uint8_t *blob,
-                                                     const fr *msc, const fr *domain, fr *rows, uint32_t stride,
-                                                     uint32_t *nterms) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  VerifyItem it = items[i];
+__global__ void __launch_bounds__(ROW_THREADS) k_verify_rows(VerifyItem *items, const uint8_t *blob, const fr *msc,
+                                                             const fr *domain, fr *rows, uint32_t stride,
+                                                             uint32_t *nterms) {
+  const uint32_t i = blockIdx.x, t = threadIdx.x;
+  const VerifyItem it = items[i];
   fr e;
-  bool ok = it.status == ST_OK && it.pk_status != DEC_BAD && fr_raw_from_be32(blob + it.sig_off + 48, e);
-  if (!ok) {
-    if (items[i].status == ST_OK) items[i].status = ST_INVALID;
-    nterms[i] = 0;
-    return;
+  const bool ok = it.status == ST_OK && it.pk_status != DEC_BAD && fr_raw_from_be32(blob + it.sig_off + 48, e);
+  __syncthreads();  // every thread has read the item
+  if (t == 0) {
+    if (!ok && it.status == ST_OK) items[i].status = ST_INVALID;
+    nterms[i] = ok ? it.L + 2 : 0;
   }
+  if (!ok) return;
   fr *row = rows + (size_t)i * stride;
-  nterms[i] = it.L + 2;
-  row[0] = frr_one();
-  row[1] = domain[i];
   #pragma unroll 1
-  for (uint32_t k = 0; k < it.L; k++) row[2 + k] = msc[it.msg_base + k];
+  for (uint32_t g = t; g < it.L + 2; g += ROW_THREADS)
+    row[g] = g == 0 ? frr_one() : g == 1 ? domain[i] : msc[it.msg_base + g - 2];
 }
 
 // The variable-base job -e * A of each signature, from the untouched input
@@ -798,15 +817,13 @@ __global__ void __launch_bounds__(64) k_pg_random(const PgItem *items, uint32_t 
     sha_byte(c, 0);
     sha_bytes(c, dst, DST_MOCK_LEN);
     sha_byte(c, DST_MOCK_LEN);
-    uint8_t b0[32];
-    sha_final(c, b0);
+    uint32_t x0[8];
+    sha_final_words(c, x0);
     // b_i = SHA-256((b_0 xor b_(i-1)) || I2OSP(i, 1) || DST || I2OSP(68, 1)): 102 bytes
     // in two blocks.  Block 1 is 8 words of b_0 xor b_(i-1), then i and DST[0..30];
     // block 2 (DST[31..67], the DST length, the padding, the bit length 816) is the
     // same for every i.
-    uint32_t x0[8], bi[8] = {0, 0, 0, 0, 0, 0, 0, 0}, tail1[7], blk2[16];
-    for (int k = 0; k < 8; k++)
-      x0[k] = (uint32_t)b0[4 * k] << 24 | (uint32_t)b0[4 * k + 1] << 16 | (uint32_t)b0[4 * k + 2] << 8 | b0[4 * k + 3];
+    uint32_t bi[8] = {0, 0, 0, 0, 0, 0, 0, 0}, tail1[7], blk2[16];
     const uint32_t dst3 = (uint32_t)dst[0] << 16 | (uint32_t)dst[1] << 8 | dst[2];
     for (int k = 0; k < 7; k++)
       tail1[k] = (uint32_t)dst[3 + 4 * k] << 24 | (uint32_t)dst[4 + 4 * k] << 16 | (uint32_t)dst[5 + 4 * k] << 8 |
@@ -822,8 +839,7 @@ __global__ void __launch_bounds__(64) k_pg_random(const PgItem *items, uint32_t 
       for (int k = 0; k < 16; k++)
         blk2[k] = (uint32_t)t[4 * k] << 24 | (uint32_t)t[4 * k + 1] << 16 | (uint32_t)t[4 * k + 2] << 8 | t[4 * k + 3];
     }
-    uint8_t okm[48];
-    uint32_t fill = 0, produced = 0;
+    uint32_t okm[12], fill = 0, produced = 0;
     uint32_t ell = (nbytes + 31) / 32;
     #pragma unroll 1
     for (uint32_t b = 1; b <= ell; b++) {
@@ -837,10 +853,10 @@ __global__ void __launch_bounds__(64) k_pg_random(const PgItem *items, uint32_t 
       for (int k = 0; k < 16; k++) w[k] = blk2[k];
       sha256_compress(h, w);
       for (int k = 0; k < 8; k++) bi[k] = h[k];
-      for (int j = 0; j < 32; j++) {
-        okm[fill++] = (uint8_t)(bi[j >> 2] >> (24 - 8 * (j & 3)));
-        if (fill == 48) {
-          out[c0 + produced] = fr_raw_from_okm(okm);
+      for (int j = 0; j < 8; j++) {
+        okm[fill++] = bi[j];
+        if (fill == 12) {
+          out[c0 + produced] = fr_raw_from_okm_words(okm);
           produced++;
           fill = 0;
         }
@@ -852,54 +868,46 @@ __global__ void __launch_bounds__(64) k_pg_random(const PgItem *items, uint32_t 
 // Row i: B = P1 + Q1 domain + sum H_i m_i.  Needs neither the decoded signature
 // point (k_pg_vars rejects a signature whose A does not decode) nor the blinding
 // scalars, so the B-MSM starts as soon as the messages are hashed.
-__global__ void __launch_bounds__(128) k_pg_rows_b(PgItem *items, uint32_t n, const uint8_t *blob, const fr *msc,
-                                                   const fr *domain, fr *rows, uint32_t stride, uint32_t *nterms) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  PgItem it = items[i];
+__global__ void __launch_bounds__(ROW_THREADS) k_pg_rows_b(PgItem *items, const uint8_t *blob, const fr *msc,
+                                                           const fr *domain, fr *rows, uint32_t stride,
+                                                           uint32_t *nterms) {
+  const uint32_t i = blockIdx.x, t = threadIdx.x;
+  const PgItem it = items[i];
   fr e;
-  bool ok = it.status == ST_OK && it.pk_status != DEC_BAD && fr_raw_from_be32(blob + it.sig_off + 48, e);
-  if (!ok) {
-    items[i].status = ST_ERROR;
-    nterms[i] = 0;
-    return;
+  const bool ok = it.status == ST_OK && it.pk_status != DEC_BAD && fr_raw_from_be32(blob + it.sig_off + 48, e);
+  __syncthreads();  // every thread has read the item
+  if (t == 0) {
+    if (!ok) items[i].status = ST_ERROR;
+    nterms[i] = ok ? it.L + 2 : 0;
   }
-  fr *rb = rows + (size_t)i * stride;
-  nterms[i] = it.L + 2;
-  rb[0] = frr_one();
-  rb[1] = domain[i];
+  if (!ok) return;
+  fr *row = rows + (size_t)i * stride;
   #pragma unroll 1
-  for (uint32_t m = 0; m < it.L; m++) rb[2 + m] = msc[it.msg_base + m];
+  for (uint32_t g = t; g < it.L + 2; g += ROW_THREADS)
+    row[g] = g == 0 ? frr_one() : g == 1 ? domain[i] : msc[it.msg_base + g - 2];
 }
 
 // Row n + i: the fixed part of T2, sum_{j not disclosed} H_j m~_j, from the
 // untouched input items and the blinding scalars.
-__global__ void __launch_bounds__(128) k_pg_rows_t2(const PgItem *items0, uint32_t n, const uint8_t *blob,
-                                                    const fr *rs, uint32_t rs_stride, fr *rows, uint32_t stride,
-                                                    uint32_t *nterms) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+__global__ void __launch_bounds__(ROW_THREADS) k_pg_rows_t2(const PgItem *items0, uint32_t n, const uint8_t *blob,
+                                                            const fr *rs, uint32_t rs_stride, fr *rows,
+                                                            uint32_t stride, uint32_t *nterms) {
+  const uint32_t i = blockIdx.x, t = threadIdx.x;
   const PgItem it = items0[i];
-  if (it.status != ST_OK) {
-    nterms[n + i] = 0;
-    return;
-  }
-  fr *rt = rows + (size_t)(n + i) * stride;
-  nterms[n + i] = it.L + 2;
-  rt[0] = fr_zero();
-  rt[1] = fr_zero();
+  const bool ok = it.status == ST_OK;
+  if (t == 0) nterms[n + i] = ok ? it.L + 2 : 0;
+  if (!ok) return;
+  fr *row = rows + (size_t)(n + i) * stride;
   const uint32_t *idx = reinterpret_cast<const uint32_t *>(blob + it.idx_off);
   const fr *r = rs + (size_t)i * rs_stride;
-  uint32_t k = 0, u = 0;
   #pragma unroll 1
-  for (uint32_t m = 0; m < it.L; m++) {
-    if (k < it.R && idx[k] == m) {
-      rt[2 + m] = fr_zero();
-      k++;
-    } else {
-      rt[2 + m] = r[5 + u];
-      u++;
+  for (uint32_t g = t; g < it.L + 2; g += ROW_THREADS) {
+    fr s = fr_zero();
+    if (g >= 2) {
+      const uint32_t m = g - 2, k = count_below(idx, it.R, m);
+      if (k >= it.R || idx[k] != m) s = r[5 + m - k];
     }
+    row[g] = s;
   }
 }
 
@@ -987,23 +995,34 @@ __global__ void __launch_bounds__(64) k_pg_finish(PgItem *items, uint32_t n, con
   fr_raw_to_be32(fr_add(et, frr_mul(e, ch)), o + 144);
   fr_raw_to_be32(fr_sub(r1t, frr_mul(r1, ch)), o + 176);
   fr_raw_to_be32(fr_sub(r3t, frr_mul(r3, ch)), o + 208);
-  uint32_t k = 0, u = 0;
-  #pragma unroll 1
-  for (uint32_t m = 0; m < it.L; m++) {
-    if (k < it.R && idx[k] == m) {
-      k++;
-      continue;
-    }
-    fr_raw_to_be32(fr_add(r[5 + u], frr_mul(msc[it.msg_base + m], ch)), o + 240 + 32 * u);
-    u++;
-  }
   fr_raw_to_be32(ch, o + 240 + 32 * it.U);
+}
+
+// The responses m^_j = m~_j + c m_j of the undisclosed messages, from the
+// challenge that k_pg_finish wrote behind them.
+__global__ void __launch_bounds__(ROW_THREADS) k_pg_responses(const PgItem *items, const uint8_t *blob, const fr *msc,
+                                                              const fr *rs, uint32_t rs_stride, uint8_t *out) {
+  const uint32_t i = blockIdx.x;
+  const PgItem it = items[i];
+  if (it.status != ST_OK) return;
+  uint8_t *o = out + it.out_off + 240;
+  fr c;
+  fr_raw_from_be32(o + 32 * it.U, c);
+  const fr cm = fr_to_mont(c);
+  const uint32_t *idx = reinterpret_cast<const uint32_t *>(blob + it.idx_off);
+  const fr *r = rs + (size_t)i * rs_stride + 5;
+  #pragma unroll 1
+  for (uint32_t m = threadIdx.x; m < it.L; m += ROW_THREADS) {
+    const uint32_t k = count_below(idx, it.R, m), u = m - k;
+    if (k < it.R && idx[k] == m) continue;
+    fr_raw_to_be32(fr_add(r[u], fr_mul(msc[it.msg_base + m], cm)), o + 32 * u);
+  }
 }
 
 // Work of k_pg_finish that needs neither the MSMs nor the proof's points, done
 // beside them: the challenge hash's leading part (R, the disclosed indexes and
 // message scalars: about 31 SHA-256 blocks at 50 disclosed messages), kept as
-// the expander's state per item, and r3 = r2^-1 (a Fermat inversion in Fr).
+// the expander's state per item, and r3 = r2^-1 in Fr.
 // It reads the input items as packed; an item the host rejected is skipped
 // (k_pg_finish skips it as well).
 template <int S>
@@ -1024,7 +1043,7 @@ __global__ void __launch_bounds__(64) k_pg_early(const PgItem *items0, uint32_t 
     msg_fr_be(c, msc[it.msg_base + idx[k]]);
   }
   chal[i] = c;
-  r3inv[i] = frr_inv(rs[(size_t)i * rs_stride + 1]);  // r2 == 0 gives 0; k_pg_finish reports it
+  r3inv[i] = fr_inv_raw(rs[(size_t)i * rs_stride + 1]);  // r2 == 0 gives 0; k_pg_finish reports it
 }
 
 // ============================================================================ host side
@@ -1512,7 +1531,7 @@ void run_pverify(Runtime &rt, OpBatch &b, uint8_t *dmapdst) {
   CUBBS_CHECK(cudaEventRecord(rt.ev_side, s2));
   SPAN(s, "domain", launch_domain(s, b.ddj, N, b.dblob, rt.d_gens_c(), rt.ss().d_dom_prefix, b.domain, rt.suite));
   SPAN(s, "scalar_prep",
-       k_pv_rows<<<blocks_for(n, 128), 128, 0, s>>>(it, N, b.dblob, b.msc, b.domain, b.rows, stride, b.nterms));
+       k_pv_rows<<<N, ROW_THREADS, 0, s>>>(it, b.dblob, b.msc, b.domain, b.rows, stride, b.nterms));
   SPAN(s, "fixed_msm", launch_fixed_msm(s, rt.table(), b.rows, stride, b.nterms, N, b.fixed));
   CUBBS_CHECK(cudaStreamWaitEvent(s, rt.ev_side, 0));
   CUBBS_CHECK(cudaStreamWaitEvent(s, rt.ev_sub, 0));
@@ -1546,7 +1565,7 @@ void run_pgen(Runtime &rt, OpBatch &b, uint8_t *dmapdst) {
   SPAN(s2, "random_scalars", CUBBS_SUITE_DISPATCH(rt.suite, k_pg_random<S><<<blocks_for(n, 64), 64, 0, s2>>>(it0, N, b.dblob, b.rs, rss)));
   CUBBS_CHECK(cudaEventRecord(rt.ev_mid, s2));
   SPAN(s2, "fixed_msm_t2",
-       k_pg_rows_t2<<<blocks_for(n, 128), 128, 0, s2>>>(it0, N, b.dblob, b.rs, rss, b.rows, stride, b.nterms);
+       k_pg_rows_t2<<<N, ROW_THREADS, 0, s2>>>(it0, N, b.dblob, b.rs, rss, b.rows, stride, b.nterms);
        launch_fixed_msm(s2, rt.table(), b.rows + (size_t)n * stride, stride, b.nterms + n, N, b.fixed + n));
   CUBBS_CHECK(cudaEventRecord(rt.ev_side, s2));
   if (nm)
@@ -1555,7 +1574,7 @@ void run_pgen(Runtime &rt, OpBatch &b, uint8_t *dmapdst) {
                          reinterpret_cast<uint32_t *>(b.dmsg) + nm, (uint32_t)nm, dmapdst, map_dst_len(rt), b.msc, rt.suite));
   SPAN(s, "domain", launch_domain(s, b.ddj, N, b.dblob, rt.d_gens_c(), rt.ss().d_dom_prefix, b.domain, rt.suite));
   SPAN(s, "fixed_msm",
-       k_pg_rows_b<<<blocks_for(n, 128), 128, 0, s>>>(it, N, b.dblob, b.msc, b.domain, b.rows, stride, b.nterms);
+       k_pg_rows_b<<<N, ROW_THREADS, 0, s>>>(it, b.dblob, b.msc, b.domain, b.rows, stride, b.nterms);
        launch_fixed_msm(s, rt.table(), b.rows, stride, b.nterms, N, b.fixed));
   CUBBS_CHECK(cudaStreamWaitEvent(s, rt.ev_mid, 0));  // the blinding scalars
   SPAN(s, "finish_early",
@@ -1570,8 +1589,9 @@ void run_pgen(Runtime &rt, OpBatch &b, uint8_t *dmapdst) {
   SPAN(s, "var_mul", launch_var_mul(s, b.vpts, b.jobs, b.jscal, 7 * N, b.v));
   SPAN(s, "finish",
        CUBBS_SUITE_DISPATCH(rt.suite, k_pg_finish<S><<<blocks_for(n, 64), 64, 0, s>>>(it, N, b.dblob, b.msc, b.domain, b.rs, rss, b.fixed + n, b.v,
-                                                    b.out, reinterpret_cast<const hash_ctx<S> *>(b.chal), b.r3inv)));
-  b.launches_per_run = (nm ? 1 : 0) + (npts ? 2 : 0) + 10;
+                                                    b.out, reinterpret_cast<const hash_ctx<S> *>(b.chal), b.r3inv));
+       k_pg_responses<<<N, ROW_THREADS, 0, s>>>(it, b.dblob, b.msc, b.rs, rss, b.out));
+  b.launches_per_run = (nm ? 1 : 0) + (npts ? 2 : 0) + 11;
 }
 
 // Verify on three streams, as ProofVerify: the signature decode (stream2, no
@@ -1601,7 +1621,7 @@ void run_verify(Runtime &rt, OpBatch &b, uint8_t *dmapdst) {
                          reinterpret_cast<uint32_t *>(b.dmsg) + nm, (uint32_t)nm, dmapdst, map_dst_len(rt), b.msc, rt.suite));
   SPAN(s, "domain", launch_domain(s, b.ddj, N, b.dblob, rt.d_gens_c(), rt.ss().d_dom_prefix, b.domain, rt.suite));
   SPAN(s, "scalar_prep",
-       k_verify_rows<<<blocks_for(n, 128), 128, 0, s>>>(it, N, b.dblob, b.msc, b.domain, b.rows, stride, b.nterms));
+       k_verify_rows<<<N, ROW_THREADS, 0, s>>>(it, b.dblob, b.msc, b.domain, b.rows, stride, b.nterms));
   SPAN(s, "fixed_msm", launch_fixed_msm(s, rt.table(), b.rows, stride, b.nterms, N, b.fixed));
   CUBBS_CHECK(cudaStreamWaitEvent(s, rt.ev_side, 0));
   CUBBS_CHECK(cudaStreamWaitEvent(s, rt.ev_sub, 0));
@@ -1668,10 +1688,11 @@ void run(Runtime &rt, OpBatch &b, uint8_t *dmapdst) {
       SignItem *it = reinterpret_cast<SignItem *>(b.ditems);
       SPAN(s, "scalar_prep",
            CUBBS_SUITE_DISPATCH(rt.suite, k_sign_prep<S><<<blocks_for(n, 64), 64, 0, s>>>(it, N, b.dblob, b.msc, b.domain, b.rows, stride, b.nterms,
-                                                        b.e)));
+                                                        b.e));
+           k_sign_rows<<<N, ROW_THREADS, 0, s>>>(it, b.msc, b.domain, b.rows, stride, b.nterms));
       SPAN(s, "fixed_msm", launch_fixed_msm(s, rt.table(), b.rows, stride, b.nterms, N, b.fixed));
       SPAN(s, "finish", k_sign_finish<<<blocks_for(n, 64), 64, 0, s>>>(it, N, b.fixed, b.e, b.out));
-      launches += 3;
+      launches += 4;
       break;
     }
     case OP_VERIFY:
@@ -2469,7 +2490,7 @@ __global__ void k_h2s_scalars_test(const uint8_t *be, uint32_t n, fr *out) {
   for (uint32_t k = 0; k < n; k++) {
     fr s;
     fr_raw_from_be32(be + 32 * k, s);
-    sha_fr_be(c, s);
+    msg_fr_be(c, s);
   }
   out[0] = h2s_finish(c, DST_H2S, DST_H2S_LEN);
 }
@@ -2509,7 +2530,7 @@ __global__ void k_pairs_test(const uint8_t *blob, uint32_t idx_off, uint32_t R, 
     sha_u64be(c, idx[k], 8);
     fr m;
     fr_raw_from_be32(mbe + 32 * k, m);
-    sha_fr_be(c, m);
+    msg_fr_be(c, m);
   }
   out[0] = h2s_finish(c, DST_H2S, DST_H2S_LEN);
 }

@@ -133,11 +133,7 @@ __global__ void k_sign_e(const SignEJob *jobs, uint32_t n, const uint8_t *blob, 
   xmd_begin(c);
   sha_bytes(c, blob + j.blob_off, 32);
   #pragma unroll 1
-  for (uint32_t k = 0; k < j.count; k++) {
-    uint8_t b[32];
-    fr_raw_to_be32(scalars[j.scalar_off + k], b);
-    sha_bytes(c, b, 32);
-  }
+  for (uint32_t k = 0; k < j.count; k++) msg_fr_be(c, scalars[j.scalar_off + k]);
   sha_bytes(c, blob + j.blob_off + 32, 32);
   out[i] = h2s_finish(c, dst, dlen);
 }

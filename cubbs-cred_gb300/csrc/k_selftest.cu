@@ -54,13 +54,23 @@ DEV g1 zabs_unrolled_bits(g1 p) {
 }
 
 // op 0: Fp product of canonical BE inputs; op 1: Fp inverse; op 2: Fp sqrt (0 if none);
-// op 3: variable-time Fp inverse; op 4: Fp product by CIOS carry chains; op 5: Fp square
+// op 3: variable-time Fp inverse; op 4: Fp product by CIOS carry chains; op 5: Fp square;
+// op 6: the Fr inverse of a residue mod r
 __global__ void k_fp_test(const uint8_t *a, const uint8_t *b, uint32_t n, int op, uint8_t *out, int32_t *st) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   fp x, y, r = fp_zero();
   bool ok = fp_from_be48(a + 48 * (size_t)i, x) && fp_from_be48(b + 48 * (size_t)i, y);
   if (ok) {
+    if (op == 6) {
+      fr v;
+      ok = fr_raw_from_be32(a + 48 * (size_t)i + 16, v);
+      v = fr_inv_raw(v);
+      st[i] = ok ? 0 : 1;
+      for (int k = 0; k < 16; k++) out[48 * (size_t)i + k] = 0;
+      fr_raw_to_be32(v, out + 48 * (size_t)i + 16);
+      return;
+    }
     if (op == 0) r = fp_mul(x, y);
     else if (op == 4) r = fp_mul_cios(x, y);
     else if (op == 5) r = fp_sqr(x);

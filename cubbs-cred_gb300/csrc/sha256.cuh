@@ -58,51 +58,67 @@ DEV void sha_init(sha_ctx &c) {
   c.fill = 0;
   c.total = 0;
 }
-DEV void sha_byte(sha_ctx &c, uint8_t b) {
-  c.w[c.fill >> 2] |= (uint32_t)b << (24 - 8 * (c.fill & 3));
-  c.fill++;
-  c.total++;
-  if (c.fill == 64) {
+// Absorbs nbytes = 1..4 bytes, the top bytes of v (the others zero).  Every
+// piece of a BBS hash input is fed through this, four bytes at a time whatever
+// the block position: the words lie in local memory, and a byte at a time cost
+// a read-modify-write each (Sign's e over 90 messages: 16 thousand cycles a
+// block where the compression takes 4).
+DEV void sha_put(sha_ctx &c, uint32_t v, uint32_t nbytes) {
+  const uint32_t i = c.fill >> 2, r = 8 * (c.fill & 3);
+  c.w[i] |= v >> r;
+  const uint32_t rest = __funnelshift_l(0u, v, 32 - r);  // v << (32 - r), 0 for r = 0: what goes past word i
+  const bool past = (c.fill & 3) + nbytes > 4;
+  c.fill += nbytes;
+  c.total += nbytes;
+  if (c.fill >= 64) {
     sha256_compress(c.h, c.w);
-    for (int i = 0; i < 16; i++) c.w[i] = 0;
-    c.fill = 0;
+    c.fill -= 64;
+#pragma unroll
+    for (int k = 1; k < 16; k++) c.w[k] = 0;
+    c.w[0] = past ? rest : 0;
+  } else if (past) {
+    c.w[i + 1] = rest;
   }
 }
+DEV void sha_byte(sha_ctx &c, uint8_t b) { sha_put(c, (uint32_t)b << 24, 1); }
 DEV void sha_bytes(sha_ctx &c, const uint8_t *p, uint32_t n) {
-  // word-at-a-time when the block position is 4-aligned (bytes are assembled
-  // individually: the source may be a byte array just written by this thread)
   uint32_t i = 0;
-  if ((c.fill & 3) == 0) {
 #pragma unroll 1
-    while (i + 4 <= n) {
-      c.w[c.fill >> 2] = ((uint32_t)p[i] << 24) | ((uint32_t)p[i + 1] << 16) | ((uint32_t)p[i + 2] << 8) | p[i + 3];
-      c.fill += 4;
-      c.total += 4;
-      i += 4;
-      if (c.fill == 64) {
-        sha256_compress(c.h, c.w);
-        for (int k = 0; k < 16; k++) c.w[k] = 0;
-        c.fill = 0;
-      }
-    }
+  for (; i < n; i += 4) {
+    const uint32_t m = min(n - i, 4u);
+    uint32_t v = (uint32_t)p[i] << 24;
+    if (m > 1) v |= (uint32_t)p[i + 1] << 16;
+    if (m > 2) v |= (uint32_t)p[i + 2] << 8;
+    if (m > 3) v |= p[i + 3];
+    sha_put(c, v, m);
   }
-#pragma unroll 1
-  for (; i < n; i++) sha_byte(c, p[i]);
 }
-DEV void sha_u64be(sha_ctx &c, uint64_t x, int nbytes) {
-  #pragma unroll 1
-  for (int i = nbytes - 1; i >= 0; i--) sha_byte(c, (uint8_t)(x >> (8 * i)));
+DEV void sha_u64be(sha_ctx &c, uint64_t x, int nbytes) {  // the low nbytes (4 or 8) bytes of x
+  if (nbytes == 8) sha_put(c, (uint32_t)(x >> 32), 4);
+  sha_put(c, (uint32_t)x, 4);
 }
-DEV void sha_final(sha_ctx &c, uint8_t out[32]) {
-  uint64_t bits = (uint64_t)c.total * 8;
+// out = the digest as eight big-endian words
+DEV void sha_final_words(sha_ctx &c, uint32_t out[8]) {
+  const uint64_t bits = (uint64_t)c.total * 8;
   sha_byte(c, 0x80);
-  while (c.fill != 56) sha_byte(c, 0);
+  if (c.fill > 56) {
+    sha256_compress(c.h, c.w);
+#pragma unroll
+    for (int k = 0; k < 14; k++) c.w[k] = 0;
+  }
   c.w[14] = (uint32_t)(bits >> 32);
   c.w[15] = (uint32_t)bits;
   sha256_compress(c.h, c.w);
+#pragma unroll
+  for (int k = 0; k < 8; k++) out[k] = c.h[k];
+}
+DEV void sha_final(sha_ctx &c, uint8_t out[32]) {
+  uint32_t w[8];
+  sha_final_words(c, w);
+#pragma unroll
   for (int i = 0; i < 8; i++) {
-    out[4 * i] = (uint8_t)(c.h[i] >> 24); out[4 * i + 1] = (uint8_t)(c.h[i] >> 16);
-    out[4 * i + 2] = (uint8_t)(c.h[i] >> 8); out[4 * i + 3] = (uint8_t)c.h[i];
+    out[4 * i] = (uint8_t)(w[i] >> 24); out[4 * i + 1] = (uint8_t)(w[i] >> 16);
+    out[4 * i + 2] = (uint8_t)(w[i] >> 8); out[4 * i + 3] = (uint8_t)w[i];
   }
 }
 
@@ -115,36 +131,49 @@ DEV void xmd_begin(sha_ctx &c) {
   for (int i = 0; i < 16; i++) c.w[i] = 0;
   c.total = 64;
 }
-// Finishes b_0 and writes n output bytes (n <= 255*32).
-DEV void xmd_finish(sha_ctx &c, const uint8_t *dst, uint32_t dlen, uint32_t n, uint8_t *out) {
-  sha_byte(c, (uint8_t)(n >> 8));
-  sha_byte(c, (uint8_t)n);
-  sha_byte(c, 0);
+// Finishes b_0 for n output bytes (n <= 255*32); block(i, b_i) gets the output
+// blocks i = 1, 2, .. as eight words each.
+template <class Block>
+DEV void xmd_blocks(sha_ctx &c, const uint8_t *dst, uint32_t dlen, uint32_t n, const Block &block) {
+  sha_put(c, n << 16, 3);  // I2OSP(n, 2), then a zero byte
   sha_bytes(c, dst, dlen);
   sha_byte(c, (uint8_t)dlen);
-  uint8_t b0[32], bi[32];
-  sha_final(c, b0);
-  uint32_t ell = (n + 31) / 32;
+  uint32_t b0[8], bi[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  sha_final_words(c, b0);
+  const uint32_t ell = (n + 31) / 32;
   #pragma unroll 1
   for (uint32_t i = 1; i <= ell; i++) {
     sha_ctx s;
     sha_init(s);
-    for (int j = 0; j < 32; j++) sha_byte(s, i == 1 ? b0[j] : (uint8_t)(b0[j] ^ bi[j]));
+#pragma unroll
+    for (int k = 0; k < 8; k++) s.w[k] = b0[k] ^ bi[k];  // b_1 takes b_0 alone
+    s.fill = s.total = 32;
     sha_byte(s, (uint8_t)i);
     sha_bytes(s, dst, dlen);
     sha_byte(s, (uint8_t)dlen);
-    sha_final(s, bi);
-    uint32_t off = (i - 1) * 32;
-    #pragma unroll 1
-    for (uint32_t j = 0; j < 32 && off + j < n; j++) out[off + j] = bi[j];
+    sha_final_words(s, bi);
+    block(i, bi);
   }
+}
+DEV void xmd_finish(sha_ctx &c, const uint8_t *dst, uint32_t dlen, uint32_t n, uint8_t *out) {
+  xmd_blocks(c, dst, dlen, n, [&](uint32_t i, const uint32_t *b) {
+    const uint32_t off = (i - 1) * 32;
+    #pragma unroll 1
+    for (uint32_t j = 0; j < 32 && off + j < n; j++) out[off + j] = (uint8_t)(b[j >> 2] >> (24 - 8 * (j & 3)));
+  });
 }
 // hash_to_scalar (util.rs:104-129): OS2IP(expand_message_xmd(msg, dst, 48)) mod r,
 // returned as the canonical raw residue.
 DEV fr h2s_finish(sha_ctx &c, const uint8_t *dst, uint32_t dlen) {
-  uint8_t okm[48];
-  xmd_finish(c, dst, dlen, 48, okm);
-  return fr_raw_from_okm(okm);
+  uint32_t okm[16];
+  xmd_blocks(c, dst, dlen, 48, [&](uint32_t i, const uint32_t *b) {
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      if (i == 1) okm[k] = b[k];
+      else okm[8 + k] = b[k];
+    }
+  });
+  return fr_raw_from_okm_words(okm);
 }
 
 // The suite-generic names used by the kernels (the SHAKE-256 forms are in keccak.cuh).
@@ -152,6 +181,10 @@ DEV void msg_begin(sha_ctx &c) { xmd_begin(c); }
 DEV void msg_byte(sha_ctx &c, uint8_t b) { sha_byte(c, b); }
 DEV void msg_bytes(sha_ctx &c, const uint8_t *p, uint32_t n) { sha_bytes(c, p, n); }
 DEV void msg_u64be(sha_ctx &c, uint64_t x, int nbytes) { sha_u64be(c, x, nbytes); }
+DEV void msg_fr_be(sha_ctx &c, const fr &raw) {  // 32 bytes, big-endian
+#pragma unroll 1
+  for (int k = 7; k >= 0; k--) sha_put(c, raw.w[k], 4);
+}
 DEV void msg_finish(sha_ctx &c, const uint8_t *dst, uint32_t dlen, uint32_t n, uint8_t *out) {
   xmd_finish(c, dst, dlen, n, out);
 }

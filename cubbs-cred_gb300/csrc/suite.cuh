@@ -15,7 +15,7 @@ template <int S> struct HashCtxOf { using type = sha_ctx; };
 template <> struct HashCtxOf<SUITE_SHAKE256> { using type = shake_ctx; };
 template <int S> using hash_ctx = typename HashCtxOf<S>::type;
 
-template <class C> DEV void msg_fr_be(C &c, const fr &raw) {
+DEV void msg_fr_be(shake_ctx &c, const fr &raw) {  // (the SHA-256 form is in sha256.cuh)
   uint8_t b[32];
   fr_raw_to_be32(raw, b);
   msg_bytes(c, b, 32);

@@ -51,6 +51,16 @@ def test_fp_inv_sqrt(gpu, oracle):
         assert st == 0 and oracle.fp_mul(r, r) == s
 
 
+def test_fr_inv(gpu, oracle):
+    """The constant-time inverse mod r: 0, +-1, powers of two, and random residues."""
+    r = oracle.R_MOD
+    xs = [0, 1, 2, 3, r - 1, r - 2, (r - 1) // 2] + [(1 << k) % r for k in range(30, 256, 15)]
+    xs += [int.from_bytes(scalar(b"frinv", b"x", i), "big") for i in range(512)]
+    a = [x.to_bytes(48, "big") for x in xs]
+    want = [(0, (pow(x, -1, r) if x else 0).to_bytes(48, "big")) for x in xs]
+    assert gpu.fp_op_for_test(6, a, a) == want
+
+
 def test_fp_inv_vartime_matches_fermat(gpu, oracle):
     a = rand_fp(oracle, b"vinv", 48) + [(1).to_bytes(48, "big"), (oracle.P_MOD - 1).to_bytes(48, "big"),
                                         (2).to_bytes(48, "big"), bytes(48)]
