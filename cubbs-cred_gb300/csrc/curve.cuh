@@ -526,20 +526,29 @@ DEV g1 warp_sum_g1(g1 acc) {
 #define DEC_BAD 2
 // G1Affine::from_compressed (unchecked decode + torsion check).  Returns DEC_OK
 // with the affine point, DEC_INF for the canonical identity encoding, DEC_BAD otherwise.
-DEV int g1_decompress(const uint8_t in[48], g1a &out, bool check_subgroup = true) {
+// g1_x: the flags and the x coordinate; DEC_OK when a y is to be found, with
+// rhs = x^3 + 4 and the sign flag.
+DEV int g1_x(const uint8_t in[48], fp &x, fp &rhs, bool &sort) {
   uint8_t f = in[0];
-  bool comp = f & 0x80, inf = f & 0x40, sort = f & 0x20;
+  bool comp = f & 0x80, inf = f & 0x40;
+  sort = f & 0x20;
   uint8_t t[48];
   t[0] = f & 0x1f;
   #pragma unroll 1
   for (int i = 1; i < 48; i++) t[i] = in[i];
-  fp x;
   if (!fp_from_be48(t, x)) return DEC_BAD;
   if (inf) return (comp && !sort && fp_is_zero(x)) ? DEC_INF : DEC_BAD;
   if (!comp) return DEC_BAD;
   const fp four = C_FP_FOUR;
-  fp y;
-  if (!fp_sqrt(fp_add(fp_mul(fp_sqr(x), x), four), y)) return DEC_BAD;
+  rhs = fp_add(fp_mul(fp_sqr(x), x), four);
+  return DEC_OK;
+}
+DEV int g1_decompress(const uint8_t in[48], g1a &out, bool check_subgroup = true) {
+  fp x, y, rhs;
+  bool sort;
+  const int st = g1_x(in, x, rhs, sort);
+  if (st != DEC_OK) return st;
+  if (!fp_sqrt(rhs, y)) return DEC_BAD;
   if (fp_lex_largest(y) != sort) y = fp_neg(y);
   out.x = x;
   out.y = y;

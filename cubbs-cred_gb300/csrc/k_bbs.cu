@@ -1560,7 +1560,9 @@ void run_pgen(Runtime &rt, OpBatch &b, uint8_t *dmapdst) {
   CUBBS_CHECK(cudaStreamWaitEvent(s2, rt.ev_fork, 0));
   CUBBS_CHECK(cudaStreamWaitEvent(s3, rt.ev_fork, 0));
   SPAN(s3, "g1_decode", launch_g1_decode(s3, b.dpts48, 48, (uint32_t)npts, b.pts, b.dec, false));
-  SPAN(s3, "g1_subgroup", launch_g1_subgroup(s3, b.pts, b.dec, (uint32_t)npts, b.sub));
+  // the check is done long before the MSMs are, so it takes the form with the
+  // fewest instructions at any size (1024 proofs: 3.66 -> 3.58 ms)
+  SPAN(s3, "g1_subgroup", launch_g1_subgroup(s3, b.pts, b.dec, (uint32_t)npts, b.sub, npts > 512 ? 2 : 0));
   CUBBS_CHECK(cudaEventRecord(rt.ev_join, s3));
   SPAN(s2, "random_scalars", CUBBS_SUITE_DISPATCH(rt.suite, k_pg_random<S><<<blocks_for(n, 64), 64, 0, s2>>>(it0, N, b.dblob, b.rs, rss)));
   CUBBS_CHECK(cudaEventRecord(rt.ev_mid, s2));
@@ -1653,6 +1655,20 @@ void run_verify(Runtime &rt, OpBatch &b, uint8_t *dmapdst) {
   }
   b.launches_per_run = (nm ? 1 : 0) + (npts ? 2 : 0) + 7 + (G ? (agg_by_buckets(b) ? 6 : 5) : 0);
 }
+
+template <int S> static void share_carveout_suite() {
+  share_carveout(k_pv_chal_prefix<S>, k_pv_finish<S>, k_sign_prep<S>, k_pg_random<S>, k_pg_early<S>, k_pg_finish<S>);
+}
+}  // namespace
+void share_carveout_bbs() {
+  share_carveout(k_pv_rows, k_pv_jobs, k_pv_pairjobs, k_pv_pairjobs_agg, k_vf_pairjobs_agg, k_agg_prep_pv,
+                 k_agg_prep_vf, k_agg_sort, k_agg_buckets, k_agg_combine, k_agg_ladder, k_agg_sum, k_sign_rows,
+                 k_sign_finish, k_verify_rows, k_verify_jobs, k_verify_finish, k_pg_rows_b, k_pg_rows_t2, k_pg_vars,
+                 k_pg_responses);
+  share_carveout_suite<SUITE_SHA256>();
+  share_carveout_suite<SUITE_SHAKE256>();
+}
+namespace {
 
 // The whole device pipeline of one batch (no host work, no transfers).
 void run(Runtime &rt, OpBatch &b, uint8_t *dmapdst) {

@@ -12,6 +12,7 @@
 #include <cmath>
 #include <cstdlib>
 
+#include "bipartite.cuh"
 #include "g1_ladder.cuh"
 #include "runtime.cuh"
 
@@ -29,6 +30,37 @@ __global__ void __launch_bounds__(128) k_g1_decode(const uint8_t *pts, uint32_t 
     a.x = fp_zero();
     a.y = fp_zero();
   }
+  out[i] = a;
+  status[i] = st;
+}
+
+// The same without the subgroup check, on pairs of warps (bipartite.cuh): lane l
+// of both warps of a block decodes point 32 blockIdx + l.  Bound by the chain of
+// 376 squares and 86 products of one square root; 1 to 3072 points: 0.41 -> 0.26 ms.
+__global__ void __launch_bounds__(64) k_g1_decode_pair(const uint8_t *pts, uint32_t stride, uint32_t n, g1a *out,
+                                                       int32_t *status) {
+  __shared__ __align__(16) bp::Exchange ex;
+  __shared__ __align__(16) bp::Powers pow;
+  const uint32_t lane = threadIdx.x & 31, i = 32 * blockIdx.x + lane;
+  if (n == 0) return;
+  uint8_t b[48];
+  const uint8_t *src = pts + (size_t)min(i, n - 1) * stride;  // spare lanes repeat the last point
+  for (int k = 0; k < 48; k++) b[k] = src[k];
+  g1a a;
+  fp rhs = fp_zero();
+  bool sort;
+  int st = g1_x(b, a.x, rhs, sort);
+  const fp in = C_FP_BP_IN, back = C_FP_BP_OUT;
+  __syncwarp();  // the rounds' barriers want whole warps
+  bp::Pair w{&ex, (int)(threadIdx.x >> 5), (int)lane, 1, 0};
+  const fp root = bp::sqrt_power(w, pow, fp_mul(rhs, in));
+  if (w.half || i >= n) return;
+  if (st == DEC_OK) {
+    a.y = fp_mul(root, back);
+    if (!fp_eq(fp_sqr(a.y), rhs)) st = DEC_BAD;
+    else if (fp_lex_largest(a.y) != sort) a.y = fp_neg(a.y);
+  }
+  if (st != DEC_OK) a.x = a.y = fp_zero();
   out[i] = a;
   status[i] = st;
 }
@@ -288,36 +320,45 @@ __global__ void __launch_bounds__(128) k_g1_compress(const g1 *pts, uint32_t n, 
 }
 
 // Subgroup check of points decoded without it: bad[i] = 1 when point i
-// decoded to an affine point outside G1 (status DEC_OK), else 0.
-__global__ void __launch_bounds__(32) k_g1_subgroup_lane(const g1a *pts, const int32_t *status, uint32_t n,
-                                                          int32_t *bad) {
+// decoded to an affine point outside G1 (status DEC_OK), else 0.  Without
+// `bad` the point itself is marked as not decoded (DEC_BAD, zero coordinates).
+DEV void subgroup_result(g1a *pts, int32_t *status, uint32_t i, int32_t *bad, bool outside) {
+  if (bad) {
+    bad[i] = outside ? 1 : 0;
+  } else if (outside) {
+    status[i] = DEC_BAD;
+    pts[i].x = pts[i].y = fp_zero();
+  }
+}
+__global__ void __launch_bounds__(32) k_g1_subgroup_lane(g1a *pts, int32_t *status, uint32_t n, int32_t *bad) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  bad[i] = (status[i] == DEC_OK && !g1_in_subgroup(pts[i])) ? 1 : 0;
+  subgroup_result(pts, status, i, bad, status[i] == DEC_OK && !g1_in_subgroup(pts[i]));
 }
 // One lane pair per point.
-__global__ void __launch_bounds__(32) k_g1_subgroup(const g1a *pts, const int32_t *status, uint32_t n, int32_t *bad) {
+__global__ void __launch_bounds__(32) k_g1_subgroup(g1a *pts, int32_t *status, uint32_t n, int32_t *bad) {
   const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 1;
   if (i >= n) return;  // both lanes of a pair leave together
   const LanePair lp = LanePair::here();
   const bool outside = status[i] == DEC_OK && !g1_in_subgroup_pair(lp, pts[i]);
-  if (lp.role == 0) bad[i] = outside ? 1 : 0;
+  __syncwarp(lp.mask);  // the other lane has read the point
+  if (lp.role == 0) subgroup_result(pts, status, i, bad, outside);
 }
 // One lane quad per point.
-__global__ void __launch_bounds__(64) k_g1_subgroup_quad(const g1a *pts, const int32_t *status, uint32_t n,
-                                                         int32_t *bad) {
+__global__ void __launch_bounds__(64) k_g1_subgroup_quad(g1a *pts, int32_t *status, uint32_t n, int32_t *bad) {
   const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 2;
   if (i >= n) return;  // the four lanes of a quad leave together
   const LaneQuad lq = LaneQuad::here();
   const bool outside = status[i] == DEC_OK && !g1_in_subgroup_quad(lq, pts[i]);
-  if (lq.role == 0) bad[i] = outside ? 1 : 0;
+  __syncwarp(lq.mask);  // the other lanes have read the point
+  if (lq.role == 0) subgroup_result(pts, status, i, bad, outside);
 }
 
 // One ladder of eight lanes per point (g1_ladder.cuh), four points a warp, one
 // warp a block: phi(P) == -[z^2]P, that is [z^2]P == (beta x, -y).
-__global__ void __launch_bounds__(32) k_g1_subgroup_ladder(const g1a *pts, const int32_t *status, uint32_t n,
-                                                           int32_t *bad) {
+__global__ void __launch_bounds__(32) k_g1_subgroup_ladder(g1a *pts, int32_t *status, uint32_t n, int32_t *bad) {
   __shared__ __align__(16) gl::Mem mem;
+  if (n == 0) return;
   const int lane = threadIdx.x & 31, role = lane & 7;
   const uint32_t i = 4 * blockIdx.x + (lane >> 3), j = min(i, n - 1);
   const bool ok = status[j] == DEC_OK;
@@ -336,7 +377,7 @@ __global__ void __launch_bounds__(32) k_g1_subgroup_ladder(const g1a *pts, const
     fp_csub1(x.w, x.w);
     fp_csub1(y.w, y.w);
     const bool in = !fp_is_zero(Z) && fp_eq(X, fp_mul(fp_mul(x, beta), Z)) && fp_eq(Y, fp_mul(fp_neg(y), Z));
-    bad[i] = ok && !in ? 1 : 0;
+    subgroup_result(pts, status, i, bad, ok && !in);
   }
 }
 
@@ -363,7 +404,7 @@ static int lanes_for(uint32_t n) {
   return l ? l : n <= 2048 ? 8 : 2;
 }
 
-void launch_g1_subgroup(cudaStream_t s, const g1a *pts, const int32_t *status, uint32_t n, int32_t *bad, int lanes) {
+void launch_g1_subgroup(cudaStream_t s, g1a *pts, int32_t *status, uint32_t n, int32_t *bad, int lanes) {
   if (!n) return;
   if (lanes == 0) lanes = lanes_for(n);
   if (lanes == 8) k_g1_subgroup_ladder<<<blocks_for(n, 4), 32, 0, s>>>(pts, status, n, bad);
@@ -373,7 +414,17 @@ void launch_g1_subgroup(cudaStream_t s, const g1a *pts, const int32_t *status, u
 }
 void launch_g1_decode(cudaStream_t s, const uint8_t *pts48, uint32_t stride, uint32_t n, g1a *out, int32_t *status,
                       bool check_subgroup) {
-  if (n) k_g1_decode<<<blocks_for(n, 128), 128, 0, s>>>(pts48, stride, n, out, status, check_subgroup);
+  if (!n) return;
+  // Up to one warp per SM sub-partition (152 x 4, two warps per 32 points) the
+  // launch is bound by one square root's chain, which pairs of warps shorten
+  // (0.41 -> 0.26 ms), with the subgroup check as a launch of its own; beyond
+  // that the one-lane form has fewer multiply-adds a point.
+  if (n > 9728) {
+    k_g1_decode<<<blocks_for(n, 128), 128, 0, s>>>(pts48, stride, n, out, status, check_subgroup);
+    return;
+  }
+  k_g1_decode_pair<<<blocks_for(n, 32), 64, 0, s>>>(pts48, stride, n, out, status);
+  if (check_subgroup) launch_g1_subgroup(s, out, status, n, nullptr);
 }
 void launch_build_table(cudaStream_t s, const g1a *gens, int g0, int g1n, FixedTable t, g1a *bases, g1 *scratch,
                         fp *prod) {
@@ -438,9 +489,19 @@ void launch_var_mul(cudaStream_t s, const g1a *points, const VarJob *jobs, const
   else if (lanes == 2) k_var_mul_pair<<<blocks_for(2 * (size_t)n, 128), 128, 0, s>>>(points, jobs, scalars, n, out);
   else k_var_mul<<<blocks_for(n, 128), 128, 0, s>>>(points, jobs, scalars, n, out);
 }
+void share_carveout_g1() {
+  share_carveout(k_g1_decode, k_g1_decode_pair, k_fixed_msm<128>, k_fixed_msm<512>, k_var_mul, k_var_mul_pair,
+                 k_var_mul_quad, k_var_mul_ladder, k_g1_subgroup_lane, k_g1_subgroup, k_g1_subgroup_quad,
+                 k_g1_subgroup_ladder, k_g1_compress);
+}
 cudaError_t warm_decode_and_var_mul_kernels(uint8_t *any_device_buffer) {
   // n = 0: every thread returns before touching memory
   k_g1_decode<<<1, 128>>>(any_device_buffer, 48, 0, nullptr, nullptr, true);
+  k_g1_decode_pair<<<1, 64>>>(any_device_buffer, 48, 0, nullptr, nullptr);
+  k_g1_subgroup_lane<<<1, 32>>>(nullptr, nullptr, 0, nullptr);
+  k_g1_subgroup<<<1, 32>>>(nullptr, nullptr, 0, nullptr);
+  k_g1_subgroup_quad<<<1, 64>>>(nullptr, nullptr, 0, nullptr);
+  k_g1_subgroup_ladder<<<1, 32>>>(nullptr, nullptr, 0, nullptr);
   k_var_mul<<<1, 128>>>(nullptr, nullptr, nullptr, 0, nullptr);
   k_var_mul_pair<<<1, 128>>>(nullptr, nullptr, nullptr, 0, nullptr);
   k_var_mul_quad<<<1, 128>>>(nullptr, nullptr, nullptr, 0, nullptr);

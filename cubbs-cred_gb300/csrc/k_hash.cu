@@ -164,6 +164,10 @@ void launch_h2s_flat(cudaStream_t s, const uint8_t *msgs, const uint32_t *offs, 
     CUBBS_SUITE_DISPATCH(suite, k_h2s_flat<S><<<blocks_for(n, 128), 128, 0, s>>>(msgs, offs, lens, n, dst, dlen,
                                                                                   out));
 }
+void share_carveout_hash() {
+  share_carveout(k_h2s_flat<SUITE_SHA256>, k_h2s_flat<SUITE_SHAKE256>, k_domain<SUITE_SHA256>,
+                 k_domain<SUITE_SHAKE256>);
+}
 void launch_domain(cudaStream_t s, const DomainJob *jobs, uint32_t n, const uint8_t *blob,
                    const uint8_t *gens_c, const uint8_t *prefixes, fr *out, int suite) {
   if (n)

@@ -119,6 +119,8 @@ static bool wide_pair_teams() {
   return v;
 }
 
+void share_carveout_pairing() { share_carveout(k_pairing_check_team); }
+
 void launch_pairing_check_split(cudaStream_t s, const PairJob *jobs, uint32_t n, const line2 *lines, uint8_t *ok) {
   const size_t smem = 2 * (size_t)PP_SLOTS * sizeof(fp);
   static const bool attr = [smem] {

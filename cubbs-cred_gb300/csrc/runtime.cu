@@ -515,6 +515,10 @@ Runtime::Runtime(SharedState &s)
   CUBBS_CHECK(cudaStreamCreateWithFlags(&stream4, cudaStreamNonBlocking));
   CUBBS_CHECK(cudaEventCreateWithFlags(&ev_sub, cudaEventDisableTiming));
   CUBBS_CHECK(cudaEventCreateWithFlags(&ev_hash, cudaEventDisableTiming));
+  share_carveout_bbs();
+  share_carveout_g1();
+  share_carveout_hash();
+  share_carveout_pairing();
   arena.reserve((size_t)256 << 20);
   staging.reserve((size_t)64 << 20);
   pack.reserve((size_t)64 << 20);

@@ -294,7 +294,8 @@ void launch_build_table(cudaStream_t s, const g1a *gens, int g0, int g1n, FixedT
                         g1 *scratch_xyzz, fp *scratch_prod);
 // decode N compressed G1 points: status DEC_*; affine out
 // lanes per point: 1, 2, 4 or 8 (0: chosen by the point count or CUBBS_BBS_VAR_LANES)
-void launch_g1_subgroup(cudaStream_t s, const g1a *pts, const int32_t *status, uint32_t n, int32_t *bad,
+// bad: 1 for a point outside G1; null: such a point's status becomes DEC_BAD
+void launch_g1_subgroup(cudaStream_t s, g1a *pts, int32_t *status, uint32_t n, int32_t *bad,
                         int lanes = 0);
 int var_lanes_setting();
 void launch_g1_decode(cudaStream_t s, const uint8_t *pts48, uint32_t stride, uint32_t n, g1a *out,
@@ -311,6 +312,21 @@ struct VarJob {
 void launch_var_mul(cudaStream_t s, const g1a *points, const VarJob *jobs, const fr *scalars, uint32_t n,
                     g1 *out, int lanes = 0);
 void launch_g1_compress(cudaStream_t s, const g1 *pts, uint32_t n, uint8_t *out48);
+// One split of L1 and shared memory for the kernels that calls run beside one
+// another: an SM changes its split only when it is idle, so a kernel that wants
+// another one waits for the SMs it meets to drain, which made calls of the same
+// batch differ by up to 0.5 ms (Verify of 1000: 2.5 or 3.0 ms, now 2.5).  Half
+// of the memory holds every block that fits by its registers; a quarter does
+// not (Sign of 4096: 1.97 -> 2.36 ms), and all of it leaves the point kernels'
+// local arrays less L1 (ProofGen of 1024: 3.66 -> 3.76 ms).
+template <typename... K> inline void share_carveout(K *...kernel) {
+  for (const void *k : {reinterpret_cast<const void *>(kernel)...})
+    CUBBS_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributePreferredSharedMemoryCarveout, 50));
+}
+void share_carveout_bbs();
+void share_carveout_g1();
+void share_carveout_hash();
+void share_carveout_pairing();
 // Launches k_g1_decode and every variable-base kernel over zero items on the
 // legacy default stream of the current device (module load and local-memory
 // sizing ahead of real work; nothing is read or written).

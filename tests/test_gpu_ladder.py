@@ -56,3 +56,23 @@ def test_fixed_rows(gpu, oracle, rows):
     assert all(c == 0 for c, _, _ in got)
     for i in sorted({0, 1, 2, 7, 8, 15, 16, 31, 32, 98, rows // 2, rows - 2, rows - 1} & set(range(rows))):
         assert got[i][2] == oracle.g1_msm(pts, scalars[i]), i
+
+
+@pytest.mark.parametrize("n", [1, 31, 33, 70])
+def test_decode_pairs(gpu, oracle, n):
+    """Points decoded on pairs of warps, spare lanes in the last block: both signs, the identity, an x off the curve, an
+    x that is not reduced, bad flag bits, and points outside G1, through the checked MSM decode."""
+    p1, gens = oracle.generators(4)
+    neg = [bytes([p[0] ^ 0x20]) + p[1:] for p in (p1, gens[0])]
+    off = next(bytes([0x80]) + x.to_bytes(47, "big") for x in range(1, 99)
+               if pow(x ** 3 + 4, (oracle.P_MOD - 1) // 2, oracle.P_MOD) != 1)
+    big = bytearray((oracle.P_MOD + 1).to_bytes(48, "big"))
+    big[0] |= 0x80
+    kinds = [(p1, 0), (neg[0], 0), (off, 1), (gens[1], 0), (INF, 0), (bytes(big), 1), (neg[1], 0),
+             (bytes([p1[0] & 0x7F]) + p1[1:], 1), (_on_curve_outside_g1(oracle, b"pairs"), 1),
+             (bytes([0xE0]) + bytes(47), 1), (bytes([0x80]) + bytes(47), 1)]
+    one = (1).to_bytes(32, "big")
+    want = [(p if not bad else None) for p, bad in (kinds[i % len(kinds)] for i in range(n))]
+    got = gpu.g1_msm_batch([([kinds[i % len(kinds)][0]], [one]) for i in range(n)])
+    assert [c for c, _ in got] == [0 if w is not None else 1 for w in want]
+    assert [p for (_, p), w in zip(got, want) if w is not None] == [w for w in want if w is not None]
