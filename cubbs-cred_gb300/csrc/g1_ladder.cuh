@@ -285,6 +285,17 @@ DEV void mul_z2(const Ladders &l) {
   }
 }
 
+// The accumulator, taken back from E' as an XYZZ point, by the ladder's lanes
+// 0 and 1: (X Z, s^2 Z^2) and (Y Z^2, s^3 Z^3).
+DEV void leave(const fp *sl, int role, fp v[2]) {
+  const fp s2 = C_B3_S2, s3 = C_B3_S3;
+  const fp z = sl[AZ];
+  fp zz = z;
+  if (role == 1) zz = fp_mul(z, z);
+  v[0] = fp_mul(sl[AX + role], zz);
+  v[1] = fp_mul(fp_mul(zz, z), role ? s3 : s2);
+}
+
 // ---- sums of many points
 // Projective triples (X, Y, Z) in shared memory, added in place by the lane
 // octets of a warp: a level of a tree sum is one complete addition of two

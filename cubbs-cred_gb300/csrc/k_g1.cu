@@ -281,13 +281,8 @@ __global__ void __launch_bounds__(32) k_var_mul_ladder(const g1a *points, const 
     if (!half && role < 3) sl[gl::TAB + (role == 2 ? 3 : role)] = mem.slot[(lane >> 3) + 1][gl::AX + role];
   });
   if (!half && role < 2) {
-    const fp s2 = C_B3_S2, s3 = C_B3_S3;
-    fp v[2];  // (X Z, s^2 Z^2) or (Y Z^2, s^3 Z^3)
-    const fp z = sl[gl::AZ];
-    fp zz = z;
-    if (role == 1) zz = fp_mul(z, z);
-    v[0] = fp_mul(sl[gl::AX + role], zz);
-    v[1] = fp_mul(fp_mul(zz, z), role ? s3 : s2);
+    fp v[2];
+    gl::leave(sl, role, v);
     if (i < n) {
       if (inf) {
         const g1 o = g1_inf();

@@ -20,7 +20,10 @@
 // launch.  A second kernel sums the partials of each MSM (one warp per MSM)
 // and compresses the result.  Mode, chunk length t and window c are chosen
 // per size class of K by an autotuner (t >= K: one lane per MSM; t < K: the
-// MSM is spread over several lanes and joined by the reduction).  The
+// MSM is spread over several lanes and joined by the reduction).  While the
+// settings are the initial ones and no pairing checks share the launch, the
+// MSMs are split over lanes by window and chunk instead (k_msm_windows), which
+// is faster at every size measured.  The
 // general MSM entry point replays the engine's kernels from captured CUDA
 // graphs (k_prims.cu).
 //
@@ -31,6 +34,7 @@
 #include <cstring>
 #include <vector>
 
+#include "g1_ladder.cuh"
 #include "pairing_team.cuh"
 #include "runtime.cuh"
 
@@ -41,7 +45,7 @@ namespace cubbs {
 // Per term: phi(P) and the offset forms k' = k + M of the two 128-bit GLV
 // halves for the window width c of the term's MSM (5 words each; with
 // nwin = ceil(130 / c) windows, k' < 2^(nwin c) <= 2^136).  An identity
-// point gets all-zero offset forms, which the chunk kernel skips.
+// point gets the forms of zero, all of whose digits are zero.
 __global__ void __launch_bounds__(128) k_msm_prep(const g1a *pts, const VarJob *jobs,
                                                   const fr *scalars, const uint8_t *term_c, uint32_t n, g1a *phi,
                                                   uint32_t *koff) {
@@ -49,18 +53,16 @@ __global__ void __launch_bounds__(128) k_msm_prep(const g1a *pts, const VarJob *
   if (j >= n) return;
   uint32_t *o = koff + 10 * (size_t)j;
   const VarJob jb = jobs[j];
-  if (jb.flags & 1) {  // identity point: the term contributes nothing
-    for (int k = 0; k < 10; k++) o[k] = 0;
-    return;
+  uint32_t s[4] = {0, 0, 0, 0}, q[4] = {0, 0, 0, 0};  // an identity point contributes nothing
+  if (!(jb.flags & 1)) {
+    const g1a p = pts[jb.point];
+    const fp beta = C_GLV_BETA;
+    g1a f;
+    f.x = fp_mul(p.x, beta);
+    f.y = fp_neg(p.y);
+    phi[j] = f;
+    glv_split(scalars[j], s, q);
   }
-  const g1a p = pts[jb.point];
-  const fp beta = C_GLV_BETA;
-  g1a f;
-  f.x = fp_mul(p.x, beta);
-  f.y = fp_neg(p.y);
-  phi[j] = f;
-  uint32_t s[4], q[4];
-  glv_split(scalars[j], s, q);
   const int c = term_c[j];
   // M = sum_{w < nwin} 2^(c-1) 2^(wc); nwin c >= 130 keeps k + M below 2^(nwin c)
   uint32_t m[5] = {0, 0, 0, 0, 0};
@@ -394,7 +396,184 @@ __global__ void __launch_bounds__(128) k_msm_reduce(const g1 *partials, const ui
   }
 }
 
+// ---------------------------------------------------------------- split windows
+// Without settings of the caller's own, an MSM is split over lanes by window as
+// well as by chunk: a lane takes one window of one chunk, so it doubles nothing,
+// and a batch of a thousand MSMs has tens of thousands of lanes (thread mode:
+// 4700, a quarter of the GPU's sub-partitions with one warp each).  The lanes of
+// a warp are neighbouring windows of the same chunk: they read the same points.
+// A lane sorts its digits by magnitude, largest first, and adds the points in
+// that order into one sum; its value where a magnitude b begins is S_b, and the
+// window's sum is that of the S_b.  Every lane then has the same mixed
+// additions to do in the same loop, and writes a bucket once instead of reading
+// and writing one at each addition (5.3 ms for 1024 MSMs of 2 to 257 terms: the
+// buckets of the resident lanes exceed L2).  What bounds it: the products, ten
+// for each nonzero digit and 14 a bucket.  The windows' sums are joined per MSM
+// by a ladder of eight lanes (g1_ladder.cuh).
+// Measured, all kernels after the decode, against the best settings of the
+// persistent engine: 32 MSMs of 8 terms 10.2 -> 0.70 ms; 1024 of 8 to 16
+// 13.8 -> 1.11; 1024 of 2 to 257 16.9 -> 4.08; 16384 of 2 to 257 84 -> 47.6 (two
+// thirds of what the products take at the full rate for this kernel alone).
+constexpr uint32_t msm_windows(uint32_t c) { return (130 + c - 1) / c; }
+#define MSM_SPLIT_T_MAX 120  // terms of a chunk: its half-terms' indices fit eight bits
+// bytes 0 .. 15 of a lane's counters
+struct Bytes16 {
+  uint64_t lo = 0, hi = 0;
+  DEV uint32_t get(int b) const { return (uint32_t)((b < 8 ? lo : hi) >> (8 * (b & 7))) & 0xff; }
+  DEV void add(int b, uint32_t v) {
+    const uint64_t x = (uint64_t)v << (8 * (b & 7));
+    if (b < 8) lo += x;
+    else hi += x;
+  }
+};
+template <int C>
+__global__ void __launch_bounds__(64) k_msm_windows(const g1a *pts, const VarJob *jobs, const g1a *phi,
+                                                    const uint32_t *koff, const MsmChunk *chunks, uint32_t nchunks,
+                                                    g1 *partials) {
+  constexpr uint32_t NWIN = (130 + C - 1) / C;
+  constexpr int NB = 1 << (C - 1);
+  static_assert(NB <= 16, "Bytes16");
+  const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x, ci = e / NWIN, w = e - ci * NWIN;
+  if (ci >= nchunks) return;
+  const MsmChunk ch = chunks[ci];
+  const uint32_t *k5 = koff + 10 * (size_t)ch.first;
+  const uint32_t halves = 2 * ch.count;
+  // counting sort: (half-term, bucket, sign) of every nonzero digit
+  Bytes16 cnt, pos;
+  uint16_t order[2 * MSM_SPLIT_T_MAX];
+#pragma unroll 1
+  for (uint32_t h = 0; h < halves; h++) {
+    const int d = msm_digit(k5 + 5 * h, (int)w, C);
+    if (d) cnt.add((d < 0 ? -d : d) - 1, 1);
+  }
+  uint32_t m = 0;
+#pragma unroll 1
+  for (int b = NB - 1; b >= 0; b--) {
+    pos.add(b, m);
+    m += cnt.get(b);
+  }
+#pragma unroll 1
+  for (uint32_t h = 0; h < halves; h++) {
+    const int d = msm_digit(k5 + 5 * h, (int)w, C);
+    if (!d) continue;
+    const int b = (d < 0 ? -d : d) - 1;
+    order[pos.get(b)] = (uint16_t)(h | b << 8 | (d < 0 ? 0x1000 : 0));
+    pos.add(b, 1);
+  }
+  g1 S[NB], run = g1_inf();
+  g1a next;
+  auto fetch = [&](uint32_t k) {
+    if (k >= m) return;
+    const uint32_t o = order[k], j = ch.first + ((o & 0xff) >> 1);
+    next = (o & 1) ? phi[j] : pts[jobs[j].point];
+    if (o & 0x1000) next.y = fp_neg(next.y);
+  };
+  fetch(0);
+  int cur = NB - 1;
+#pragma unroll 1
+  for (uint32_t k = 0; k < m; k++) {
+    const g1a p = next;
+    const int b = (order[k] >> 8) & 15;
+#pragma unroll 1
+    for (; cur > b; cur--) S[cur] = run;
+    fetch(k + 1);
+    run = g1_add_aff_inl(run, p);
+  }
+#pragma unroll 1
+  for (; cur > 0; cur--) S[cur] = run;
+#pragma unroll 1
+  for (int b = 1; b < NB; b++) run = g1_add_inl(run, S[b]);
+  partials[(size_t)ch.slot * NWIN + w] = run;
+}
+
+// A lane per window of an MSM: the chunks' partials added, as a projective
+// triple on the ladders' curve.
+__global__ void __launch_bounds__(64) k_msm_join(const uint32_t *pstart, uint32_t n, uint32_t nwin, const g1 *partials,
+                                                 fp *triples) {
+  const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x, i = e / nwin, w = e - i * nwin;
+  if (i >= n) return;
+  g1 acc = g1_inf();
+#pragma unroll 1
+  for (uint32_t k = pstart[i]; k < pstart[i + 1]; k++) acc = g1_add_inl(acc, partials[(size_t)k * nwin + w]);
+  const fp s2 = C_B3_S2, s3 = C_B3_S3;
+  fp t[3];
+  gl::put_triple(t, acc);
+  fp *o = triples + 3 * (size_t)e;
+  o[0] = fp_mul(t[0], s2);
+  o[1] = fp_mul(t[1], s3);
+  o[2] = t[2];
+}
+
+// sum_w 2^(c w) W_w: a ladder of eight lanes per MSM, four a warp.
+__global__ void __launch_bounds__(32) k_msm_horner(const fp *triples, uint32_t n, uint32_t nwin, uint32_t c, g1 *out) {
+  __shared__ __align__(16) gl::Mem mem;
+  const int lane = threadIdx.x & 31, role = lane & 7;
+  const uint32_t i = 4 * blockIdx.x + (lane >> 3);
+  const fp *t = triples + 3 * (size_t)min(i, n - 1) * nwin;  // a warp's spare ladders repeat the last MSM
+  g1a any;
+  any.x = any.y = fp_one();
+  const gl::Ladders l = gl::start(&mem, any, false);
+  fp *sl = l.sl;
+  if (role < 3) sl[gl::AX + role] = t[3 * (nwin - 1) + role];
+  __syncwarp();
+#pragma unroll 1
+  for (int w = (int)nwin - 2, k = 0; w >= 0;) {
+    const bool doubling = k < (int)c;
+    if (!doubling) {
+      if (role < 3) sl[gl::TAB + (role == 2 ? 3 : role)] = t[3 * w + role];
+      __syncwarp();
+      w--;
+    }
+    k = doubling ? k + 1 : 0;
+    l.step(doubling, 1);
+  }
+  if (role < 2 && i < n) {
+    fp v[2];
+    gl::leave(sl, role, v);
+    (role ? out[i].Y : out[i].X) = v[0];
+    (role ? out[i].ZZZ : out[i].ZZ) = v[1];
+  }
+}
+
 // ------------------------------------------------------------------ host plan
+// Window and chunk length of a batch in split windows: the least of what the
+// products take when every sub-partition has several warps (1215 cycles a
+// product, field.cuh) plus half of the longest lane, which runs alone at the
+// end (1816), over windows 3 .. 5 and chunks of 8 .. 120 terms.
+void MsmPlan::build_split(const std::vector<uint32_t> &K) {
+  const size_t n = K.size();
+  uint32_t longest = 0, best_t = 0;
+  for (uint32_t k : K) longest = std::max(longest, k);
+  double best = 0;
+  for (uint32_t t : {8u, 16u, 32u, 64u, (uint32_t)MSM_SPLIT_T_MAX}) {
+    double parts = 0;
+    for (uint32_t k : K) parts += (k + t - 1) / t;
+    for (uint32_t c = 3; c <= 5; c++) {
+      const double digit = 20 * (1 - 1.0 / (1u << c)), fold = 14.0 * ((1u << (c - 1)) - 1);
+      const double lane = digit * std::min(t, longest) + fold, join = 14.0 * ((longest + t - 1) / t);
+      const double all = (digit * terms + fold * parts) * msm_windows(c) * 1215 / (128.0 * sms);
+      const double cost = std::max(all + 0.5 * 1816 * lane, 1816 * lane) + 1816 * join;
+      if (best_t == 0 || cost < best) {
+        best = cost;
+        best_t = t;
+        split_c = c;
+      }
+    }
+  }
+  std::fill(term_c.begin(), term_c.end(), (uint8_t)split_c);
+  for (size_t i = 0; i < n; i++) {
+    const uint32_t nch = (K[i] + best_t - 1) / best_t;
+    pstart[i + 1] = pstart[i] + nch;
+    for (uint32_t k = 0; k < nch; k++) {  // chunks of equal length, give or take one
+      const uint32_t a = (uint32_t)((uint64_t)K[i] * k / nch), b = (uint32_t)((uint64_t)K[i] * (k + 1) / nch);
+      chunks.push_back({start[i] + a, b - a, pstart[i] + k, 0});
+    }
+  }
+  // longest first: the last lanes to run are the shortest
+  std::stable_sort(chunks.begin(), chunks.end(), [](const MsmChunk &a, const MsmChunk &b) { return a.count > b.count; });
+  nparts = pstart[n] * msm_windows(split_c);
+}
+
 int msm_size_class(uint32_t K) { return K <= 8 ? 0 : K <= 32 ? 1 : K <= 96 ? 2 : 3; }
 
 void MsmPlan::build(const std::vector<uint32_t> &K, const MsmTuning &tune, uint32_t pairings) {
@@ -409,6 +588,11 @@ void MsmPlan::build(const std::vector<uint32_t> &K, const MsmTuning &tune, uint3
   pair_units = pairings;
   units.clear();
   chunks.clear();
+  split_c = 0;
+  if (pairings == 0 && tune == MsmTuning()) {
+    build_split(K);
+    return;
+  }
   // pairing checks first: each takes a warp for milliseconds, so they must
   // not be the launch's tail
   for (uint32_t k = 0; k < pairings; k++) units.push_back({MSM_UNIT_PAIR << 8, k});
@@ -462,6 +646,11 @@ namespace {
 // occupancy the device reports.
 void engine_shape(const MsmPlan &p, int sm_count, uint32_t &wpb, uint32_t &smem_per_warp, uint32_t &grid,
                   uint32_t &gstride) {
+  if (p.split_c) {
+    wpb = grid = 1;
+    smem_per_warp = gstride = 0;
+    return;
+  }
   // A warp unit keeps its buckets in shared memory when its window is at most
   // MSM_WARP_SMEM_C_MAX, in its warp's slot of the global buckets otherwise;
   // one plan may hold both kinds (windows differ between size classes).
@@ -515,13 +704,20 @@ void MsmDevice::upload(Runtime &rt, const MsmPlan &p, cudaStream_t s) {
   partials = rt.arena.alloc<g1>(p.nparts ? p.nparts : 1);
   counter = rt.arena.alloc<uint32_t>(2);  // [0] next unit, [1] units skipped for want of room
   engine_shape(p, rt.sm_count, warps_per_block, smem_per_warp, grid, gbucket_stride);
+  split_c = p.split_c;
+  if (split_c) {
+    triples = rt.arena.alloc<fp>(3 * (size_t)n * msm_windows(split_c));
+    sums = rt.arena.alloc<g1>(n ? n : 1);
+  }
   gbuckets = gbucket_stride ? rt.arena.alloc<g1>((size_t)grid * warps_per_block * gbucket_stride) : nullptr;
 }
 
 size_t MsmDevice::arena_bytes(const MsmPlan &p, int sm_count) {
   uint32_t wpb, per, grid, gstride;
   engine_shape(p, sm_count, wpb, per, grid, gstride);
-  const size_t g = (size_t)grid * wpb * gstride * sizeof(g1) + 256;
+  const size_t n = p.pstart.size() - 1;
+  const size_t g = (size_t)grid * wpb * gstride * sizeof(g1) + 256 +
+                   (p.split_c ? n * (3 * sizeof(fp) * msm_windows(p.split_c) + sizeof(g1)) + 512 : 0);
   return p.term_c.size() + p.chunks.size() * sizeof(MsmChunk) + p.units.size() * sizeof(MsmUnit) +
          p.pstart.size() * 4 + p.start.size() * 4 + (size_t)p.terms * (sizeof(g1a) + 40) +
          (size_t)p.nparts * sizeof(g1) + g + 10 * 256;
@@ -536,6 +732,21 @@ void launch_msm_main(cudaStream_t s, const MsmDevice &d, const g1a *pts, const V
                      uint8_t *out48) {
   (void)sm_count;
   CUBBS_CHECK(cudaMemsetAsync(d.counter, 0, 8, s));
+  if (d.split_c) {
+    const uint32_t nwin = msm_windows(d.split_c);
+    const unsigned blocks = blocks_for((size_t)d.nchunks * nwin, 64);
+    if (d.nchunks) {
+      if (d.split_c == 3) k_msm_windows<3><<<blocks, 64, 0, s>>>(pts, jobs, d.phi, d.koff, d.chunks, d.nchunks, d.partials);
+      else if (d.split_c == 4) k_msm_windows<4><<<blocks, 64, 0, s>>>(pts, jobs, d.phi, d.koff, d.chunks, d.nchunks, d.partials);
+      else k_msm_windows<5><<<blocks, 64, 0, s>>>(pts, jobs, d.phi, d.koff, d.chunks, d.nchunks, d.partials);
+    }
+    if (!d.n) return;
+    g1 *sums = out ? out : d.sums;
+    k_msm_join<<<blocks_for((size_t)d.n * nwin, 64), 64, 0, s>>>(d.pstart, d.n, nwin, d.partials, d.triples);
+    k_msm_horner<<<blocks_for(d.n, 4), 32, 0, s>>>(d.triples, d.n, nwin, d.split_c, sums);
+    if (out48) launch_g1_compress(s, sums, d.n, out48);
+    return;
+  }
   if (d.nunits) {
     EngineArgs a{pts, jobs, d.phi, d.koff, d.chunks, d.nchunks, d.units, d.nunits, d.start, d.counter, d.partials,
                  d.pstart, d.gbuckets, d.gbucket_stride, d.smem_per_warp, d.pjobs, d.lines, d.pok};
@@ -721,9 +932,11 @@ extern "C" int32_t cubbs_bbs_gpu_msm_uneven_bench_v2(uint32_t abi, size_t n_msms
       }
       widest.build(std::vector<uint32_t>(1, 2), t);
     }
+    MsmPlan split;  // and for split windows, of this workload or of the tuner's sample
+    split.build(K, MsmTuning());
     rt.arena.reserve(terms * (sizeof(fr) + 2 * sizeof(g1a) + sizeof(VarJob) + 48 + 4 + 40 + sizeof(g1)) +
                      n_msms * (sizeof(g1) * 4 + 64) + ((size_t)64 << 20) +
-                     MsmDevice::arena_bytes(widest, rt.sm_count));
+                     MsmDevice::arena_bytes(widest, rt.sm_count) + 2 * MsmDevice::arena_bytes(split, rt.sm_count));
     rt.staging.reserve(((size_t)64 << 20) + n_msms * 64 + terms * 8);
     cudaEvent_t e0, e1;
     CUBBS_CHECK(cudaEventCreate(&e0));

@@ -219,10 +219,10 @@ void run_engine_graph(Runtime &rt, cudaStream_t s, const MsmPlan &mp, MsmDevice 
   for (uint32_t v : mp.start) mix(v);
   for (uint32_t v : mp.pstart) mix(v);
   const void *ptrs[] = {pts, djobs, vsc, dout, md.term_c, md.chunks, md.units, md.pstart, md.start, md.koff,
-                        md.counter, md.phi, md.partials, md.gbuckets, md.pjobs, md.lines, md.pok};
+                        md.counter, md.phi, md.partials, md.gbuckets, md.pjobs, md.lines, md.pok, md.triples, md.sums};
   for (const void *q : ptrs) mix((uint64_t)(uintptr_t)q);
   mix((uint64_t)md.grid << 32 | md.warps_per_block);
-  mix(md.smem_per_warp);
+  mix((uint64_t)md.split_c << 32 | md.smem_per_warp);
   auto it = rt.msm_graphs.find(key);
   if (it == rt.msm_graphs.end()) {
     if (rt.msm_graphs.size() >= 32) {

@@ -97,6 +97,10 @@ struct MsmTuning {
   uint32_t chunk[MSM_CLASSES] = {8, 16, 32, 32};
   uint32_t window[MSM_CLASSES] = {4, 4, 4, 4};
   uint32_t mode[MSM_CLASSES] = {MSM_MODE_THREAD, MSM_MODE_THREAD, MSM_MODE_THREAD, MSM_MODE_THREAD};
+  bool operator==(const MsmTuning &o) const {
+    return std::equal(chunk, chunk + MSM_CLASSES, o.chunk) && std::equal(window, window + MSM_CLASSES, o.window) &&
+           std::equal(mode, mode + MSM_CLASSES, o.mode);
+  }
 };
 struct MsmChunk {
   uint32_t first, count;  // term range
@@ -122,6 +126,9 @@ struct MsmPlan {
   uint32_t max_warp_c = 0;        // widest warp-mode window (0: no warp units)
   uint32_t max_warp_smem_c = 0;   // widest warp-mode window with buckets in shared memory (0: none)
   uint32_t pair_units = 0;
+  uint32_t split_c = 0;           // split windows of this width (k_msm_windows); 0: the persistent engine
+  uint32_t sms = 152;             // of the device the plan is for
+  void build_split(const std::vector<uint32_t> &K);
   void build(const std::vector<uint32_t> &K, const MsmTuning &tune, uint32_t pairings = 0);
 };
 // Prepared state of one ciphersuite (the generators and everything built on
@@ -342,6 +349,9 @@ struct MsmDevice {
   g1 *partials = nullptr;
   g1 *gbuckets = nullptr;  // global buckets of warp units whose window exceeds MSM_WARP_SMEM_C_MAX
   uint32_t warps_per_block = 4, smem_per_warp = 0, grid = 0, gbucket_stride = 0;
+  uint32_t split_c = 0;
+  fp *triples = nullptr;  // split windows: the windows' sums,
+  g1 *sums = nullptr;     // the MSMs' results
   // pairing units: e(pa, Q_slot_a) e(pb, Q_slot_b) == 1 for pjobs[0 .. pair_units)
   const PairJob *pjobs = nullptr;
   const line2 *lines = nullptr;
