@@ -236,14 +236,59 @@ DEV g1 g1_mul_zabs(g1 p) {
   }
   return acc;
 }
-// G1 membership for a curve point: phi(P) == -[z^2]P  <=>  [z^2]P == (beta x, -y)
+// Jacobian coordinates (x = X / Z^2, y = Y / Z^3, Z == 0 is infinity; EFD
+// formulas dbl-2009-l, add-1998-cmo-2) for chains of doublings on one lane: two
+// products and five squares a doubling, against six and three in XYZZ.
+struct g1j { fp X, Y, Z; };
+DEV g1j g1j_dbl(const g1j &p) {
+  const fp A = fp_sqr(p.X), B = fp_sqr(p.Y), C = fp_sqr(B);
+  const fp D = fp_dbl(fp_sub(fp_sub(fp_sqr(fp_add(p.X, B)), A), C));
+  const fp E = fp_add(fp_dbl(A), A);
+  g1j r;
+  r.Z = fp_dbl(fp_mul(p.Y, p.Z));
+  r.X = fp_sub(fp_sqr(E), fp_dbl(D));
+  r.Y = fp_sub(fp_mul(E, fp_sub(D, r.X)), fp_dbl(fp_dbl(fp_dbl(C))));
+  return r;
+}
+DEVNI g1j g1j_add(g1j p, g1j q) {
+  if (fp_is_zero(p.Z)) return q;
+  if (fp_is_zero(q.Z)) return p;
+  const fp Z1 = fp_sqr(p.Z), Z2 = fp_sqr(q.Z);
+  const fp U1 = fp_mul(p.X, Z2), S1 = fp_mul(fp_mul(p.Y, Z2), q.Z);
+  const fp H = fp_sub(fp_mul(q.X, Z1), U1), R = fp_sub(fp_mul(fp_mul(q.Y, Z1), p.Z), S1);
+  g1j r;
+  if (fp_is_zero(H)) {
+    if (fp_is_zero(R)) return g1j_dbl(p);
+    r.X = r.Y = fp_one();
+    r.Z = fp_zero();
+    return r;
+  }
+  const fp HH = fp_sqr(H), HHH = fp_mul(H, HH), V = fp_mul(U1, HH);
+  r.X = fp_sub(fp_sub(fp_sqr(R), HHH), fp_dbl(V));
+  r.Y = fp_sub(fp_mul(R, fp_sub(V, r.X)), fp_mul(S1, HHH));
+  r.Z = fp_mul(fp_mul(p.Z, q.Z), H);
+  return r;
+}
+// G1 membership for a curve point: phi(P) == -[z^2]P  <=>  [z^2]P == (beta x, -y).
+// base: room for the chain's base point, kept out of registers.
+DEV bool g1_in_subgroup(g1a a, g1j *base) {
+  g1j t;
+  t.X = a.x;
+  t.Y = a.y;
+  t.Z = fp_one();
+  #pragma unroll 1
+  for (int i = 125; i >= 0; i--) {  // [|z|] twice: bits 62 .. 0 below the leading one
+    if (i == 125 || i == 62) *base = t;
+    t = g1j_dbl(t);
+    if (zabs_bit(i > 62 ? i - 63 : i)) t = g1j_add(t, *base);
+  }
+  if (fp_is_zero(t.Z)) return false;
+  const fp beta = C_GLV_BETA, zz = fp_sqr(t.Z);
+  return fp_eq(t.X, fp_mul(fp_mul(a.x, beta), zz)) && fp_eq(t.Y, fp_mul(fp_neg(a.y), fp_mul(zz, t.Z)));
+}
 DEV bool g1_in_subgroup(g1a a) {
-  g1 t = g1_mul_zabs(g1_mul_zabs(g1_from_aff(a)));
-  if (g1_is_inf(t)) return false;
-  const fp beta = C_GLV_BETA;
-  fp bx = fp_mul(a.x, beta);
-  fp ny = fp_neg(a.y);
-  return fp_eq(t.X, fp_mul(bx, t.ZZ)) && fp_eq(t.Y, fp_mul(ny, t.ZZZ));
+  g1j base;
+  return g1_in_subgroup(a, &base);
 }
 
 // ---- point arithmetic on a lane pair

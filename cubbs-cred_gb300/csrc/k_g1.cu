@@ -18,14 +18,14 @@
 
 namespace cubbs {
 
-__global__ void __launch_bounds__(128) k_g1_decode(const uint8_t *pts, uint32_t stride, uint32_t n, g1a *out,
-                                                   int32_t *status, bool check_subgroup) {
+__global__ void __launch_bounds__(64) k_g1_decode(const uint8_t *pts, uint32_t stride, uint32_t n, g1a *out,
+                                                   int32_t *status) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   uint8_t b[48];
   for (int k = 0; k < 48; k++) b[k] = pts[(size_t)i * stride + k];
   g1a a;
-  int st = g1_decompress(b, a, check_subgroup);
+  int st = g1_decompress(b, a, false);
   if (st != DEC_OK) {
     a.x = fp_zero();
     a.y = fp_zero();
@@ -34,8 +34,7 @@ __global__ void __launch_bounds__(128) k_g1_decode(const uint8_t *pts, uint32_t 
   status[i] = st;
 }
 
-// The same without the subgroup check, on pairs of warps (bipartite.cuh): lane l
-// of both warps of a block decodes point 32 blockIdx + l.  Bound by the chain of
+// The same on pairs of warps (bipartite.cuh): lane l of both warps of a block decodes point 32 blockIdx + l.  Bound by the chain of
 // 376 squares and 86 products of one square root; 1 to 3072 points: 0.41 -> 0.26 ms.
 __global__ void __launch_bounds__(64) k_g1_decode_pair(const uint8_t *pts, uint32_t stride, uint32_t n, g1a *out,
                                                        int32_t *status) {
@@ -325,10 +324,16 @@ DEV void subgroup_result(g1a *pts, int32_t *status, uint32_t i, int32_t *bad, bo
     pts[i].x = pts[i].y = fp_zero();
   }
 }
-__global__ void __launch_bounds__(32) k_g1_subgroup_lane(g1a *pts, int32_t *status, uint32_t n, int32_t *bad) {
+// One lane per point: for launches that fill every SM sub-partition several
+// times.  Bound by the products (126 doublings of two products and five
+// squares); the base point waits in shared memory so that ten warps fit an SM
+// (133 thousand points beside other kernels: 5.3 -> 4.7 ms; twelve or sixteen
+// spill: 4.9, 5.0).
+__global__ void __launch_bounds__(32, 10) k_g1_subgroup_lane(g1a *pts, int32_t *status, uint32_t n, int32_t *bad) {
+  __shared__ g1j base[32];
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  subgroup_result(pts, status, i, bad, status[i] == DEC_OK && !g1_in_subgroup(pts[i]));
+  subgroup_result(pts, status, i, bad, status[i] == DEC_OK && !g1_in_subgroup(pts[i], &base[threadIdx.x]));
 }
 // One lane pair per point.
 __global__ void __launch_bounds__(32) k_g1_subgroup(g1a *pts, int32_t *status, uint32_t n, int32_t *bad) {
@@ -401,7 +406,9 @@ static int lanes_for(uint32_t n) {
 
 void launch_g1_subgroup(cudaStream_t s, g1a *pts, int32_t *status, uint32_t n, int32_t *bad, int lanes) {
   if (!n) return;
-  if (lanes == 0) lanes = lanes_for(n);
+  // Above one warp per SM sub-partition (152 x 4) of points, one lane each: the
+  // Jacobian doublings there cost seven products' time, the pair's ten.
+  if (lanes == 0) lanes = n > 19456 && !var_lanes_setting() ? 1 : lanes_for(n);
   if (lanes == 8) k_g1_subgroup_ladder<<<blocks_for(n, 4), 32, 0, s>>>(pts, status, n, bad);
   else if (lanes == 4) k_g1_subgroup_quad<<<blocks_for(4 * (size_t)n, 64), 64, 0, s>>>(pts, status, n, bad);
   else if (lanes == 2) k_g1_subgroup<<<blocks_for(2 * (size_t)n, 32), 32, 0, s>>>(pts, status, n, bad);
@@ -412,13 +419,10 @@ void launch_g1_decode(cudaStream_t s, const uint8_t *pts48, uint32_t stride, uin
   if (!n) return;
   // Up to one warp per SM sub-partition (152 x 4, two warps per 32 points) the
   // launch is bound by one square root's chain, which pairs of warps shorten
-  // (0.41 -> 0.26 ms), with the subgroup check as a launch of its own; beyond
-  // that the one-lane form has fewer multiply-adds a point.
-  if (n > 9728) {
-    k_g1_decode<<<blocks_for(n, 128), 128, 0, s>>>(pts48, stride, n, out, status, check_subgroup);
-    return;
-  }
-  k_g1_decode_pair<<<blocks_for(n, 32), 64, 0, s>>>(pts48, stride, n, out, status);
+  // (0.41 -> 0.26 ms); beyond that the one-lane form has fewer multiply-adds a
+  // point.
+  if (n > 9728) k_g1_decode<<<blocks_for(n, 64), 64, 0, s>>>(pts48, stride, n, out, status);
+  else k_g1_decode_pair<<<blocks_for(n, 32), 64, 0, s>>>(pts48, stride, n, out, status);
   if (check_subgroup) launch_g1_subgroup(s, out, status, n, nullptr);
 }
 void launch_build_table(cudaStream_t s, const g1a *gens, int g0, int g1n, FixedTable t, g1a *bases, g1 *scratch,
@@ -491,7 +495,7 @@ void share_carveout_g1() {
 }
 cudaError_t warm_decode_and_var_mul_kernels(uint8_t *any_device_buffer) {
   // n = 0: every thread returns before touching memory
-  k_g1_decode<<<1, 128>>>(any_device_buffer, 48, 0, nullptr, nullptr, true);
+  k_g1_decode<<<1, 64>>>(any_device_buffer, 48, 0, nullptr, nullptr);
   k_g1_decode_pair<<<1, 64>>>(any_device_buffer, 48, 0, nullptr, nullptr);
   k_g1_subgroup_lane<<<1, 32>>>(nullptr, nullptr, 0, nullptr);
   k_g1_subgroup<<<1, 32>>>(nullptr, nullptr, 0, nullptr);

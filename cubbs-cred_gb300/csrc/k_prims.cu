@@ -61,6 +61,40 @@ __global__ void __launch_bounds__(128) k_row_sum(const g1 *fixed, const g1 *var,
   if (lane == 0) out[row] = fixed ? g1_add(acc, fixed[row]) : acc;
 }
 
+// a variable-base job per term; a point that is not affine contributes nothing
+__global__ void k_var_jobs(const uint32_t *point, const int32_t *status, uint32_t n, VarJob *jobs) {
+  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j < n) jobs[j] = {point[j], status[point[j]] != DEC_OK ? 1u : 0u};
+}
+
+// ok[r] = 1 when every input of row r is valid: its points decoded and in G1,
+// its scalars canonical.  A warp per row.
+struct RowChecks {
+  const uint32_t *var_point;
+  const int32_t *point_st, *outside, *scalar_st;
+  const uint32_t *start;
+  const int32_t *fixed_st, *scale_st;  // null: none
+  const uint32_t *fixed_nterms;
+  uint32_t fixed_stride;
+};
+__global__ void __launch_bounds__(128) k_row_checks(RowChecks c, uint32_t rows, uint8_t *ok) {
+  const uint32_t row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (row >= rows) return;
+  bool bad = false;
+  for (uint32_t j = c.start[row] + lane; j < c.start[row + 1]; j += 32) {
+    const uint32_t p = c.var_point[j];
+    bad |= c.point_st[p] == DEC_BAD || c.outside[p] != 0 || c.scalar_st[j] != 0;
+  }
+  if (c.fixed_st) {
+    const uint32_t terms = c.fixed_nterms[row];
+    for (uint32_t g = lane; g < terms; g += 32) bad |= c.fixed_st[(size_t)row * c.fixed_stride + g] != 0;
+    if (c.scale_st && terms) bad |= c.scale_st[row] != 0;
+  }
+  const bool any = __any_sync(0xffffffffu, bad);
+  if (lane == 0) ok[row] = any ? 0 : 1;
+}
+
 // negate the second G1 point of pairing jobs (e(a,b) == e(c,d) <=> e(a,b) e(-c,d) == 1)
 __global__ void k_negate_pb(PairJob *j, uint32_t n) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -273,55 +307,54 @@ void run_plan(Runtime &rt, Plan &pl, std::vector<uint8_t> &out48, std::vector<ui
     pok = rt.arena.alloc<uint8_t>(np);
   }
   if (pl.has_fixed) rt.ensure_table((int)pl.fixed_stride);
-  // decode points
+  // decode points; the sums need only the affine points, and a row with a point
+  // outside G1 is rejected at the end
   uint8_t *dpb = upload(rt, pl.points_be.data(), pl.points_be.size());
   g1a *pts = rt.arena.alloc<g1a>(npts);
-  int32_t *pst = rt.arena.alloc<int32_t>(npts);
-  launch_g1_decode(s, dpb, 48, (uint32_t)npts, pts, pst, true);
-  // var scalars
+  int32_t *pst = rt.arena.alloc<int32_t>(npts), *outside = rt.arena.alloc<int32_t>(npts);
+  launch_g1_decode(s, dpb, 48, (uint32_t)npts, pts, pst, false);
+  if (npts) {
+    // the subgroup check beside the sums (their last kernels leave most of the GPU free)
+    CUBBS_CHECK(cudaEventRecord(rt.ev_fork, s));
+    CUBBS_CHECK(cudaStreamWaitEvent(rt.stream2, rt.ev_fork, 0));
+    launch_g1_subgroup(rt.stream2, pts, pst, (uint32_t)npts, outside);
+    CUBBS_CHECK(cudaEventRecord(rt.ev_join, rt.stream2));
+  }
+  // var scalars and jobs
   uint8_t *dvs = upload(rt, pl.var_scalars_be.data(), pl.var_scalars_be.size());
   fr *vsc = rt.arena.alloc<fr>(nvar);
   int32_t *vst = rt.arena.alloc<int32_t>(nvar);
-  if (nvar) k_parse_scalars<<<blocks_for(nvar, 128), 128, 0, s>>>(dvs, (uint32_t)nvar, vsc, vst);
-  // host needs point statuses to build job flags: fetch them
-  std::vector<int32_t> hpst(npts);
-  if (npts) CUBBS_CHECK(cudaMemcpyAsync(hpst.data(), pst, 4 * npts, cudaMemcpyDeviceToHost, s));
-  std::vector<int32_t> hvst(nvar);
-  if (nvar) CUBBS_CHECK(cudaMemcpyAsync(hvst.data(), vst, 4 * nvar, cudaMemcpyDeviceToHost, s));
+  uint32_t *dvp = upload(rt, pl.var_point.data(), nvar);
+  VarJob *djobs = rt.arena.alloc<VarJob>(nvar);
+  if (nvar) {
+    k_parse_scalars<<<blocks_for(nvar, 128), 128, 0, s>>>(dvs, (uint32_t)nvar, vsc, vst);
+    k_var_jobs<<<blocks_for(nvar, 128), 128, 0, s>>>(dvp, pst, (uint32_t)nvar, djobs);
+  }
+  uint32_t *dstart = upload(rt, pl.var_start.data(), R + 1);
   // fixed scalars
   g1 *fixed = nullptr;
-  std::vector<int32_t> hfst;
+  RowChecks chk{dvp, pst, outside, vst, dstart, nullptr, nullptr, nullptr, 0};
   if (pl.has_fixed) {
     uint8_t *dfs = upload(rt, pl.fixed_scalars_be.data(), pl.fixed_scalars_be.size());
     fr *fsc = rt.arena.alloc<fr>(nfix);
     int32_t *fst = rt.arena.alloc<int32_t>(nfix);
     k_parse_scalars<<<blocks_for(nfix, 128), 128, 0, s>>>(dfs, (uint32_t)nfix, fsc, fst);
-    hfst.resize(nfix);
-    CUBBS_CHECK(cudaMemcpyAsync(hfst.data(), fst, 4 * nfix, cudaMemcpyDeviceToHost, s));
     uint32_t *dnt = upload(rt, pl.fixed_nterms.data(), R);
+    chk.fixed_st = fst;
+    chk.fixed_nterms = dnt;
+    chk.fixed_stride = pl.fixed_stride;
     if (!pl.fixed_scale_be.empty()) {
       uint8_t *dsc = upload(rt, pl.fixed_scale_be.data(), pl.fixed_scale_be.size());
       fr *scale = rt.arena.alloc<fr>(R);
       int32_t *sst = rt.arena.alloc<int32_t>(R);
       k_parse_scalars<<<blocks_for(R, 128), 128, 0, s>>>(dsc, (uint32_t)R, scale, sst);
       k_scale_rows<<<blocks_for(nfix, 128), 128, 0, s>>>(fsc, pl.fixed_stride, dnt, scale, (uint32_t)R);
-      std::vector<int32_t> hs(R);
-      CUBBS_CHECK(cudaMemcpyAsync(hs.data(), sst, 4 * R, cudaMemcpyDeviceToHost, s));
-      CUBBS_CHECK(cudaStreamSynchronize(s));
-      for (size_t r = 0; r < R; r++)
-        if (hs[r]) hfst[r * pl.fixed_stride] |= 1;
+      chk.scale_st = sst;
     }
     fixed = rt.arena.alloc<g1>(R);
     launch_fixed_msm(s, rt.table(), fsc, pl.fixed_stride, dnt, (uint32_t)R, fixed);
   }
-  CUBBS_CHECK(cudaStreamSynchronize(s));
-  std::vector<VarJob> jobs(nvar);
-  for (size_t j = 0; j < nvar; j++) {
-    uint32_t p = pl.var_point[j];
-    jobs[j] = {p, (uint32_t)(hpst[p] != DEC_OK ? 1 : 0)};
-  }
-  VarJob *djobs = upload(rt, jobs.data(), nvar);
-  uint8_t *dout = rt.arena.alloc<uint8_t>(48 * R);
+  uint8_t *dout = rt.arena.alloc<uint8_t>(49 * R);  // the rows' points, then a byte each: every input valid
   uint32_t *engine_err = nullptr, herr = 0;
   if (engine) {
     MsmDevice md;
@@ -336,14 +369,15 @@ void run_plan(Runtime &rt, Plan &pl, std::vector<uint8_t> &out48, std::vector<ui
   } else {
     g1 *v = rt.arena.alloc<g1>(nvar);
     launch_var_mul(s, pts, djobs, vsc, (uint32_t)nvar, v);
-    uint32_t *dstart = upload(rt, pl.var_start.data(), R + 1);
     g1 *res = rt.arena.alloc<g1>(R);
     if (R) k_row_sum<<<blocks_for(R * 32, 128), 128, 0, s>>>(fixed, v, dstart, (uint32_t)R, res);
     launch_g1_compress(s, res, (uint32_t)R, dout);
   }
+  if (npts) CUBBS_CHECK(cudaStreamWaitEvent(s, rt.ev_join, 0));
+  if (R) k_row_checks<<<blocks_for(R * 32, 128), 128, 0, s>>>(chk, (uint32_t)R, dout + 48 * R);
   CUBBS_CHECK(cudaGetLastError());
-  out48.resize(48 * R);
-  if (R) CUBBS_CHECK(cudaMemcpyAsync(out48.data(), dout, 48 * R, cudaMemcpyDeviceToHost, s));
+  out48.resize(49 * R);
+  if (R) CUBBS_CHECK(cudaMemcpyAsync(out48.data(), dout, 49 * R, cudaMemcpyDeviceToHost, s));
   if (np) {
     pairs->ok.resize(np);
     CUBBS_CHECK(cudaMemcpyAsync(pairs->ok.data(), pok, np, cudaMemcpyDeviceToHost, s));
@@ -351,14 +385,8 @@ void run_plan(Runtime &rt, Plan &pl, std::vector<uint8_t> &out48, std::vector<ui
   if (engine_err) CUBBS_CHECK(cudaMemcpyAsync(&herr, engine_err, 4, cudaMemcpyDeviceToHost, s));
   CUBBS_CHECK(cudaStreamSynchronize(s));
   if (herr) throw CudaError(cudaErrorInvalidValue, "uneven-MSM engine: a unit had no room in its launch");
-  row_ok.assign(R, 1);
-  for (size_t r = 0; r < R; r++) {
-    for (uint32_t j = pl.var_start[r]; j < pl.var_start[r + 1]; j++)
-      if (hpst[pl.var_point[j]] == DEC_BAD || hvst[j]) row_ok[r] = 0;
-    if (pl.has_fixed)
-      for (uint32_t g = 0; g < pl.fixed_nterms[r]; g++)
-        if (hfst[r * pl.fixed_stride + g]) row_ok[r] = 0;
-  }
+  row_ok.assign(out48.begin() + 48 * R, out48.end());
+  out48.resize(48 * R);
 }
 
 // Is points[0..K) == [P1, Q1, H1, ...][0..K)?

@@ -76,3 +76,40 @@ def test_decode_pairs(gpu, oracle, n):
     got = gpu.g1_msm_batch([([kinds[i % len(kinds)][0]], [one]) for i in range(n)])
     assert [c for c, _ in got] == [0 if w is not None else 1 for w in want]
     assert [p for (_, p), w in zip(got, want) if w is not None] == [w for w in want if w is not None]
+
+
+@pytest.mark.parametrize("n", [19456, 19457])
+def test_membership_of_many(gpu, oracle, n):
+    """A lane per point, in Jacobian coordinates, and the lane pairs just below: points in and out of G1, of order 3 and
+    of order 11 or 121 (sums with equal and opposite points, and the identity, within the chain)."""
+    p, q = oracle.P_MOD, oracle.R_MOD
+
+    def add(a, b):
+        if a is None or b is None:
+            return a or b
+        if a[0] == b[0]:
+            if (a[1] + b[1]) % p == 0:
+                return None
+            m = 3 * a[0] * a[0] * pow(2 * a[1], -1, p)
+        else:
+            m = (b[1] - a[1]) * pow(b[0] - a[0], -1, p)
+        x = (m * m - a[0] - b[0]) % p
+        return x, (m * (a[0] - x) - a[1]) % p
+    order = 0x396C8C005555E1568C00AAAB0000AAAB * q
+    assert order % 121 == 0
+    small, x = [], 0
+    while len(small) < 2:
+        x += 1
+        y = pow(x ** 3 + 4, (p + 1) // 4, p)
+        if (y * y - x ** 3 - 4) % p:
+            continue
+        r, k, b = None, order // 121, (x, y)
+        while k:
+            r, b, k = add(r, b) if k & 1 else r, add(b, b), k >> 1
+        if r:
+            small.append(bytes([r[0].to_bytes(48, "big")[0] | 0x80 | (0x20 if r[1] > p // 2 else 0)]) +
+                         r[0].to_bytes(48, "big")[1:])
+    p1, gens = oracle.generators(2)
+    pts = [(p1, 0), (_on_curve_outside_g1(oracle, b"many"), 1), (bytes([0x80]) + bytes(47), 1), (small[0], 1),
+           (gens[0], 0), (small[1], 1), (gens[1], 0)]
+    assert gpu.g1_subgroup_for_test([pts[i % 7][0] for i in range(n)]) == [(0, pts[i % 7][1]) for i in range(n)]
