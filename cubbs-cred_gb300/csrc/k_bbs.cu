@@ -763,110 +763,116 @@ struct PgItem {
 // with expand_message_xmd more than 170 scalars are drawn in chunks keyed by
 // seed || I2OSP(chunk, 2); with expand_message_xof one call covers up to 1365
 // (65535 bytes) and larger counts are chunked the same way.
+// A thread per item and chunk (blockIdx.y).  Bound by the chain of compressions
+// of one chunk, so the first five scalars, which the products with A and B need,
+// come from a launch of their own (head), and the rest beside those products.
+constexpr uint32_t PG_HEAD = 5;
+template <int S> constexpr uint32_t pg_chunk() { return S == SUITE_SHAKE256 ? 1365 : 170; }
 template <int S>
 __global__ void __launch_bounds__(64) k_pg_random(const PgItem *items, uint32_t n, const uint8_t *blob,
-                                                  fr *rs, uint32_t rs_stride) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+                                                  fr *rs, uint32_t rs_stride, bool head) {
+  __shared__ __align__(16) uint32_t kw2[64];
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  constexpr uint32_t CH = S == SUITE_SHAKE256 ? 1365 : 170;
+  if constexpr (S != SUITE_SHAKE256) {
+    // b_i = SHA-256((b_0 xor b_(i-1)) || I2OSP(i, 1) || DST || I2OSP(68, 1)): 102 bytes
+    // in two blocks.  Block 1 is 8 words of b_0 xor b_(i-1), then i and DST[0..30];
+    // block 2 (DST[31..67], the DST length, the padding, the bit length 816) is the
+    // same for every i, item and chunk.
+    if (threadIdx.x == 0) {
+      uint32_t w[16];
+      for (int k = 0; k < 16; k++) {
+        w[k] = 0;
+        for (int q = 0; q < 4; q++) {
+          const int t = 4 * k + q;
+          const uint32_t v = t < 37 ? DST_MOCK[31 + t] : t == 37 ? DST_MOCK_LEN : t == 38 ? 0x80
+                             : t == 62 ? (102 * 8) >> 8 : t == 63 ? (102 * 8) & 0xff : 0;
+          w[k] = w[k] << 8 | v;
+        }
+      }
+      sha256_schedule(w, kw2);
+    }
+    __syncthreads();
+  }
   if (i >= n) return;
-  PgItem it = items[i];
-  if (it.status != ST_OK) return;
+  const PgItem it = items[i];
+  const uint32_t count = 5 + it.U, c0 = CH * blockIdx.y;
+  if (it.status != ST_OK || c0 >= count) return;
+  const uint32_t m = min(CH, count - c0), first = head || c0 ? 0 : PG_HEAD, last = head ? PG_HEAD : m;
+  if (first >= last) return;
+  fr *out = rs + (size_t)i * rs_stride + c0;
   if constexpr (S == SUITE_SHAKE256) {
-    const uint32_t count = 5 + it.U, CH = 1365;
-    fr *out = rs + (size_t)i * rs_stride;
+    shake_ctx c;
+    xof_begin(c);
+    shake_bytes(c, blob + it.seed_off, 32);
+    if (count > CH) {
+      shake_byte(c, (uint8_t)(blockIdx.y >> 8));
+      shake_byte(c, (uint8_t)blockIdx.y);
+    }
+    xof_start_output(c, SuiteDst<S>::dst_mock(), SuiteDst<S>::dst_mock_len, 48 * m);
 #pragma unroll 1
-    for (uint32_t c0 = 0; c0 < count; c0 += CH) {
-      const uint32_t m = min(CH, count - c0);
-      shake_ctx c;
-      xof_begin(c);
-      shake_bytes(c, blob + it.seed_off, 32);
-      if (count > CH) {
-        shake_byte(c, (uint8_t)((c0 / CH) >> 8));
-        shake_byte(c, (uint8_t)(c0 / CH));
-      }
-      xof_start_output(c, SuiteDst<S>::dst_mock(), SuiteDst<S>::dst_mock_len, 48 * m);
-#pragma unroll 1
-      for (uint32_t k = 0; k < m; k++) {
-        uint8_t okm[48];
-        shake_squeeze(c, okm, 48);
-        out[c0 + k] = fr_raw_from_okm(okm);
-      }
+    for (uint32_t k = 0; k < last; k++) {
+      uint8_t okm[48];
+      shake_squeeze(c, okm, 48);
+      if (k >= first) out[k] = fr_raw_from_okm(okm);
     }
     return;
   }
   const uint8_t *dst = DST_MOCK;
-  uint32_t count = 5 + it.U;
-  const uint32_t CH = 170;
-  fr *out = rs + (size_t)i * rs_stride;
+  sha_ctx c;
+  xmd_begin(c);
+  sha_bytes(c, blob + it.seed_off, 32);
+  if (count > CH) {
+    sha_byte(c, (uint8_t)(blockIdx.y >> 8));
+    sha_byte(c, (uint8_t)blockIdx.y);
+  }
+  // expand 48*m bytes, one 32-byte block at a time, reducing every 48 bytes
+  // (xmd_finish into a per-thread buffer of at most 8160 bytes would not fit in
+  // registers; stream the b_i blocks instead)
+  const uint32_t nbytes = 48 * m;
+  sha_byte(c, (uint8_t)(nbytes >> 8));
+  sha_byte(c, (uint8_t)nbytes);
+  sha_byte(c, 0);
+  sha_bytes(c, dst, DST_MOCK_LEN);
+  sha_byte(c, DST_MOCK_LEN);
+  uint32_t x0[8];
+  sha_final_words(c, x0);
+  uint32_t bi[8] = {0, 0, 0, 0, 0, 0, 0, 0}, tail1[7];
+  const uint32_t dst3 = (uint32_t)dst[0] << 16 | (uint32_t)dst[1] << 8 | dst[2];
+  for (int k = 0; k < 7; k++)
+    tail1[k] = (uint32_t)dst[3 + 4 * k] << 24 | (uint32_t)dst[4 + 4 * k] << 16 | (uint32_t)dst[5 + 4 * k] << 8 |
+               dst[6 + 4 * k];
+  uint32_t okm[12], fill = 0, produced = 0;
   #pragma unroll 1
-  for (uint32_t c0 = 0; c0 < count; c0 += CH) {
-    uint32_t m = min(CH, count - c0);
-    sha_ctx c;
-    xmd_begin(c);
-    sha_bytes(c, blob + it.seed_off, 32);
-    if (count > CH) {
-      uint32_t chunk = c0 / CH;
-      sha_byte(c, (uint8_t)(chunk >> 8));
-      sha_byte(c, (uint8_t)chunk);
-    }
-    // expand 48*m bytes, one 32-byte block at a time, reducing every 48 bytes
-    // (xmd_finish into a per-thread buffer of at most 8160 bytes would not fit in
-    // registers; stream the b_i blocks instead)
-    uint32_t nbytes = 48 * m;
-    sha_byte(c, (uint8_t)(nbytes >> 8));
-    sha_byte(c, (uint8_t)nbytes);
-    sha_byte(c, 0);
-    sha_bytes(c, dst, DST_MOCK_LEN);
-    sha_byte(c, DST_MOCK_LEN);
-    uint32_t x0[8];
-    sha_final_words(c, x0);
-    // b_i = SHA-256((b_0 xor b_(i-1)) || I2OSP(i, 1) || DST || I2OSP(68, 1)): 102 bytes
-    // in two blocks.  Block 1 is 8 words of b_0 xor b_(i-1), then i and DST[0..30];
-    // block 2 (DST[31..67], the DST length, the padding, the bit length 816) is the
-    // same for every i.
-    uint32_t bi[8] = {0, 0, 0, 0, 0, 0, 0, 0}, tail1[7], blk2[16];
-    const uint32_t dst3 = (uint32_t)dst[0] << 16 | (uint32_t)dst[1] << 8 | dst[2];
-    for (int k = 0; k < 7; k++)
-      tail1[k] = (uint32_t)dst[3 + 4 * k] << 24 | (uint32_t)dst[4 + 4 * k] << 16 | (uint32_t)dst[5 + 4 * k] << 8 |
-                 dst[6 + 4 * k];
-    {
-      uint8_t t[64];
-      for (int k = 0; k < 37; k++) t[k] = dst[31 + k];
-      t[37] = DST_MOCK_LEN;
-      t[38] = 0x80;
-      for (int k = 39; k < 64; k++) t[k] = 0;
-      t[62] = (uint8_t)((102 * 8) >> 8);
-      t[63] = (uint8_t)(102 * 8);
-      for (int k = 0; k < 16; k++)
-        blk2[k] = (uint32_t)t[4 * k] << 24 | (uint32_t)t[4 * k + 1] << 16 | (uint32_t)t[4 * k + 2] << 8 | t[4 * k + 3];
-    }
-    uint32_t okm[12], fill = 0, produced = 0;
-    uint32_t ell = (nbytes + 31) / 32;
-    #pragma unroll 1
-    for (uint32_t b = 1; b <= ell; b++) {
-      uint32_t h[8] = {0x6a09e667u, 0xbb67ae85u, 0x3c6ef372u, 0xa54ff53au,
-                       0x510e527fu, 0x9b05688cu, 0x1f83d9abu, 0x5be0cd19u};
-      uint32_t w[16];
-      for (int k = 0; k < 8; k++) w[k] = x0[k] ^ bi[k];  // bi = 0 before b_1
-      w[8] = b << 24 | dst3;
-      for (int k = 0; k < 7; k++) w[9 + k] = tail1[k];
-      sha256_compress(h, w);
-      for (int k = 0; k < 16; k++) w[k] = blk2[k];
-      sha256_compress(h, w);
-      for (int k = 0; k < 8; k++) bi[k] = h[k];
-      for (int j = 0; j < 8; j++) {
-        okm[fill++] = bi[j];
-        if (fill == 12) {
-          out[c0 + produced] = fr_raw_from_okm_words(okm);
-          produced++;
-          fill = 0;
-        }
+  for (uint32_t b = 1; produced < last; b++) {
+    uint32_t h[8] = {0x6a09e667u, 0xbb67ae85u, 0x3c6ef372u, 0xa54ff53au,
+                     0x510e527fu, 0x9b05688cu, 0x1f83d9abu, 0x5be0cd19u};
+    uint32_t w[16];
+    for (int k = 0; k < 8; k++) w[k] = x0[k] ^ bi[k];  // bi = 0 before b_1
+    w[8] = b << 24 | dst3;
+    for (int k = 0; k < 7; k++) w[9 + k] = tail1[k];
+    sha256_compress(h, w);
+    sha256_compress_scheduled(h, kw2);
+    for (int k = 0; k < 8; k++) bi[k] = h[k];
+    for (int j = 0; j < 8; j++) {
+      okm[fill++] = bi[j];
+      if (fill == 12) {
+        if (produced >= first && produced < last) out[produced] = fr_raw_from_okm_words(okm);
+        produced++;
+        fill = 0;
       }
     }
   }
 }
+template <int S>
+static void launch_pg_random(cudaStream_t s, const PgItem *items, uint32_t n, const uint8_t *blob, fr *rs,
+                             uint32_t rs_stride, bool head) {
+  const uint32_t chunks = head ? 1 : (rs_stride + pg_chunk<S>() - 1) / pg_chunk<S>();
+  k_pg_random<S><<<dim3(blocks_for(n, 64), chunks), 64, 0, s>>>(items, n, blob, rs, rs_stride, head);
+}
 
 // Row i: B = P1 + Q1 domain + sum H_i m_i.  Needs neither the decoded signature
-// point (k_pg_vars rejects a signature whose A does not decode) nor the blinding
+// point (k_pg_finish rejects a signature whose A does not decode) nor the blinding
 // scalars, so the B-MSM starts as soon as the messages are hashed.
 __global__ void __launch_bounds__(ROW_THREADS) k_pg_rows_b(PgItem *items, const uint8_t *blob, const fr *msc,
                                                            const fr *domain, fr *rows, uint32_t stride,
@@ -911,55 +917,65 @@ __global__ void __launch_bounds__(ROW_THREADS) k_pg_rows_t2(const PgItem *items0
   }
 }
 
-// Variable-base jobs on B (affine) and A: D = r2 B, Abar = r1r2 A,
-// Bbar = r1r2 B - e r1r2 A, T1 = r1~ r2 B + e~ r1r2 A, T2 += r3~ r2 B.
-__global__ void __launch_bounds__(64) k_pg_vars(PgItem *items, uint32_t n, const uint8_t *blob, const g1 *Bx,
-                                                const g1a *A, const int32_t *dec_status, const int32_t *outside_g1,
-                                                const fr *rs, uint32_t rs_stride, g1a *pts, VarJob *jobs, fr *jscal) {
+// Variable-base jobs: D = r2 B, Abar = r1r2 A, Bbar = r1r2 B - e r1r2 A,
+// T1 = r1~ r2 B + e~ r1r2 A, T2 += r3~ r2 B.  The three products with A follow
+// its decode and the four with B its MSM, side by side; an item that is rejected
+// later gets jobs all the same.
+__global__ void __launch_bounds__(64) k_pg_vars_a(const PgItem *items0, uint32_t n, const uint8_t *blob,
+                                                  const g1a *A, const int32_t *dec_status, const fr *rs,
+                                                  uint32_t rs_stride, g1a *pts, VarJob *jobs, fr *jscal) {
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  PgItem it = items[i];
-  for (int k = 0; k < 7; k++) jobs[7 * i + k] = {2 * i, 1};
-  if (it.status != ST_OK) return;
-  if (dec_status[i] == DEC_BAD || outside_g1[i]) {  // signature A does not decode to a point of G1
-    items[i].status = ST_ERROR;
-    return;
-  }
-  g1a b;
-  bool binf = !g1_to_aff(Bx[i], b);
-  pts[2 * i] = A[i];
-  pts[2 * i + 1] = binf ? A[i] : b;
-  uint32_t fa = dec_status[i] == DEC_INF ? 1 : 0, fb = binf ? 1 : 0;
+  const PgItem it = items0[i];
+  const bool ok = it.status == ST_OK && dec_status[i] == DEC_OK;
+  for (int k = 0; k < 3; k++) jobs[3 * i + k] = {n + i, ok ? 0u : 1u};
+  if (!ok) return;
+  pts[n + i] = A[i];
   fr e;
   fr_raw_from_be32(blob + it.sig_off + 48, e);
   const fr *r = rs + (size_t)i * rs_stride;
-  fr r1 = r[0], r2 = r[1], et = r[2], r1t = r[3], r3t = r[4];
-  fr r1r2 = frr_mul(r1, r2);
-  jobs[7 * i + 0] = {2 * i + 1, fb}; jscal[7 * i + 0] = r2;
-  jobs[7 * i + 1] = {2 * i, fa};     jscal[7 * i + 1] = r1r2;
-  jobs[7 * i + 2] = {2 * i + 1, fb}; jscal[7 * i + 2] = r1r2;
-  jobs[7 * i + 3] = {2 * i, fa};     jscal[7 * i + 3] = frr_neg(frr_mul(e, r1r2));
-  jobs[7 * i + 4] = {2 * i + 1, fb}; jscal[7 * i + 4] = frr_mul(r1t, r2);
-  jobs[7 * i + 5] = {2 * i, fa};     jscal[7 * i + 5] = frr_mul(et, r1r2);
-  jobs[7 * i + 6] = {2 * i + 1, fb}; jscal[7 * i + 6] = frr_mul(r3t, r2);
+  const fr r1r2 = frr_mul(r[0], r[1]);
+  jscal[3 * i + 0] = r1r2;
+  jscal[3 * i + 1] = frr_neg(frr_mul(e, r1r2));
+  jscal[3 * i + 2] = frr_mul(r[2], r1r2);
+}
+__global__ void __launch_bounds__(64) k_pg_vars_b(const PgItem *items0, uint32_t n, const g1 *Bx, const fr *rs,
+                                                  uint32_t rs_stride, g1a *pts, VarJob *jobs, fr *jscal) {
+  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  g1a b;
+  const bool ok = items0[i].status == ST_OK && g1_to_aff(Bx[i], b);
+  for (int k = 0; k < 4; k++) jobs[4 * i + k] = {i, ok ? 0u : 1u};
+  if (!ok) return;
+  pts[i] = b;
+  const fr *r = rs + (size_t)i * rs_stride;
+  jscal[4 * i + 0] = r[1];
+  jscal[4 * i + 1] = frr_mul(r[0], r[1]);
+  jscal[4 * i + 2] = frr_mul(r[3], r[1]);
+  jscal[4 * i + 3] = frr_mul(r[4], r[1]);
 }
 
 template <int S>
 __global__ void __launch_bounds__(64) k_pg_finish(PgItem *items, uint32_t n, const uint8_t *blob, const fr *msc,
                                                   const fr *domain, const fr *rs, uint32_t rs_stride,
-                                                  const g1 *t2fix, const g1 *v, uint8_t *out, const hash_ctx<S> *chal,
+                                                  const g1 *t2fix, const g1 *v, const int32_t *dec_status,
+                                                  const int32_t *outside_g1, uint8_t *out, const hash_ctx<S> *chal,
                                                   const fr *r3inv) {
   // every lane of the warp reaches the shared affine conversion below
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool act = i < n && items[i].status == ST_OK;
+  bool act = i < n && items[i].status == ST_OK;
+  if (act && (dec_status[i] == DEC_BAD || outside_g1[i])) {  // signature A does not decode to a point of G1
+    items[i].status = ST_ERROR;
+    act = false;
+  }
   g1 P[5] = {g1_inf(), g1_inf(), g1_inf(), g1_inf(), g1_inf()};  // Abar, Bbar, D, T1, T2
   if (act) {
-    const g1 *vi = v + 7 * (size_t)i;
-    P[0] = vi[1];
-    P[1] = g1_add(vi[2], vi[3]);
-    P[2] = vi[0];
-    P[3] = g1_add(vi[4], vi[5]);
-    P[4] = g1_add(t2fix[i], vi[6]);
+    const g1 *va = v + 3 * (size_t)i, *vb = v + 3 * (size_t)n + 4 * (size_t)i;
+    P[0] = va[0];
+    P[1] = g1_add(vb[1], va[1]);
+    P[2] = vb[0];
+    P[3] = g1_add(vb[2], va[2]);
+    P[4] = g1_add(t2fix[i], vb[3]);
   }
   g1a aff[5];
   bool fin[5];
@@ -1546,54 +1562,88 @@ void run_pverify(Runtime &rt, OpBatch &b, uint8_t *dmapdst) {
   b.launches_per_run = (nm ? 1 : 0) + (npts ? 2 : 0) + 9 + (G ? (agg_by_buckets(b) ? 5 : 4) : 0);
 }
 
-// ProofGen on three streams: the signature decode (stream3) runs beside
-// everything before the variable-base terms; the B-MSM follows the message hash
-// and the domain (stream) while the blinding scalars and the T2 fixed-base MSM
-// run on stream2; the variable-base terms need all of them.
+// ProofGen on four streams.  The products with A (stream) need the signature's
+// decode and the first blinding scalars, those with B (stream3, whose blocks go
+// first) its MSM and the same scalars; the T2 fixed-base MSM (stream2) needs all blinding scalars, a
+// chain of hashes that is the longest part of a small batch.  Stream4 has the
+// first scalars, the challenge hash's prefix and the subgroup check, whose
+// result only the finish reads.
+// With all seven products in one launch after the check and both MSMs one item
+// took 1.24 ms (now 0.90) and 1024 took 3.03.
+// From PG_APART_JOBS on the products fill the GPU's sub-partitions a warp each
+// and the MSMs fill them several times: one launch for both bases then, with the
+// T2 MSM in what it leaves free.
+const size_t PG_APART_JOBS = 2048;  // the ladders' limit, k_g1.cu
 void run_pgen(Runtime &rt, OpBatch &b, uint8_t *dmapdst) {
-  cudaStream_t s = rt.stream, s2 = rt.stream2, s3 = rt.stream3;
+  cudaStream_t s = rt.stream3, s2 = rt.stream2, sa = rt.stream, s4 = rt.stream4;
   size_t n = b.n, nm = b.ml.count(), npts = b.pts48.size() / 48;
   uint32_t N = (uint32_t)n, stride = (uint32_t)b.stride, rss = (uint32_t)b.rs_stride;
   PgItem *it = reinterpret_cast<PgItem *>(b.ditems);
   const PgItem *it0 = reinterpret_cast<const PgItem *>(b.ditems0);
-  CUBBS_CHECK(cudaEventRecord(rt.ev_fork, s));
+  CUBBS_CHECK(cudaEventRecord(rt.ev_fork, sa));
+  CUBBS_CHECK(cudaStreamWaitEvent(s, rt.ev_fork, 0));
   CUBBS_CHECK(cudaStreamWaitEvent(s2, rt.ev_fork, 0));
-  CUBBS_CHECK(cudaStreamWaitEvent(s3, rt.ev_fork, 0));
-  SPAN(s3, "g1_decode", launch_g1_decode(s3, b.dpts48, 48, (uint32_t)npts, b.pts, b.dec, false));
-  // the check is done long before the MSMs are, so it takes the form with the
-  // fewest instructions at any size (1024 proofs: 3.66 -> 3.58 ms)
-  SPAN(s3, "g1_subgroup", launch_g1_subgroup(s3, b.pts, b.dec, (uint32_t)npts, b.sub, npts > 512 ? 2 : 0));
-  CUBBS_CHECK(cudaEventRecord(rt.ev_join, s3));
-  SPAN(s2, "random_scalars", CUBBS_SUITE_DISPATCH(rt.suite, k_pg_random<S><<<blocks_for(n, 64), 64, 0, s2>>>(it0, N, b.dblob, b.rs, rss)));
-  CUBBS_CHECK(cudaEventRecord(rt.ev_mid, s2));
-  SPAN(s2, "fixed_msm_t2",
-       k_pg_rows_t2<<<N, ROW_THREADS, 0, s2>>>(it0, N, b.dblob, b.rs, rss, b.rows, stride, b.nterms);
-       launch_fixed_msm(s2, rt.table(), b.rows + (size_t)n * stride, stride, b.nterms + n, N, b.fixed + n));
-  CUBBS_CHECK(cudaEventRecord(rt.ev_side, s2));
+  CUBBS_CHECK(cudaStreamWaitEvent(s4, rt.ev_fork, 0));
+  SPAN(sa, "g1_decode", launch_g1_decode(sa, b.dpts48, 48, (uint32_t)npts, b.pts, b.dec, false));
+  CUBBS_CHECK(cudaEventRecord(rt.ev_dec, sa));
+  SPAN(s4, "first_scalars", CUBBS_SUITE_DISPATCH(rt.suite, launch_pg_random<S>(s4, it0, N, b.dblob, b.rs, rss, true)));
+  CUBBS_CHECK(cudaEventRecord(rt.ev_mid, s4));
+  SPAN(s2, "random_scalars", CUBBS_SUITE_DISPATCH(rt.suite, launch_pg_random<S>(s2, it0, N, b.dblob, b.rs, rss, false)));
+  const size_t na = 3 * n;
+  const bool apart = 7 * n <= PG_APART_JOBS;
+  auto fixed_t2 = [&] {
+    SPAN(s2, "fixed_msm_t2",
+         k_pg_rows_t2<<<N, ROW_THREADS, 0, s2>>>(it0, N, b.dblob, b.rs, rss, b.rows, stride, b.nterms);
+         launch_fixed_msm(s2, rt.table(), b.rows + (size_t)n * stride, stride, b.nterms + n, N, b.fixed + n));
+  };
+  if (apart) fixed_t2();
+  CUBBS_CHECK(cudaStreamWaitEvent(sa, rt.ev_mid, 0));  // the first scalars
+  SPAN(sa, "var_mul_a",
+       k_pg_vars_a<<<blocks_for(n, 64), 64, 0, sa>>>(it0, N, b.dblob, b.pts, b.dec, b.rs, rss, b.vpts, b.jobs,
+                                                     b.jscal);
+       if (apart) launch_var_mul(sa, b.vpts, b.jobs, b.jscal, 3 * N, b.v));
+  if (!apart) CUBBS_CHECK(cudaEventRecord(rt.ev_dec, sa));
   if (nm)
     SPAN(s, "hash_messages",
          launch_h2s_flat(s, b.dmsg + 8 * nm, reinterpret_cast<uint32_t *>(b.dmsg),
                          reinterpret_cast<uint32_t *>(b.dmsg) + nm, (uint32_t)nm, dmapdst, map_dst_len(rt), b.msc, rt.suite));
+  CUBBS_CHECK(cudaEventRecord(rt.ev_hash, s));
   SPAN(s, "domain", launch_domain(s, b.ddj, N, b.dblob, rt.d_gens_c(), rt.ss().d_dom_prefix, b.domain, rt.suite));
   SPAN(s, "fixed_msm",
        k_pg_rows_b<<<N, ROW_THREADS, 0, s>>>(it, b.dblob, b.msc, b.domain, b.rows, stride, b.nterms);
        launch_fixed_msm(s, rt.table(), b.rows, stride, b.nterms, N, b.fixed));
-  CUBBS_CHECK(cudaStreamWaitEvent(s, rt.ev_mid, 0));  // the blinding scalars
-  SPAN(s, "finish_early",
-       CUBBS_SUITE_DISPATCH(rt.suite, k_pg_early<S><<<blocks_for(n, 64), 64, 0, s>>>(
+  CUBBS_CHECK(cudaStreamWaitEvent(s4, rt.ev_hash, 0));
+  SPAN(s4, "finish_early",
+       CUBBS_SUITE_DISPATCH(rt.suite, k_pg_early<S><<<blocks_for(n, 64), 64, 0, s4>>>(
                                           it0, N, b.dblob, b.msc, b.rs, rss, reinterpret_cast<hash_ctx<S> *>(b.chal),
                                           b.r3inv)));
-  CUBBS_CHECK(cudaStreamWaitEvent(s, rt.ev_side, 0));
-  CUBBS_CHECK(cudaStreamWaitEvent(s, rt.ev_join, 0));
-  SPAN(s, "var_prep",
-       k_pg_vars<<<blocks_for(n, 64), 64, 0, s>>>(it, N, b.dblob, b.fixed, b.pts, b.dec, b.sub, b.rs, rss, b.vpts,
-                                                  b.jobs, b.jscal));
-  SPAN(s, "var_mul", launch_var_mul(s, b.vpts, b.jobs, b.jscal, 7 * N, b.v));
-  SPAN(s, "finish",
-       CUBBS_SUITE_DISPATCH(rt.suite, k_pg_finish<S><<<blocks_for(n, 64), 64, 0, s>>>(it, N, b.dblob, b.msc, b.domain, b.rs, rss, b.fixed + n, b.v,
-                                                    b.out, reinterpret_cast<const hash_ctx<S> *>(b.chal), b.r3inv));
-       k_pg_responses<<<N, ROW_THREADS, 0, s>>>(it, b.dblob, b.msc, b.rs, rss, b.out));
-  b.launches_per_run = (nm ? 1 : 0) + (npts ? 2 : 0) + 11;
+  CUBBS_CHECK(cudaStreamWaitEvent(s4, rt.ev_dec, 0));
+  // the check is done long before the MSMs are, so it takes the form with the
+  // fewest instructions at any size (1024 proofs: 3.66 -> 3.58 ms)
+  SPAN(s4, "g1_subgroup", launch_g1_subgroup(s4, b.pts, b.dec, (uint32_t)npts, b.sub, npts > 512 ? 2 : 0));
+  CUBBS_CHECK(cudaEventRecord(rt.ev_sub, s4));
+  CUBBS_CHECK(cudaStreamWaitEvent(s, rt.ev_mid, 0));
+  SPAN(s, "var_mul",
+       k_pg_vars_b<<<blocks_for(n, 64), 64, 0, s>>>(it0, N, b.fixed, b.rs, rss, b.vpts, b.jobs + na, b.jscal + na);
+       if (apart) {
+         launch_var_mul(s, b.vpts, b.jobs + na, b.jscal + na, 4 * N, b.v + na);
+       } else {
+         CUBBS_CHECK(cudaStreamWaitEvent(s, rt.ev_dec, 0));
+         CUBBS_CHECK(cudaEventRecord(rt.ev_join, s));
+         launch_var_mul(s, b.vpts, b.jobs, b.jscal, 7 * N, b.v);
+         CUBBS_CHECK(cudaStreamWaitEvent(s2, rt.ev_join, 0));
+         fixed_t2();
+       });
+  CUBBS_CHECK(cudaEventRecord(rt.ev_side, s2));
+  CUBBS_CHECK(cudaEventRecord(rt.ev_join, s));
+  CUBBS_CHECK(cudaStreamWaitEvent(sa, rt.ev_join, 0));
+  CUBBS_CHECK(cudaStreamWaitEvent(sa, rt.ev_side, 0));
+  CUBBS_CHECK(cudaStreamWaitEvent(sa, rt.ev_sub, 0));
+  SPAN(sa, "finish",
+       CUBBS_SUITE_DISPATCH(rt.suite, k_pg_finish<S><<<blocks_for(n, 64), 64, 0, sa>>>(it, N, b.dblob, b.msc, b.domain, b.rs, rss, b.fixed + n, b.v,
+                                                    b.dec, b.sub, b.out, reinterpret_cast<const hash_ctx<S> *>(b.chal), b.r3inv));
+       k_pg_responses<<<N, ROW_THREADS, 0, sa>>>(it, b.dblob, b.msc, b.rs, rss, b.out));
+  b.launches_per_run = (nm ? 1 : 0) + (npts ? 2 : 0) + 14;
 }
 
 // Verify on three streams, as ProofVerify: the signature decode (stream2, no
@@ -1663,8 +1713,8 @@ template <int S> static void share_carveout_suite() {
 void share_carveout_bbs() {
   share_carveout(k_pv_rows, k_pv_jobs, k_pv_pairjobs, k_pv_pairjobs_agg, k_vf_pairjobs_agg, k_agg_prep_pv,
                  k_agg_prep_vf, k_agg_sort, k_agg_buckets, k_agg_combine, k_agg_ladder, k_agg_sum, k_sign_rows,
-                 k_sign_finish, k_verify_rows, k_verify_jobs, k_verify_finish, k_pg_rows_b, k_pg_rows_t2, k_pg_vars,
-                 k_pg_responses);
+                 k_sign_finish, k_verify_rows, k_verify_jobs, k_verify_finish, k_pg_rows_b, k_pg_rows_t2, k_pg_vars_a,
+                 k_pg_vars_b, k_pg_responses);
   share_carveout_suite<SUITE_SHA256>();
   share_carveout_suite<SUITE_SHAKE256>();
 }

@@ -514,6 +514,7 @@ Runtime::Runtime(SharedState &s)
   CUBBS_CHECK(cudaEventCreateWithFlags(&ev_side, cudaEventDisableTiming));
   CUBBS_CHECK(cudaStreamCreateWithFlags(&stream4, cudaStreamNonBlocking));
   CUBBS_CHECK(cudaEventCreateWithFlags(&ev_sub, cudaEventDisableTiming));
+  CUBBS_CHECK(cudaEventCreateWithFlags(&ev_dec, cudaEventDisableTiming));
   CUBBS_CHECK(cudaEventCreateWithFlags(&ev_hash, cudaEventDisableTiming));
   share_carveout_bbs();
   share_carveout_g1();

@@ -44,6 +44,35 @@ DEVNI void sha256_compress(uint32_t h[8], uint32_t w[16]) {
   h[0] += a; h[1] += b; h[2] += c; h[3] += d; h[4] += e; h[5] += f; h[6] += g; h[7] += hh;
 }
 
+// A block that many hashes share: kw[i] = its schedule's word i + K[i], made by
+// one thread, and the compression from it (two thirds of the instructions).
+DEV void sha256_schedule(const uint32_t block[16], uint32_t kw[64]) {
+  uint32_t w[16];
+  for (int i = 0; i < 16; i++) w[i] = block[i];
+#pragma unroll
+  for (int i = 0; i < 64; i++) {
+    if (i >= 16) {
+      const uint32_t w15 = w[(i - 15) & 15], w2 = w[(i - 2) & 15];
+      w[i & 15] += (sha_rotr(w15, 7) ^ sha_rotr(w15, 18) ^ (w15 >> 3)) + w[(i - 7) & 15] +
+                   (sha_rotr(w2, 17) ^ sha_rotr(w2, 19) ^ (w2 >> 10));
+    }
+    kw[i] = w[i & 15] + SHA256_K[i];
+  }
+}
+DEV void sha256_compress_scheduled(uint32_t h[8], const uint32_t *kw) {
+  uint32_t a = h[0], b = h[1], c = h[2], d = h[3], e = h[4], f = h[5], g = h[6], hh = h[7];
+#pragma unroll
+  for (int i = 0; i < 64; i++) {
+    const uint32_t S1 = sha_rotr(e, 6) ^ sha_rotr(e, 11) ^ sha_rotr(e, 25);
+    const uint32_t ch = (e & f) ^ (~e & g);
+    const uint32_t t1 = hh + S1 + ch + kw[i];
+    const uint32_t S0 = sha_rotr(a, 2) ^ sha_rotr(a, 13) ^ sha_rotr(a, 22);
+    const uint32_t mj = (a & b) ^ (a & c) ^ (b & c);
+    hh = g; g = f; f = e; e = d + t1; d = c; c = b; b = a; a = t1 + S0 + mj;
+  }
+  h[0] += a; h[1] += b; h[2] += c; h[3] += d; h[4] += e; h[5] += f; h[6] += g; h[7] += hh;
+}
+
 struct sha_ctx {
   uint32_t h[8];
   uint32_t w[16];
