@@ -319,10 +319,10 @@ struct Adder {
   Operand operand;
   uint32_t mul_p;
   bool acc_a, acc_a2, acc_out;  // which of the lane's slots lie in the accumulator
-  DEV static Adder on(uint32_t tmp, uint32_t mul_p) {
+  DEV static Adder on(uint32_t tmp, uint32_t mul_p, const Op &op = ADD4) {
     const uint32_t oct = (threadIdx.x & 31) >> 3, t = tmp + oct * TMP_BYTES;
-    const Mul f = ADD4.first[threadIdx.x & 7], g = ADD4.second[threadIdx.x & 7];
-    return {role_of(ADD4, 0, 0, 0, 0, t), Operand::of(ADD4), mul_p, f.a - AX < 3u, f.a2 - AX < 3u, g.out != NONE};
+    const Mul f = op.first[threadIdx.x & 7], g = op.second[threadIdx.x & 7];
+    return {role_of(op, 0, 0, 0, 0, t), Operand::of(op), mul_p, f.a - AX < 3u, f.a2 - AX < 3u, g.out != NONE};
   }
   // For e < count: the triple (e / d) stride + e % d (in steps of `step` bytes
   // from base) takes the one d further on.  One warp, all lanes.

@@ -25,6 +25,7 @@
 #include <cstring>
 
 #include "bbs_dst.cuh"
+#include "g1_ladder.cuh"
 #include "runtime.cuh"
 #include "suite.cuh"
 
@@ -431,7 +432,116 @@ __global__ void __launch_bounds__(128) k_agg_combine(const g1 *part, const int32
   a = warp_sum_pairs(lp, lane < 8 ? win[lane >> 1] : g1_inf());
   if (lane == 0) agg_write_job(a, g, s, gslot, gjobs);
 }
-// Small groups: one ladder per point instead of the bucket MSM, whose
+// Up to a warp of ladders per SM sub-partition (AGG_OCT_WARPS warps a set, four
+// points a warp): a ladder of eight lanes per (item, set) for a P + b phi(P)
+// (g1_ladder.cuh; Shamir's trick over the 32 bits of a and b, one table entry of
+// P, phi(P), P + phi(P) or the identity a step), and the warp's four results
+// added as one triple: 63 additions' depth, then the trees of k_agg_oct_sum.
+// Bound by that chain at any size in range.  The sums of 1000 items of one key,
+// affine: 0.53 ms by buckets (four windows of 256 buckets, a pair of lanes each)
+// -> 0.27; 64 keys of 16 items: 1.0 ms by lane pairs (below) -> 0.35.
+// Positions of a group (perm[goff[g]] ..) are taken four at a time: warp
+// woff[g] + k has positions 4 k .. 4 k + 3 of group g.
+constexpr uint32_t AGG_OCT_WARPS = 304;
+__global__ void __launch_bounds__(32) k_agg_oct_ladder(const g1a *pts4, const uint2 *sc, const uint32_t *perm,
+                                                       const uint32_t *goff, const uint32_t *woff, uint32_t groups,
+                                                       fp *part) {
+  __shared__ __align__(16) gl::Mem mem;
+  __shared__ __align__(16) uint8_t tmp[4 * gl::TMP_BYTES];
+  const uint32_t w = blockIdx.x, s = blockIdx.y, lane = threadIdx.x, oct = lane >> 3, role = lane & 7;
+  uint32_t lo = 0, hi = groups;  // woff[lo] <= w < woff[hi]
+  while (hi - lo > 1) {
+    const uint32_t m = (lo + hi) / 2;
+    if (woff[m] <= w) lo = m;
+    else hi = m;
+  }
+  const uint32_t at = goff[lo] + 4 * (w - woff[lo]) + oct, end = goff[lo + 1];
+  const uint32_t i = perm[min(at, end - 1)];
+  const uint2 v = at < end ? sc[2 * i + s] : make_uint2(0u, 0u);
+  const bool use = v.x != 0;  // a has its top bit set when the point takes part
+  g1a p;
+  p.x = p.y = fp_one();
+  if (use) p = pts4[4 * i + 2 * s];
+  const gl::Ladders l = gl::start(&mem, p, false);
+  fp *sl = l.sl, *tab = sl + gl::TAB;
+  // entry 1: phi(P) = (beta x, -y); entry 2: P + phi(P)
+  if (role == 0) {
+    const fp beta = C_GLV_BETA;
+    tab[4] = fp_mul(tab[0], beta);
+    *reinterpret_cast<fp *>(tmp + oct * gl::TMP_BYTES + gl::at(gl::ZERO)) = fp_zero();
+  } else if (role < 4) {
+    tab[4 + role] = tab[role == 1 ? 2 : role == 2 ? 1 : 3];
+  }
+  __syncwarp();
+  l.step(false, 2);
+  gl::store_entry(sl, (int)role, 2);
+  if (!(v.y >> 31) && role < 3) sl[gl::AX + role] = tab[role == 2 ? 3 : role];
+  __syncwarp();
+#pragma unroll 1
+  for (int k = 61; k >= 0; k--) {
+    const bool doubling = k & 1;
+    const uint32_t bit = (uint32_t)k >> 1;
+    l.step(doubling, (int)(((v.x >> bit) & 1) | (((v.y >> bit) & 1) << 1)));
+  }
+  if (!use && role < 3) sl[gl::AX + role] = role == 1 ? fp_one() : fp_zero();
+  __syncwarp();
+  const gl::Adder adder = gl::Adder::on(slots::addr(tmp), l.mul_p, gl::ADD);
+  const uint32_t base = slots::addr(&mem.slot[0][gl::AX]), step = sizeof(mem.slot[0]);
+  adder.level(base, 2, 2, 4, step);
+  adder.level(base, 1, 1, 4, step);
+  if (lane < 3) part[3 * ((size_t)s * gridDim.x + w) + lane] = mem.slot[0][gl::AX + lane];
+}
+// Grid (groups, 2): the group's triples added, a tree of 32 a warp and then of
+// the warps' sums, and written as its half of the pairing job.
+constexpr uint32_t AGG_SUM_THREADS = (AGG_OCT_WARPS + 31) / 32 * 32;
+constexpr uint32_t AGG_SUM_SMEM = AGG_SUM_THREADS * gl::TRIPLE + AGG_SUM_THREADS / 8 * gl::TMP_BYTES;
+__global__ void __launch_bounds__(AGG_SUM_THREADS) k_agg_oct_sum(const fp *part, const uint32_t *woff, uint32_t warps,
+                                                                 const int32_t *gslot, PairJob *gjobs) {
+  extern __shared__ __align__(16) uint8_t sum_mem[];
+  __shared__ __align__(16) fp mul_p[slots::QMAX];
+  const uint32_t g = blockIdx.x, s = blockIdx.y, t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const uint32_t first = woff[g], count = woff[g + 1] - first;
+  fp *mine = reinterpret_cast<fp *>(sum_mem) + 3 * t;
+  for (int k = 0; k < 3; k++)
+    mine[k] = t < count ? part[3 * ((size_t)s * warps + first + t) + k] : k == 1 ? fp_one() : fp_zero();
+  for (uint32_t k = t; k < slots::QMAX; k += blockDim.x) mul_p[k] = slots::multiple_of_p(k);
+  const uint32_t tmp = AGG_SUM_THREADS * gl::TRIPLE + 4 * warp * gl::TMP_BYTES;
+  if ((lane & 7) == 0)
+    *reinterpret_cast<fp *>(sum_mem + tmp + (lane >> 3) * gl::TMP_BYTES + gl::at(gl::ZERO)) = fp_zero();
+  __syncthreads();
+  const gl::Adder adder = gl::Adder::on(slots::addr(sum_mem) + tmp, slots::addr(mul_p), gl::ADD);
+  const uint32_t base = slots::addr(sum_mem), used = (count + 31) / 32;  // warps with triples
+  uint32_t left = used;
+  uint32_t d = warp < used ? 16 : 0, at = base + 32 * warp * gl::TRIPLE, step = gl::TRIPLE, span = 32;
+#pragma unroll 1
+  for (bool across = false;; d >>= 1) {
+    if (d == 0) {
+      if (across) break;
+      across = true;
+      __syncthreads();
+      if (warp != 0) return;
+      at = base;
+      step = 32 * gl::TRIPLE;
+      span = 16;
+      d = used > 8 ? 8 : used > 4 ? 4 : used > 2 ? 2 : used > 1 ? 1 : 0;
+      if (d == 0) break;
+    }
+    // (across the warps: entry e of d takes e + d, where there is one)
+    const uint32_t pairs = across ? min(d, left - d) : d;
+    adder.level(at, pairs, d, span, step);
+    if (across) left = d;
+  }
+  __shared__ g1 sum;
+  if (lane < 2) {
+    fp v[2];
+    gl::leave(reinterpret_cast<const fp *>(sum_mem) - gl::AX, (int)lane, v);
+    (lane ? sum.Y : sum.X) = v[0];
+    (lane ? sum.ZZZ : sum.ZZ) = v[1];
+  }
+  __syncwarp();
+  if (lane == 0) agg_write_job(sum, g, s, gslot, gjobs);
+}
+// Small groups of larger batches: one ladder per point instead of the bucket MSM, whose
 // 255 bucket weights per (set, window) cost the same whatever the group size
 // (per group about 16 n mixed additions plus 8 x 255 x 15 point operations,
 // against 2 n x 62 for the ladders: the buckets win from about 280 items).
@@ -1247,7 +1357,9 @@ struct OpBatch {
   int32_t *dec = nullptr, *sub = nullptr;  // decode status; 1 = decoded outside G1 (ProofVerify)
   // ProofVerify pairing groups (items under one public key, checked together)
   std::vector<int32_t> h_group_of, h_gslot;
-  std::vector<uint32_t> h_perm, h_goff;
+  std::vector<uint32_t> h_perm, h_goff, h_woff;
+  uint32_t *woff = nullptr, agg_warps = 0;  // eight-lane ladders: four items of a group a warp
+  fp *agg_triples = nullptr;
   int32_t *group_of = nullptr, *gslot = nullptr;
   uint32_t *perm = nullptr, *goff = nullptr;
   PairJob *gjobs = nullptr;
@@ -1297,6 +1409,7 @@ template <typename ItemT> void plan_groups_of(Runtime &rt, OpBatch &b) {
   b.h_group_of.assign(n, -1);
   b.h_perm.clear();
   b.h_goff.assign(1, 0);
+  b.h_woff.assign(1, 0);
   b.h_gslot.clear();
   if (n >= AGG_MIN_BATCH) {
     std::unordered_map<int32_t, std::vector<uint32_t>> by_slot;
@@ -1317,6 +1430,7 @@ template <typename ItemT> void plan_groups_of(Runtime &rt, OpBatch &b) {
       }
       b.h_gslot.push_back(slot);
       b.h_goff.push_back((uint32_t)b.h_perm.size());
+      b.h_woff.push_back(b.h_woff.back() + (uint32_t)(v.size() + 3) / 4);
     }
   }
   const size_t G = b.h_gslot.size();
@@ -1324,6 +1438,9 @@ template <typename ItemT> void plan_groups_of(Runtime &rt, OpBatch &b) {
   if (G) {
     b.perm = upload(rt, b.h_perm.data(), b.h_perm.size());
     b.goff = upload(rt, b.h_goff.data(), G + 1);
+    b.woff = upload(rt, b.h_woff.data(), G + 1);
+    b.agg_warps = b.h_woff.back();
+    b.agg_triples = rt.arena.alloc<fp>(6 * std::min(b.agg_warps, AGG_OCT_WARPS));
     b.gslot = upload(rt, b.h_gslot.data(), G);
     b.gjobs = rt.arena.alloc<PairJob>(G);
     b.gok = rt.arena.alloc<uint8_t>(G);
@@ -1348,7 +1465,7 @@ void upload(Runtime &rt, OpBatch &b) {
                 (b.pts48.size() / 48) * (sizeof(g1a) + 8) + 2 * n * sizeof(g1) + 2 * n * sizeof(g1a) +
                 n * b.rs_stride * sizeof(fr) + b.out_total + n * (2 * sizeof(g1) + 16 + sizeof(PairJob) + 8) +
                 n * (4 * sizeof(g1a) + 2 * sizeof(uint2) + 4 * 2 * AGG_SLAB) +
-                (n / AGG_MIN_GROUP + 1) * AGG_SLAB * (257 * 4 + 16 * sizeof(g1)) +
+                (n / AGG_MIN_GROUP + 1) * (AGG_SLAB * (257 * 4 + 16 * sizeof(g1)) + 4) + AGG_OCT_WARPS * 6 * sizeof(fp) +
                 n * std::max(sizeof(sha_ctx), sizeof(shake_ctx)) + 64 * 256;
   rt.arena.reserve(need);
   // (room for the results too: the host reads them from pinned memory)
@@ -1438,14 +1555,18 @@ void span_end(cudaStream_t s, int k, const char *name) {
 // The group sums of a batch (k_agg_prep_* has filled agg_pts / agg_sc): the
 // bucket MSM when a group has AGG_BUCKET_MIN items or more, else the ladders.
 const size_t AGG_BUCKET_MIN = 256;
+bool agg_by_octets(const OpBatch &b) { return b.agg_warps <= AGG_OCT_WARPS; }
 bool agg_by_buckets(const OpBatch &b) {
+  if (agg_by_octets(b)) return false;
   for (size_t g = 0; g + 1 < b.h_goff.size(); g++)
     if (b.h_goff[g + 1] - b.h_goff[g] >= AGG_BUCKET_MIN) return true;
   return false;
 }
 void launch_agg_buckets(cudaStream_t s, OpBatch &b, uint32_t G) {
   const uint32_t M = (uint32_t)b.h_perm.size();
-  if (agg_by_buckets(b)) {
+  if (agg_by_octets(b)) {
+    k_agg_oct_ladder<<<dim3(b.agg_warps, 2), 32, 0, s>>>(b.agg_pts, b.agg_sc, b.perm, b.goff, b.woff, G, b.agg_triples);
+  } else if (agg_by_buckets(b)) {
     k_agg_sort<<<dim3(G, AGG_SLAB), 256, 0, s>>>(b.perm, b.goff, b.agg_sc, M, b.agg_ent, b.agg_boff);
     k_agg_buckets<<<AGG_SLAB * G * 8, 64, 0, s>>>(b.agg_pts, b.agg_ent, b.agg_boff, M, b.agg_part);
   } else {
@@ -1454,7 +1575,15 @@ void launch_agg_buckets(cudaStream_t s, OpBatch &b, uint32_t G) {
 }
 void launch_agg_combine(cudaStream_t s, OpBatch &b, uint32_t G) {
   CUBBS_CHECK(cudaMemsetAsync(b.gjobs, 0, G * sizeof(PairJob), s));
-  if (agg_by_buckets(b))
+  if (agg_by_octets(b)) {
+    static const bool attr = [] {
+      CUBBS_CHECK(cudaFuncSetAttribute(k_agg_oct_sum, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AGG_SUM_SMEM));
+      return true;
+    }();
+    (void)attr;
+    k_agg_oct_sum<<<dim3(G, 2), AGG_SUM_THREADS, AGG_SUM_SMEM, s>>>(b.agg_triples, b.woff, b.agg_warps, b.gslot,
+                                                                    b.gjobs);
+  } else if (agg_by_buckets(b))
     k_agg_combine<<<dim3(G, 2), 128, 0, s>>>(b.agg_part, b.gslot, b.gjobs);
   else
     k_agg_sum<<<dim3(G, 2), 256, 0, s>>>(b.scaled, b.perm, b.goff, b.gslot, b.gjobs);
@@ -1515,16 +1644,20 @@ void run_pverify(Runtime &rt, OpBatch &b, uint8_t *dmapdst) {
       if (r <= 0) throw CudaError(cudaErrorUnknown, "getrandom");
       got += (size_t)r;
     }
-    // the group sums and the group checks run on the small partition
-    cudaStream_t sa = part ? rt.part_check : s3;
-    if (part) {
+    // the group sums and the group checks run on the small partition, but for
+    // the eight-lane ladders, which want a warp on most of the SMs
+    cudaStream_t sa = part ? rt.part_check : s3, sg = agg_by_octets(b) ? s3 : sa;
+    auto to_small = [&] {
+      if (!part) return;
       CUBBS_CHECK(cudaEventRecord(rt.ev_gc, s3));
       CUBBS_CHECK(cudaStreamWaitEvent(sa, rt.ev_gc, 0));
-    }
-    SPAN(sa, "agg_buckets",
-         k_agg_prep_pv<<<blocks_for(n, 128), 128, 0, sa>>>(it0, N, b.pts, b.dec, b.group_of, seed, b.agg_pts,
+    };
+    if (sg == sa) to_small();
+    SPAN(sg, "agg_buckets",
+         k_agg_prep_pv<<<blocks_for(n, 128), 128, 0, sg>>>(it0, N, b.pts, b.dec, b.group_of, seed, b.agg_pts,
                                                             b.agg_sc);
-         launch_agg_buckets(sa, b, G));
+         launch_agg_buckets(sg, b, G));
+    if (sg != sa) to_small();
     SPAN(sa, "agg_sum", launch_agg_combine(sa, b, G));
     SPAN(sa, "pairing_check", launch_pairing_check_split(sa, b.gjobs, G, rt.d_lines, b.gok));
     if (part) {
@@ -1712,7 +1845,8 @@ template <int S> static void share_carveout_suite() {
 }  // namespace
 void share_carveout_bbs() {
   share_carveout(k_pv_rows, k_pv_jobs, k_pv_pairjobs, k_pv_pairjobs_agg, k_vf_pairjobs_agg, k_agg_prep_pv,
-                 k_agg_prep_vf, k_agg_sort, k_agg_buckets, k_agg_combine, k_agg_ladder, k_agg_sum, k_sign_rows,
+                 k_agg_prep_vf, k_agg_sort, k_agg_buckets, k_agg_combine, k_agg_ladder, k_agg_sum, k_agg_oct_ladder,
+                 k_agg_oct_sum, k_sign_rows,
                  k_sign_finish, k_verify_rows, k_verify_jobs, k_verify_finish, k_pg_rows_b, k_pg_rows_t2, k_pg_vars_a,
                  k_pg_vars_b, k_pg_responses);
   share_carveout_suite<SUITE_SHA256>();
