@@ -93,9 +93,11 @@ __global__ void __launch_bounds__(64) k_pairing_check_split(const PairJob *jobs,
 
 // One check per block of four warps (pairing_quad.cuh).  Calls of n checks
 // through the pairing-equality entry point (decode included), one warp per
-// check -> this: 1: 3.86 -> 2.44 ms, 152: 3.95 -> 2.53, 608: 4.09 -> 3.04, 1216: 4.94 -> 4.33,
-// 4864: 12.4 -> 12.0; no size prefers the one-warp form, which is left for CUBBS_BBS_PAIR_TEAM=32
+// check with the decode of that form -> this: 1: 3.86 -> 1.29 ms, 152: 3.95 -> 1.33,
+// 608: 4.09 -> 1.91, 1216: 4.94 -> 3.63, 4864: 12.4 -> 11.2; no size prefers the
+// one-warp form, which is left for CUBBS_BBS_PAIR_TEAM=32
 // and for the units of the uneven-MSM engine.
+template <bool HALVES>
 __global__ void __launch_bounds__(128) k_pairing_check_team(const PairJob *jobs, uint32_t n, const line2 *lines,
                                                             uint8_t *ok) {
   __shared__ __align__(16) pq::Mem mem;
@@ -106,7 +108,7 @@ __global__ void __launch_bounds__(128) k_pairing_check_team(const PairJob *jobs,
     if (threadIdx.x == 0 && j.active == 0) ok[item] = 0;
     return;
   }
-  const bool one = pq::pairing_check(&mem, j, lines);
+  const bool one = pq::pairing_check<HALVES>(&mem, j, lines);
   if (threadIdx.x == 0) ok[item] = one ? 1 : 0;
 }
 
@@ -119,7 +121,14 @@ static bool wide_pair_teams() {
   return v;
 }
 
-void share_carveout_pairing() { share_carveout(k_pairing_check_team); }
+// Half products on a second warp up to two checks an SM (152 SMs); from three on
+// the warps fill each other's gaps, and the half products' extra multiply-adds
+// cost 1 to 2 %.
+static void launch_team(cudaStream_t s, const PairJob *jobs, uint32_t n, const line2 *lines, uint8_t *ok) {
+  if (n <= 304) k_pairing_check_team<true><<<n, 128, 0, s>>>(jobs, n, lines, ok);
+  else k_pairing_check_team<false><<<n, 128, 0, s>>>(jobs, n, lines, ok);
+}
+void share_carveout_pairing() { share_carveout(k_pairing_check_team<true>, k_pairing_check_team<false>); }
 
 void launch_pairing_check_split(cudaStream_t s, const PairJob *jobs, uint32_t n, const line2 *lines, uint8_t *ok) {
   const size_t smem = 2 * (size_t)PP_SLOTS * sizeof(fp);
@@ -129,7 +138,7 @@ void launch_pairing_check_split(cudaStream_t s, const PairJob *jobs, uint32_t n,
   }();
   (void)attr;
   if (!n) return;
-  if (wide_pair_teams()) k_pairing_check_team<<<n, 128, 0, s>>>(jobs, n, lines, ok);
+  if (wide_pair_teams()) launch_team(s, jobs, n, lines, ok);
   else k_pairing_check_split<<<n, 64, smem, s>>>(jobs, n, lines, ok);
 }
 
@@ -210,7 +219,7 @@ void launch_pairing_check(cudaStream_t s, const PairJob *jobs, uint32_t n, const
   }();
   (void)attr;
   if (!n) return;
-  if (wide_pair_teams()) k_pairing_check_team<<<n, 128, 0, s>>>(jobs, n, lines, ok);
+  if (wide_pair_teams()) launch_team(s, jobs, n, lines, ok);
   else k_pairing_check_warp<<<n, 32, smem, s>>>(jobs, n, lines, ok);
 }
 
