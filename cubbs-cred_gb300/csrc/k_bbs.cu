@@ -669,43 +669,46 @@ __global__ void __launch_bounds__(64) k_pv_finish(PvItem *items, uint32_t n, con
                                                   const fr *domain, const int32_t *dec_status,
                                                   const int32_t *outside_g1, const g1 *t2fix, const g1 *v,
                                                   const hash_ctx<S> *chal) {
+  __shared__ uint8_t enc[32][2 * 48];
   // every lane of the warp reaches the shared affine conversion below
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) >> 1, role = threadIdx.x & 1;
+  uint8_t *t12 = enc[threadIdx.x >> 1];
   bool act = i < n;
   PvItem it;
   if (act) {
     it = items[i];
     act = it.status == ST_OK;
-    if (act && (dec_status[3 * i] == DEC_BAD || dec_status[3 * i + 1] == DEC_BAD ||
-                dec_status[3 * i + 2] == DEC_BAD || outside_g1[3 * i] || outside_g1[3 * i + 1] ||
-                outside_g1[3 * i + 2])) {
-      items[i].status = ST_INVALID;
-      act = false;
-    }
   }
-  g1 T1 = g1_inf(), T2 = g1_inf();
+  __syncwarp();  // both lanes have read the item
+  if (act && (dec_status[3 * i] == DEC_BAD || dec_status[3 * i + 1] == DEC_BAD || dec_status[3 * i + 2] == DEC_BAD ||
+              outside_g1[3 * i] || outside_g1[3 * i + 1] || outside_g1[3 * i + 2])) {
+    if (role == 0) items[i].status = ST_INVALID;
+    act = false;
+  }
+  g1 T = g1_inf();
   if (act) {
-    T1 = g1_add(g1_add(v[3 * i], v[3 * i + 1]), v[3 * i + 2]);
-    T2 = g1_add(t2fix[i], v[3 * n + i]);
+    T = g1_add(role ? t2fix[i] : v[3 * i], role ? v[3 * n + i] : v[3 * i + 1]);
+    if (!role) T = g1_add(T, v[3 * i + 2]);
   }
-  const g1 T[2] = {T1, T2};
-  g1a aff[2];
-  bool fin[2];
-  warp_to_aff<2>(T, aff, fin);
-  if (!act) return;
-  uint8_t t1c[48], t2c[48];
-  g1_compress_aff_or_inf(aff[0], fin[0], t1c);
-  g1_compress_aff_or_inf(aff[1], fin[1], t2c);
+  g1a aff;
+  bool fin;
+  warp_to_aff<1>(&T, &aff, &fin);
+  if (act) {
+    uint8_t b[48];
+    g1_compress_aff_or_inf(aff, fin, b);
+    for (int k = 0; k < 48; k++) t12[48 * role + k] = b[k];
+  }
+  __syncwarp();
+  if (!act || role) return;
   const uint8_t *pr = blob + it.proof_off;
   const uint32_t *idx = reinterpret_cast<const uint32_t *>(blob + it.idx_off);
   hash_ctx<S> c = chal[i];
-  msg_bytes(c, t1c, 48);
-  msg_bytes(c, t2c, 48);
+  msg_bytes(c, t12, 96);
   msg_fr_be(c, domain[i]);
   msg_u64be(c, it.ph_len, 8);
   msg_bytes(c, blob + it.ph_off, it.ph_len);
   fr ch = h2s_api<S>(c);
-  if (i == 0) debug_record(t1c, t2c, domain[i], ch, it.R, idx, it.R ? &msc[it.msg_base] : nullptr);
+  if (i == 0) debug_record(t12, t12 + 48, domain[i], ch, it.R, idx, it.R ? &msc[it.msg_base] : nullptr);
   fr cp;
   fr_raw_from_be32(pr + 240 + 32 * it.U, cp);
   if (!fr_eq(ch, cp)) items[i].status = ST_INVALID;
@@ -1065,63 +1068,79 @@ __global__ void __launch_bounds__(64) k_pg_vars_b(const PgItem *items0, uint32_t
   jscal[4 * i + 3] = frr_mul(r[4], r[1]);
 }
 
+// Eight lanes per item: one each for Abar, Bbar, D, T1 and T2 up to their
+// encodings (one lane for all five took 204 us of a single item, 121 like this),
+// then one for the challenge and three for the responses of e, r1 and r3.
+constexpr uint32_t PG_LANES = 8;
 template <int S>
 __global__ void __launch_bounds__(64) k_pg_finish(PgItem *items, uint32_t n, const uint8_t *blob, const fr *msc,
                                                   const fr *domain, const fr *rs, uint32_t rs_stride,
                                                   const g1 *t2fix, const g1 *v, const int32_t *dec_status,
                                                   const int32_t *outside_g1, uint8_t *out, const hash_ctx<S> *chal,
                                                   const fr *r3inv) {
+  __shared__ uint8_t enc[64 / PG_LANES][5 * 48];
   // every lane of the warp reaches the shared affine conversion below
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  bool act = i < n && items[i].status == ST_OK;
+  const uint32_t i = (blockIdx.x * blockDim.x + threadIdx.x) / PG_LANES, role = threadIdx.x % PG_LANES;
+  uint8_t *e5 = enc[threadIdx.x / PG_LANES];
+  bool act = false;
+  PgItem it;
+  if (i < n) {
+    it = items[i];
+    act = it.status == ST_OK;
+  }
+  __syncwarp();  // every lane has read the item
   if (act && (dec_status[i] == DEC_BAD || outside_g1[i])) {  // signature A does not decode to a point of G1
-    items[i].status = ST_ERROR;
+    if (role == 0) items[i].status = ST_ERROR;
     act = false;
   }
-  g1 P[5] = {g1_inf(), g1_inf(), g1_inf(), g1_inf(), g1_inf()};  // Abar, Bbar, D, T1, T2
-  if (act) {
+  g1 P = g1_inf();
+  if (act && role < 5) {
     const g1 *va = v + 3 * (size_t)i, *vb = v + 3 * (size_t)n + 4 * (size_t)i;
-    P[0] = va[0];
-    P[1] = g1_add(vb[1], va[1]);
-    P[2] = vb[0];
-    P[3] = g1_add(vb[2], va[2]);
-    P[4] = g1_add(t2fix[i], vb[3]);
+    P = role == 0 ? va[0] : role == 1 ? vb[1] : role == 2 ? vb[0] : role == 3 ? vb[2] : t2fix[i];
+    if (role == 1 || role >= 3) P = g1_add(P, role == 1 ? va[1] : role == 3 ? va[2] : vb[3]);
   }
-  g1a aff[5];
-  bool fin[5];
-  warp_to_aff<5>(P, aff, fin);
-  if (!act) return;
-  const PgItem it = items[i];
+  g1a aff;
+  bool fin;
+  warp_to_aff<1>(&P, &aff, &fin);
   uint8_t *o = out + it.out_off;
-  g1_compress_aff_or_inf(aff[0], fin[0], o);
-  g1_compress_aff_or_inf(aff[1], fin[1], o + 48);
-  g1_compress_aff_or_inf(aff[2], fin[2], o + 96);
-  uint8_t t1c[48], t2c[48];
-  g1_compress_aff_or_inf(aff[3], fin[3], t1c);
-  g1_compress_aff_or_inf(aff[4], fin[4], t2c);
-  const uint32_t *idx = reinterpret_cast<const uint32_t *>(blob + it.idx_off);
-  hash_ctx<S> c = chal[i];  // R and the disclosed messages, absorbed by k_pg_early
-  msg_bytes(c, o, 144);
-  msg_bytes(c, t1c, 48);
-  msg_bytes(c, t2c, 48);
-  msg_fr_be(c, domain[i]);
-  msg_u64be(c, it.ph_len, 8);
-  msg_bytes(c, blob + it.ph_off, it.ph_len);
-  fr ch = h2s_api<S>(c);
-  if (i == 0) debug_record(t1c, t2c, domain[i], ch, it.R, idx, it.R ? &msc[it.msg_base + idx[0]] : nullptr);
+  if (act && role < 5) {
+    uint8_t b[48];
+    g1_compress_aff_or_inf(aff, fin, b);
+    for (int k = 0; k < 48; k++) e5[48 * role + k] = b[k];
+    if (role < 3)
+      for (int k = 0; k < 48; k++) o[48 * role + k] = b[k];
+  }
+  __syncwarp();
+  fr ch = fr_zero();
+  if (act && role == 0) {
+    hash_ctx<S> c = chal[i];  // R and the disclosed messages, absorbed by k_pg_early
+    msg_bytes(c, e5, 240);
+    msg_fr_be(c, domain[i]);
+    msg_u64be(c, it.ph_len, 8);
+    msg_bytes(c, blob + it.ph_off, it.ph_len);
+    ch = h2s_api<S>(c);
+    const uint32_t *idx = reinterpret_cast<const uint32_t *>(blob + it.idx_off);
+    if (i == 0) debug_record(e5 + 144, e5 + 192, domain[i], ch, it.R, idx, it.R ? &msc[it.msg_base + idx[0]] : nullptr);
+  }
+  __syncwarp();
+  for (int k = 0; k < 8; k++) ch.w[k] = __shfl_sync(0xffffffffu, ch.w[k], (int)(threadIdx.x & 31 & ~(PG_LANES - 1)));
+  if (!act) return;
   const fr *r = rs + (size_t)i * rs_stride;
-  fr r1 = r[0], r2 = r[1], et = r[2], r1t = r[3], r3t = r[4];
-  if (fr_is_zero(r2)) {  // "Invert scalar failed" (proof.rs:2340-2341)
-    items[i].status = ST_ERROR;
+  if (fr_is_zero(r[1])) {  // "Invert scalar failed" (proof.rs:2340-2341)
+    if (role == 0) items[i].status = ST_ERROR;
     return;
   }
-  fr e;
-  fr_raw_from_be32(blob + it.sig_off + 48, e);
-  const fr r3 = r3inv[i];
-  fr_raw_to_be32(fr_add(et, frr_mul(e, ch)), o + 144);
-  fr_raw_to_be32(fr_sub(r1t, frr_mul(r1, ch)), o + 176);
-  fr_raw_to_be32(fr_sub(r3t, frr_mul(r3, ch)), o + 208);
-  fr_raw_to_be32(ch, o + 240 + 32 * it.U);
+  if (role == 0) {
+    fr e;
+    fr_raw_from_be32(blob + it.sig_off + 48, e);
+    fr_raw_to_be32(fr_add(r[2], frr_mul(e, ch)), o + 144);
+  } else if (role == 1) {
+    fr_raw_to_be32(fr_sub(r[3], frr_mul(r[0], ch)), o + 176);
+  } else if (role == 2) {
+    fr_raw_to_be32(fr_sub(r[4], frr_mul(r3inv[i], ch)), o + 208);
+  } else if (role == 3) {
+    fr_raw_to_be32(ch, o + 240 + 32 * it.U);
+  }
 }
 
 // The responses m^_j = m~_j + c m_j of the undisclosed messages, from the
@@ -1685,7 +1704,7 @@ void run_pverify(Runtime &rt, OpBatch &b, uint8_t *dmapdst) {
   CUBBS_CHECK(cudaStreamWaitEvent(s, rt.ev_side, 0));
   CUBBS_CHECK(cudaStreamWaitEvent(s, rt.ev_sub, 0));
   SPAN(s, "challenge",
-       CUBBS_SUITE_DISPATCH(rt.suite, k_pv_finish<S><<<blocks_for(n, 64), 64, 0, s>>>(it, N, b.dblob, b.msc, b.domain, b.dec, b.sub, b.fixed, b.v,
+       CUBBS_SUITE_DISPATCH(rt.suite, k_pv_finish<S><<<blocks_for(2 * n, 64), 64, 0, s>>>(it, N, b.dblob, b.msc, b.domain, b.dec, b.sub, b.fixed, b.v,
                                                                                       reinterpret_cast<const hash_ctx<S> *>(b.chal))));
   CUBBS_CHECK(cudaStreamWaitEvent(s, rt.ev_join, 0));
   if (part) {
@@ -1773,7 +1792,7 @@ void run_pgen(Runtime &rt, OpBatch &b, uint8_t *dmapdst) {
   CUBBS_CHECK(cudaStreamWaitEvent(sa, rt.ev_side, 0));
   CUBBS_CHECK(cudaStreamWaitEvent(sa, rt.ev_sub, 0));
   SPAN(sa, "finish",
-       CUBBS_SUITE_DISPATCH(rt.suite, k_pg_finish<S><<<blocks_for(n, 64), 64, 0, sa>>>(it, N, b.dblob, b.msc, b.domain, b.rs, rss, b.fixed + n, b.v,
+       CUBBS_SUITE_DISPATCH(rt.suite, k_pg_finish<S><<<blocks_for(PG_LANES * n, 64), 64, 0, sa>>>(it, N, b.dblob, b.msc, b.domain, b.rs, rss, b.fixed + n, b.v,
                                                     b.dec, b.sub, b.out, reinterpret_cast<const hash_ctx<S> *>(b.chal), b.r3inv));
        k_pg_responses<<<N, ROW_THREADS, 0, sa>>>(it, b.dblob, b.msc, b.rs, rss, b.out));
   b.launches_per_run = (nm ? 1 : 0) + (npts ? 2 : 0) + 14;
