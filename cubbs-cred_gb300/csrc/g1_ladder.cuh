@@ -24,6 +24,7 @@
 // cost 4500.
 #pragma once
 #include "curve.cuh"
+#include "fp_bipartite.cuh"
 #include "slots.cuh"
 
 namespace gl {
@@ -120,38 +121,88 @@ struct Operand {
   }
 };
 
+// The second warp's halves of the products where two warps share a launch's
+// ladders (HALVES): both compute half of each product (fp_bipartite.cuh), the
+// first does the rest.  Slots then hold x 2^256 instead of x 2^384 (mod p).
+struct Halves {
+  uint4 v[3][32];
+  uint32_t top[32];
+};
+DEV void pair_sync() { asm volatile("bar.sync 1, 64;" ::: "memory"); }
+// t = x y on the first warp
+DEV void halved(uint32_t halves, bool second, const fp &x, const fp &y, fp &t) {
+  uint32_t m[13];
+  const uint32_t at_v = halves + 16 * (threadIdx.x & 31), at_top = halves + 3 * 32 * 16 + 4 * (threadIdx.x & 31);
+  if (second) {
+    fp_bp_mul_hi(m, x.w, y.w);
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+      asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(at_v + 512 * k), "r"(m[4 * k]), "r"(m[4 * k + 1]),
+                   "r"(m[4 * k + 2]), "r"(m[4 * k + 3])
+                   : "memory");
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(at_top), "r"(m[12]) : "memory");
+  } else {
+    fp_bp_mul_lo(m, x.w, y.w);
+  }
+  __syncwarp();
+  pair_sync();
+  if (!second) {
+    uint32_t o[13];
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+      asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                   : "=r"(o[4 * k]), "=r"(o[4 * k + 1]), "=r"(o[4 * k + 2]), "=r"(o[4 * k + 3])
+                   : "r"(at_v + 512 * k)
+                   : "memory");
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(o[12]) : "r"(at_top) : "memory");
+    fp_bp_finish(t.w, m, o);
+  }
+}
+
 // The operation on the slots of `r`; octets with `live` false compute and store
-// nothing.  All lanes of the warp call it.
-DEV void apply(const Role &r, uint32_t mul_p, bool live) {
+// nothing.  All lanes of the warp (of both warps, with HALVES) call it.
+template <bool HALVES = false> DEV void apply(const Role &r, uint32_t mul_p, bool live, uint32_t halves = 0) {
+  const bool second = HALVES && threadIdx.x >= 32;
   uint32_t v[13], w[12];
+  if constexpr (HALVES) {
+    __syncwarp();
+    pair_sync();  // the first warp has written the operands
+  }
   {
     fp x = ld(r.a), y = ld(r.b);
     const fp x2 = ld(r.a2), y2 = ld(r.b2);
     fp_acc_add(x.w, x.w, x2.w);
     fp_acc_add(y.w, y.w, y2.w);
     fp t;
-    fp_mont_mul(t.w, x.w, y.w);
-    scale(v, t.w, r.k1);
-    reduce13(mul_p, v, w);
-    __syncwarp();  // every lane has read its operands
-    if (live && r.out1 >= 0) st((uint32_t)r.out1, w);
-    __syncwarp();
+    if constexpr (HALVES) halved(halves, second, x, y, t);
+    else fp_mont_mul(t.w, x.w, y.w);
+    if (!second) {
+      scale(v, t.w, r.k1);
+      reduce13(mul_p, v, w);
+      __syncwarp();  // every lane has read its operands
+      if (live && r.out1 >= 0) st((uint32_t)r.out1, w);
+      __syncwarp();
+    }
   }
-  {
+  if (!second) {
     const fp t = lane_sum(r.p0, r.p1, r.m0, r.m1);
     if (live && r.sum >= 0) st((uint32_t)r.sum, t.w);
     __syncwarp();
   }
+  if constexpr (HALVES) pair_sync();  // and the second round's
   {
     const fp x = ld(r.c), y = ld(r.d);
     fp t;
-    fp_mont_mul(t.w, x.w, y.w);
-    scale(v, t.w, r.k2);
-    add_lane(v, 1);
-    reduce13(mul_p, v, w);
-    __syncwarp();
-    if (live && r.out2 >= 0) st((uint32_t)r.out2, w);
-    __syncwarp();
+    if constexpr (HALVES) halved(halves, second, x, y, t);
+    else fp_mont_mul(t.w, x.w, y.w);
+    if (!second) {
+      scale(v, t.w, r.k2);
+      add_lane(v, 1);
+      reduce13(mul_p, v, w);
+      __syncwarp();
+      if (live && r.out2 >= 0) st((uint32_t)r.out2, w);
+      __syncwarp();
+    }
   }
 }
 
@@ -169,12 +220,16 @@ DEV void store_entry(fp *sl, int role, int k) {
 }
 
 // A warp's four ladders: the lanes' parts of a doubling and of an addition.
-struct Ladders {
+// With HALVES a second warp runs the same code for its half of the products;
+// only the first (`first`) writes slots.
+template <bool HALVES> struct LaddersOf {
   Role dbl, add;
   Operand operand;
   uint32_t tab, mul_p;  // addresses of table entry 0 and of the multiples of p
   fp *sl;
   int role;
+  uint32_t halves;
+  bool first;
   // acc *= 2, or acc += digit * P for digit in -8 .. 8 (entry |digit| - 1; 0
   // adds the identity).  One copy in the code: the loops select the operation.
   DEV void step(bool doubling, int digit) const {
@@ -182,30 +237,43 @@ struct Ladders {
     const uint32_t e = tab + at(4 * (uint32_t)(abs(digit) - 1)), zero = tab - at(TAB);
     operand.set(r, digit ? e : zero, digit ? e + at(digit < 0 ? 2 : 1) : tab + at(ONE - TAB), digit ? e + at(3) : zero);
     if (doubling) r = dbl;
-    apply(r, mul_p, true);
+    apply<HALVES>(r, mul_p, true, halves);
+  }
+  // table entry k = acc
+  DEV void entry(int k) const {
+    if (first) store_entry(sl, role, k);
   }
 };
+using Ladders = LaddersOf<false>;
 
 // The constants, ladder state and base point: acc = entry 0 = the image on E'
-// of (x, y), or of phi(x, y) = (beta x, -y).  All lanes of the warp call it.
-DEV Ladders start(Mem *m, const g1a &p, bool phi) {
+// of (x, y), or of phi(x, y) = (beta x, -y).  All lanes of the warp (of both
+// warps, with HALVES, where h is room for the halves) call it.
+template <bool HALVES = false> DEV LaddersOf<HALVES> start(Mem *m, const g1a &p, bool phi, Halves *h = nullptr) {
   const int lane = threadIdx.x & 31, role = lane & 7;
   fp *sl = m->slot[lane >> 3];
-  for (int k = lane; k < QMAX; k += 32) m->mul_p[k] = multiple_of_p((uint32_t)k);
-  if (role == 0) {
-    const fp s2 = C_B3_S2, bs2 = C_B3_BETA_S2;
-    sl[AX] = fp_mul(p.x, phi ? bs2 : s2);
-    sl[ZERO] = fp_zero();
-  } else if (role == 1) {
-    const fp s3 = C_B3_S3;
-    sl[AY] = fp_mul(phi ? fp_neg(p.y) : p.y, s3);
-    sl[ONE] = fp_one();
-  } else if (role == 2) {
-    sl[AZ] = fp_one();
+  LaddersOf<HALVES> l;
+  l.first = !HALVES || threadIdx.x < 32;
+  l.halves = HALVES ? addr(h) : 0;
+  if (l.first) {
+    for (int k = lane; k < QMAX; k += 32) m->mul_p[k] = multiple_of_p((uint32_t)k);
+    const fp form = C_FP_BP_IN;  // 2^256: a Montgomery product with it leaves x 2^256
+    if (role == 0) {
+      const fp s2 = C_B3_S2, bs2 = C_B3_BETA_S2;
+      fp x = fp_mul(p.x, phi ? bs2 : s2);
+      sl[AX] = HALVES ? fp_mul(x, form) : x;
+      sl[ZERO] = fp_zero();
+    } else if (role == 1) {
+      const fp s3 = C_B3_S3;
+      fp y = fp_mul(phi ? fp_neg(p.y) : p.y, s3);
+      sl[AY] = HALVES ? fp_mul(y, form) : y;
+      sl[ONE] = HALVES ? form : fp_one();
+    } else if (role == 2) {
+      sl[AZ] = HALVES ? form : fp_one();
+    }
+    __syncwarp();
+    store_entry(sl, role, 0);
   }
-  __syncwarp();
-  store_entry(sl, role, 0);
-  Ladders l;
   const uint32_t a = addr(sl);
   l.dbl = role_of(DBL, a + at(AX), a, a, a, a);
   l.add = role_of(ADD, a + at(AX), a, a, a, a);
@@ -219,7 +287,8 @@ DEV Ladders start(Mem *m, const g1a &p, bool phi) {
 
 // acc = k P on each of the four ladders (sh: k's 128-bit half of a GLV term),
 // then acc += the point that `join` has stored as entry 0.
-template <class Join> DEV void ladder128(const Ladders &l, const uint32_t sh[4], const Join &join) {
+template <bool HALVES, class Join>
+DEV void ladder128(const LaddersOf<HALVES> &l, const uint32_t sh[4], const Join &join) {
   // signed digits: nibbles of sh + 0x888...8, less 8
   uint32_t d[5];
   uint64_t c = 0;
@@ -240,12 +309,12 @@ template <class Join> DEV void ladder128(const Ladders &l, const uint32_t sh[4],
     int digit = 1;
     if (i == BUILD) {
       digit = (int)d[4];
-      if (l.role == 0) l.sl[AX] = fp_zero();
-      if (l.role == 1) l.sl[AY] = fp_one();
-      if (l.role == 2) l.sl[AZ] = fp_zero();
+      if (l.first && l.role == 0) l.sl[AX] = fp_zero();
+      if (l.first && l.role == 1) l.sl[AY] = l.sl[ONE];
+      if (l.first && l.role == 2) l.sl[AZ] = fp_zero();
       __syncwarp();
     } else if (i == END) {
-      join();
+      if (l.first) join();
       __syncwarp();
     } else if (i >= MAIN) {
       doubling = quint < 4;
@@ -259,7 +328,7 @@ template <class Join> DEV void ladder128(const Ladders &l, const uint32_t sh[4],
       }
     }
     l.step(doubling, digit);
-    if (i < BUILD) store_entry(l.sl, l.role, i + 1);
+    if (i < BUILD) l.entry(i + 1);
   }
 }
 
@@ -287,12 +356,16 @@ DEV void mul_z2(const Ladders &l) {
 
 // The accumulator, taken back from E' as an XYZZ point, by the ladder's lanes
 // 0 and 1: (X Z, s^2 Z^2) and (Y Z^2, s^3 Z^3).
-DEV void leave(const fp *sl, int role, fp v[2]) {
-  const fp s2 = C_B3_S2, s3 = C_B3_S3;
-  const fp z = sl[AZ];
+template <bool HALVES = false> DEV void leave(const fp *sl, int role, fp v[2]) {
+  const fp s2 = C_B3_S2, s3 = C_B3_S3, form = C_FP_BP_OUT;
+  fp z = sl[AZ], xy = sl[AX + role];
+  if (HALVES) {  // to x 2^384
+    z = fp_mul(z, form);
+    xy = fp_mul(xy, form);
+  }
   fp zz = z;
   if (role == 1) zz = fp_mul(z, z);
-  v[0] = fp_mul(sl[AX + role], zz);
+  v[0] = fp_mul(xy, zz);
   v[1] = fp_mul(fp_mul(zz, z), role ? s3 : s2);
 }
 

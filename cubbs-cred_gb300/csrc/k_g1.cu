@@ -258,10 +258,12 @@ __global__ void __launch_bounds__(128) k_var_mul_quad(const g1a *points, const V
   if (lq.role == 0) out[i] = r;
 }
 // Two ladders of eight lanes per job (g1_ladder.cuh), one per GLV half; two
-// jobs a warp, one warp a block.
-__global__ void __launch_bounds__(32) k_var_mul_ladder(const g1a *points, const VarJob *jobs, const fr *scalars,
-                                                       uint32_t n, g1 *out) {
+// jobs a block of one warp, or of two that share the products (HALVES).
+template <bool HALVES>
+__global__ void __launch_bounds__(HALVES ? 64 : 32) k_var_mul_ladder(const g1a *points, const VarJob *jobs,
+                                                                     const fr *scalars, uint32_t n, g1 *out) {
   __shared__ __align__(16) gl::Mem mem;
+  __shared__ __align__(16) gl::Halves halves;
   if (n == 0) return;
   const int lane = threadIdx.x & 31, role = lane & 7, half = (lane >> 3) & 1;
   const uint32_t i = 2 * blockIdx.x + (lane >> 4);
@@ -271,7 +273,7 @@ __global__ void __launch_bounds__(32) k_var_mul_ladder(const g1a *points, const 
   g1a p;
   p.x = p.y = fp_one();
   if (!inf) p = points[job.point];
-  const gl::Ladders l = gl::start(&mem, p, half != 0);
+  const gl::LaddersOf<HALVES> l = gl::start<HALVES>(&mem, p, half != 0, &halves);
   uint32_t s[4], q[4];
   glv_split(scalars[j], s, q);
   fp *sl = l.sl;
@@ -279,9 +281,10 @@ __global__ void __launch_bounds__(32) k_var_mul_ladder(const g1a *points, const 
   gl::ladder128(l, half ? q : s, [&] {
     if (!half && role < 3) sl[gl::TAB + (role == 2 ? 3 : role)] = mem.slot[(lane >> 3) + 1][gl::AX + role];
   });
+  if (!l.first) return;
   if (!half && role < 2) {
     fp v[2];
-    gl::leave(sl, role, v);
+    gl::leave<HALVES>(sl, role, v);
     if (i < n) {
       if (inf) {
         const g1 o = g1_inf();
@@ -483,14 +486,17 @@ void launch_var_mul(cudaStream_t s, const g1a *points, const VarJob *jobs, const
                     int lanes) {
   if (!n) return;
   if (lanes == 0) lanes = lanes_for(n);
-  if (lanes == 8) k_var_mul_ladder<<<blocks_for(n, 2), 32, 0, s>>>(points, jobs, scalars, n, out);
+  // Products shared by two warps while those still find a sub-partition each
+  // (152 x 4): 64 terms 0.39 -> 0.33 ms.
+  if (lanes == 8 && n <= 608) k_var_mul_ladder<true><<<blocks_for(n, 2), 64, 0, s>>>(points, jobs, scalars, n, out);
+  else if (lanes == 8) k_var_mul_ladder<false><<<blocks_for(n, 2), 32, 0, s>>>(points, jobs, scalars, n, out);
   else if (lanes == 4) k_var_mul_quad<<<blocks_for(4 * (size_t)n, 128), 128, 0, s>>>(points, jobs, scalars, n, out);
   else if (lanes == 2) k_var_mul_pair<<<blocks_for(2 * (size_t)n, 128), 128, 0, s>>>(points, jobs, scalars, n, out);
   else k_var_mul<<<blocks_for(n, 128), 128, 0, s>>>(points, jobs, scalars, n, out);
 }
 void share_carveout_g1() {
   share_carveout(k_g1_decode, k_g1_decode_pair, k_fixed_msm<128>, k_fixed_msm<512>, k_var_mul, k_var_mul_pair,
-                 k_var_mul_quad, k_var_mul_ladder, k_g1_subgroup_lane, k_g1_subgroup, k_g1_subgroup_quad,
+                 k_var_mul_quad, k_var_mul_ladder<true>, k_var_mul_ladder<false>, k_g1_subgroup_lane, k_g1_subgroup, k_g1_subgroup_quad,
                  k_g1_subgroup_ladder, k_g1_compress);
 }
 cudaError_t warm_decode_and_var_mul_kernels(uint8_t *any_device_buffer) {
@@ -504,7 +510,8 @@ cudaError_t warm_decode_and_var_mul_kernels(uint8_t *any_device_buffer) {
   k_var_mul<<<1, 128>>>(nullptr, nullptr, nullptr, 0, nullptr);
   k_var_mul_pair<<<1, 128>>>(nullptr, nullptr, nullptr, 0, nullptr);
   k_var_mul_quad<<<1, 128>>>(nullptr, nullptr, nullptr, 0, nullptr);
-  k_var_mul_ladder<<<1, 32>>>(nullptr, nullptr, nullptr, 0, nullptr);
+  k_var_mul_ladder<true><<<1, 64>>>(nullptr, nullptr, nullptr, 0, nullptr);
+  k_var_mul_ladder<false><<<1, 32>>>(nullptr, nullptr, nullptr, 0, nullptr);
   return cudaGetLastError();
 }
 void launch_g1_compress(cudaStream_t s, const g1 *pts, uint32_t n, uint8_t *out48) {

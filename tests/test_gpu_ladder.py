@@ -24,6 +24,19 @@ def test_terms(gpu, oracle, n):
     assert gpu.g1_msm_batch([([INF], [ks[3].to_bytes(32, "big")])] * n) == [(0, INF)] * n
 
 
+@pytest.mark.parametrize("n", [608, 609])
+def test_terms_shared_products(gpu, oracle, n):
+    """The most terms whose products two warps share, and one more."""
+    p1, gens = oracle.generators(4)
+    pts = [p1] + gens[:3]
+    ks = [scalar(b"shared", b"k", i) for i in range(n)]
+    ks[5], ks[n - 1] = bytes(32), (oracle.R_MOD - 1).to_bytes(32, "big")
+    got = gpu.g1_msm_batch([([pts[i % 4]], [ks[i]]) for i in range(n)])
+    assert all(c == 0 for c, _ in got)
+    for i in (0, 1, 5, 6, n // 2, n - 2, n - 1):
+        assert got[i][1] == oracle.g1_mul(pts[i % 4], ks[i]), i
+
+
 @pytest.mark.parametrize("n", [1, 3, 4, 6])
 def test_membership(gpu, oracle, n):
     p1, gens = oracle.generators(4)
