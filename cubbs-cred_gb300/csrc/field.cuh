@@ -421,7 +421,7 @@ DEV bool fr_lt_mod(const fr &a) {
 // A batch takes its steps on the low words of f and g, which gives a matrix of
 // entries at most 2^30 in absolute value, then applies it to f and g (exact
 // division by 2^30) and to d, e (mod r), which keep f = d x and g = e x; at the
-// end f = +-1.  About 45 thousand cycles on one lane where the 4-bit window
+// end f = +-1.  About 56 thousand cycles on one lane where the 4-bit window
 // x^(r-2) took 290 thousand.
 namespace inv_detail {
 struct signed288 { uint32_t w[9]; };

@@ -235,8 +235,7 @@ def wide_chain(lines, acc, xs, y, first_carry=False, carry_out=True, fresh=False
 
 
 def gen_mont(name, mod, n):
-    """{name}_mont_mul(r, a, b) = a b / 2^(32n) mod mod up to one mod too large, and {name}_mont_mul2(r, a, b, c, d)
-    = (a b + c d) / 2^(32n) the same way.
+    """{name}_mont_mul(r, a, b) = a b / 2^(32n) mod mod up to one mod too large.
 
     The running sum is kept in two arrays of n words: E at limbs 0..n-1 holds the products of even limb distance, O
     at limbs 1..n those of odd distance, so a row b_i adds its n products as two carry chains of n/2 64-bit
@@ -244,45 +243,37 @@ def gen_mont(name, mod, n):
     zero.  Dropping that limb turns O into the next E and E's words 2.. into the next O; the word E_1 left over is
     added to the next E_0 and its carry enters the next row's O chain.
     Bounds: the sum before a shift is below 2^32 (a + mod + the sum before), so operands with
-    a (+ c) < 2^(32n) - 3 mod never carry out of limb n, and the result is below mod + (a b (+ c d)) / 2^(32n)."""
+    a < 2^(32n) - 3 mod never carry out of limb n, and the result is below mod + a b / 2^(32n)."""
     assert n % 2 == 0
     ml = limbs(mod, n)
     pinv = (-pow(mod, -1, 1 << 32)) % (1 << 32)
     odd = [f"0x{ml[j]:08x}" for j in range(1, n, 2)]
     even = [f"0x{ml[j]:08x}" for j in range(0, n, 2)]
 
-    def build(pairs):
-        body = [f"{{ .reg .u32 x<{n}>; .reg .u32 y<{n}>; .reg .u32 m;"]
-        op = [[f"%{n * (k + 1) + j}" for j in range(n)] for k in range(2 * pairs)]
-        E, O = [f"x{j}" for j in range(n)], [f"y{j}" for j in range(n)]
-        for i in range(n):
-            for k in range(pairs):
-                a, b = op[2 * k], op[2 * k + 1][i]
-                if i == 0 and k == 0:
-                    wide_chain(body, O, a[1::2], b, fresh=True)
-                    wide_chain(body, E, a[0::2], b, fresh=True)
-                    continue
-                if k == 0:
-                    body.append(f"add.cc.u32 {E[0]}, {E[0]}, {left};")
-                wide_chain(body, O, a[1::2], b, first_carry=k == 0, carry_out=False, fresh_top=k == 0 and i > 0)
-                wide_chain(body, E, a[0::2], b)
-                body.append(f"addc.u32 {O[n - 1]}, {O[n - 1]}, 0;")
-            body.append(f"mul.lo.u32 m, {E[0]}, 0x{pinv:08x};")
-            wide_chain(body, O, odd, "m", carry_out=False)
-            wide_chain(body, E, even, "m")
+    body = [f"{{ .reg .u32 x<{n}>; .reg .u32 y<{n}>; .reg .u32 m;"]
+    a, b = [f"%{n + j}" for j in range(n)], [f"%{2 * n + j}" for j in range(n)]
+    E, O = [f"x{j}" for j in range(n)], [f"y{j}" for j in range(n)]
+    for i in range(n):
+        if i == 0:
+            wide_chain(body, O, a[1::2], b[i], fresh=True)
+            wide_chain(body, E, a[0::2], b[i], fresh=True)
+        else:
+            body.append(f"add.cc.u32 {E[0]}, {E[0]}, {left};")
+            wide_chain(body, O, a[1::2], b[i], first_carry=True, carry_out=False, fresh_top=True)
+            wide_chain(body, E, a[0::2], b[i])
             body.append(f"addc.u32 {O[n - 1]}, {O[n - 1]}, 0;")
-            left = E[1]
-            E, O = O, E[2:] + E[:2]  # the two top words of the new O count as zero (fresh_top)
-        body.append(f"add.cc.u32 %0, {E[0]}, {left};")
-        for j in range(1, n):
-            body.append(f"addc{'.cc' if j < n - 1 else ''}.u32 %{j}, {E[j]}, {O[j - 1] if j < n - 1 else '0'};")
-        body.append("}")
-        return body
-
+        body.append(f"mul.lo.u32 m, {E[0]}, 0x{pinv:08x};")
+        wide_chain(body, O, odd, "m", carry_out=False)
+        wide_chain(body, E, even, "m")
+        body.append(f"addc.u32 {O[n - 1]}, {O[n - 1]}, 0;")
+        left = E[1]
+        E, O = O, E[2:] + E[:2]  # the two top words of the new O count as zero (fresh_top)
+    body.append(f"add.cc.u32 %0, {E[0]}, {left};")
+    for j in range(1, n):
+        body.append(f"addc{'.cc' if j < n - 1 else ''}.u32 %{j}, {E[j]}, {O[j - 1] if j < n - 1 else '0'};")
+    body.append("}")
     return (f"// r = a b / 2^{32 * n} mod p, up to one p too large (interleaved Montgomery rows on even / odd carry "
-            f"chains).\n" + asm_fn(f"{name}_mont_mul", n, build(1), "ab")
-            + f"// r = (a b + c d) / 2^{32 * n} mod p, up to one p too large: one reduction for both products.\n"
-            + asm_fn(f"{name}_mont_mul2", n, build(2), "abcd"))
+            f"chains).\n" + asm_fn(f"{name}_mont_mul", n, body, "ab"))
 
 
 def gen_mont_sqr(name, mod, n):

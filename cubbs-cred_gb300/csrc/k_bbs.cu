@@ -1618,10 +1618,9 @@ void launch_agg_combine(cudaStream_t s, OpBatch &b, uint32_t G) {
 // fills only part of the GPU, so running them side by side shortens the step.
 // The SM partition is used when the batch's key groups fit its small part
 // two to an SM: the four streams are then those of the larger partition and
-// the aggregated pairing chain (the group sums and one check per key group,
+// the aggregated pairing chain (the last sums and one check per key group,
 // made of kernels that fill only a few SMs) runs alone on the smaller one;
-// sharing SMs with the MSM kernels stretched that chain from about 3.5 ms to
-// 5 ms.  With the third partition, stream2 (the decode and the variable-base
+// 1024 proofs of one key take 2.76 ms on the plain streams, 2.50 like this.  With the third partition, stream2 (the decode and the variable-base
 // terms) runs on it and the other three streams on the SMs left.  A batch with
 // more groups runs on the plain streams (64 keys of 16 proofs: 1.5 % faster on
 // the whole GPU than with the chain beside the MSM kernels on the larger part).

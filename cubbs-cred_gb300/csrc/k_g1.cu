@@ -396,12 +396,11 @@ int var_lanes_setting() {
 // Lanes per job for a launch of n jobs: the CUBBS_BBS_VAR_LANES setting, else
 // by size.  Few jobs leave the GPU idle, so each takes ladders of eight lanes
 // (g1_ladder.cuh); thousands fill it, where lane pairs spend fewer
-// instructions a job.  Measured on GB300, 8 lanes against 2: Verify of 64
-// (64 terms) 1.72 ms against 2.45 on the lane octets before the ladders,
-// Verify of 1000 (1000 terms) 2.79 against 3.43; ProofVerify of 1024 over 64
-// keys (4096 terms, 3072 points) 3.36 against 3.37; ProofGen of 1024 (7168
-// terms) 6.21 against 5.91.  Lane quads were slower than one or the other at
-// every size (3.78, 3.66 and 6.29 ms) and are left for the setting.
+// instructions a job.  Terms on GB300, 8 lanes against 2: 64 0.39 ms against
+// 1.16, 1000 0.49 against 1.16, 7168 1.46 against 1.16; whole calls at 4096
+// terms (ProofVerify of 1024 over 64 keys) were 3 % slower on 8 lanes, and
+// lane quads at every size slower than one or the other; those are left for
+// the setting.
 static int lanes_for(uint32_t n) {
   const int l = var_lanes_setting();
   return l ? l : n <= 2048 ? 8 : 2;

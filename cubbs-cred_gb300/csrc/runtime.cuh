@@ -222,11 +222,11 @@ struct Runtime {
   g1a *d_gens() const { return ss().d_gens; }
   uint8_t *d_gens_c() const { return ss().d_gens_c; }
   cudaStream_t stream = nullptr, stream2 = nullptr, stream3 = nullptr, stream4 = nullptr;
-  // stream -> stream2 (ev_fork), stream2 -> stream3, stream4 (ev_mid), back to stream
+  // stream -> the others (ev_fork), between them (ev_mid, ev_hash, ev_dec), back to stream
   // (ev_side, ev_join, ev_sub)
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_mid = nullptr, ev_side = nullptr, ev_sub = nullptr,
               ev_dec = nullptr;
-  cudaEvent_t ev_hash = nullptr;  // ProofVerify: message scalars ready (stream -> stream4)
+  cudaEvent_t ev_hash = nullptr;  // message scalars ready
   // ProofVerify on the SM partition: part[0..3] play stream..stream4 on the
   // larger partition, part_check runs the aggregated pairing chain on the
   // smaller one (all null without a partition)
