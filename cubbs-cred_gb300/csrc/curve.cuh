@@ -400,24 +400,61 @@ DEV g1 g1_add_pair(const LanePair &lp, const g1 &p, const g1 &q) {
   return r;
 }
 
-// [|z|]P on a lane pair.
-DEV g1 g1_mul_zabs_pair(const LanePair &lp, const g1 &p) {
-  g1 acc = p;
-  #pragma unroll 1
-  for (int i = 62; i >= 0; i--) {
-    acc = g1_dbl_pair(lp, acc);
-    if (zabs_bit(i)) acc = g1_add_pair(lp, acc, p);
+// g1j_dbl and g1j_add on a lane pair: four rounds a doubling, two of them
+// squares (XYZZ: five, one a square).
+DEV g1j g1j_dbl_pair(const LanePair &lp, const g1j &p) {
+  fp A, B, C, t, F, YZ;
+  pair_sqr(lp, p.X, p.Y, A, B);
+  pair_sqr(lp, B, fp_add(p.X, B), C, t);
+  const fp D = fp_dbl(fp_sub(fp_sub(t, A), C)), E = fp_add(fp_dbl(A), A);
+  pair_mul(lp, E, E, p.Y, p.Z, F, YZ);
+  g1j r;
+  r.X = fp_sub(F, fp_dbl(D));
+  r.Y = fp_sub(fp_mul(E, fp_sub(D, r.X)), fp_dbl(fp_dbl(fp_dbl(C))));  // same product on both lanes
+  r.Z = fp_dbl(YZ);
+  return r;
+}
+DEV g1j g1j_add_pair(const LanePair &lp, const g1j &p, const g1j &q) {
+  if (fp_is_zero(p.Z)) return q;
+  if (fp_is_zero(q.Z)) return p;
+  fp Z1, Z2, U1, U2, a, b, S1, S2;
+  pair_sqr(lp, p.Z, q.Z, Z1, Z2);
+  pair_mul(lp, p.X, Z2, q.X, Z1, U1, U2);
+  pair_mul(lp, p.Y, Z2, q.Y, Z1, a, b);
+  pair_mul(lp, a, q.Z, b, p.Z, S1, S2);
+  const fp H = fp_sub(U2, U1), R = fp_sub(S2, S1);
+  g1j r;
+  if (fp_is_zero(H)) {
+    if (fp_is_zero(R)) return g1j_dbl_pair(lp, p);
+    r.X = r.Y = fp_one();
+    r.Z = fp_zero();
+    return r;
   }
-  return acc;
+  fp HH, RR, HHH, V, ZZ, SH, T;
+  pair_sqr(lp, H, R, HH, RR);
+  pair_mul(lp, H, HH, U1, HH, HHH, V);
+  r.X = fp_sub(fp_sub(RR, HHH), fp_dbl(V));
+  pair_mul(lp, p.Z, q.Z, S1, HHH, ZZ, SH);
+  pair_mul(lp, ZZ, H, R, fp_sub(V, r.X), r.Z, T);
+  r.Y = fp_sub(T, SH);
+  return r;
 }
 // g1_in_subgroup on a lane pair.
 DEV bool g1_in_subgroup_pair(const LanePair &lp, g1a a) {
-  g1 t = g1_mul_zabs_pair(lp, g1_mul_zabs_pair(lp, g1_from_aff(a)));
-  if (g1_is_inf(t)) return false;
-  const fp beta = C_GLV_BETA;
-  fp bx = fp_mul(a.x, beta);
-  fp ny = fp_neg(a.y);
-  return fp_eq(t.X, fp_mul(bx, t.ZZ)) && fp_eq(t.Y, fp_mul(ny, t.ZZZ));
+  g1j t, p;
+  t.X = a.x;
+  t.Y = a.y;
+  t.Z = fp_one();
+  p = t;
+  #pragma unroll 1
+  for (int i = 125; i >= 0; i--) {
+    if (i == 62) p = t;
+    t = g1j_dbl_pair(lp, t);
+    if (zabs_bit(i > 62 ? i - 63 : i)) t = g1j_add_pair(lp, t, p);
+  }
+  if (fp_is_zero(t.Z)) return false;
+  const fp beta = C_GLV_BETA, zz = fp_sqr(t.Z);
+  return fp_eq(t.X, fp_mul(fp_mul(a.x, beta), zz)) && fp_eq(t.Y, fp_mul(fp_neg(a.y), fp_mul(zz, t.Z)));
 }
 // ---- point arithmetic on a lane quad
 // Lanes 4k .. 4k+3 hold the same operands and split each formula's
