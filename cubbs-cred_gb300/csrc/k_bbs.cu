@@ -1620,7 +1620,7 @@ void launch_agg_combine(cudaStream_t s, OpBatch &b, uint32_t G) {
 // two to an SM: the four streams are then those of the larger partition and
 // the aggregated pairing chain (the last sums and one check per key group,
 // made of kernels that fill only a few SMs) runs alone on the smaller one;
-// 1024 proofs of one key take 2.76 ms on the plain streams, 2.50 like this.  With the third partition, stream2 (the decode and the variable-base
+// 1024 proofs of one key take 2.76 ms on the plain streams, 2.40 like this.  With the third partition, stream2 (the decode and the variable-base
 // terms) runs on it and the other three streams on the SMs left.  A batch with
 // more groups runs on the plain streams (64 keys of 16 proofs: 1.5 % faster on
 // the whole GPU than with the chain beside the MSM kernels on the larger part).
@@ -1692,9 +1692,13 @@ void run_pverify(Runtime &rt, OpBatch &b, uint8_t *dmapdst) {
          launch_pairing_check(s3, b.pj, N, rt.d_lines, b.ok));
   }
   CUBBS_CHECK(cudaEventRecord(rt.ev_join, s3));
+  // on their own partition the ladders (a warp per two terms) last as long as
+  // one lane pair does from four warps a sub-partition on (512 proofs, 48 SMs:
+  // 2.22 -> 1.90 ms)
+  const int lanes = part && rt.sh.green_var && var_lanes_setting() == 0 && 4 * N > 32u * (uint32_t)rt.sh.var_sms ? 2 : 0;
   SPAN(s2, "var_mul",
        k_pv_jobs<<<blocks_for(n, 128), 128, 0, s2>>>(it0, N, b.dblob, b.dec, b.jobs, b.jscal);
-       launch_var_mul(s2, b.pts, b.jobs, b.jscal, 4 * N, b.v));
+       launch_var_mul(s2, b.pts, b.jobs, b.jscal, 4 * N, b.v, lanes));
   CUBBS_CHECK(cudaEventRecord(rt.ev_side, s2));
   SPAN(s, "domain", launch_domain(s, b.ddj, N, b.dblob, rt.d_gens_c(), rt.ss().d_dom_prefix, b.domain, rt.suite));
   SPAN(s, "scalar_prep",

@@ -204,14 +204,15 @@ void SharedState::init_partition() {
     destroy(gs);
     return (void)fail(10, r);
   }
-  // Optionally a third partition: CUBBS_BBS_VAR_SMS SMs (default 32; 0:
+  // Optionally a third partition: CUBBS_BBS_VAR_SMS SMs (default 48; 0:
   // none) taken from the larger one for the point decode and the
   // variable-base terms of ProofVerify, whose lane pairs then stop sharing
-  // issue slots with the fixed-base MSM and the subgroup check.  Measured on
-  // GB300 (1024 proofs, L = 100): 32 SMs 3.87 ms per step, 48 / 56 SMs 3.9 ms,
-  // 64 SMs 4.2 ms (the terms at one warp per SM sub-partition take 1.9 ms
-  // instead of 2.8, but the subgroup check on the 72 SMs left takes 3.2 ms),
-  // no third partition 4.2 ms.  The device's SMs are split into groups of 8
+  // issue slots with the fixed-base MSM and the subgroup check.  Whole calls
+  // on GB300 (1024 proofs, L = 100): 32 SMs 2.48 ms, 40 2.48, 48 2.40, 56
+  // 2.41, 64 2.6 or more, no partition 2.76: the decode's two warps per 32 points
+  // find a sub-partition each from 48 SMs on (0.36 -> 0.27 ms), and the
+  // fixed-base MSM lacks the SMs from 64 on.  512 proofs 2.81 ms on 32 SMs,
+  // 2.24 on 48, and 1.90 with lane pairs for their terms (run_pverify).  The device's SMs are split into groups of 8
   // in one call and the groups are joined into the three partitions (the
   // chain's partition then holds the first groups, as many SMs as the two-way
   // split gave it, and replaces that split's own small partition so that the
@@ -219,7 +220,7 @@ void SharedState::init_partition() {
   // is off; any failure here leaves the two-way split as it is.
   CUgreenCtx gv = nullptr, gr2 = nullptr, gs3 = nullptr;
   int var_count = 0, small3 = 0;
-  const int var_want = env_int("CUBBS_BBS_VAR_SMS", 32);
+  const int var_want = env_int("CUBBS_BBS_VAR_SMS", 48);
   var_status = 1;
   if (var_want > 0 && var_want + 16 <= (int)rest.sm.smCount) {
     constexpr unsigned GMAX = 64;
