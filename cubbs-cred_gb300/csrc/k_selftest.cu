@@ -461,3 +461,41 @@ extern "C" int32_t cubbs_bbs_gpu_int_peaks_v2(double *tera_imad, double *giga_fp
     return CUBBS_BBS_GPU_ERR_INTERNAL;
   }
 }
+
+// ------------------------------------------------------------------------- failed calls
+// About ten milliseconds of one warp.
+__global__ void k_busy(uint32_t *out) {
+#pragma unroll 1
+  for (int i = 0; i < 10000; i++) __nanosleep(1000);
+  *out = 1;
+}
+
+// A call that throws with work under way, kind 0: kernels on the side streams;
+// 1: a stream capture.  *idle = 1 when the workspace it gave back has no work,
+// no capture and no error left.
+extern "C" int32_t cubbs_bbs_gpu_failed_call_for_test_v2(int32_t kind, int32_t *idle) {
+  if (!idle || kind < 0 || kind > 1) return CUBBS_BBS_GPU_ERR_INVALID_INPUT;
+  *idle = 0;
+  Runtime *used = nullptr;
+  try {
+    CallScope scope;
+    Runtime &rt = scope.rt;
+    used = &rt;
+    uint32_t *o = rt.arena.alloc<uint32_t>(4);
+    if (kind == 1) CUBBS_CHECK(cudaStreamBeginCapture(rt.stream, cudaStreamCaptureModeThreadLocal));
+    k_busy<<<1, 1, 0, kind == 1 ? rt.stream : rt.stream2>>>(o);
+    if (kind == 0) k_busy<<<1, 1, 0, rt.stream4>>>(o + 1);
+    CUBBS_CHECK(cudaGetLastError());
+    throw CudaError(cudaErrorUnknown, "a call that fails");
+  } catch (const CudaError &) {
+    if (!used) return CUBBS_BBS_GPU_ERR_INTERNAL;
+  }
+  bool ok = cudaGetLastError() == cudaSuccess;
+  for (cudaStream_t s : {used->stream, used->stream2, used->stream3, used->stream4}) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusActive;
+    ok = ok && cudaStreamIsCapturing(s, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone &&
+         cudaStreamQuery(s) == cudaSuccess;
+  }
+  *idle = ok ? 1 : 0;
+  return 0;
+}

@@ -5,6 +5,7 @@
 // kernels/common_cache.cuh:112-486 and the canary probe cubbs_bbs_cuda.cu:719-824.
 #include <cstdlib>
 #include <cstring>
+#include <exception>
 
 #include "runtime.cuh"
 
@@ -526,6 +527,19 @@ Runtime::Runtime(SharedState &s)
   pack.reserve((size_t)64 << 20);
 }
 
+void Runtime::settle() {
+  for (cudaStream_t s : {stream, stream2, stream3, stream4, part[0], part[1], part[2], part[3], part_check}) {
+    if (!s) continue;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone) {
+      cudaGraph_t g = nullptr;
+      if (cudaStreamEndCapture(s, &g) == cudaSuccess && g) cudaGraphDestroy(g);
+    }
+    (void)cudaStreamSynchronize(s);
+  }
+  (void)cudaGetLastError();
+}
+
 // The workspace's streams on the SM partition, made the first time a call on
 // this workspace can use them (the workspace belongs to one call at a time).
 bool Runtime::use_partition() {
@@ -706,7 +720,7 @@ void release_workspace(Runtime &rt) {
 }
 }  // namespace
 
-CallScope::CallScope() : rt(acquire_workspace()), lock(rt.sh.mu) {
+CallScope::CallScope() : rt(acquire_workspace()), lock(rt.sh.mu), unwinding(std::uncaught_exceptions()) {
   rt.lock = &lock;
   rt.suite = SUITE_SHA256;
   rt.arena.reset();
@@ -715,6 +729,7 @@ CallScope::CallScope() : rt(acquire_workspace()), lock(rt.sh.mu) {
 }
 
 CallScope::~CallScope() {
+  if (std::uncaught_exceptions() > unwinding) rt.settle();
   rt.lock = nullptr;
   lock.unlock();
   release_workspace(rt);

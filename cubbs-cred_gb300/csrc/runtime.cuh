@@ -241,6 +241,10 @@ struct Runtime {
   std::shared_lock<std::shared_mutex> *lock = nullptr;  // the running call's shared hold
 
   explicit Runtime(SharedState &s);
+  // Drops a stream capture under way and waits for every stream.  Work that a
+  // failed call has left on one stream is not ordered before the next call's
+  // work on another, which would use the same arena.
+  void settle();
   // true when part[] / part_check exist (makes the shared partition and this
   // workspace's streams on it the first time)
   bool use_partition();
@@ -257,10 +261,12 @@ struct Runtime {
 
 // Takes a free workspace from the pool (waiting while all are busy), makes the
 // device current on the calling thread, holds the prepared state shared and
-// resets the workspace's arena and staging.  Released on destruction.
+// resets the workspace's arena and staging.  Released on destruction; a call
+// that leaves by an exception waits for its streams first (Runtime::settle).
 struct CallScope {
   Runtime &rt;
   std::shared_lock<std::shared_mutex> lock;
+  const int unwinding;  // exceptions in flight when the call began
   CallScope();
   ~CallScope();
   CallScope(const CallScope &) = delete;
