@@ -1729,6 +1729,10 @@ void run_pverify(Runtime &rt, OpBatch &b, uint8_t *dmapdst) {
 // and the MSMs fill them several times: one launch for both bases then, with the
 // T2 MSM in what it leaves free.
 const size_t PG_APART_JOBS = 2048;  // the ladders' limit, k_g1.cu
+// Lanes per point of the subgroup check there.  It is done long before the MSMs
+// are, so it takes the form with the fewest instructions at any size (1024
+// proofs: 3.66 -> 3.58 ms), unless CUBBS_BBS_VAR_LANES says otherwise.
+int pg_subgroup_lanes(uint32_t npts) { return npts > 512 && !var_lanes_setting() ? 2 : subgroup_lanes(npts); }
 void run_pgen(Runtime &rt, OpBatch &b, uint8_t *dmapdst) {
   cudaStream_t s = rt.stream3, s2 = rt.stream2, sa = rt.stream, s4 = rt.stream4;
   size_t n = b.n, nm = b.ml.count(), npts = b.pts48.size() / 48;
@@ -1773,9 +1777,7 @@ void run_pgen(Runtime &rt, OpBatch &b, uint8_t *dmapdst) {
                                           it0, N, b.dblob, b.msc, b.rs, rss, reinterpret_cast<hash_ctx<S> *>(b.chal),
                                           b.r3inv)));
   CUBBS_CHECK(cudaStreamWaitEvent(s4, rt.ev_dec, 0));
-  // the check is done long before the MSMs are, so it takes the form with the
-  // fewest instructions at any size (1024 proofs: 3.66 -> 3.58 ms)
-  SPAN(s4, "g1_subgroup", launch_g1_subgroup(s4, b.pts, b.dec, (uint32_t)npts, b.sub, npts > 512 ? 2 : 0));
+  SPAN(s4, "g1_subgroup", launch_g1_subgroup(s4, b.pts, b.dec, (uint32_t)npts, b.sub, pg_subgroup_lanes((uint32_t)npts)));
   CUBBS_CHECK(cudaEventRecord(rt.ev_sub, s4));
   CUBBS_CHECK(cudaStreamWaitEvent(s, rt.ev_mid, 0));
   SPAN(s, "var_mul",
@@ -2606,6 +2608,9 @@ extern "C" int32_t cubbs_bbs_gpu_proof_gen_seeded_batch_cs_v2(uint32_t abi, uint
   if (n == 0) return CUBBS_BBS_GPU_SUCCESS;
   return proof_gen_impl((int)suite, items, n, seeds, results);
 }
+
+// Test export: lanes per point of the subgroup check in a ProofGen call of n items.
+extern "C" int32_t cubbs_bbs_gpu_proof_gen_check_lanes_for_test_v2(size_t n) { return pg_subgroup_lanes((uint32_t)n); }
 
 // ----------------------------------------------------------------------------- device-resident timing
 // Benchmark entry (outside the reference ABI): packs and uploads one batch of

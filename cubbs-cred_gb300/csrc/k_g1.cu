@@ -406,11 +406,13 @@ static int lanes_for(uint32_t n) {
   return l ? l : n <= 2048 ? 8 : 2;
 }
 
+// Above one warp per SM sub-partition (152 x 4) of points, one lane each: the
+// Jacobian doublings there cost seven products' time, the pair's ten.
+int subgroup_lanes(uint32_t n) { return n > 19456 && !var_lanes_setting() ? 1 : lanes_for(n); }
+
 void launch_g1_subgroup(cudaStream_t s, g1a *pts, int32_t *status, uint32_t n, int32_t *bad, int lanes) {
   if (!n) return;
-  // Above one warp per SM sub-partition (152 x 4) of points, one lane each: the
-  // Jacobian doublings there cost seven products' time, the pair's ten.
-  if (lanes == 0) lanes = n > 19456 && !var_lanes_setting() ? 1 : lanes_for(n);
+  if (lanes == 0) lanes = subgroup_lanes(n);
   if (lanes == 8) k_g1_subgroup_ladder<<<blocks_for(n, 4), 32, 0, s>>>(pts, status, n, bad);
   else if (lanes == 4) k_g1_subgroup_quad<<<blocks_for(4 * (size_t)n, 64), 64, 0, s>>>(pts, status, n, bad);
   else if (lanes == 2) k_g1_subgroup<<<blocks_for(2 * (size_t)n, 32), 32, 0, s>>>(pts, status, n, bad);

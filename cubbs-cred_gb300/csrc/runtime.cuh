@@ -312,6 +312,7 @@ void launch_build_table(cudaStream_t s, const g1a *gens, int g0, int g1n, FixedT
 void launch_g1_subgroup(cudaStream_t s, g1a *pts, int32_t *status, uint32_t n, int32_t *bad,
                         int lanes = 0);
 int var_lanes_setting();
+int subgroup_lanes(uint32_t n);  // what 0 stands for
 void launch_g1_decode(cudaStream_t s, const uint8_t *pts48, uint32_t stride, uint32_t n, g1a *out,
                       int32_t *status, bool check_subgroup);
 // fixed-base MSM rows: scalars raw Fr [row * stride + g] for g < nterms[row]

@@ -112,6 +112,9 @@ int32_t cubbs_bbs_gpu_hash_to_scalar_shake256_batch_for_test_v2(uint32_t abi_ver
 int32_t cubbs_bbs_gpu_proof_verify_phases_for_test_v2(const CuBbsBbsGpuProofVerifyItem *items, size_t n,
                                                       CuBbsBbsGpuResult *results, double *ms6);
 
+/* Lanes per point of the subgroup check in a ProofGen call of n items (no device work). */
+int32_t cubbs_bbs_gpu_proof_gen_check_lanes_for_test_v2(size_t n);
+
 /* A call that throws with work under way (kind 0: kernels on the side streams, 1: a stream capture);
  * *idle = 1 when the workspace it gave back has neither work nor a capture left. */
 int32_t cubbs_bbs_gpu_failed_call_for_test_v2(int32_t kind, int32_t *idle);
