@@ -493,7 +493,8 @@ def prepared_common_points_call(points, rows):
 def msm_uneven_bench(n_msms=16384, k_min=2, k_max=257, seed=4, tune=True, warmup=3, steps=5):
     """Uneven variable-base MSM benchmark (points u*P1 and scalars generated on the
     device from `seed`).  Returns dict(ms=[per replay], decode_ms, chunk=[per size
-    class], window=[per size class], checked, mismatch)."""
+    class], window=[per size class], mode=[per size class] as msm_tuning() gives
+    them, checked, mismatch)."""
     ms = (ctypes.c_float * steps)()
     dec = ctypes.c_float(0)
     tun = (ctypes.c_uint32 * 12)()
@@ -516,7 +517,8 @@ def msm_tuning(chunk=None, window=None, mode=None):
     """Uneven-MSM engine settings per size class (K <= 8, <= 32, <= 96, larger):
     with chunk, window and mode (4 values each; mode 0 thread, 1 warp; mode
     defaults to thread) they replace the process's settings.  Returns the
-    (chunk, window, mode) lists in force."""
+    (chunk, window, mode) lists in force; mode 2 of every class: no settings,
+    the MSMs are split by window and chunk (as input: settings taken back)."""
     fn = lib().cubbs_bbs_gpu_msm_tuning_v2
     fn.restype = ctypes.c_int32
     fn.argtypes = [ctypes.c_void_p] * 6

@@ -20,10 +20,10 @@
 // launch.  A second kernel sums the partials of each MSM (one warp per MSM)
 // and compresses the result.  Mode, chunk length t and window c are chosen
 // per size class of K by an autotuner (t >= K: one lane per MSM; t < K: the
-// MSM is spread over several lanes and joined by the reduction).  While the
-// settings are the initial ones and no pairing checks share the launch, the
-// MSMs are split over lanes by window and chunk instead (k_msm_windows), which
-// is faster at every size measured.  The
+// MSM is spread over several lanes and joined by the reduction).  While no
+// caller has made settings and no pairing checks share the launch, the MSMs are
+// split over lanes by window and chunk instead (k_msm_windows), which was the
+// faster way at every size measured.  The
 // general MSM entry point replays the engine's kernels from captured CUDA
 // graphs (k_prims.cu).
 //
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(128) k_msm_reduce(const g1 *partials, const ui
 }
 
 // ---------------------------------------------------------------- split windows
-// Without settings of the caller's own, an MSM is split over lanes by window as
+// Without settings made by a caller, an MSM is split over lanes by window as
 // well as by chunk: a lane takes one window of one chunk, so it doubles nothing,
 // and a batch of a thousand MSMs has tens of thousands of lanes (thread mode:
 // 4700, a quarter of the GPU's sub-partitions with one warp each).  The lanes of
@@ -589,7 +589,7 @@ void MsmPlan::build(const std::vector<uint32_t> &K, const MsmTuning &tune, uint3
   units.clear();
   chunks.clear();
   split_c = 0;
-  if (pairings == 0 && tune == MsmTuning()) {
+  if (pairings == 0 && tune.split) {
     build_split(K);
     return;
   }
@@ -862,8 +862,8 @@ MsmWork make_work(Runtime &rt, cudaStream_t s, uint64_t seed, const std::vector<
   return w;
 }
 
-// mean ms of `reps` engine runs (prep + persistent launch + reduction) on `w` with `tune`;
-// the kernels are the same for every candidate, so no warm-up run is needed
+// mean ms of `reps` runs (prep, MSMs, join or reduction) on `w` with `tune`; the kernels are
+// the same for every candidate of the engine, so only the first needs a warm-up run
 float time_engine(Runtime &rt, cudaStream_t s, const MsmWork &w, const MsmTuning &tune, int reps, uint8_t *out48,
                   cudaEvent_t e0, cudaEvent_t e1) {
   MsmPlan p;
@@ -895,18 +895,19 @@ using namespace cubbs;
 
 // Uneven MSM benchmark (config 4): n_msms MSMs with K ~ U{k_min..k_max} drawn
 // from `seed`, points u * P1 and scalars uniform mod r generated on the
-// device.  With tune != 0 the mode, chunk length and window of each size
-// class are chosen by timing candidates on a sample of the same size and K
-// distribution (coordinate descent, largest class first), and kept for later
-// g1_msm_batch_v2 calls.  The engine (prep + persistent launch +
-// reduction) is captured in a CUDA graph and replayed warmup + steps times
+// device.  With tune != 0 the engine's mode, chunk length and window of each
+// size class are chosen by timing candidates on a sample of the same size and
+// K distribution (coordinate descent, largest class first); then split windows
+// are timed on the sample, and the faster way is kept for later
+// g1_msm_batch_v2 calls.  The kernels of the way in use (prep, MSMs, join or
+// reduction) are captured in a CUDA graph and replayed warmup + steps times
 // with a 256 MiB L2 flush before each; ms_out gets the timed replays.
 // decode_ms: decompression with subgroup check of all points (the work the
 // ABI path adds).  checked/mismatch: the first 64 MSMs recomputed with one GLV
 // multiplication per term and compared.  tuning_out[3 * MSM_CLASSES]: chunk
-// lengths, windows, then modes (0 thread, 1 warp) per size class.  The
-// autotuner tries thread mode (chunks of 4..64 terms, windows 4..7) and warp
-// mode (windows 4..12) for every class.
+// lengths, windows, then modes (0 thread, 1 warp) per size class, or mode 2 of
+// every class for split windows.  The autotuner tries thread mode (chunks of
+// 4..64 terms, windows 4..7) and warp mode (windows 4..12) for every class.
 extern "C" int32_t cubbs_bbs_gpu_msm_uneven_bench_v2(uint32_t abi, size_t n_msms, uint32_t k_min, uint32_t k_max,
                                                     uint64_t seed, int32_t tune, int32_t warmup, int32_t steps,
                                                     float *ms_out, float *decode_ms, uint32_t *tuning_out,
@@ -926,6 +927,7 @@ extern "C" int32_t cubbs_bbs_gpu_msm_uneven_bench_v2(uint32_t abi, size_t n_msms
     MsmPlan widest;
     {
       MsmTuning t;
+      t.split = false;
       for (int c = 0; c < MSM_CLASSES; c++) {
         t.mode[c] = MSM_MODE_WARP;
         t.window[c] = MSM_WARP_C_MAX;
@@ -953,6 +955,7 @@ extern "C" int32_t cubbs_bbs_gpu_msm_uneven_bench_v2(uint32_t abi, size_t n_msms
       size_t mark = rt.arena.used;
       MsmWork w = make_work(rt, s, seed ^ 0x77ull, draw_k(seed + 99, ns, k_min, k_max));
       uint8_t *o = rt.arena.alloc<uint8_t>(48 * ns);
+      best.split = false;
       time_engine(rt, s, w, best, 1, o, e0, e1);  // first launch of the kernels, untimed
       float cur = time_engine(rt, s, w, best, 1, o, e0, e1);
       for (int cls = MSM_CLASSES - 1; cls >= 0; cls--) {
@@ -984,14 +987,12 @@ extern "C" int32_t cubbs_bbs_gpu_msm_uneven_bench_v2(uint32_t abi, size_t n_msms
           }
         }
       }
+      time_engine(rt, s, w, MsmTuning(), 1, o, e0, e1);
+      if (time_engine(rt, s, w, MsmTuning(), 1, o, e0, e1) <= cur) best = MsmTuning();
       rt.arena.used = mark;
       rt.set_msm_tuning(best);
     }
-    for (int c = 0; c < MSM_CLASSES; c++) {
-      tuning_out[c] = best.chunk[c];
-      tuning_out[MSM_CLASSES + c] = best.window[c];
-      tuning_out[2 * MSM_CLASSES + c] = best.mode[c];
-    }
+    best.write(tuning_out, tuning_out + MSM_CLASSES, tuning_out + 2 * MSM_CLASSES);
     // ---- the workload
     MsmWork w = make_work(rt, s, seed, K);
     // decode cost of the same points (compress, then decompress + subgroup check)
@@ -1068,39 +1069,43 @@ extern "C" int32_t cubbs_bbs_gpu_msm_uneven_bench_v2(uint32_t abi, size_t n_msms
 // larger): mode (0 thread, 1 warp), chunk length (terms per lane, 1..256;
 // thread mode) and window width (4..7 in thread mode, 4..12 in warp mode).
 // Non-null chunk_in / window_in / mode_in replace the process's settings (all
-// three or none; out-of-range values are rejected), then the settings in
-// force are written to the non-null outputs.
+// three or none; out-of-range values are rejected), whatever their values; mode
+// 2 of every class takes settings back (split windows, chunk and window not
+// read), so that what the outputs gave can be set again.  Then the settings in
+// force are written to the non-null outputs: mode 2 of every class while there
+// are none.
 extern "C" int32_t cubbs_bbs_gpu_msm_tuning_v2(const uint32_t *chunk_in, const uint32_t *window_in,
                                                const uint32_t *mode_in, uint32_t *chunk_out, uint32_t *window_out,
                                                uint32_t *mode_out) {
   if ((chunk_in == nullptr) != (window_in == nullptr) || (chunk_in == nullptr) != (mode_in == nullptr))
     return CUBBS_BBS_GPU_ERR_INVALID_INPUT;
-  if (chunk_in)
-    for (int c = 0; c < MSM_CLASSES; c++) {
-      const uint32_t cmax = mode_in[c] == MSM_MODE_WARP ? MSM_WARP_C_MAX : MSM_THREAD_C_MAX;
-      if (mode_in[c] > MSM_MODE_WARP || chunk_in[c] < 1 || chunk_in[c] > 256 || window_in[c] < 4 ||
-          window_in[c] > cmax)
-        return CUBBS_BBS_GPU_ERR_INVALID_INPUT;
-    }
+  MsmTuning t;
+  if (chunk_in && !t.read(chunk_in, window_in, mode_in)) return CUBBS_BBS_GPU_ERR_INVALID_INPUT;
   try {
     CallScope scope;
     Runtime &rt = scope.rt;
-    if (chunk_in) {
-      MsmTuning t;
-      for (int c = 0; c < MSM_CLASSES; c++) {
-        t.chunk[c] = chunk_in[c];
-        t.window[c] = window_in[c];
-        t.mode[c] = mode_in[c];
-      }
-      rt.set_msm_tuning(t);
-    }
-    for (int c = 0; c < MSM_CLASSES; c++) {
-      if (chunk_out) chunk_out[c] = rt.sh.msm_tuning.chunk[c];
-      if (window_out) window_out[c] = rt.sh.msm_tuning.window[c];
-      if (mode_out) mode_out[c] = rt.sh.msm_tuning.mode[c];
-    }
+    if (chunk_in) rt.set_msm_tuning(t);
+    rt.sh.msm_tuning.write(chunk_out, window_out, mode_out);
     return CUBBS_BBS_GPU_SUCCESS;
   } catch (const CudaError &) {
     return CUBBS_BBS_GPU_ERR_INTERNAL;
   }
+}
+
+// Test export: the plan of a batch of MSMs of K[0..n) terms (host work alone).
+extern "C" int32_t cubbs_bbs_gpu_msm_plan_for_test_v2(const uint32_t *K, size_t n, int32_t sms,
+                                                      const uint32_t *chunk_in, const uint32_t *window_in,
+                                                      const uint32_t *mode_in, uint64_t *plan8) {
+  if ((n && !K) || sms <= 0 || !plan8 || (chunk_in == nullptr) != (window_in == nullptr) ||
+      (chunk_in == nullptr) != (mode_in == nullptr))
+    return CUBBS_BBS_GPU_ERR_INVALID_INPUT;
+  MsmTuning t;
+  if (chunk_in && !t.read(chunk_in, window_in, mode_in)) return CUBBS_BBS_GPU_ERR_INVALID_INPUT;
+  MsmPlan p;
+  p.build(std::vector<uint32_t>(K, K + n), t);
+  uint32_t longest = 0;
+  for (const MsmChunk &c : p.chunks) longest = std::max(longest, c.count);
+  const uint64_t v[8] = {p.split_c, longest, p.chunks.size(), p.units.size(), 0, 0, 0, 0};
+  std::copy(v, v + 8, plan8);
+  return CUBBS_BBS_GPU_SUCCESS;
 }

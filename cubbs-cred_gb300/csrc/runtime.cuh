@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <condition_variable>
 #include <memory>
 #include <mutex>
@@ -89,17 +90,41 @@ struct PkSlot {
 #define MSM_CLASSES 4  // K <= 8, <= 32, <= 96, larger
 #define MSM_MODE_THREAD 0u
 #define MSM_MODE_WARP 1u
+#define MSM_MODE_SPLIT 2u  // of every class together: no settings made (MsmTuning::split)
 #define MSM_THREAD_C_MAX 7
 #define MSM_WARP_C_MAX 12
 #define MSM_WARP_SMEM_C_MAX 10  // warp-mode buckets in shared memory up to this window, global memory beyond
 struct MsmTuning {
+  // No caller has made settings: MSMs alone in a launch take split windows
+  // (k_msm_windows), and the values below are for those beside pairing checks.
+  bool split = true;
   // measured on GB300 over 16384 MSMs with K ~ U{2..257}: 120.7k MSMs/s
   uint32_t chunk[MSM_CLASSES] = {8, 16, 32, 32};
   uint32_t window[MSM_CLASSES] = {4, 4, 4, 4};
   uint32_t mode[MSM_CLASSES] = {MSM_MODE_THREAD, MSM_MODE_THREAD, MSM_MODE_THREAD, MSM_MODE_THREAD};
-  bool operator==(const MsmTuning &o) const {
-    return std::equal(chunk, chunk + MSM_CLASSES, o.chunk) && std::equal(window, window + MSM_CLASSES, o.window) &&
-           std::equal(mode, mode + MSM_CLASSES, o.mode);
+  // The settings as chunk[], window[], mode[] values: `split` is mode 2 of every class.
+  void write(uint32_t *chunk_out, uint32_t *window_out, uint32_t *mode_out) const {
+    for (int c = 0; c < MSM_CLASSES; c++) {
+      if (chunk_out) chunk_out[c] = chunk[c];
+      if (window_out) window_out[c] = window[c];
+      if (mode_out) mode_out[c] = split ? MSM_MODE_SPLIT : mode[c];
+    }
+  }
+  // From such values; false when one is out of range.
+  bool read(const uint32_t *chunk_in, const uint32_t *window_in, const uint32_t *mode_in) {
+    *this = MsmTuning();
+    if (std::all_of(mode_in, mode_in + MSM_CLASSES, [](uint32_t m) { return m == MSM_MODE_SPLIT; })) return true;
+    split = false;
+    for (int c = 0; c < MSM_CLASSES; c++) {
+      const uint32_t cmax = mode_in[c] == MSM_MODE_WARP ? MSM_WARP_C_MAX : MSM_THREAD_C_MAX;
+      if (mode_in[c] > MSM_MODE_WARP || chunk_in[c] < 1 || chunk_in[c] > 256 || window_in[c] < 4 ||
+          window_in[c] > cmax)
+        return false;
+      chunk[c] = chunk_in[c];
+      window[c] = window_in[c];
+      mode[c] = mode_in[c];
+    }
+    return true;
   }
 };
 struct MsmChunk {

@@ -47,15 +47,17 @@ int32_t cubbs_bbs_gpu_fixed_msm_autotune_v2(uint32_t abi_version, const uint8_t 
 /* Uneven-MSM engine settings per size class (K <= 8, <= 32, <= 96, larger):
  * mode (0: thread per chunk of `chunk` terms, window 4..7; 1: warp per MSM,
  * window 4..12), chunk length and window width; non-null inputs replace them,
- * non-null outputs receive the settings in force. */
+ * non-null outputs receive the settings in force.  Mode 2 of every class: no
+ * settings, MSMs alone in a launch are split by window and chunk. */
 int32_t cubbs_bbs_gpu_msm_tuning_v2(const uint32_t *chunk_in, const uint32_t *window_in, const uint32_t *mode_in,
                                     uint32_t *chunk_out, uint32_t *window_out, uint32_t *mode_out);
 
 /* ---- benchmarks */
 
 /* Uneven variable-base MSM benchmark: n_msms MSMs with K ~ U{k_min..k_max}
- * generated on the device from `seed`; optional autotuning (tuning_out: 12
- * values, chunk / window / mode per size class); CUDA-graph replays
+ * generated on the device from `seed`; optional autotuning (the engine's
+ * settings, then those against split windows; tuning_out: 12 values, chunk /
+ * window / mode per size class, as msm_tuning_v2 gives them); CUDA-graph replays
  * (ms_out[steps]); decode cost; the first 64 MSMs rechecked. */
 int32_t cubbs_bbs_gpu_msm_uneven_bench_v2(uint32_t abi_version, size_t n_msms, uint32_t k_min, uint32_t k_max,
                                          uint64_t seed, int32_t tune, int32_t warmup, int32_t steps, float *ms_out,
@@ -114,6 +116,12 @@ int32_t cubbs_bbs_gpu_proof_verify_phases_for_test_v2(const CuBbsBbsGpuProofVeri
 
 /* Lanes per point of the subgroup check in a ProofGen call of n items (no device work). */
 int32_t cubbs_bbs_gpu_proof_gen_check_lanes_for_test_v2(size_t n);
+
+/* How an MSM batch of K[0..n) terms is run on `sms` SMs under the settings (as msm_tuning_v2 takes
+ * them; null: none made), without device work: plan8 = window width of split windows (0: the
+ * engine), terms of the largest chunk, chunks, units of the engine, and four zeros. */
+int32_t cubbs_bbs_gpu_msm_plan_for_test_v2(const uint32_t *K, size_t n, int32_t sms, const uint32_t *chunk_in,
+                                           const uint32_t *window_in, const uint32_t *mode_in, uint64_t *plan8);
 
 /* A call that throws with work under way (kind 0: kernels on the side streams, 1: a stream capture);
  * *idle = 1 when the workspace it gave back has neither work nor a capture left. */
