@@ -593,9 +593,11 @@ DEV g1 shfl_down_g1(const g1 &p, int delta) {
   }
   return r;
 }
-DEV g1 warp_sum_g1(g1 acc) {
+// Sum over groups of `lanes` lanes (a power of two), on each group's first lane;
+// every lane of the warp calls it.
+DEV g1 group_sum_g1(g1 acc, uint32_t lanes) {
   #pragma unroll 1
-  for (int d = 16; d > 0; d >>= 1) {
+  for (int d = (int)lanes / 2; d > 0; d >>= 1) {
     g1 o = shfl_down_g1(acc, d);
     acc = g1_add(acc, o);
   }

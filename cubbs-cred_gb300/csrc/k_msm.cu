@@ -31,6 +31,7 @@
 // 337-644) and the Pippenger kernel (kernels/large_msm.cuh:322-416).
 #include <algorithm>
 #include <cstdlib>
+#include <cmath>
 #include <cstring>
 #include <vector>
 
@@ -486,15 +487,23 @@ __global__ void __launch_bounds__(64) k_msm_windows(const g1a *pts, const VarJob
   partials[(size_t)ch.slot * NWIN + w] = run;
 }
 
-// A lane per window of an MSM: the chunks' partials added, as a projective
-// triple on the ladders' curve.
-__global__ void __launch_bounds__(64) k_msm_join(const uint32_t *pstart, uint32_t n, uint32_t nwin, const g1 *partials,
-                                                 fp *triples) {
-  const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x, i = e / nwin, w = e - i * nwin;
-  if (i >= n) return;
+// A lane per window of an MSM, or `lanes` of them where the longest MSM has more
+// than eight chunks (msm_join_lanes): the chunks' partials added, as a projective
+// triple on the ladders' curve.  Bound by one lane's chain of additions: one MSM
+// of 524288 terms among 39 of 8 spent 54 ms of a 132 ms call here on one lane
+// (a call of 74 ms now; the persistent engine's took 130).
+__global__ void __launch_bounds__(64) k_msm_join(const uint32_t *pstart, uint32_t n, uint32_t nwin, uint32_t lanes,
+                                                 const g1 *partials, fp *triples) {
+  const size_t x = (size_t)blockIdx.x * blockDim.x + threadIdx.x, e = x / lanes;
+  const uint32_t sub = (uint32_t)x & (lanes - 1), i = (uint32_t)min(e / nwin, (size_t)n), w = (uint32_t)(e % nwin);
   g1 acc = g1_inf();
+  if (i < n) {
 #pragma unroll 1
-  for (uint32_t k = pstart[i]; k < pstart[i + 1]; k++) acc = g1_add_inl(acc, partials[(size_t)k * nwin + w]);
+    for (uint32_t k = pstart[i] + sub; k < pstart[i + 1]; k += lanes)
+      acc = g1_add_inl(acc, partials[(size_t)k * nwin + w]);
+  }
+  acc = group_sum_g1(acc, lanes);
+  if (i >= n || sub) return;
   const fp s2 = C_B3_S2, s3 = C_B3_S3;
   fp t[3];
   gl::put_triple(t, acc);
@@ -536,6 +545,12 @@ __global__ void __launch_bounds__(32) k_msm_horner(const fp *triples, uint32_t n
 }
 
 // ------------------------------------------------------------------ host plan
+// Lanes that add the partials of one window of an MSM of at most `chunks` chunks.
+static uint32_t msm_join_lanes(uint32_t chunks) {
+  uint32_t lanes = 1;
+  while (lanes < 32 && 8 * lanes < chunks) lanes *= 2;
+  return lanes;
+}
 // Window and chunk length of a batch in split windows: the least of what the
 // products take when every sub-partition has several warps (1215 cycles a
 // product, field.cuh) plus half of the longest lane, which runs alone at the
@@ -550,13 +565,16 @@ void MsmPlan::build_split(const std::vector<uint32_t> &K) {
     for (uint32_t k : K) parts += (k + t - 1) / t;
     for (uint32_t c = 3; c <= 5; c++) {
       const double digit = 20 * (1 - 1.0 / (1u << c)), fold = 14.0 * ((1u << (c - 1)) - 1);
-      const double lane = digit * std::min(t, longest) + fold, join = 14.0 * ((longest + t - 1) / t);
+      const uint32_t chunks = (longest + t - 1) / t, lanes = msm_join_lanes(chunks);
+      const double lane = digit * std::min(t, longest) + fold,
+                   join = 14.0 * ((chunks + lanes - 1) / lanes + std::log2(lanes));
       const double all = (digit * terms + fold * parts) * msm_windows(c) * 1215 / (128.0 * sms);
       const double cost = std::max(all + 0.5 * 1816 * lane, 1816 * lane) + 1816 * join;
       if (best_t == 0 || cost < best) {
         best = cost;
         best_t = t;
         split_c = c;
+        join_lanes = lanes;
       }
     }
   }
@@ -589,6 +607,7 @@ void MsmPlan::build(const std::vector<uint32_t> &K, const MsmTuning &tune, uint3
   units.clear();
   chunks.clear();
   split_c = 0;
+  join_lanes = 1;
   if (pairings == 0 && tune.split) {
     build_split(K);
     return;
@@ -705,6 +724,7 @@ void MsmDevice::upload(Runtime &rt, const MsmPlan &p, cudaStream_t s) {
   counter = rt.arena.alloc<uint32_t>(2);  // [0] next unit, [1] units skipped for want of room
   engine_shape(p, rt.sm_count, warps_per_block, smem_per_warp, grid, gbucket_stride);
   split_c = p.split_c;
+  join_lanes = p.join_lanes;
   if (split_c) {
     triples = rt.arena.alloc<fp>(3 * (size_t)n * msm_windows(split_c));
     sums = rt.arena.alloc<g1>(n ? n : 1);
@@ -742,7 +762,8 @@ void launch_msm_main(cudaStream_t s, const MsmDevice &d, const g1a *pts, const V
     }
     if (!d.n) return;
     g1 *sums = out ? out : d.sums;
-    k_msm_join<<<blocks_for((size_t)d.n * nwin, 64), 64, 0, s>>>(d.pstart, d.n, nwin, d.partials, d.triples);
+    k_msm_join<<<blocks_for((size_t)d.n * nwin * d.join_lanes, 64), 64, 0, s>>>(d.pstart, d.n, nwin, d.join_lanes,
+                                                                                d.partials, d.triples);
     k_msm_horner<<<blocks_for(d.n, 4), 32, 0, s>>>(d.triples, d.n, nwin, d.split_c, sums);
     if (out48) launch_g1_compress(s, sums, d.n, out48);
     return;
@@ -1105,7 +1126,7 @@ extern "C" int32_t cubbs_bbs_gpu_msm_plan_for_test_v2(const uint32_t *K, size_t 
   p.build(std::vector<uint32_t>(K, K + n), t);
   uint32_t longest = 0;
   for (const MsmChunk &c : p.chunks) longest = std::max(longest, c.count);
-  const uint64_t v[8] = {p.split_c, longest, p.chunks.size(), p.units.size(), 0, 0, 0, 0};
+  const uint64_t v[8] = {p.split_c, longest, p.chunks.size(), p.units.size(), p.join_lanes, 0, 0, 0};
   std::copy(v, v + 8, plan8);
   return CUBBS_BBS_GPU_SUCCESS;
 }

@@ -152,6 +152,7 @@ struct MsmPlan {
   uint32_t max_warp_smem_c = 0;   // widest warp-mode window with buckets in shared memory (0: none)
   uint32_t pair_units = 0;
   uint32_t split_c = 0;           // split windows of this width (k_msm_windows); 0: the persistent engine
+  uint32_t join_lanes = 1;        // lanes that add a window's partials (k_msm_join)
   uint32_t sms = 152;             // of the device the plan is for
   void build_split(const std::vector<uint32_t> &K);
   void build(const std::vector<uint32_t> &K, const MsmTuning &tune, uint32_t pairings = 0);
@@ -382,7 +383,7 @@ struct MsmDevice {
   g1 *partials = nullptr;
   g1 *gbuckets = nullptr;  // global buckets of warp units whose window exceeds MSM_WARP_SMEM_C_MAX
   uint32_t warps_per_block = 4, smem_per_warp = 0, grid = 0, gbucket_stride = 0;
-  uint32_t split_c = 0;
+  uint32_t split_c = 0, join_lanes = 1;
   fp *triples = nullptr;  // split windows: the windows' sums,
   g1 *sums = nullptr;     // the MSMs' results
   // pairing units: e(pa, Q_slot_a) e(pb, Q_slot_b) == 1 for pjobs[0 .. pair_units)

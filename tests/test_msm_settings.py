@@ -1,10 +1,12 @@
 """Which way an uneven MSM batch takes: split windows while no caller has made settings, the persistent engine under
 settings whatever their values, and what the settings and the autotuner report."""
 import ctypes
+import random
 
 import pytest
 
 from conftest import load_package
+from helpers import R_MOD
 
 INITIAL = ([8, 16, 32, 32], [4] * 4, [0] * 4)
 SPLIT = [2] * 4
@@ -37,6 +39,35 @@ def test_way_taken(settings, split):
 def test_mixed_modes_are_refused(mode):
     with pytest.raises(ValueError):
         plan([8] * 32, ([8] * 4, [4] * 4, mode))
+
+
+@pytest.mark.parametrize("longest", [8, 257, 4096, 524288])
+def test_long_msm_among_short_ones(longest):
+    """No lane adds many chunks one after another, however long one MSM is: at most 8, or a 32nd of them."""
+    c, t, _, _, lanes, *_ = plan([longest] + [8] * 39)
+    chunks = -(-longest // t)
+    assert c and lanes in (1, 2, 4, 8, 16, 32) and -(-chunks // lanes) <= max(8, -(-chunks // 32))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("longest", [63, 70, 130, 260, 520, 1100, 2100])
+def test_joined_chunks(gpu, oracle, longest):
+    """One long MSM among short ones, in chunks joined by 1, 2, .. 32 lanes: equal, opposite and identity points."""
+    rng = random.Random(longest)
+    p1, gens = oracle.generators(5)
+    base = [p1] + list(gens)
+    base += [bytes([p[0] ^ 0x20]) + p[1:] for p in base[:2]] + [bytes([0xC0]) + bytes(47)]
+    sizes = [8] * 40
+    sizes[7], sizes[9], sizes[11] = longest, 0, 40
+    msms = [([rng.choice(base) for _ in range(k)], [rng.randrange(R_MOD).to_bytes(32, "big") for _ in range(k)])
+            for k in sizes]
+    # one MSM of the long one's points and summed scalars: at most nine terms
+    total = {}
+    for p, k in zip(*msms[7]):
+        total[p] = (total.get(p, 0) + int.from_bytes(k, "big")) % R_MOD
+    want = [oracle.g1_msm(*m) if i != 7 else oracle.g1_msm(list(total), [v.to_bytes(32, "big") for v in total.values()])
+            for i, m in enumerate(msms)]
+    assert gpu.g1_msm_batch(msms) == [(0, w) for w in want]
 
 
 @pytest.mark.gpu
