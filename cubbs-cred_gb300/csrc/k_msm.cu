@@ -743,6 +743,12 @@ size_t MsmDevice::arena_bytes(const MsmPlan &p, int sm_count) {
          (size_t)p.nparts * sizeof(g1) + g + 10 * 256;
 }
 
+// Pinned bytes that upload() takes for one plan.
+size_t MsmDevice::host_bytes(const MsmPlan &p) {
+  return p.term_c.size() + p.chunks.size() * sizeof(MsmChunk) + p.units.size() * sizeof(MsmUnit) +
+         p.pstart.size() * 4 + p.start.size() * 4 + 5 * 16;
+}
+
 void launch_msm_prep(cudaStream_t s, const MsmDevice &d, const g1a *pts, const VarJob *jobs, const fr *scalars) {
   if (d.nterms)
     k_msm_prep<<<blocks_for(d.nterms, 128), 128, 0, s>>>(pts, jobs, scalars, d.term_c, d.nterms, d.phi, d.koff);
@@ -1111,22 +1117,4 @@ extern "C" int32_t cubbs_bbs_gpu_msm_tuning_v2(const uint32_t *chunk_in, const u
   } catch (const CudaError &) {
     return CUBBS_BBS_GPU_ERR_INTERNAL;
   }
-}
-
-// Test export: the plan of a batch of MSMs of K[0..n) terms (host work alone).
-extern "C" int32_t cubbs_bbs_gpu_msm_plan_for_test_v2(const uint32_t *K, size_t n, int32_t sms,
-                                                      const uint32_t *chunk_in, const uint32_t *window_in,
-                                                      const uint32_t *mode_in, uint64_t *plan8) {
-  if ((n && !K) || sms <= 0 || !plan8 || (chunk_in == nullptr) != (window_in == nullptr) ||
-      (chunk_in == nullptr) != (mode_in == nullptr))
-    return CUBBS_BBS_GPU_ERR_INVALID_INPUT;
-  MsmTuning t;
-  if (chunk_in && !t.read(chunk_in, window_in, mode_in)) return CUBBS_BBS_GPU_ERR_INVALID_INPUT;
-  MsmPlan p;
-  p.build(std::vector<uint32_t>(K, K + n), t);
-  uint32_t longest = 0;
-  for (const MsmChunk &c : p.chunks) longest = std::max(longest, c.count);
-  const uint64_t v[8] = {p.split_c, longest, p.chunks.size(), p.units.size(), p.join_lanes, 0, 0, 0};
-  std::copy(v, v + 8, plan8);
-  return CUBBS_BBS_GPU_SUCCESS;
 }

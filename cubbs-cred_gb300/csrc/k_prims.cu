@@ -277,6 +277,13 @@ void run_engine_graph(Runtime &rt, cudaStream_t s, const MsmPlan &mp, MsmDevice 
   CUBBS_CHECK(cudaGraphLaunch(it->second, s));
 }
 
+// Pinned bytes that the uploads of a plan take (those of its MsmPlan and pairing checks aside).
+size_t plan_host_bytes(const Plan &pl) {
+  const size_t R = pl.rows;
+  return 65536 + pl.points_be.size() + pl.var_scalars_be.size() + pl.fixed_scalars_be.size() +
+         pl.fixed_scale_be.size() + 4 * pl.var_point.size() + 8 * (R + 1);
+}
+
 // Runs the plan; returns per-row compressed outputs and per-row ok flags.
 // With pairs (or force_engine) the MSMs take the persistent engine, and the
 // pairing checks run as units of the same launch.
@@ -298,8 +305,8 @@ void run_plan(Runtime &rt, Plan &pl, std::vector<uint8_t> &out48, std::vector<ui
   const size_t np = pairs ? pairs->n : 0;
   rt.arena.reserve(8192 + npts * (sizeof(g1a) + 64) + nvar * (sizeof(g1) + sizeof(fr) + 48) +
                    nfix * (sizeof(fr) + 40) + R * (2 * sizeof(g1) + 128) + eng_bytes + 65536 + np * 512);
-  rt.staging.reserve(65536 + pl.points_be.size() + pl.var_scalars_be.size() + pl.fixed_scalars_be.size() +
-                     R * 128 + nvar * 16 + eng_bytes + 65536 + np * 256);
+  rt.staging.reserve(plan_host_bytes(pl) + (engine ? MsmDevice::host_bytes(mp) : 0) +
+                     np * (96 + sizeof(PairJob)) + 2 * 16);
   const PairJob *pjobs = nullptr;
   uint8_t *pok = nullptr;
   if (np) {
@@ -500,6 +507,30 @@ extern "C" int32_t cubbs_bbs_gpu_g1_msm_batch_v2(uint32_t abi, CuBbsBbsGpuG1MsmI
   for (size_t i = 0; i < n; i++) items[i].point_out.len = outs[i].len;
   return CUBBS_BBS_GPU_SUCCESS;
   ABI_GUARD_END
+}
+
+// Test export: the plan of a batch of MSMs of K[0..n) terms (host work alone).
+extern "C" int32_t cubbs_bbs_gpu_msm_plan_for_test_v2(const uint32_t *K, size_t n, int32_t sms,
+                                                      const uint32_t *chunk_in, const uint32_t *window_in,
+                                                      const uint32_t *mode_in, uint64_t *plan8) {
+  if ((n && !K) || sms <= 0 || !plan8 || (chunk_in == nullptr) != (window_in == nullptr) ||
+      (chunk_in == nullptr) != (mode_in == nullptr))
+    return CUBBS_BBS_GPU_ERR_INVALID_INPUT;
+  MsmTuning t;
+  if (chunk_in && !t.read(chunk_in, window_in, mode_in)) return CUBBS_BBS_GPU_ERR_INVALID_INPUT;
+  MsmPlan p;
+  p.build(std::vector<uint32_t>(K, K + n), t);
+  Plan pl;
+  pl.rows = n;
+  pl.points_be.resize(48 * (size_t)p.terms);
+  pl.var_scalars_be.resize(32 * (size_t)p.terms);
+  pl.var_point.resize(p.terms);
+  uint32_t longest = 0;
+  for (const MsmChunk &c : p.chunks) longest = std::max(longest, c.count);
+  const uint64_t v[8] = {p.split_c, longest, p.chunks.size(), p.units.size(), p.join_lanes,
+                         plan_host_bytes(pl) + MsmDevice::host_bytes(p), 0, 0};
+  std::copy(v, v + 8, plan8);
+  return CUBBS_BBS_GPU_SUCCESS;
 }
 
 // ----------------------------------------------------------------------------- MSMs and pairings in one launch

@@ -392,6 +392,7 @@ struct MsmDevice {
   uint8_t *pok = nullptr;
   void upload(Runtime &rt, const MsmPlan &p, cudaStream_t s);
   static size_t arena_bytes(const MsmPlan &p, int sm_count);
+  static size_t host_bytes(const MsmPlan &p);
 };
 // term j of the flat term list uses point jobs[j].point (skipped when flags & 1)
 // and scalar scalars[j]; MSM i owns terms [start[i], start[i+1]).

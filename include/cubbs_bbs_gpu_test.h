@@ -120,7 +120,7 @@ int32_t cubbs_bbs_gpu_proof_gen_check_lanes_for_test_v2(size_t n);
 /* How an MSM batch of K[0..n) terms is run on `sms` SMs under the settings (as msm_tuning_v2 takes
  * them; null: none made), without device work: plan8 = window width of split windows (0: the
  * engine), terms of the largest chunk, chunks, units of the engine, lanes that join a window's
- * chunks, and three zeros. */
+ * chunks, pinned bytes that the call reserves, and two zeros. */
 int32_t cubbs_bbs_gpu_msm_plan_for_test_v2(const uint32_t *K, size_t n, int32_t sms, const uint32_t *chunk_in,
                                            const uint32_t *window_in, const uint32_t *mode_in, uint64_t *plan8);
 

@@ -49,6 +49,17 @@ def test_long_msm_among_short_ones(longest):
     assert c and lanes in (1, 2, 4, 8, 16, 32) and -(-chunks // lanes) <= max(8, -(-chunks // 32))
 
 
+@pytest.mark.parametrize("settings", [None, INITIAL])
+@pytest.mark.parametrize("n,hi", [(32, 8), (1024, 257), (16384, 257), (40, 20000)])
+def test_pinned_bytes_are_those_uploaded(n, hi, settings):
+    """A call page-locks what it copies (points, scalars, indexes, chunks), not the plan's device buffers."""
+    K = [2 + (i * 7919) % (hi - 1) for i in range(n)]
+    _, _, chunks, units, _, pinned, *_ = plan(K, settings)
+    terms = sum(K)
+    copied = (48 + 32 + 4 + 1) * terms + 16 * chunks + 8 * units + 16 * (n + 1)
+    assert copied <= pinned <= copied + 70000
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("longest", [63, 70, 130, 260, 520, 1100, 2100])
 def test_joined_chunks(gpu, oracle, longest):
