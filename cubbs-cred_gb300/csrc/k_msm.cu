@@ -894,6 +894,7 @@ MsmWork make_work(Runtime &rt, cudaStream_t s, uint64_t seed, const std::vector<
 float time_engine(Runtime &rt, cudaStream_t s, const MsmWork &w, const MsmTuning &tune, int reps, uint8_t *out48,
                   cudaEvent_t e0, cudaEvent_t e1) {
   MsmPlan p;
+  p.sms = (uint32_t)rt.sm_count;
   p.build(w.K, tune);
   size_t mark = rt.arena.used;
   MsmDevice d;
@@ -962,6 +963,7 @@ extern "C" int32_t cubbs_bbs_gpu_msm_uneven_bench_v2(uint32_t abi, size_t n_msms
       widest.build(std::vector<uint32_t>(1, 2), t);
     }
     MsmPlan split;  // and for split windows, of this workload or of the tuner's sample
+    split.sms = (uint32_t)rt.sm_count;
     split.build(K, MsmTuning());
     rt.arena.reserve(terms * (sizeof(fr) + 2 * sizeof(g1a) + sizeof(VarJob) + 48 + 4 + 40 + sizeof(g1)) +
                      n_msms * (sizeof(g1) * 4 + 64) + ((size_t)64 << 20) +
@@ -1039,6 +1041,7 @@ extern "C" int32_t cubbs_bbs_gpu_msm_uneven_bench_v2(uint32_t abi, size_t n_msms
     CUBBS_CHECK(cudaMemcpyAsync(&hbad, bad, 4, cudaMemcpyDeviceToHost, s));
     // ---- plan, graph capture, timed replays
     MsmPlan p;
+    p.sms = (uint32_t)rt.sm_count;
     p.build(K, best);
     MsmDevice d;
     d.upload(rt, p, s);

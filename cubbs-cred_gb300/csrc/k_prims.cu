@@ -299,6 +299,7 @@ void run_plan(Runtime &rt, Plan &pl, std::vector<uint8_t> &out48, std::vector<ui
   if (engine) {
     std::vector<uint32_t> K(R);
     for (size_t r = 0; r < R; r++) K[r] = pl.var_start[r + 1] - pl.var_start[r];
+    mp.sms = (uint32_t)rt.sm_count;
     mp.build(K, rt.sh.msm_tuning, pairs ? pairs->n : 0);
   }
   const size_t eng_bytes = engine ? MsmDevice::arena_bytes(mp, rt.sm_count) : 0;
@@ -519,6 +520,7 @@ extern "C" int32_t cubbs_bbs_gpu_msm_plan_for_test_v2(const uint32_t *K, size_t 
   MsmTuning t;
   if (chunk_in && !t.read(chunk_in, window_in, mode_in)) return CUBBS_BBS_GPU_ERR_INVALID_INPUT;
   MsmPlan p;
+  p.sms = (uint32_t)sms;
   p.build(std::vector<uint32_t>(K, K + n), t);
   Plan pl;
   pl.rows = n;

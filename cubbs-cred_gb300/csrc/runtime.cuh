@@ -153,7 +153,7 @@ struct MsmPlan {
   uint32_t pair_units = 0;
   uint32_t split_c = 0;           // split windows of this width (k_msm_windows); 0: the persistent engine
   uint32_t join_lanes = 1;        // lanes that add a window's partials (k_msm_join)
-  uint32_t sms = 152;             // of the device the plan is for
+  uint32_t sms = 152;             // of the device the plan is for, set before build()
   void build_split(const std::vector<uint32_t> &K);
   void build(const std::vector<uint32_t> &K, const MsmTuning &tune, uint32_t pairings = 0);
 };

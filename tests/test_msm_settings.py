@@ -49,6 +49,12 @@ def test_long_msm_among_short_ones(longest):
     assert c and lanes in (1, 2, 4, 8, 16, 32) and -(-chunks // lanes) <= max(8, -(-chunks // 32))
 
 
+def test_plan_is_for_the_devices_sms():
+    """On fewer SMs the same batch fills the GPU earlier, so its MSMs are cut into fewer chunks."""
+    K = [2 + (i * 7919) % 256 for i in range(700)]
+    assert plan(K, sms=16)[1] > plan(K, sms=152)[1] > plan(K, sms=1000)[1]
+
+
 @pytest.mark.parametrize("settings", [None, INITIAL])
 @pytest.mark.parametrize("n,hi", [(32, 8), (1024, 257), (16384, 257), (40, 20000)])
 def test_pinned_bytes_are_those_uploaded(n, hi, settings):
