@@ -17,6 +17,7 @@
 #include <algorithm>
 #include <atomic>
 #include <chrono>
+#include <exception>
 #include <thread>
 #include <mutex>
 #include <condition_variable>
@@ -1278,7 +1279,10 @@ class PackPool {
   PackPool() {
     const unsigned hw = std::thread::hardware_concurrency();
     const unsigned n = hw > 1 ? std::min(7u, hw - 1) : 0;
-    for (unsigned k = 0; k < n; k++) workers_.emplace_back([this] { worker(); });
+    try {
+      for (unsigned k = 0; k < n; k++) workers_.emplace_back([this] { worker(); });
+    } catch (const std::exception &) {  // no more threads to be had: the calls pack with those there are
+    }
   }
   ~PackPool() {
     {
@@ -2607,6 +2611,15 @@ extern "C" int32_t cubbs_bbs_gpu_proof_gen_seeded_batch_cs_v2(uint32_t abi, uint
     return CUBBS_BBS_GPU_ERR_INVALID_INPUT;
   if (n == 0) return CUBBS_BBS_GPU_SUCCESS;
   return proof_gen_impl((int)suite, items, n, seeds, results);
+}
+
+// Test export: the sum of 1 .. ranges, a range each on the packing workers.
+extern "C" int32_t cubbs_bbs_gpu_pack_pool_for_test_v2(size_t ranges, uint64_t *sum) {
+  if (!sum) return CUBBS_BBS_GPU_ERR_INVALID_INPUT;
+  std::atomic<uint64_t> total{0};
+  PackPool::get().parallel_for(ranges, [&](size_t r) { total += r + 1; });
+  *sum = total;
+  return CUBBS_BBS_GPU_SUCCESS;
 }
 
 // Test export: lanes per point of the subgroup check in a ProofGen call of n items.

@@ -114,6 +114,9 @@ int32_t cubbs_bbs_gpu_hash_to_scalar_shake256_batch_for_test_v2(uint32_t abi_ver
 int32_t cubbs_bbs_gpu_proof_verify_phases_for_test_v2(const CuBbsBbsGpuProofVerifyItem *items, size_t n,
                                                       CuBbsBbsGpuResult *results, double *ms6);
 
+/* 1 + 2 + .. + ranges, a range each on the workers that pack large batches (no device work). */
+int32_t cubbs_bbs_gpu_pack_pool_for_test_v2(size_t ranges, uint64_t *sum);
+
 /* Lanes per point of the subgroup check in a ProofGen call of n items (no device work). */
 int32_t cubbs_bbs_gpu_proof_gen_check_lanes_for_test_v2(size_t n);
 
