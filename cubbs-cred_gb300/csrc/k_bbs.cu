@@ -1804,7 +1804,7 @@ void run_pgen(Runtime &rt, OpBatch &b, uint8_t *dmapdst) {
        CUBBS_SUITE_DISPATCH(rt.suite, k_pg_finish<S><<<blocks_for(PG_LANES * n, 64), 64, 0, sa>>>(it, N, b.dblob, b.msc, b.domain, b.rs, rss, b.fixed + n, b.v,
                                                     b.dec, b.sub, b.out, reinterpret_cast<const hash_ctx<S> *>(b.chal), b.r3inv));
        k_pg_responses<<<N, ROW_THREADS, 0, sa>>>(it, b.dblob, b.msc, b.rs, rss, b.out));
-  b.launches_per_run = (nm ? 1 : 0) + (npts ? 2 : 0) + 14;
+  b.launches_per_run = (nm ? 1 : 0) + (npts ? 2 : 0) + (apart ? 14 : 13);
 }
 
 // Verify on three streams, as ProofVerify: the signature decode (stream2, no
