@@ -187,6 +187,7 @@ def lib():
             "cubbs_bbs_gpu_proof_gen_batch_cs_v2": [U32, U32, P, S, P],
             "cubbs_bbs_gpu_proof_gen_seeded_batch_cs_v2": [U32, U32, P, S, P, P],
             "cubbs_bbs_gpu_proof_verify_batch_cs_v2": [U32, U32, P, S, P],
+            "cubbs_bbs_gpu_g1_msm_split_for_test_v2": [U32, U32, U32, P, S, P],
             "cubbs_bbs_gpu_expand_xof_shake256_48_batch_for_test_v2": [U32, P, P, P, S, P, S, P],
             "cubbs_bbs_gpu_hash_to_scalar_shake256_batch_for_test_v2": [U32, P, P, P, S, P, S, P],
         }
@@ -214,7 +215,7 @@ _SYMBOLS = [
     "cubbs_bbs_gpu_sign_batch_cs_v2", "cubbs_bbs_gpu_verify_batch_cs_v2", "cubbs_bbs_gpu_proof_gen_batch_cs_v2",
     "cubbs_bbs_gpu_proof_gen_seeded_batch_cs_v2", "cubbs_bbs_gpu_proof_verify_batch_cs_v2",
     "cubbs_bbs_gpu_expand_xof_shake256_48_batch_for_test_v2",
-    "cubbs_bbs_gpu_hash_to_scalar_shake256_batch_for_test_v2",
+    "cubbs_bbs_gpu_hash_to_scalar_shake256_batch_for_test_v2", "cubbs_bbs_gpu_g1_msm_split_for_test_v2",
 ]
 
 
@@ -392,8 +393,9 @@ def hash_to_scalar_batch(msgs, dst, suite=SUITE_SHA256):
     return [out.raw[32 * i:32 * i + 32] for i in range(len(msgs))]
 
 
-def g1_msm_batch(msms):
-    """msms: list of ([points48], [scalars32]) -> list of (code, point48)."""
+def g1_msm_batch(msms, split=None):
+    """msms: list of ([points48], [scalars32]) -> list of (code, point48).  split (window, chunk),
+    for the tests: by split windows of that width over chunks of up to that many terms."""
     k = _Keep()
     items = (G1MsmItem * len(msms))()
     outs = []
@@ -402,7 +404,10 @@ def g1_msm_batch(msms):
         outs.append(buf)
         items[i] = G1MsmItem(k.slices(pts), k.slices(scs), len(pts), ob)
     res = (Result * len(msms))()
-    _call("cubbs_bbs_gpu_g1_msm_batch_v2", ABI_VERSION, items, len(msms), res)
+    if split is None:
+        _call("cubbs_bbs_gpu_g1_msm_batch_v2", ABI_VERSION, items, len(msms), res)
+    else:
+        _call("cubbs_bbs_gpu_g1_msm_split_for_test_v2", ABI_VERSION, *split, items, len(msms), res)
     return [(res[i].code, outs[i].raw[:48]) for i in range(len(msms))]
 
 

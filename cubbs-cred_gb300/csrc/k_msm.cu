@@ -555,15 +555,17 @@ static uint32_t msm_join_lanes(uint32_t chunks) {
 // products take when every sub-partition has several warps (1215 cycles a
 // product, field.cuh) plus half of the longest lane, which runs alone at the
 // end (1816), over windows 3 .. 5 and chunks of 8 .. 120 terms.
-void MsmPlan::build_split(const std::vector<uint32_t> &K) {
+void MsmPlan::build_split(const std::vector<uint32_t> &K, const MsmTuning &tune) {
   const size_t n = K.size();
   uint32_t longest = 0, best_t = 0;
   for (uint32_t k : K) longest = std::max(longest, k);
   double best = 0;
   for (uint32_t t : {8u, 16u, 32u, 64u, (uint32_t)MSM_SPLIT_T_MAX}) {
+    if (tune.split_t && t != tune.split_t) continue;
     double parts = 0;
     for (uint32_t k : K) parts += (k + t - 1) / t;
     for (uint32_t c = 3; c <= 5; c++) {
+      if (tune.split_c && c != tune.split_c) continue;
       const double digit = 20 * (1 - 1.0 / (1u << c)), fold = 14.0 * ((1u << (c - 1)) - 1);
       const uint32_t chunks = (longest + t - 1) / t, lanes = msm_join_lanes(chunks);
       const double lane = digit * std::min(t, longest) + fold,
@@ -609,7 +611,7 @@ void MsmPlan::build(const std::vector<uint32_t> &K, const MsmTuning &tune, uint3
   split_c = 0;
   join_lanes = 1;
   if (pairings == 0 && tune.split) {
-    build_split(K);
+    build_split(K, tune);
     return;
   }
   // pairing checks first: each takes a warp for milliseconds, so they must

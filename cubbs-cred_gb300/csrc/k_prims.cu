@@ -285,22 +285,23 @@ size_t plan_host_bytes(const Plan &pl) {
 }
 
 // Runs the plan; returns per-row compressed outputs and per-row ok flags.
-// With pairs (or force_engine) the MSMs take the persistent engine, and the
-// pairing checks run as units of the same launch.
+// With pairs the MSMs take the persistent engine, and the pairing checks run as
+// units of the same launch.  `tuning` replaces the process's settings and makes
+// a batch of any size take the way that they select (for the tests).
 void run_plan(Runtime &rt, Plan &pl, std::vector<uint8_t> &out48, std::vector<uint8_t> &row_ok,
-              PairRequest *pairs = nullptr) {
+              PairRequest *pairs = nullptr, const MsmTuning *tuning = nullptr) {
   cudaStream_t s = rt.stream;
   size_t R = pl.rows, npts = pl.points_be.size() / 48, nvar = pl.var_point.size();
   size_t nfix = pl.has_fixed ? R * pl.fixed_stride : 0;
-  // Many variable-only rows: the persistent bucket-method engine (k_msm.cu)
-  // instead of one GLV multiplication per term plus a row sum.
-  const bool engine = (pairs && pairs->n && !pl.has_fixed) || (!pl.has_fixed && R >= 32 && nvar >= 8 * R);
+  // Many variable-only rows: split windows or the persistent bucket-method
+  // engine (k_msm.cu) instead of one GLV multiplication per term plus a row sum.
+  const bool engine = (pairs && pairs->n && !pl.has_fixed) || (!pl.has_fixed && R >= 32 && nvar >= 8 * R) || tuning;
   MsmPlan mp;
   if (engine) {
     std::vector<uint32_t> K(R);
     for (size_t r = 0; r < R; r++) K[r] = pl.var_start[r + 1] - pl.var_start[r];
     mp.sms = (uint32_t)rt.sm_count;
-    mp.build(K, rt.sh.msm_tuning, pairs ? pairs->n : 0);
+    mp.build(K, tuning ? *tuning : rt.sh.msm_tuning, pairs ? pairs->n : 0);
   }
   const size_t eng_bytes = engine ? MsmDevice::arena_bytes(mp, rt.sm_count) : 0;
   const size_t np = pairs ? pairs->n : 0;
@@ -477,8 +478,8 @@ using namespace cubbs;
   }
 
 // ----------------------------------------------------------------------------- g1_msm_batch (route 4)
-extern "C" int32_t cubbs_bbs_gpu_g1_msm_batch_v2(uint32_t abi, CuBbsBbsGpuG1MsmItem *items, size_t n,
-                                                 CuBbsBbsGpuResult *results) {
+static int32_t g1_msm_batch(uint32_t abi, CuBbsBbsGpuG1MsmItem *items, size_t n, CuBbsBbsGpuResult *results,
+                            const MsmTuning *tuning) {
   if (!abi_ok(abi) || (n > 0 && (items == nullptr || results == nullptr))) return CUBBS_BBS_GPU_ERR_INVALID_INPUT;
   for (size_t i = 0; i < n; i++) {
     const auto &it = items[i];
@@ -501,13 +502,28 @@ extern "C" int32_t cubbs_bbs_gpu_g1_msm_batch_v2(uint32_t abi, CuBbsBbsGpuG1MsmI
   }
   pl.var_start.push_back((uint32_t)pl.var_point.size());
   std::vector<uint8_t> out, ok;
-  run_plan(rt, pl, out, ok);
+  run_plan(rt, pl, out, ok, nullptr, tuning);
   std::vector<CuBbsBbsGpuByteBuffer> outs(n);
   for (size_t i = 0; i < n; i++) outs[i] = items[i].point_out;
   finish_rows(out, ok, outs.data(), results, n, CUBBS_BBS_MSM_ROUTE_CUBBS_UNIVERSAL);
   for (size_t i = 0; i < n; i++) items[i].point_out.len = outs[i].len;
   return CUBBS_BBS_GPU_SUCCESS;
   ABI_GUARD_END
+}
+extern "C" int32_t cubbs_bbs_gpu_g1_msm_batch_v2(uint32_t abi, CuBbsBbsGpuG1MsmItem *items, size_t n,
+                                                 CuBbsBbsGpuResult *results) {
+  return g1_msm_batch(abi, items, n, results, nullptr);
+}
+// Test export: the same by split windows of width c (3 .. 5) over chunks of up
+// to t (8, 16, 32, 64 or 120) terms, whatever the batch's size and the settings.
+extern "C" int32_t cubbs_bbs_gpu_g1_msm_split_for_test_v2(uint32_t abi, uint32_t c, uint32_t t,
+                                                          CuBbsBbsGpuG1MsmItem *items, size_t n,
+                                                          CuBbsBbsGpuResult *results) {
+  if (c < 3 || c > 5 || (t != 8 && t != 16 && t != 32 && t != 64 && t != 120)) return CUBBS_BBS_GPU_ERR_INVALID_INPUT;
+  MsmTuning tuning;
+  tuning.split_c = c;
+  tuning.split_t = t;
+  return g1_msm_batch(abi, items, n, results, &tuning);
 }
 
 // Test export: the plan of a batch of MSMs of K[0..n) terms (host work alone).

@@ -98,6 +98,7 @@ struct MsmTuning {
   // No caller has made settings: MSMs alone in a launch take split windows
   // (k_msm_windows), and the values below are for those beside pairing checks.
   bool split = true;
+  uint32_t split_c = 0, split_t = 0;  // its window and chunk (0: by the cost model; for the tests)
   // measured on GB300 over 16384 MSMs with K ~ U{2..257}: 120.7k MSMs/s
   uint32_t chunk[MSM_CLASSES] = {8, 16, 32, 32};
   uint32_t window[MSM_CLASSES] = {4, 4, 4, 4};
@@ -154,7 +155,7 @@ struct MsmPlan {
   uint32_t split_c = 0;           // split windows of this width (k_msm_windows); 0: the persistent engine
   uint32_t join_lanes = 1;        // lanes that add a window's partials (k_msm_join)
   uint32_t sms = 152;             // of the device the plan is for, set before build()
-  void build_split(const std::vector<uint32_t> &K);
+  void build_split(const std::vector<uint32_t> &K, const MsmTuning &tune);
   void build(const std::vector<uint32_t> &K, const MsmTuning &tune, uint32_t pairings = 0);
 };
 // Prepared state of one ciphersuite (the generators and everything built on

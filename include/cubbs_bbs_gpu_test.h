@@ -114,6 +114,11 @@ int32_t cubbs_bbs_gpu_hash_to_scalar_shake256_batch_for_test_v2(uint32_t abi_ver
 int32_t cubbs_bbs_gpu_proof_verify_phases_for_test_v2(const CuBbsBbsGpuProofVerifyItem *items, size_t n,
                                                       CuBbsBbsGpuResult *results, double *ms6);
 
+/* g1_msm_batch_v2 by split windows of width c (3..5) over chunks of up to t (8, 16, 32, 64, 120)
+ * terms, whatever the batch's size and the settings. */
+int32_t cubbs_bbs_gpu_g1_msm_split_for_test_v2(uint32_t abi_version, uint32_t c, uint32_t t,
+                                               CuBbsBbsGpuG1MsmItem *items, size_t n, CuBbsBbsGpuResult *results);
+
 /* 1 + 2 + .. + ranges, a range each on the workers that pack large batches (no device work). */
 int32_t cubbs_bbs_gpu_pack_pool_for_test_v2(size_t ranges, uint64_t *sum);
 
