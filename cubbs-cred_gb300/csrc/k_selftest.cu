@@ -471,10 +471,11 @@ __global__ void k_busy(uint32_t *out) {
 }
 
 // A call that throws with work under way, kind 0: kernels on the side streams;
-// 1: a stream capture.  *idle = 1 when the workspace it gave back has no work,
+// 1: a stream capture; 2: as 0, with the prepared state not held, as when it
+// fails to grow.  *idle = 1 when the workspace it gave back has no work,
 // no capture and no error left.
 extern "C" int32_t cubbs_bbs_gpu_failed_call_for_test_v2(int32_t kind, int32_t *idle) {
-  if (!idle || kind < 0 || kind > 1) return CUBBS_BBS_GPU_ERR_INVALID_INPUT;
+  if (!idle || kind < 0 || kind > 2) return CUBBS_BBS_GPU_ERR_INVALID_INPUT;
   *idle = 0;
   Runtime *used = nullptr;
   try {
@@ -484,8 +485,9 @@ extern "C" int32_t cubbs_bbs_gpu_failed_call_for_test_v2(int32_t kind, int32_t *
     uint32_t *o = rt.arena.alloc<uint32_t>(4);
     if (kind == 1) CUBBS_CHECK(cudaStreamBeginCapture(rt.stream, cudaStreamCaptureModeThreadLocal));
     k_busy<<<1, 1, 0, kind == 1 ? rt.stream : rt.stream2>>>(o);
-    if (kind == 0) k_busy<<<1, 1, 0, rt.stream4>>>(o + 1);
+    if (kind != 1) k_busy<<<1, 1, 0, rt.stream4>>>(o + 1);
     CUBBS_CHECK(cudaGetLastError());
+    if (kind == 2) scope.lock.unlock();
     throw CudaError(cudaErrorUnknown, "a call that fails");
   } catch (const CudaError &) {
     if (!used) return CUBBS_BBS_GPU_ERR_INTERNAL;

@@ -731,7 +731,7 @@ CallScope::CallScope() : rt(acquire_workspace()), lock(rt.sh.mu), unwinding(std:
 CallScope::~CallScope() {
   if (std::uncaught_exceptions() > unwinding) rt.settle();
   rt.lock = nullptr;
-  lock.unlock();
+  if (lock.owns_lock()) lock.unlock();  // (not held when the prepared state failed to grow)
   release_workspace(rt);
 }
 

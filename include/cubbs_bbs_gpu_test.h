@@ -132,7 +132,8 @@ int32_t cubbs_bbs_gpu_proof_gen_check_lanes_for_test_v2(size_t n);
 int32_t cubbs_bbs_gpu_msm_plan_for_test_v2(const uint32_t *K, size_t n, int32_t sms, const uint32_t *chunk_in,
                                            const uint32_t *window_in, const uint32_t *mode_in, uint64_t *plan8);
 
-/* A call that throws with work under way (kind 0: kernels on the side streams, 1: a stream capture);
+/* A call that throws with work under way (kind 0: kernels on the side streams, 1: a stream capture,
+ * 2: kernels, and the prepared state not held);
  * *idle = 1 when the workspace it gave back has neither work nor a capture left. */
 int32_t cubbs_bbs_gpu_failed_call_for_test_v2(int32_t kind, int32_t *idle);
 

@@ -8,7 +8,7 @@ from helpers import scalar
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("kind", [0, 1, 2])
 def test_workspace_is_idle_after_a_failed_call(gpu, oracle, kind):
     idle = ctypes.c_int32(-1)
     fn = gpu.lib().cubbs_bbs_gpu_failed_call_for_test_v2
