@@ -390,21 +390,8 @@ DEV fr fr_mul_inl(const fr &a, const fr &b) {
   fr_reduce_once(r.w, t.w);
   return r;
 }
-// The CIOS form (carry chains of field_ptx.cuh), kept for the tests.
-DEV fr fr_mul_cios_inl(const fr &a, const fr &b) {
-  uint32_t t[17];
-  _Pragma("unroll") for (int i = 0; i < 9; i++) t[i] = 0;
-  _Pragma("unroll") for (int i = 0; i < 8; i++) {
-    t[i + 8] = 0;
-    fr_cios_row(&t[i], a.w, b.w[i]);
-  }
-  fr r;
-  fr_reduce_once(r.w, &t[8]);
-  return r;
-}
 DEVNI fr fr_mul(fr a, fr b) { return fr_mul_inl(a, b); }
 DEV fr fr_to_mont(const fr &a) { const fr r2 = FR_R2_INIT; return fr_mul(a, r2); }
-DEV fr fr_from_mont(const fr &a) { fr one = fr_zero(); one.w[0] = 1; return fr_mul(a, one); }
 DEV bool fr_lt_mod(const fr &a) {
   const fr m = FR_MOD_INIT;
   _Pragma("unroll") for (int i = 7; i >= 0; i--) {

@@ -22,7 +22,7 @@ def limbs(x, n):
     return [(x >> (32 * i)) & 0xFFFFFFFF for i in range(n)]
 
 
-def gen_field(name, mod, n):
+def gen_field(name, mod, n, cios):
     ml = limbs(mod, n)
     pinv = (-pow(mod, -1, 1 << 32)) % (1 << 32)
     Rm = (1 << (32 * n)) % mod
@@ -70,13 +70,14 @@ def gen_field(name, mod, n):
     body.append(f"madc.hi.u32 {regs_t[n]}, m, 0x{ml[n - 1]:08x}, {regs_t[n]};")
     body.append("}")
     asm_text = "\\n\\t".join(body)
-    w(f"// t[0..{n}] += a*b + m*mod with m = t0*pinv; afterwards t0 == 0 and the value is t[1..{n}].")
-    w(f"__device__ __forceinline__ void {name}_cios_row(uint32_t *t, const uint32_t *a, uint32_t b) {{")
-    outs = ", ".join(f'"+&r"(t[{i}])' for i in range(n + 1))
-    ins = ", ".join(f'"r"(a[{i}])' for i in range(n)) + ', "r"(b)'
-    w(f'  asm volatile("{asm_text}" : {outs} : {ins});')
-    w("}")
-    w("")
+    if cios:
+        w(f"// t[0..{n}] += a*b + m*mod with m = t0*pinv; afterwards t0 == 0 and the value is t[1..{n}].")
+        w(f"__device__ __forceinline__ void {name}_cios_row(uint32_t *t, const uint32_t *a, uint32_t b) {{")
+        outs = ", ".join(f'"+&r"(t[{i}])' for i in range(n + 1))
+        ins = ", ".join(f'"r"(a[{i}])' for i in range(n)) + ', "r"(b)'
+        w(f'  asm volatile("{asm_text}" : {outs} : {ins});')
+        w("}")
+        w("")
     # ---- conditional subtract: r = t >= mod ? t - mod : t  (t < 2*mod)
     body = []
     body.append("{ .reg .u32 d<%d>; .reg .u32 bw; .reg .pred ge;" % n)
@@ -352,11 +353,11 @@ def main():
         "#pragma once",
         "#include <stdint.h>",
         "",
-        gen_field("fp", P, 12),
+        gen_field("fp", P, 12, cios=True),
         gen_lazy("fp", P, 12),
         gen_mont("fp", P, 12),
         gen_mont_sqr("fp", P, 12),
-        gen_field("fr", R, 8),
+        gen_field("fr", R, 8, cios=False),
         gen_mont("fr", R, 8),
     ]
     dst = pathlib.Path(__file__).with_name("field_ptx.cuh")
