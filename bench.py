@@ -53,11 +53,11 @@ MODEL_M = {
 
 # DRAM bytes per launch of a stage's kernel at this workload, from one ncu capture
 # of the 1024-proof, L = 100 step (dram__bytes_read.sum + dram__bytes_write.sum):
-# k_var_mul_pair moved 0.638 + 0.004 MB for its 4096 terms (points, scalars, jobs);
-# k_fixed_msm<32> moved 170.4 + 3.5 MB with the table narrowed to window 14 (19
+# k_var_mul_pair moved 0.636 + 0.094 MB for its 4096 terms (points, scalars, jobs);
+# k_fixed_msm<128> moved 320.6 + 3.0 MB with the table narrowed to window 14 (19
 # windows per term, so that the capture fits); table reads scale with the windows,
-# so the window-20 launch (13 windows) moves about 173.9 MB x 13 / 19 = 119 MB.
-TRAFFIC_BYTES = {"fixed_msm": 173.9e6 * 13 / 19, "var_mul": 0.6415e6}
+# so the window-20 launch (13 windows) moves about 323.6 MB x 13 / 19 = 221 MB.
+TRAFFIC_BYTES = {"fixed_msm": 323.6e6 * 13 / 19, "var_mul": 0.7301e6}
 
 
 def drbg(seed: bytes, label: bytes, i: int, n: int) -> bytes:

@@ -1070,7 +1070,7 @@ __global__ void __launch_bounds__(64) k_pg_vars_b(const PgItem *items0, uint32_t
 }
 
 // Eight lanes per item: one each for Abar, Bbar, D, T1 and T2 up to their
-// encodings (one lane for all five took 204 us of a single item, 121 like this),
+// encodings (one lane for all five took 204 us of a single item, 125 like this),
 // then one for the challenge and three for the responses of e, r1 and r3.
 constexpr uint32_t PG_LANES = 8;
 template <int S>
@@ -1728,7 +1728,7 @@ void run_pverify(Runtime &rt, OpBatch &b, uint8_t *dmapdst) {
 // first scalars, the challenge hash's prefix and the subgroup check, whose
 // result only the finish reads.
 // With all seven products in one launch after the check and both MSMs one item
-// took 1.24 ms (now 0.90) and 1024 took 3.03.
+// took 1.24 ms (now 0.76) and 1024 took 3.03 (2.54).
 // From PG_APART_JOBS on the products fill the GPU's sub-partitions a warp each
 // and the MSMs fill them several times: one launch for both bases then, with the
 // T2 MSM in what it leaves free.

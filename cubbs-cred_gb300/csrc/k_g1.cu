@@ -1,7 +1,7 @@
-// G1 kernels: point decoding (decompress + subgroup check), fixed-base window
-// tables over the resident generators, the fixed-base MSM (one warp per MSM
-// row, signed w-bit windows, affine table entries, mixed XYZZ additions),
-// GLV variable-base multiplication and point compression.
+// G1 kernels: point decoding, the subgroup check, fixed-base window tables over
+// the resident generators, the fixed-base MSM (4 to 512 lanes per MSM row,
+// signed w-bit windows, affine table entries, mixed XYZZ additions, octet tree
+// sums), GLV variable-base multiplication and point compression.
 //
 // Reference counterparts: comb tables and comb MSMs
 // (native/cuda/src/kernels/comb_precompute.cuh:8-268, comb_msm.cuh:3-363),
@@ -155,12 +155,15 @@ DEV uint32_t fixed_digit(const uint32_t *s, int k, int w, uint32_t half, bool &n
 // take one); each nonzero digit costs one table lookup and one mixed addition,
 // and the next unit's table entry (a random 96-byte read from HBM) is fetched
 // while the current one is added.  The lanes' sums are added as projective
-// triples by the lane octets (g1_ladder.cuh, tree_level): 9 levels of a 32-lane
+// triples by the lane octets (g1_ladder.cuh, Adder::level): 9 levels of a 32-lane
 // row take 41 thousand cycles where five rounds of shuffled full additions
 // took 140 thousand, so that short rows can spread over many lanes.
 // Dynamic shared memory: fixed_smem of the block's warps.
 constexpr uint32_t fixed_smem(uint32_t warps) { return warps * (32 * gl::TRIPLE + 4 * gl::TMP_BYTES); }
-template <int THREADS>  // the largest block: few rows spread over 256 or 512 lanes take the form with fewer registers
+// THREADS: the largest block.  Few rows spread over 256 or 512 lanes take the
+// form with 128 registers, which spills (396 bytes stored, 508 loaded a thread);
+// the other has 204 and spills nothing.
+template <int THREADS>
 __global__ void __launch_bounds__(THREADS) k_fixed_msm(FixedTable t, const fr *scalars, uint32_t stride,
                                                    const uint32_t *nterms, uint32_t rows, uint32_t L, g1 *out) {
   extern __shared__ __align__(16) uint8_t fixed_mem[];
@@ -400,7 +403,9 @@ int var_lanes_setting() {
 // 1.16, 1000 0.49 against 1.16, 7168 1.46 against 1.16; whole calls at 4096
 // terms (ProofVerify of 1024 over 64 keys) were 3 % slower on 8 lanes, and
 // lane quads at every size slower than one or the other; those are left for
-// the setting.
+// the setting.  The line counts the whole GPU's SMs, as do the other lines of
+// this file; ProofVerify of a few keys makes these launches on partitions of 48
+// and 88 SMs, where they would lie lower (run_pverify has one of its own).
 static int lanes_for(uint32_t n) {
   const int l = var_lanes_setting();
   return l ? l : n <= 2048 ? 8 : 2;

@@ -1,6 +1,5 @@
 // Uneven variable-base G1 MSMs: many independent MSMs of different term
-// counts (config 4 of the benchmark plan: 16384 MSMs, K ~ U{2..257}) in one
-// persistent launch.
+// counts (the benchmark's: 16384 MSMs, K ~ U{2..257}).
 //
 // Every term k_j * P_j is GLV-split as k_j = q_j * lambda + s_j (lambda = z^2,
 // so k_j P_j = s_j P_j + q_j phi(P_j) with phi(x, y) = (beta x, -y)), which
@@ -12,7 +11,7 @@
 // Signed digits come from k' = k + sum_w 2^(c-1) 2^(wc): digit_w =
 // field_w(k') - 2^(c-1) in [-2^(c-1), 2^(c-1)).
 //
-// Work is grouped into units: 32 chunks of the same window width (thread
+// In the persistent engine, work is grouped into units: 32 chunks of the same window width (thread
 // mode), one whole MSM (warp mode: the warp's lanes share the MSM's buckets,
 // each lane owning the buckets of its index mod 32; windows 4..12), or one
 // pairing check.  The persistent kernel's warps take units from an atomic
@@ -23,9 +22,8 @@
 // MSM is spread over several lanes and joined by the reduction).  While no
 // caller has made settings and no pairing checks share the launch, the MSMs are
 // split over lanes by window and chunk instead (k_msm_windows), which was the
-// faster way at every size measured.  The
-// general MSM entry point replays the engine's kernels from captured CUDA
-// graphs (k_prims.cu).
+// faster way at every size measured.  The general MSM entry point replays the
+// kernels of either way from captured CUDA graphs (k_prims.cu).
 //
 // Reference counterpart: route 4 (native/cuda/src/kernels/variable_base_universal.cuh:
 // 337-644) and the Pippenger kernel (kernels/large_msm.cuh:322-416).
@@ -923,7 +921,7 @@ float time_engine(Runtime &rt, cudaStream_t s, const MsmWork &w, const MsmTuning
 
 using namespace cubbs;
 
-// Uneven MSM benchmark (config 4): n_msms MSMs with K ~ U{k_min..k_max} drawn
+// Uneven MSM benchmark: n_msms MSMs with K ~ U{k_min..k_max} drawn
 // from `seed`, points u * P1 and scalars uniform mod r generated on the
 // device.  With tune != 0 the engine's mode, chunk length and window of each
 // size class are chosen by timing candidates on a sample of the same size and

@@ -62,9 +62,8 @@ __global__ void __launch_bounds__(32) k_pairing_check_warp(const PairJob *jobs, 
   if (lane == 0) ok[item] = one ? 1 : 0;
 }
 
-// One pairing check per block of two warps (for the few group checks of an
-// aggregated batch, where one check's latency is the step's critical path):
-// warp w runs the Miller loop of pair w, then warp 0 multiplies the two values
+// One pairing check per block of two warps (CUBBS_BBS_PAIR_TEAM=32, for the few
+// group checks of an aggregated batch): warp w runs the Miller loop of pair w, then warp 0 multiplies the two values
 // and runs the final exponentiation.  Dynamic shared memory: 2 * PP_SLOTS Fp slots.
 __global__ void __launch_bounds__(64) k_pairing_check_split(const PairJob *jobs, uint32_t n, const line2 *lines,
                                                             uint8_t *ok) {

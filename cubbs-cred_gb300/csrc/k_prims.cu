@@ -236,8 +236,8 @@ PairJob *prepare_pair_jobs(Runtime &rt, const CuBbsBbsGpuPairingEqItem *items, s
   return dj;
 }
 
-// The engine's kernels (prep, persistent launch, reduction) for a plan, from a
-// CUDA graph: one is captured the first time a workspace meets the plan's
+// The kernels of a plan (prep, split windows or the persistent launch, join or
+// reduction), from a CUDA graph: one is captured the first time a workspace meets the plan's
 // shape and device buffers (the arena hands out the same addresses to the same
 // sequence of allocations) and replayed afterwards.  At most 32 graphs per
 // workspace are kept.

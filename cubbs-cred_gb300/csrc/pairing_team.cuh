@@ -23,8 +23,9 @@
 // A team is one warp or two: the programs are compiled for both widths, and a
 // two-warp team runs phases of up to 64 entries between named barriers, so an
 // Fp12 product or a Miller step's squaring (36..54 products) takes one round of
-// products instead of two.  Latency-bound checks (the group checks of an
-// aggregated batch, small batches) use two-warp teams.
+// products instead of two.  Calls take the four-warp form (pairing_quad.cuh),
+// which runs the inverse here on two warps; the one-warp programs are for
+// CUBBS_BBS_PAIR_TEAM=32 and the uneven-MSM engine's pairing units.
 #pragma once
 #include "pairing.cuh"
 #include "pairing_program.cuh"

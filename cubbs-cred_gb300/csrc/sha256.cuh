@@ -95,7 +95,7 @@ DEV void sha_init(sha_ctx &c) {
 DEV void sha_put(sha_ctx &c, uint32_t v, uint32_t nbytes) {
   const uint32_t i = c.fill >> 2, r = 8 * (c.fill & 3);
   c.w[i] |= v >> r;
-  const uint32_t rest = __funnelshift_l(0u, v, 32 - r);  // v << (32 - r), 0 for r = 0: what goes past word i
+  const uint32_t rest = __funnelshift_l(0u, v, 32 - r);  // v << (32 - r): what goes past word i (unused at r = 0)
   const bool past = (c.fill & 3) + nbytes > 4;
   c.fill += nbytes;
   c.total += nbytes;

@@ -1,7 +1,9 @@
 // Fp values in shared-memory slots: the vector loads, small signed sums and
 // reductions that the four-warp pairing (pairing_quad.cuh) and the G1 ladders
 // (g1_ladder.cuh) share.  Between rounds a slot holds a value below 1.42 p
-// (products) or 1.001 p (reduced sums).
+// (products of the pairing) or 1.001 p (reduced sums); the ladders also keep
+// unreduced sums of four slots there (lane_sum, below 5.01 p) and multiply those,
+// up to 53.7 p of the QMAX p that reduce13 takes.
 #pragma once
 #include "field.cuh"
 
